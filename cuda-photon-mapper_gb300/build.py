@@ -76,10 +76,10 @@ def build_reference():
     its photon-mapping code as serial host C++ (the legacy oracle's pin) and
     its CUDA file unmodified as an sm_103a module (the measured reference-GPU
     bar; the module travels to GPU hosts, the checkout does not)."""
-    if not os.path.isdir(REF_DIR):
+    src = os.path.join(REF_DIR, "photonMappingKernel.cu")
+    if not os.path.isfile(src):
         return None
     _run(["make", "-s", "-C", ROOT, "-f", "oracle/ref.mk", "REF=" + REF_DIR])
-    src = os.path.join(REF_DIR, "photonMappingKernel.cu")
     shims = glob.glob(os.path.join(ORACLE_DIR, "ref_gpu", "*.h"))
     if _newer(REF_CUBIN, [src] + shims):
         _run([NVCC] + ARCH + ["-O3", "-cubin", "-w", "-I", os.path.join(ORACLE_DIR, "ref_gpu"), "-o",
