@@ -206,7 +206,6 @@ struct pm_batch {
     ExtentJob *ext_jobs = nullptr;     // 2 per scene
     uint32_t *scan_tmp = nullptr;
     uint32_t *words = nullptr;         // kWords per scene
-    uint32_t *capn = nullptr;          // 2 per scene: map capacities (device n of the builds)
     unsigned long long *gathers = nullptr;  // 2 per scene
     uint32_t *work = nullptr;
     float4 *rad = nullptr;
@@ -215,10 +214,8 @@ struct pm_batch {
     TraceParams *count_dev = nullptr, *write_dev = nullptr;
     BatchRenderScene *render_dev = nullptr;
     uint32_t *prefix_dev = nullptr;
-    struct Sort {
-        uint64_t *keys = nullptr, *keys_tmp = nullptr;
-        uint32_t *vals = nullptr, *vals_tmp = nullptr, *hist = nullptr;
-    } sort;  // the autotuner's per-scene rebuilds
+    void *kd_one = nullptr;  // build scratch of the autotuner's per-scene rebuilds
+    size_t kd_one_bytes = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     unsigned long long graph_kernels = 0;
@@ -269,8 +266,8 @@ struct pm_batch {
         bool on = false;
     } ar;
     std::vector<uint32_t> nsurf;  // diffuse queries per scene
-    // the radix-sorted levels of every map's tree in shared launches (one
-    // plan per set of leaf sizes; re-planned when a tune changes one)
+    // every map's tree in shared launches (one plan per set of leaf sizes;
+    // re-planned when a tune changes one)
     KdMulti kd;
     // per-scene radiance caches (pm_batch_cache_enable): one network per
     // scene; the frame's picks and the per-step scratch are shared (scenes
@@ -318,11 +315,10 @@ void free_batch(pm_batch *b) {
     cudaFree(b->cnt); cudaFree(b->off); cudaFree(b->scan_tmp); cudaFree(b->words);
     seg_runs_free(b->cnt_runs);
     cudaFree(b->ext_jobs);
-    cudaFree(b->capn); cudaFree(b->gathers); cudaFree(b->work); cudaFree(b->rad); cudaFree(b->rgba);
+    cudaFree(b->gathers); cudaFree(b->work); cudaFree(b->rad); cudaFree(b->rgba);
     cudaFree(b->scenes_dev); cudaFree(b->count_dev); cudaFree(b->write_dev);
     cudaFree(b->render_dev); cudaFree(b->prefix_dev);
-    cudaFree(b->sort.keys); cudaFree(b->sort.keys_tmp); cudaFree(b->sort.vals); cudaFree(b->sort.vals_tmp);
-    cudaFree(b->sort.hist);
+    cudaFree(b->kd_one);
     auto &q = b->q;
     cudaFree(q.cnt); cudaFree(q.off); cudaFree(q.scnt); cudaFree(q.soff); cudaFree(q.slist);
     cudaFree(q.scan_tmp); cudaFree(q.qa); cudaFree(q.qd); cudaFree(q.val); cudaFree(q.key);
@@ -600,7 +596,7 @@ cudaError_t enqueue_lists(pm_batch *b, cudaStream_t st) {
         Q_TRY(list_keys_multi(ar.lists, ar.tile_scene, run.first, run.n, keys + run.first, ar.ord + run.first, st));
         uint32_t *ok_keys = nullptr, *ok_vals = nullptr;
         Q_TRY(radix_sort_pairs_u32(keys + run.first, ar.ord + run.first, keys_tmp + run.first, ar.defer + run.first,
-                                   ar.q_runs.n_dev + r, run.n, 0, 31, ar.hist, st, &ok_keys, &ok_vals, 0,
+                                   ar.q_runs.n_dev + r, run.n, 0, 31, ar.hist, st, &ok_keys, &ok_vals,
                                    ar.q_runs.tab + run.first / kSortTile));
         if (ok_vals != ar.ord + run.first)
             Q_TRY(cudaMemcpyAsync(ar.ord + run.first, ok_vals, sizeof(uint32_t) * run.n, cudaMemcpyDeviceToDevice,
@@ -755,18 +751,14 @@ cudaError_t size_query_buffers(pm_batch *b) {
     return cudaSuccess;
 }
 
-// Pads and builds the two trees of scene s on `st` with sort scratch `so`.
-// The build arguments of map m of scene s (sort scratch so; nullable for a
-// plan of the shared levels).
-KdBuildArgs map_args(const pm_batch *b, int s, int m, const pm_batch::Sort *so) {
+// The build arguments of map m of scene s.
+KdBuildArgs map_args(const pm_batch *b, int s, int m) {
     const auto &mp = b->maps[2 * s + m];
     KdBuildArgs a;
     a.n = mp.cap;
-    a.n_dev = b->capn + 2 * s + m;
     const pm_scene &sc = b->scenes[s];
     a.lo = make_float3(sc.box_min[0], sc.box_min[1], sc.box_min[2]);
     a.hi = make_float3(sc.box_max[0], sc.box_max[1], sc.box_max[2]);
-    a.box_dev = nullptr;
     a.pos_in = mp.pos;
     a.pow_in = mp.pow;
     a.pos_out = mp.tpos;
@@ -774,37 +766,44 @@ KdBuildArgs map_args(const pm_batch *b, int s, int m, const pm_batch::Sort *so) 
     a.dir_out = mp.tdir;
     a.node_lo = mp.lo;
     a.node_hi = mp.hi;
-    a.keys = so ? so->keys : nullptr;
-    a.keys_tmp = so ? so->keys_tmp : nullptr;
-    a.vals = so ? so->vals : nullptr;
-    a.vals_tmp = so ? so->vals_tmp : nullptr;
-    a.hist = so ? so->hist : nullptr;
-    a.order_out = nullptr;
     a.leaf_shift = shift_of(b->tune[s].leaf_size);
     a.pad_count = b->words + s * kWords + (m == 0 ? W_EXT_S : W_EXT_V);
     return a;
 }
 
-// Pads and builds the two trees of scene s on `st` with sort scratch `so`.
-cudaError_t build_scene(pm_batch *b, int s, cudaStream_t st, const pm_batch::Sort &so) {
+// Pads and builds the two trees of scene s on `st` (the autotuner's timed
+// scenes), in scratch that grows to the largest map built so.
+cudaError_t build_scene(pm_batch *b, int s, cudaStream_t st) {
     for (int m = 0; m < 2; ++m) {
         auto &mp = b->maps[2 * s + m];
         if (mp.cap == 0) continue;
-        cudaError_t e = pad_map(mp.pos, mp.pow, b->words + s * kWords + (m == 0 ? W_EXT_S : W_EXT_V),
-                                mp.cap, st);
+        const KdBuildArgs a = map_args(b, s, m);
+        const size_t bytes = kd_scratch_bytes(&a.n, &a.leaf_shift, 1);
+        cudaError_t e = cudaSuccess;
+        if (bytes > b->kd_one_bytes) {
+            e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) return e;
+            cudaFree(b->kd_one);
+            b->kd_one = nullptr;
+            b->kd_one_bytes = 0;
+            e = cudaMalloc(&b->kd_one, bytes);
+            if (e != cudaSuccess) return e;
+            b->kd_one_bytes = bytes;
+        }
+        e = pad_map(mp.pos, mp.pow, a.pad_count, mp.cap, st);
         if (e != cudaSuccess) return e;
-        e = build_tree(map_args(b, s, m, &so), st);
+        e = build_trees(&a, 1, b->kd_one, st);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-// The plan of the shared tree levels for the current leaf sizes.
+// The plan of the shared tree builds for the current leaf sizes.
 cudaError_t plan_trees(pm_batch *b) {
     kd_multi_free(b->kd);
     std::vector<KdBuildArgs> args;
     for (int s = 0; s < b->n; ++s)
-        for (int m = 0; m < 2; ++m) args.push_back(map_args(b, s, m, nullptr));
+        for (int m = 0; m < 2; ++m) args.push_back(map_args(b, s, m));
     return kd_multi_create(args, &b->kd);
 }
 
@@ -823,12 +822,9 @@ cudaError_t enqueue_frame(pm_batch *b, cudaStream_t st) {
     note_launch();
     B_TRY(cudaGetLastError());
     B_TRY(trace_photons_batch(b->scenes_dev, b->write_dev, b->n, b->sm_count, st));
-    // the trees of every map in shared launches: records past each map's
-    // size to infinity, the radix-sorted levels, then the subtree finishes,
-    // the permutations into tree order and the boxes
-    uint32_t *order = nullptr;
-    B_TRY(kd_multi_levels(b->kd, st, &order));
-    B_TRY(kd_multi_finish(b->kd, order, st));
+    // the trees of every map in shared launches, records past each map's
+    // size at infinity
+    B_TRY(kd_multi_build(b->kd, st));
     if (b->n_pixel > 0) B_TRY(render_batch(b->render_dev, b->prefix_dev, b->n_pixel, b->work, b->sm_count, st));
     if (b->ar.n_list > 0) {
         B_TRY(enqueue_lists(b, st));
@@ -878,7 +874,6 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
     cudaError_t e = cudaSuccess;
 #define C_TRY(x) do { e = (x); if (e != cudaSuccess) { free_batch(b); return check_cuda(ctx, e, #x); } } while (0)
     size_t pix = 0;
-    uint32_t max_map = 1;
     std::vector<size_t> map_counts;  // per map: path cap (one segment of the count pools each)
     for (int s = 0; s < n; ++s) {
         const pm_config &c = cfgs[s];
@@ -896,7 +891,6 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
         for (int m = 0; m < 2; ++m) {
             auto &mp = b->maps[2 * s + m];
             mp.cap = targets[m];
-            max_map = std::max(max_map, mp.cap);
             C_TRY(dalloc(&mp.pos, mp.cap));
             C_TRY(dalloc(&mp.pow, mp.cap));
             C_TRY(dalloc(&mp.tpos, mp.cap));
@@ -919,7 +913,6 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
     C_TRY(dalloc(&b->scan_tmp, scan_tile_count(b->cnt_runs.max_n) + 1));
     C_TRY(dalloc(&b->ext_jobs, 2 * (size_t)n));
     C_TRY(dalloc(&b->words, (size_t)kWords * n));
-    C_TRY(dalloc(&b->capn, 2 * (size_t)n));
     C_TRY(dalloc(&b->gathers, 2 * (size_t)n));
     C_TRY(dalloc(&b->work, 1));
     C_TRY(dalloc(&b->rad, pix));
@@ -929,19 +922,11 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
     C_TRY(dalloc(&b->write_dev, n));
     C_TRY(dalloc(&b->render_dev, n));
     C_TRY(dalloc(&b->prefix_dev, (size_t)n + 1));
-    C_TRY(dalloc(&b->sort.keys, max_map));
-    C_TRY(dalloc(&b->sort.keys_tmp, max_map));
-    C_TRY(dalloc(&b->sort.vals, max_map));
-    C_TRY(dalloc(&b->sort.vals_tmp, max_map));
-    C_TRY(dalloc(&b->sort.hist, radix_sort_hist_words(max_map)));
     // static per-scene parameters
-    std::vector<uint32_t> capn(2 * (size_t)n);
     std::vector<TraceParams> cp(n), wp(n);
     std::vector<ExtentJob> jobs(2 * (size_t)n);
     for (int s = 0; s < n; ++s) {
         const pm_config &c = cfgs[s];
-        capn[2 * s] = b->maps[2 * s].cap;
-        capn[2 * s + 1] = b->maps[2 * s + 1].cap;
         uint32_t *w = b->words + s * kWords;
         const size_t os = b->cnt_off[2 * s], ov = b->cnt_off[2 * s + 1];
         const uint32_t cap = b->path_cap[s];
@@ -981,7 +966,6 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
         P.vpos = b->maps[2 * s + 1].pos; P.vpow = b->maps[2 * s + 1].pow;
         wp[s] = P;
     }
-    C_TRY(cudaMemcpy(b->capn, capn.data(), sizeof(uint32_t) * capn.size(), cudaMemcpyHostToDevice));
     C_TRY(cudaMemcpy(b->scenes_dev, b->dsc.data(), sizeof(PScene) * n, cudaMemcpyHostToDevice));
     C_TRY(cudaMemcpy(b->count_dev, cp.data(), sizeof(TraceParams) * n, cudaMemcpyHostToDevice));
     C_TRY(cudaMemcpy(b->write_dev, wp.data(), sizeof(TraceParams) * n, cudaMemcpyHostToDevice));
@@ -1235,7 +1219,7 @@ pm_status pm_batch_autotune(pm_batch *b, const char *json_path, cudaStream_t str
         for (int li = 0; li < 3; ++li) {
             b->tune[rep].leaf_size = leaves[li];
             b->tune[rep].query_list = 0;
-            A_TRY(build_scene(b, rep, stream, b->sort));
+            A_TRY(build_scene(b, rep, stream));
             for (int ti = 0; ti < 4; ++ti) {
                 b->tune[rep].tile = tiles[ti];
                 b->tune[rep].collect_max = 128;
@@ -1251,7 +1235,7 @@ pm_status pm_batch_autotune(pm_batch *b, const char *json_path, cudaStream_t str
             }
         }
         b->tune[rep] = best;
-        A_TRY(build_scene(b, rep, stream, b->sort));
+        A_TRY(build_scene(b, rep, stream));
         for (int ci = 0; ci < 3; ++ci)
             for (int mi = 0; mi < 3; ++mi) {
                 b->tune[rep].collect_max = collects[ci];
@@ -1271,7 +1255,7 @@ pm_status pm_batch_autotune(pm_batch *b, const char *json_path, cudaStream_t str
             b->tune[rep] = pixel_best;
             b->tune[rep].leaf_size = leaves[li];
             b->tune[rep].query_list = 1;
-            A_TRY(build_scene(b, rep, stream, b->sort));
+            A_TRY(build_scene(b, rep, stream));
             float ms;
             A_TRY(time_scene(rep, &ms));
             char buf[160];
@@ -1285,7 +1269,7 @@ pm_status pm_batch_autotune(pm_batch *b, const char *json_path, cudaStream_t str
         int members = 0;
         for (int s = 0; s < b->n; ++s)
             if (b->cfgs[s].k == kc) { b->tune[s] = best; ++members; }
-        A_TRY(build_scene(b, rep, stream, b->sort));
+        A_TRY(build_scene(b, rep, stream));
         char head[400];
         snprintf(head, sizeof(head), "%s{\"k\": %d, \"scenes\": %d, \"probe_scene\": %d, \"pixels\": %llu, "
                  "\"choice\": {\"leaf_size\": %d, \"tile\": %d, \"collect_max\": %d, \"merge_min\": %d, "

@@ -6,20 +6,30 @@
 // [j*L*2^(D-l), (j+1)*L*2^(D-l)) of the final order (j = its index within
 // the level), so no child pointers or ranges are stored.
 //
-// Top-down, one level at a time, all nodes of the level in parallel: every
-// record gets the key (node within the level, coordinate along the longest
-// axis of its node's cell, quantised to 16 bits of the cell), a stable LSD
-// radix sort orders the records by it -- which leaves each node's records
-// sorted along that axis, so the node's first half (the left child) is the
-// lower half: a median split -- and each child's cell is its parent's cell
-// cut at the coordinate of the right child's first record. Equal keys keep their previous order, so the layout is
-// deterministic. The records are then permuted into that order (SoA float4
-// pos / pow) and every node gets the tight bounding box of its records,
-// bottom-up, which is what a query tests. The cells live in the node box
-// arrays until the boxes overwrite them.
+// Top-down. A node is split at its median along the longest axis of its
+// records' bounding box (the root: of the scene box): the coordinate is cut
+// into bins of that box, a histogram finds the bin holding the median, and
+// one stable partition moves the records below the bin to the left child,
+// those above it to the right, and the bin's own records left until the
+// left child is full, in their present order. The layout is therefore
+// deterministic. It does not affect a query's result: the boxes that are
+// tested are the exact bounds of each node's records.
+//
+// Nodes of more than kSubMax records ("split levels") take three launches
+// per level over tiles of kTile records: bins and histogram, per-tile
+// counts, partition (which also collects the children's boxes). A node of
+// at most kSubMax records is finished by one CTA in shared memory: the
+// remaining levels, the records and directions in tree order and the boxes
+// of all its nodes; the last CTA of a map to finish combines the boxes of
+// the nodes above.
+//
+// Against sorting every level (two 8-bit radix passes over 12-byte pairs
+// and a key pass), a level moves each record once, 16 B read and written,
+// and its 2-byte bin three times. Measured (GB300, both maps): 2 x 8M records
+// 15.8 -> 3.4 ms, 2 x 100,000 records 1.65 -> 0.15 ms, one map of 20,011
+// 0.47 -> 0.11 ms.
 #include "launch_count.cuh"
 #include "kdtree.cuh"
-#include "radix_sort.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -27,442 +37,739 @@
 namespace pm {
 namespace {
 
-__device__ __forceinline__ int longest_axis(float4 lo, float4 hi) {
-    const float ex = hi.x - lo.x, ey = hi.y - lo.y, ez = hi.z - lo.z;
-    return (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
-}
+constexpr uint32_t kFull = 0xffffffffu;
 
-__global__ void root_cell_kernel(float3 lo, float3 hi, const float *box_dev, float4 *cell_lo,
-                                 float4 *cell_hi) {
-    if (box_dev) {
-        lo = make_float3(box_dev[0], box_dev[1], box_dev[2]);
-        hi = make_float3(box_dev[3], box_dev[4], box_dev[5]);
+// Split levels. 1024 bins: the records of the median's bin that go left by
+// their order alone are 1/1024 of the node's extent thick, a few percent of
+// a leaf's width at the root of an 8M-record map, and less below; 4 KB of
+// shared histogram.
+constexpr int kBins = 1024;
+constexpr uint32_t kTile = 4096;
+constexpr int kTileThreads = 512;
+constexpr int kTileWarps = kTileThreads / 32;
+constexpr int kTileItems = (int)(kTile / kTileThreads);
+
+// Subtrees.
+constexpr int kSubMax = 2048;
+constexpr int kSubThreads = 512;
+constexpr int kSubWarps = kSubThreads / 32;
+constexpr int kSubItems = kSubMax / kSubThreads;
+constexpr int kSubBins = 256;
+constexpr int kWarpSpan = kSubMax / kSubWarps;   // records of a warp: nodes this small are split by one warp
+constexpr int kSubLeaves = kSubMax / 32;
+static_assert(kWarpSpan == 128, "the warp-level splits sort 4 records per lane");
+
+// Up to two maps as a kernel parameter.
+struct Maps2 {
+    KdMap m[2];
+    int n;
+    __device__ __forceinline__ const KdMap &of_tile(uint32_t t) const { return m[n > 1 && t >= m[1].tile0 ? 1 : 0]; }
+    __device__ __forceinline__ const KdMap &of_sub(uint32_t b) const { return m[n > 1 && b >= m[1].sub0 ? 1 : 0]; }
+};
+// Any number of maps in device memory.
+struct MapsN {
+    const KdMap *m;
+    const uint32_t *tile_map, *sub_first;
+    int n;
+    __device__ __forceinline__ const KdMap &of_tile(uint32_t t) const { return m[tile_map[t]]; }
+    __device__ __forceinline__ const KdMap &of_sub(uint32_t b) const {
+        int lo = 0, hi = n - 1;  // the last map whose first subtree <= b
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (sub_first[mid] <= b) lo = mid; else hi = mid - 1;
+        }
+        return m[lo];
     }
-    cell_lo[1] = make_float4(lo.x, lo.y, lo.z, 0.0f);
-    cell_hi[1] = make_float4(hi.x, hi.y, hi.z, 0.0f);
-}
-
-// Key of record position i at level l: (node within the level, coordinate
-// along the longest axis of the node's cell, quantised to 16 bits of the
-// cell's extent). Records that quantise alike keep their previous order.
-__global__ void split_key_kernel(const float4 *__restrict__ pos, const uint32_t *__restrict__ order,
-                                 uint32_t n, int level, uint32_t span,
-                                 const float4 *__restrict__ cell_lo,
-                                 const float4 *__restrict__ cell_hi, uint64_t *keys,
-                                 uint32_t *vals_init) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t node = i / span;
-    const uint32_t g = (1u << level) + node;
-    const float4 lo = cell_lo[g], hi = cell_hi[g];
-    const int ax = longest_axis(lo, hi);
-    uint32_t src = i;
-    if (order) src = order[i];
-    else vals_init[i] = i;
-    const float4 p = pos[src];
-    const float c = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
-    const float l0 = ax == 0 ? lo.x : (ax == 1 ? lo.y : lo.z);
-    const float l1 = ax == 0 ? hi.x : (ax == 1 ? hi.y : hi.z);
-    const float f = (c - l0) / (l1 - l0) * 65536.0f;
-    const uint32_t qc = !(f > 0.0f) ? 0u : (f >= 65535.0f ? 65535u : (uint32_t)f);
-    keys[i] = ((uint64_t)node << 16) | qc;
-}
-
-// Children cells of every node at `level`: the parent's cell cut at the
-// coordinate of the right child's first record.
-__global__ void split_cell_kernel(const float4 *__restrict__ pos, const uint32_t *__restrict__ order,
-                                  uint32_t n, int level, uint32_t span, uint32_t nodes,
-                                  float4 *cell_lo, float4 *cell_hi) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nodes) return;
-    const uint32_t g = (1u << level) + j;
-    const float4 lo = cell_lo[g], hi = cell_hi[g];
-    const uint32_t start = j * span, half = span >> 1;
-    const uint32_t cnt = min(span, n - start);
-    float4 llo = lo, lhi = hi, rlo = lo, rhi = hi;
-    if (cnt > half) {
-        const int ax = longest_axis(lo, hi);
-        const float4 p = pos[order[start + half]];
-        const float m = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
-        if (ax == 0) { lhi.x = m; rlo.x = m; }
-        else if (ax == 1) { lhi.y = m; rlo.y = m; }
-        else { lhi.z = m; rlo.z = m; }
-    }
-    cell_lo[2 * g] = llo;
-    cell_hi[2 * g] = lhi;
-    cell_lo[2 * g + 1] = rlo;
-    cell_hi[2 * g + 1] = rhi;
-}
-
-// The levels below a node of at most kSubtreeMax records are finished by
-// one CTA in shared memory: per level, a bitonic sort of the composite keys
-// (node within the subtree, the same 16-bit quantised coordinate as
-// split_key_kernel, position before the level) -- exactly the order of the
-// global stable sort by (node, coordinate) -- then the children's cells cut
-// at the coordinate of each node's right half's first record, as
-// split_cell_kernel does. The tree comes out identical; the deep levels,
-// whose global sorts carry the most node bits, cost one pass over the
-// records instead of several per level.
-constexpr int kSubtreeMax = 2048;
-constexpr int kSubtreeThreads = 512;
-constexpr int kSubtreeNodes = kSubtreeMax / 32;  // nodes of a subtree level (leaves of >= 32)
-
-struct SubtreeScratch {
-    uint64_t key[kSubtreeMax];
-    float4 p[kSubtreeMax];
-    uint32_t idx[kSubtreeMax];
-    float4 clo[2][2 * kSubtreeNodes], chi[2][2 * kSubtreeNodes];
 };
 
-extern __shared__ __align__(16) unsigned char subtree_smem[];
+__device__ __forceinline__ float coord(float4 p, int a) { return a == 0 ? p.x : (a == 1 ? p.y : p.z); }
 
-// Subtree j of a tree (the node j at level l0); one CTA.
-__device__ __forceinline__ void subtree_finish(const float4 *__restrict__ pos, uint32_t *order, uint32_t n, int l0,
-                                               int D, uint32_t span0, const float4 *__restrict__ cell_lo,
-                                               const float4 *__restrict__ cell_hi, uint32_t j) {
-    SubtreeScratch &ss = *reinterpret_cast<SubtreeScratch *>(subtree_smem);
-    const uint32_t start = j * span0;
-    if (start >= n) return;
-    const int cnt = (int)min(span0, n - start);
-    const int tid = threadIdx.x;
-    for (int t = tid; t < cnt; t += blockDim.x) {
-        const uint32_t r = order[start + t];
-        ss.idx[t] = r;
-        ss.p[t] = pos[r];
-    }
-    if (tid == 0) {
-        ss.clo[0][0] = cell_lo[(1u << l0) + j];
-        ss.chi[0][0] = cell_hi[(1u << l0) + j];
-    }
-    int P = 2;
-    while (P < cnt) P <<= 1;
-    int cur = 0;
+// Box words of a coordinate (kd_root_box_words): zero for a value that is
+// not finite, which the box leaves out.
+__device__ __forceinline__ uint32_t min_word(float x) { return isfinite(x) ? ~kd_flip(x) : 0u; }
+__device__ __forceinline__ uint32_t max_word(float x) { return isfinite(x) ? kd_flip(x) : 0u; }
+
+// The split axis, the box's lower side along it and bins per unit length. A
+// box without finite records, or of no extent, puts every record in bin 0.
+struct Cut {
+    int axis;
+    float lo, inv;
+};
+__device__ __forceinline__ Cut cut_of(float3 lo, float3 hi, float bins) {
+    const float ex = hi.x - lo.x, ey = hi.y - lo.y, ez = hi.z - lo.z;
+    Cut c;
+    c.axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
+    c.lo = c.axis == 0 ? lo.x : (c.axis == 1 ? lo.y : lo.z);
+    const float e = c.axis == 0 ? ex : (c.axis == 1 ? ey : ez);
+    c.inv = e > 0.0f ? bins / e : 0.0f;
+    return c;
+}
+__device__ __forceinline__ Cut cut_of_words(const uint32_t *w, float bins) {
+    return cut_of(make_float3(kd_unflip(~w[0]), kd_unflip(~w[1]), kd_unflip(~w[2])),
+                  make_float3(kd_unflip(w[3]), kd_unflip(w[4]), kd_unflip(w[5])), bins);
+}
+// NaN and everything below the box: 0; +inf and above: the last bin.
+__device__ __forceinline__ uint32_t bin_of(const Cut &c, float4 p, uint32_t bins) {
+    const float f = (coord(p, c.axis) - c.lo) * c.inv;
+    return !(f > 0.0f) ? 0u : (f >= (float)(bins - 1u) ? bins - 1u : (uint32_t)f);
+}
+
+// The buffer a split level reads: level 0 the input, then the partner
+// buffer and the output in turn (level l writes the partner when l is even).
+__device__ __forceinline__ const float4 *level_src(const KdMap &m, int l) {
+    return l == 0 ? m.pos : ((l & 1) ? m.tmp : m.pos_out);
+}
+__device__ __forceinline__ float4 *level_dst(const KdMap &m, int l) { return (l & 1) ? m.pos_out : m.tmp; }
+
+struct TileNode {
+    uint32_t start, cnt;        // the tile's records within the map
+    uint32_t nstart, ncnt, half;  // its node's
+    uint32_t node;              // node words index
+};
+__device__ __forceinline__ TileNode tile_node(const KdMap &m, uint32_t t, int l) {
+    TileNode n;
+    const uint32_t span = (32u << m.leaf_shift) << (m.depth - l);
+    n.start = (t - m.tile0) * kTile;
+    n.cnt = min(kTile, m.n - n.start);
+    const uint32_t j = n.start / span;
+    n.nstart = j * span;
+    n.ncnt = min(span, m.n - n.nstart);
+    n.half = min(span >> 1, n.ncnt);
+    n.node = m.node0 + (1u << l) + j;
+    return n;
+}
+
+// Launch 1 of a split level: every record's bin, and the node's histogram.
+// Bound by the records' read (16 B each): 32 us for 8M records.
+template <class Maps>
+__global__ void __launch_bounds__(kTileThreads)
+    kd_hist_kernel(const __grid_constant__ Maps maps, int level, const uint32_t *box, uint32_t *hist) {
+    __shared__ uint32_t h[kBins];
+    const KdMap &m = maps.of_tile(blockIdx.x);
+    const TileNode n = tile_node(m, blockIdx.x, level);
+    for (int i = threadIdx.x; i < kBins; i += kTileThreads) h[i] = 0;
+    const Cut c = level == 0 && !m.root_boxed ? cut_of(m.root_lo, m.root_hi, (float)kBins)
+                                              : cut_of_words(box + 8 * (size_t)n.node, (float)kBins);
+    const float4 *src = level_src(m, level) + n.start;
+    uint16_t *bins = m.bins + n.start;
     __syncthreads();
-    for (int l = l0; l < D; ++l) {
-        const int nspan = (int)(span0 >> (l - l0));  // records per node at this level
-        // keys
-        for (int t = tid; t < P; t += blockDim.x) {
-            uint64_t key = ~0ull;
-            if (t < cnt) {
-                const int node = t / nspan;
-                const float4 lo = ss.clo[cur][node], hi = ss.chi[cur][node];
-                const int ax = longest_axis(lo, hi);
-                const float4 q = ss.p[t];
-                const float c = ax == 0 ? q.x : (ax == 1 ? q.y : q.z);
-                const float c0 = ax == 0 ? lo.x : (ax == 1 ? lo.y : lo.z);
-                const float c1 = ax == 0 ? hi.x : (ax == 1 ? hi.y : hi.z);
-                const float f = (c - c0) / (c1 - c0) * 65536.0f;
-                const uint32_t qc = !(f > 0.0f) ? 0u : (f >= 65535.0f ? 65535u : (uint32_t)f);
-                key = ((uint64_t)node << 48) | ((uint64_t)qc << 32) | (uint32_t)t;
-            }
-            ss.key[t] = key;
+#pragma unroll
+    for (int i = 0; i < kTileItems; ++i) {
+        const uint32_t r = (uint32_t)i * kTileThreads + threadIdx.x;
+        uint32_t b = kBins;
+        if (r < n.cnt) {
+            b = bin_of(c, src[r], kBins);
+            bins[r] = (uint16_t)b;
         }
-        __syncthreads();
-        for (int size = 2; size <= P; size <<= 1) {
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int t = tid; t < (P >> 1); t += blockDim.x) {
-                    const int i = ((t & ~(stride - 1)) << 1) | (t & (stride - 1));
-                    const int k = i + stride;
-                    const bool up = (i & size) == 0;
-                    const uint64_t a = ss.key[i], b = ss.key[k];
-                    if ((a > b) == up) {
-                        ss.key[i] = b;
-                        ss.key[k] = a;
-                    }
+        // records of one wall share a bin: one addition for a warp of them
+        int all;
+        __match_all_sync(kFull, b, &all);
+        if (all) {
+            if ((threadIdx.x & 31) == 0 && b < kBins) atomicAdd(&h[b], 32u);
+        } else if (b < kBins) {
+            atomicAdd(&h[b], 1u);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kBins; i += kTileThreads)
+        if (h[i]) atomicAdd(&hist[(size_t)n.node * kBins + i], h[i]);
+}
+
+// Launch 2: the node's split (every tile of the node finds the same one;
+// its first tile writes it for launch 3) and the tile's records below the
+// median's bin and in it: 12 us for 8M records (their bins, 2 B each). thr:
+// {bin, records below it, of its records those that go left, its records}.
+template <class Maps>
+__global__ void __launch_bounds__(kTileThreads)
+    kd_count_kernel(const __grid_constant__ Maps maps, int level, const uint32_t *hist, uint4 *thr,
+                    uint2 *tile_cnt) {
+    constexpr int kPer = kBins / kTileThreads;
+    __shared__ uint32_t wsum[kTileWarps];
+    __shared__ uint4 split;
+    const KdMap &m = maps.of_tile(blockIdx.x);
+    const TileNode n = tile_node(m, blockIdx.x, level);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t v[kPer], s = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        v[i] = hist[(size_t)n.node * kBins + threadIdx.x * kPer + i];
+        s += v[i];
+    }
+    if (threadIdx.x == 0) split = make_uint4(kBins, n.ncnt, 0u, 0u);  // no right child: all below
+    uint32_t incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    const uint32_t before = __reduce_add_sync(kFull, lane < warp ? wsum[lane] : 0u);
+    uint32_t run = before + incl - s;
+    if (n.ncnt > n.half) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            if (run <= n.half && n.half < run + v[i])
+                split = make_uint4(threadIdx.x * kPer + i, run, n.half - run, v[i]);
+            run += v[i];
+        }
+    }
+    __syncthreads();
+    const uint32_t tb = split.x;
+    if (threadIdx.x == 0 && n.start == n.nstart) thr[n.node] = split;
+    uint32_t less = 0, eq = 0;
+#pragma unroll
+    for (int i = 0; i < kTileItems; ++i) {
+        const uint32_t r = (uint32_t)i * kTileThreads + threadIdx.x;
+        if (r < n.cnt) {
+            const uint32_t b = m.bins[n.start + r];
+            less += b < tb ? 1u : 0u;
+            eq += b == tb ? 1u : 0u;
+        }
+    }
+    const uint32_t both = __reduce_add_sync(kFull, less | (eq << 16));  // at most 256 each
+    __syncthreads();
+    if (lane == 0) wsum[warp] = both;
+    __syncthreads();
+    if (warp == 0) {
+        // 16-bit halves hold at most kTile
+        const uint32_t t = __reduce_add_sync(kFull, lane < kTileWarps ? wsum[lane] : 0u);
+        if (lane == 0) tile_cnt[blockIdx.x] = make_uint2(t & 0xffffu, t >> 16);
+    }
+}
+
+// Launch 3: the stable partition. A warp moves 256 consecutive records; its
+// first places come from the counts of the node's earlier tiles and of the
+// block's earlier warps. Also the children's boxes when they are split
+// again. Bound by the records' read and write (32 B each): 54 us for 8M
+// records, 4.9 TB/s; the writes of a warp are runs of consecutive records.
+template <class Maps>
+__global__ void __launch_bounds__(kTileThreads)
+    kd_split_kernel(const __grid_constant__ Maps maps, int level, const uint4 *thr, const uint2 *tile_cnt,
+                    uint32_t *box) {
+    __shared__ uint32_t wcnt[kTileWarps], pre_l[kTileWarps], pre_e[kTileWarps];
+    __shared__ uint32_t bb[12];
+    const KdMap &m = maps.of_tile(blockIdx.x);
+    const TileNode n = tile_node(m, blockIdx.x, level);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint4 sp = thr[n.node];
+    const bool boxes = level + 1 < m.lf;
+    if (threadIdx.x < 12) bb[threadIdx.x] = 0u;
+    // the node's earlier tiles
+    uint32_t pl = 0, pe = 0;
+    const uint32_t first = m.tile0 + n.nstart / kTile;
+    for (uint32_t t = first + threadIdx.x; t < blockIdx.x; t += kTileThreads) {
+        const uint2 c = tile_cnt[t];
+        pl += c.x;
+        pe += c.y;
+    }
+    pl = __reduce_add_sync(kFull, pl);
+    pe = __reduce_add_sync(kFull, pe);
+    if (lane == 0) {
+        pre_l[warp] = pl;
+        pre_e[warp] = pe;
+    }
+    constexpr int kPer = kTileItems;  // records per lane
+    const uint32_t wfirst = n.start + (uint32_t)warp * (32u * kPer);
+    const float4 *src = level_src(m, level);
+    float4 *dst = level_dst(m, level);
+    float4 p[kPer];
+    uint32_t ml[kPer], me[kPer];
+    uint32_t nl = 0, ne = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t r = wfirst + 32u * i + lane;
+        const bool valid = r < m.n;
+        const uint32_t b = valid ? m.bins[r] : 0xffffu;
+        if (valid) p[i] = src[r];
+        ml[i] = __ballot_sync(kFull, b < sp.x);
+        me[i] = __ballot_sync(kFull, b == sp.x);
+        nl += __popc(ml[i]);
+        ne += __popc(me[i]);
+    }
+    if (lane == 0) wcnt[warp] = nl | (ne << 16);
+    __syncthreads();
+    uint32_t less, eq;
+    {
+        const uint32_t w = __reduce_add_sync(kFull, lane < warp ? wcnt[lane] : 0u);
+        less = (w & 0xffffu) + __reduce_add_sync(kFull, lane < kTileWarps ? pre_l[lane] : 0u);
+        eq = (w >> 16) + __reduce_add_sync(kFull, lane < kTileWarps ? pre_e[lane] : 0u);
+    }
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t wl[6] = {0, 0, 0, 0, 0, 0}, wr[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t r = wfirst + 32u * i + lane;
+        if (r < m.n) {
+            const uint32_t lb = less + __popc(ml[i] & lt), eb = eq + __popc(me[i] & lt);
+            const bool is_l = (ml[i] >> lane) & 1u, is_e = (me[i] >> lane) & 1u;
+            uint32_t at;
+            bool left = true;
+            if (is_l) {
+                at = lb;
+            } else if (is_e && eb < sp.z) {
+                at = sp.y + eb;
+            } else {
+                left = false;
+                at = is_e ? n.half + (eb - sp.z) : n.half + (sp.w - sp.z) + ((r - n.nstart) - lb - eb);
+            }
+            dst[n.nstart + at] = p[i];
+            if (boxes) {
+                const uint32_t c[6] = {min_word(p[i].x), min_word(p[i].y), min_word(p[i].z),
+                                       max_word(p[i].x), max_word(p[i].y), max_word(p[i].z)};
+#pragma unroll
+                for (int a = 0; a < 6; ++a) {
+                    if (left) wl[a] = max(wl[a], c[a]);
+                    else wr[a] = max(wr[a], c[a]);
                 }
-                __syncthreads();
             }
         }
-        // the records in the new order
-        float4 np[kSubtreeMax / kSubtreeThreads];
-        uint32_t ni[kSubtreeMax / kSubtreeThreads];
+        less += __popc(ml[i]);
+        eq += __popc(me[i]);
+    }
+    if (!boxes) return;
 #pragma unroll
-        for (int u = 0; u < kSubtreeMax / kSubtreeThreads; ++u) {
-            const int t = tid + u * kSubtreeThreads;
-            if (t < cnt) {
-                const uint32_t old = (uint32_t)ss.key[t];
-                np[u] = ss.p[old];
-                ni[u] = ss.idx[old];
+    for (int a = 0; a < 6; ++a) {
+        const uint32_t x = __reduce_max_sync(kFull, wl[a]), y = __reduce_max_sync(kFull, wr[a]);
+        if (lane == 0) {
+            if (x) atomicMax(&bb[a], x);
+            if (y) atomicMax(&bb[6 + a], y);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 12 && bb[threadIdx.x]) {
+        const uint32_t j = n.node - m.node0, side = threadIdx.x / 6, a = threadIdx.x % 6;
+        atomicMax(&box[8 * (size_t)(m.node0 + 2 * j + side) + a], bb[threadIdx.x]);
+    }
+}
+
+struct SubScratch {
+    float4 p[kSubMax];
+    union {
+        struct {
+            uint32_t hist[kSubMax / 256 * kSubBins];
+            uint32_t bb[kSubMax / 256][6];
+            uint4 thr[kSubMax / 256];
+            uint32_t wcnt[kSubWarps];
+        };
+        struct {
+            float4 lo[2 * kSubLeaves], hi[2 * kSubLeaves];
+        } nb;
+    };
+    uint16_t ord[2][kSubMax];
+    uint32_t last;
+};
+
+extern __shared__ __align__(16) unsigned char sub_smem[];
+
+// Sorts 128 keys, element lane * 4 + r in k[r], ascending within blocks of
+// kN (64 or 128) consecutive elements (bitonic; strides below 4 stay in the
+// lane).
+template <int kN>
+__device__ __forceinline__ void warp_sort4(uint32_t (&k)[4], int lane) {
+#pragma unroll
+    for (int size = 2; size <= kN; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            uint32_t o[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                o[r] = stride >= 4 ? __shfl_xor_sync(kFull, k[r], stride >> 2) : k[r ^ (stride & 3)];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int e = lane * 4 + r;
+                // the last merge of a block ascends whatever the block's place
+                const bool up = size == kN || (e & size) == 0;
+                k[r] = ((e & stride) == 0) == up ? min(k[r], o[r]) : max(k[r], o[r]);
+            }
+        }
+    }
+}
+
+// The split of a warp's nodes of kN records (one of 128 or two of 64): its
+// 128 places of ord from `base`, sorted along each node's longest axis by
+// (16-bit coordinate, place).
+template <int kN>
+__device__ __forceinline__ void warp_split(SubScratch &ss, uint16_t *ord, int base, int cnt, int lane) {
+    const unsigned mask = kN == 128 ? kFull : (lane < 16 ? 0x0000ffffu : 0xffff0000u);
+    uint32_t w[6] = {0, 0, 0, 0, 0, 0};
+    float4 p[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int at = base + lane * 4 + r;
+        if (at < cnt) {
+            p[r] = ss.p[ord[at]];
+            w[0] = max(w[0], min_word(p[r].x));
+            w[1] = max(w[1], min_word(p[r].y));
+            w[2] = max(w[2], min_word(p[r].z));
+            w[3] = max(w[3], max_word(p[r].x));
+            w[4] = max(w[4], max_word(p[r].y));
+            w[5] = max(w[5], max_word(p[r].z));
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 6; ++a) w[a] = __reduce_max_sync(mask, w[a]);
+    const Cut c = cut_of_words(w, 65536.0f);
+    uint32_t k[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int e = lane * 4 + r;
+        k[r] = base + e < cnt ? (bin_of(c, p[r], 65536u) << 16) | (uint32_t)e : 0xffffff00u | (uint32_t)e;
+    }
+    warp_sort4<kN>(k, lane);
+    // an empty place's key is above every record's, so the node's first
+    // places keep holding its records
+    uint16_t nw[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) nw[r] = base + lane * 4 + r < cnt ? ord[base + (int)(k[r] & 0x7fu)] : 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        if (base + lane * 4 + r < cnt) ord[base + lane * 4 + r] = nw[r];
+    __syncwarp();
+}
+
+// One subtree per CTA: the levels from a node of at most kSubMax records
+// down to its leaves, the records in tree order and the boxes. Nodes of
+// more than 128 records split as in the split levels, with a 256-bin shared
+// histogram per node and five barriers per level; nodes of 128 and 64 are
+// sorted by one warp in registers. Only the 2-byte places move; the records
+// stay where they were loaded. Bound by latency (barriers, shared-memory
+// round trips): 3 CTAs per SM, 0.50 ms for 8M records (sorting every level
+// of the subtree in shared memory: 2.27 ms), 32 us for a small map.
+template <class Maps>
+__global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_constant__ Maps maps) {
+    SubScratch &ss = *reinterpret_cast<SubScratch *>(sub_smem);
+    const KdMap &m = maps.of_sub(blockIdx.x);
+    const uint32_t j = blockIdx.x - m.sub0;
+    const int leaf = 32 << m.leaf_shift;
+    const int levels = m.depth - m.lf;          // below the subtree's root
+    const int span0 = leaf << levels;
+    const uint32_t start = j * (uint32_t)span0;
+    const int cnt = start < m.n ? (int)min((uint32_t)span0, m.n - start) : 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float inf = __int_as_float(0x7f800000);
+    const float4 *src = level_src(m, m.lf);
+    for (int t = tid; t < cnt; t += kSubThreads) {
+        ss.p[t] = src[start + t];
+        ss.ord[0][t] = (uint16_t)t;
+    }
+    for (int i = tid; i < kSubMax / 256 * kSubBins; i += kSubThreads) ss.hist[i] = 0;
+    for (int i = tid; i < kSubMax / 256 * 6; i += kSubThreads) (&ss.bb[0][0])[i] = 0;
+    __syncthreads();
+    int cur = 0, span = span0;
+    for (; span > kWarpSpan && span > leaf; span >>= 1) {
+        const int node = warp * kWarpSpan / span;
+        const int nodes = (cnt + span - 1) / span;
+        uint16_t o[kSubItems];
+        float4 p[kSubItems];
+        uint32_t w[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int u = 0; u < kSubItems; ++u) {
+            const int at = warp * kWarpSpan + u * 32 + lane;
+            if (at < cnt) {
+                o[u] = ss.ord[cur][at];
+                p[u] = ss.p[o[u]];
+                w[0] = max(w[0], min_word(p[u].x));
+                w[1] = max(w[1], min_word(p[u].y));
+                w[2] = max(w[2], min_word(p[u].z));
+                w[3] = max(w[3], max_word(p[u].x));
+                w[4] = max(w[4], max_word(p[u].y));
+                w[5] = max(w[5], max_word(p[u].z));
+            }
+        }
+        if (warp * kWarpSpan < cnt) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                const uint32_t x = __reduce_max_sync(kFull, w[a]);
+                if (lane == 0 && x) atomicMax(&ss.bb[node][a], x);
             }
         }
         __syncthreads();
+        uint32_t b[kSubItems];
+        if (warp * kWarpSpan < cnt) {
+            const Cut c = cut_of_words(ss.bb[node], (float)kSubBins);
 #pragma unroll
-        for (int u = 0; u < kSubtreeMax / kSubtreeThreads; ++u) {
-            const int t = tid + u * kSubtreeThreads;
-            if (t < cnt) {
-                ss.p[t] = np[u];
-                ss.idx[t] = ni[u];
+            for (int u = 0; u < kSubItems; ++u) {
+                b[u] = 0xffffu;
+                if (warp * kWarpSpan + u * 32 + lane < cnt) {
+                    b[u] = bin_of(c, p[u], kSubBins);
+                    atomicAdd(&ss.hist[node * kSubBins + b[u]], 1u);
+                }
             }
         }
         __syncthreads();
-        // the children's cells
-        const int nodes = (cnt + nspan - 1) / nspan, half = nspan >> 1;
-        for (int node = tid; node < nodes; node += blockDim.x) {
-            const float4 lo = ss.clo[cur][node], hi = ss.chi[cur][node];
-            float4 llo = lo, lhi = hi, rlo = lo, rhi = hi;
-            const int ncnt = min(nspan, cnt - node * nspan);
-            if (ncnt > half) {
-                const int ax = longest_axis(lo, hi);
-                const float4 q = ss.p[node * nspan + half];
-                const float m = ax == 0 ? q.x : (ax == 1 ? q.y : q.z);
-                if (ax == 0) { lhi.x = m; rlo.x = m; }
-                else if (ax == 1) { lhi.y = m; rlo.y = m; }
-                else { lhi.z = m; rlo.z = m; }
+        if (warp < nodes) {
+            // one warp per node: 8 consecutive bins per lane
+            const int ncnt = min(span, cnt - warp * span), half = min(span >> 1, ncnt);
+            uint32_t v[kSubBins / 32], s = 0;
+#pragma unroll
+            for (int i = 0; i < kSubBins / 32; ++i) {
+                v[i] = ss.hist[warp * kSubBins + lane * (kSubBins / 32) + i];
+                s += v[i];
             }
-            ss.clo[cur ^ 1][2 * node] = llo;
-            ss.chi[cur ^ 1][2 * node] = lhi;
-            ss.clo[cur ^ 1][2 * node + 1] = rlo;
-            ss.chi[cur ^ 1][2 * node + 1] = rhi;
+            uint32_t incl = s;
+#pragma unroll
+            for (int q = 1; q < 32; q <<= 1) {
+                const uint32_t t = __shfl_up_sync(kFull, incl, q);
+                if (lane >= q) incl += t;
+            }
+            if (ncnt == half) {
+                if (lane == 0) ss.thr[warp] = make_uint4(kSubBins, (uint32_t)ncnt, 0u, 0u);
+            } else {
+                uint32_t run = incl - s;
+#pragma unroll
+                for (int i = 0; i < kSubBins / 32; ++i) {
+                    if (run <= (uint32_t)half && (uint32_t)half < run + v[i])
+                        ss.thr[warp] = make_uint4((uint32_t)(lane * (kSubBins / 32) + i), run, (uint32_t)half - run, v[i]);
+                    run += v[i];
+                }
+            }
+        }
+        __syncthreads();
+        uint32_t ml[kSubItems], me[kSubItems], tot = 0;
+        uint4 sp = make_uint4(0u, 0u, 0u, 0u);
+        if (warp * kWarpSpan < cnt) {
+            sp = ss.thr[node];
+#pragma unroll
+            for (int u = 0; u < kSubItems; ++u) {
+                ml[u] = __ballot_sync(kFull, b[u] < sp.x);
+                me[u] = __ballot_sync(kFull, b[u] == sp.x);
+                tot += __popc(ml[u]) | ((uint32_t)__popc(me[u]) << 16);
+            }
+        }
+        if (lane == 0) ss.wcnt[warp] = tot;
+        for (int i = tid; i < kSubMax / 256 * kSubBins; i += kSubThreads) ss.hist[i] = 0;
+        for (int i = tid; i < kSubMax / 256 * 6; i += kSubThreads) (&ss.bb[0][0])[i] = 0;
+        __syncthreads();
+        if (warp * kWarpSpan < cnt) {
+            const int nwarp = node * span / kWarpSpan;  // the node's first warp
+            const uint32_t pre = __reduce_add_sync(kFull, lane >= nwarp && lane < warp ? ss.wcnt[lane] : 0u);
+            uint32_t less = pre & 0xffffu, eq = pre >> 16;
+            const unsigned lt = (1u << lane) - 1u;
+            const uint32_t half = (uint32_t)min(span >> 1, cnt - node * span);
+#pragma unroll
+            for (int u = 0; u < kSubItems; ++u) {
+                const int at = warp * kWarpSpan + u * 32 + lane;
+                if (at < cnt) {
+                    const uint32_t lb = less + __popc(ml[u] & lt), eb = eq + __popc(me[u] & lt);
+                    uint32_t to;
+                    if ((ml[u] >> lane) & 1u) to = lb;
+                    else if ((me[u] >> lane) & 1u) to = eb < sp.z ? sp.y + eb : half + (eb - sp.z);
+                    else to = half + (sp.w - sp.z) + ((uint32_t)(at - node * span) - lb - eb);
+                    ss.ord[cur ^ 1][node * span + (int)to] = o[u];
+                }
+                less += __popc(ml[u]);
+                eq += __popc(me[u]);
+            }
         }
         __syncthreads();
         cur ^= 1;
     }
-    for (int t = tid; t < cnt; t += blockDim.x) order[start + t] = ss.idx[t];
-}
-
-__global__ void __launch_bounds__(kSubtreeThreads)
-    subtree_finish_kernel(const float4 *__restrict__ pos, uint32_t *order, uint32_t n, int l0, int D,
-                          uint32_t span0, const float4 *__restrict__ cell_lo,
-                          const float4 *__restrict__ cell_hi) {
-    subtree_finish(pos, order, n, l0, D, span0, cell_lo, cell_hi, blockIdx.x);
-}
-
-__global__ void iota_kernel(uint32_t *v, uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = i;
-}
-
-__device__ __forceinline__ void permute_one(const uint32_t *__restrict__ order, uint32_t i,
-                                            const float4 *__restrict__ pos_in, const float4 *__restrict__ pow_in,
-                                            float4 *pos_out, float4 *pow_out, float4 *dir_out) {
-    uint32_t s = order[i];
-    pos_out[i] = pos_in[s];
-    if (pow_in) {
-        const float4 pw = pow_in[s];
-        pow_out[i] = pw;
-        if (dir_out) {
-            const v3 d = oct_decode(__float_as_uint(pw.w));
-            dir_out[i] = make_float4(d.x, d.y, d.z, 0.0f);
+    uint16_t *ord = ss.ord[cur];
+    const int base = warp * kWarpSpan;
+    if (base < cnt) {
+        if (span == 128 && span > leaf) {
+            warp_split<128>(ss, ord, base, cnt, lane);
+            span = 64;
+        }
+        if (span == 64 && span > leaf) warp_split<64>(ss, ord, base, cnt, lane);
+    }
+    __syncthreads();
+    // the records in tree order
+    for (int t = tid; t < cnt; t += kSubThreads) {
+        const float4 p = ss.p[ord[t]];
+        m.pos_out[start + t] = p;
+        if (m.pow) {
+            const float4 pw = __ldg(&m.pow[__float_as_uint(p.w)]);
+            m.pow_out[start + t] = pw;
+            if (m.dir_out) {
+                const v3 d = oct_decode(__float_as_uint(pw.w));
+                m.dir_out[start + t] = make_float4(d.x, d.y, d.z, 0.0f);
+            }
         }
     }
-}
-
-__global__ void permute_kernel(const uint32_t *__restrict__ order, uint32_t n,
-                               const float4 *__restrict__ pos_in, const float4 *__restrict__ pow_in,
-                               float4 *pos_out, float4 *pow_out, float4 *dir_out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) permute_one(order, i, pos_in, pow_in, pos_out, pow_out, dir_out);
-}
-
-// One warp per leaf slot: box of its (up to) 32 << leaf_shift records.
-// Leaf slot `warp` of a tree: one warp.
-__device__ __forceinline__ void leaf_box(const float4 *__restrict__ pos, uint32_t n, uint32_t first_leaf,
-                                         int leaf_shift, float4 *node_lo, float4 *node_hi, uint32_t warp) {
-    int lane = threadIdx.x & 31;
-    const float inf = __int_as_float(0x7f800000);
-    float lx = inf, ly = inf, lz = inf, hx = -inf, hy = -inf, hz = -inf;
-    for (int c = 0; c < (1 << leaf_shift); ++c) {
-        const uint32_t r = (warp << (5 + leaf_shift)) + ((uint32_t)c << 5) + lane;
-        if (r < n) {
-            float4 p = pos[r];
-            lx = fminf(lx, p.x); ly = fminf(ly, p.y); lz = fminf(lz, p.z);
-            hx = fmaxf(hx, p.x); hy = fmaxf(hy, p.y); hz = fmaxf(hz, p.z);
+    // boxes: the leaves (empty ones inverted), then each level above
+    const int leaves = 1 << levels;
+    const uint32_t root = (1u << m.lf) + j;
+    for (int f = warp; f < leaves; f += kSubWarps) {
+        float lx = inf, ly = inf, lz = inf, hx = -inf, hy = -inf, hz = -inf;
+        for (int c = 0; c < (1 << m.leaf_shift); ++c) {
+            const int t = f * leaf + c * 32 + lane;
+            if (t < cnt) {
+                const float4 p = ss.p[ord[t]];
+                lx = fminf(lx, p.x); ly = fminf(ly, p.y); lz = fminf(lz, p.z);
+                hx = fmaxf(hx, p.x); hy = fmaxf(hy, p.y); hz = fmaxf(hz, p.z);
+            }
+        }
+        const float4 lo = make_float4(kd_unflip(__reduce_min_sync(kFull, kd_flip(lx))),
+                                      kd_unflip(__reduce_min_sync(kFull, kd_flip(ly))),
+                                      kd_unflip(__reduce_min_sync(kFull, kd_flip(lz))), 0.0f);
+        const float4 hi = make_float4(kd_unflip(__reduce_max_sync(kFull, kd_flip(hx))),
+                                      kd_unflip(__reduce_max_sync(kFull, kd_flip(hy))),
+                                      kd_unflip(__reduce_max_sync(kFull, kd_flip(hz))), 0.0f);
+        if (lane == 0) {
+            ss.nb.lo[leaves + f] = lo;
+            ss.nb.hi[leaves + f] = hi;
         }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        lx = fminf(lx, __shfl_xor_sync(0xffffffffu, lx, o));
-        ly = fminf(ly, __shfl_xor_sync(0xffffffffu, ly, o));
-        lz = fminf(lz, __shfl_xor_sync(0xffffffffu, lz, o));
-        hx = fmaxf(hx, __shfl_xor_sync(0xffffffffu, hx, o));
-        hy = fmaxf(hy, __shfl_xor_sync(0xffffffffu, hy, o));
-        hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
+    __syncthreads();
+    for (int l = levels - 1; l >= 0; --l) {
+        for (int i = tid; i < (1 << l); i += kSubThreads) {
+            const int nd = (1 << l) + i;
+            const float4 a = ss.nb.lo[2 * nd], b = ss.nb.lo[2 * nd + 1];
+            const float4 c = ss.nb.hi[2 * nd], d = ss.nb.hi[2 * nd + 1];
+            ss.nb.lo[nd] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
+            ss.nb.hi[nd] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f);
+        }
+        __syncthreads();
     }
-    if (lane == 0) {
-        node_lo[first_leaf + warp] = make_float4(lx, ly, lz, 0.0f);
-        node_hi[first_leaf + warp] = make_float4(hx, hy, hz, 0.0f);
+    for (int i = tid + 1; i < 2 * leaves; i += kSubThreads) {
+        const int d = 31 - __clz(i);
+        const uint32_t g = (root << d) + (uint32_t)(i - (1 << d));
+        m.lo[g] = ss.nb.lo[i];
+        m.hi[g] = ss.nb.hi[i];
     }
-}
-
-__global__ void leaf_box_kernel(const float4 *__restrict__ pos, uint32_t n, uint32_t first_leaf,
-                                uint32_t leaf_slots, int leaf_shift, float4 *node_lo,
-                                float4 *node_hi) {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp < leaf_slots) leaf_box(pos, n, first_leaf, leaf_shift, node_lo, node_hi, warp);
-}
-
-__global__ void inner_box_kernel(uint32_t first, uint32_t count, float4 *node_lo, float4 *node_hi) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    uint32_t nd = first + i;
-    float4 a = node_lo[2 * nd], b = node_lo[2 * nd + 1];
-    float4 c = node_hi[2 * nd], d = node_hi[2 * nd + 1];
-    node_lo[nd] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
-    node_hi[nd] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f);
-}
-
-// Small levels: one CTA walks the top of the tree level by level.
-__device__ __forceinline__ void top_box(uint32_t levels, float4 *node_lo, float4 *node_hi) {
-    for (int l = (int)levels - 1; l >= 0; --l) {
-        uint32_t first = 1u << l;
-        for (uint32_t i = threadIdx.x; i < first; i += blockDim.x) {
-            uint32_t nd = first + i;
-            float4 a = node_lo[2 * nd], b = node_lo[2 * nd + 1];
-            float4 c = node_hi[2 * nd], d = node_hi[2 * nd + 1];
-            node_lo[nd] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
-            node_hi[nd] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f);
+    if (m.lf == 0) return;
+    // the last subtree of the map to get here combines the nodes above
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) ss.last = atomicAdd(m.done, 1u) == (1u << m.lf) - 1u ? 1u : 0u;
+    __syncthreads();
+    if (!ss.last) return;
+    __threadfence();
+    for (int l = m.lf - 1; l >= 0; --l) {
+        for (uint32_t i = tid; i < (1u << l); i += kSubThreads) {
+            const uint32_t nd = (1u << l) + i;
+            const float4 a = __ldcg(&m.lo[2 * nd]), b = __ldcg(&m.lo[2 * nd + 1]);
+            const float4 c = __ldcg(&m.hi[2 * nd]), d = __ldcg(&m.hi[2 * nd + 1]);
+            __stcg(&m.lo[nd], make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f));
+            __stcg(&m.hi[nd], make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f));
         }
         __syncthreads();
     }
 }
 
-__global__ void top_box_kernel(uint32_t levels, float4 *node_lo, float4 *node_hi) {
-    top_box(levels, node_lo, node_hi);
-}
-
-
-// ---- several maps at once (KdMulti) ----
-
-// Pooled position i: the map (build order) and the position within it.
-__device__ __forceinline__ int multi_map(const uint32_t *tile_map, uint32_t i) { return (int)tile_map[i / kSortTile]; }
-
-__global__ void multi_init_kernel(const KdMultiMap *maps, const uint32_t *tile_map, uint32_t total,
-                                  uint32_t *vals) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    vals[i] = i - maps[multi_map(tile_map, i)].base;
-}
-
-__global__ void multi_root_kernel(const KdMultiMap *maps, int nmaps) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= nmaps || maps[m].depth == 0) return;
-    maps[m].cell_lo[1] = maps[m].root_lo;
-    maps[m].cell_hi[1] = maps[m].root_hi;
-}
-
-// split_key_kernel over the pooled positions of the maps sorted at `level`;
-// positions past a map's records (the padding of its last tile) get the
-// largest key, so the stable sort keeps them at the end of their node.
-__global__ void split_key_multi_kernel(const KdMultiMap *maps, const uint32_t *tile_map, uint32_t total,
-                                       int level, const uint32_t *order, uint64_t *keys) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const KdMultiMap &m = maps[multi_map(tile_map, i)];
-    const uint32_t j = i - m.base;
-    if (j >= m.n) {
-        keys[i] = 0xffffu;
-        return;
-    }
-    const uint32_t span = (32u << m.leaf_shift) << (m.depth - level);
-    const uint32_t node = j / span;
-    const uint32_t g = (1u << level) + node;
-    const float4 lo = m.cell_lo[g], hi = m.cell_hi[g];
-    const int ax = longest_axis(lo, hi);
-    const float4 p = m.pos[order[i]];
-    const float c = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
-    const float l0 = ax == 0 ? lo.x : (ax == 1 ? lo.y : lo.z);
-    const float l1 = ax == 0 ? hi.x : (ax == 1 ? hi.y : hi.z);
-    const float f = (c - l0) / (l1 - l0) * 65536.0f;
-    const uint32_t qc = !(f > 0.0f) ? 0u : (f >= 65535.0f ? 65535u : (uint32_t)f);
-    keys[i] = ((uint64_t)node << 16) | qc;
-}
-
-// split_cell_kernel over the nodes of every map sorted at `level`
-// (prefix: nmaps + 1 scanned node counts).
-__global__ void split_cell_multi_kernel(const KdMultiMap *maps, int nmaps, const uint32_t *prefix,
-                                        int level, const uint32_t *order) {
-    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= prefix[nmaps]) return;
-    int lo_m = 0, hi_m = nmaps - 1;  // the last map whose prefix <= u
-    while (lo_m < hi_m) {
-        const int mid = (lo_m + hi_m + 1) >> 1;
-        if (prefix[mid] <= u) lo_m = mid; else hi_m = mid - 1;
-    }
-    const KdMultiMap &m = maps[lo_m];
-    const uint32_t j = u - prefix[lo_m];
-    const uint32_t span = (32u << m.leaf_shift) << (m.depth - level);
-    const uint32_t g = (1u << level) + j;
-    const float4 lo = m.cell_lo[g], hi = m.cell_hi[g];
-    const uint32_t start = j * span, half = span >> 1;
-    const uint32_t cnt = min(span, m.n - start);
-    float4 llo = lo, lhi = hi, rlo = lo, rhi = hi;
-    if (cnt > half) {
-        const int ax = longest_axis(lo, hi);
-        const float4 p = m.pos[order[m.base + start + half]];
-        const float c = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
-        if (ax == 0) { lhi.x = c; rlo.x = c; }
-        else if (ax == 1) { lhi.y = c; rlo.y = c; }
-        else { lhi.z = c; rlo.z = c; }
-    }
-    m.cell_lo[2 * g] = llo;
-    m.cell_hi[2 * g] = lhi;
-    m.cell_lo[2 * g + 1] = rlo;
-    m.cell_hi[2 * g + 1] = rhi;
-}
-
-
-// The last map m with prefix[m] <= u (prefix: nmaps + 1 scanned counts).
-__device__ __forceinline__ int map_at(const uint32_t *prefix, int nmaps, uint32_t u) {
-    int lo = 0, hi = nmaps - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (prefix[mid] <= u) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-__global__ void multi_pad_kernel(const KdMultiMap *maps, const uint32_t *tile_map, uint32_t total) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const KdMultiMap &m = maps[multi_map(tile_map, i)];
-    const uint32_t j = i - m.base;
-    if (!m.pad_count || j >= m.n || j < *m.pad_count) return;
+template <class Maps>
+__global__ void __launch_bounds__(kTileThreads) kd_pad_kernel(const __grid_constant__ Maps maps) {
+    const KdMap &m = maps.of_tile(blockIdx.x);
+    if (!m.pad_count) return;
+    const uint32_t first = (blockIdx.x - m.tile0) * kTile, from = *m.pad_count;
     const float inf = __int_as_float(0x7f800000);
-    m.pad_pos[j] = make_float4(inf, inf, inf, __uint_as_float(j));
-    m.pad_pow[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t r = first + threadIdx.x; r < min(first + kTile, m.n); r += kTileThreads)
+        if (r >= from) {
+            const_cast<float4 *>(m.pos)[r] = make_float4(inf, inf, inf, __uint_as_float(r));
+            const_cast<float4 *>(m.pow)[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
 }
 
-__global__ void __launch_bounds__(kSubtreeThreads)
-    multi_subtree_kernel(const KdMultiMap *maps, int nmaps, const uint32_t *prefix, uint32_t *order) {
-    const KdMultiMap &m = maps[map_at(prefix, nmaps, blockIdx.x)];
-    const uint32_t span0 = (32u << m.leaf_shift) << (m.depth - m.lf);
-    subtree_finish(m.pos, order + m.base, m.n, m.lf, m.depth, span0, m.cell_lo, m.cell_hi,
-                   blockIdx.x - prefix[map_at(prefix, nmaps, blockIdx.x)]);
+// The first level whose nodes hold at most kSubMax records.
+int first_finish_level(int depth, uint32_t leaf) {
+    int lf = depth;
+    while (lf > 0 && ((uint64_t)leaf << (depth - (lf - 1))) <= (uint64_t)kSubMax) --lf;
+    return lf;
 }
 
-__global__ void multi_permute_kernel(const KdMultiMap *maps, const uint32_t *tile_map, uint32_t total,
-                                     const uint32_t *order) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const KdMultiMap &m = maps[multi_map(tile_map, i)];
-    const uint32_t j = i - m.base;
-    if (j < m.n) permute_one(order + m.base, j, m.pos, m.pow, m.pos_out, m.pow_out, m.dir_out);
+uint32_t tiles_of(uint32_t n) { return (n + kTile - 1) / kTile; }
+
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// Scratch layout of a set of maps: the words zeroed by each build
+// (histograms, boxes, finished-subtree counters), the splits, the tile
+// counts, then the bins and the partner buffer of every map.
+struct Layout {
+    uint32_t tiles = 0, subs = 0, nodes = 0;
+    size_t hist = 0, box = 0, done = 0, clear = 0, thr = 0, tile_cnt = 0, bins = 0, tmp = 0, total = 0;
+};
+
+Layout layout_of(const uint32_t *n, const int *leaf_shift, int maps) {
+    Layout L;
+    size_t records = 0;
+    for (int i = 0; i < maps; ++i) {
+        const int D = tree_depth(n[i], leaf_shift[i]);
+        const int lf = first_finish_level(D, 32u << leaf_shift[i]);
+        if (n[i] == 0) continue;
+        L.tiles += tiles_of(n[i]);
+        L.subs += 1u << lf;
+        if (lf == 0) continue;  // never split by the level launches: no scratch
+        L.nodes += 1u << lf;
+        records += (n[i] + 127u) & ~(size_t)127u;
+    }
+    L.box = align256(L.hist + sizeof(uint32_t) * kBins * (size_t)L.nodes);
+    L.done = align256(L.box + sizeof(uint32_t) * 8 * (size_t)L.nodes);
+    L.clear = align256(L.done + sizeof(uint32_t) * (size_t)std::max(maps, 1));
+    L.thr = L.clear;
+    L.tile_cnt = align256(L.thr + sizeof(uint4) * (size_t)L.nodes);
+    L.bins = align256(L.tile_cnt + sizeof(uint2) * (size_t)L.tiles);
+    L.tmp = align256(L.bins + sizeof(uint16_t) * records);
+    L.total = align256(L.tmp + sizeof(float4) * records);
+    return L;
 }
 
-__global__ void multi_leaf_kernel(const KdMultiMap *maps, int nmaps, const uint32_t *prefix) {
-    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= prefix[nmaps]) return;  // whole warps
-    const int mi = map_at(prefix, nmaps, w);
-    const KdMultiMap &m = maps[mi];
-    leaf_box(m.pos_out, m.n, 1u << m.depth, m.leaf_shift, m.cell_lo, m.cell_hi, w - prefix[mi]);
+int finish_level_of(const KdBuildArgs &a) {
+    return first_finish_level(tree_depth(a.n, a.leaf_shift), 32u << a.leaf_shift);
 }
 
-__global__ void multi_inner_kernel(const KdMultiMap *maps, int nmaps, const uint32_t *prefix, int level) {
-    const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= prefix[nmaps]) return;
-    const int mi = map_at(prefix, nmaps, u);
-    const KdMultiMap &m = maps[mi];
-    const uint32_t nd = (1u << level) + (u - prefix[mi]);
-    const float4 a = m.cell_lo[2 * nd], b = m.cell_lo[2 * nd + 1];
-    const float4 c = m.cell_hi[2 * nd], d = m.cell_hi[2 * nd + 1];
-    m.cell_lo[nd] = make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.0f);
-    m.cell_hi[nd] = make_float4(fmaxf(c.x, d.x), fmaxf(c.y, d.y), fmaxf(c.z, d.z), 0.0f);
+// The kernel descriptors of maps a[idx[0..count)) (in that order), all with
+// records.
+void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, void *scratch, KdMap *out) {
+    unsigned char *base = (unsigned char *)scratch;
+    uint32_t tile = 0, sub = 0, node = 0;
+    size_t rec = 0;
+    for (int i = 0; i < count; ++i) {
+        const KdBuildArgs &b = a[idx[i]];
+        KdMap &m = out[i];
+        memset(&m, 0, sizeof(m));
+        m.pos = b.pos_in;
+        m.pow = b.pow_in;
+        m.pos_out = b.pos_out;
+        m.pow_out = b.pow_out;
+        m.dir_out = b.dir_out;
+        m.lo = b.node_lo;
+        m.hi = b.node_hi;
+        m.done = (uint32_t *)(base + L.done) + i;
+        m.pad_count = b.pad_count;
+        m.root_lo = b.lo;
+        m.root_hi = b.hi;
+        m.root_boxed = b.root_boxed ? 1 : 0;
+        m.n = b.n;
+        m.depth = tree_depth(b.n, b.leaf_shift);
+        m.leaf_shift = b.leaf_shift;
+        m.lf = first_finish_level(m.depth, 32u << b.leaf_shift);
+        m.tile0 = tile;
+        m.sub0 = sub;
+        m.node0 = node;
+        tile += tiles_of(b.n);
+        sub += 1u << m.lf;
+        if (m.lf > 0) {
+            m.tmp = (float4 *)(base + L.tmp) + rec;
+            m.bins = (uint16_t *)(base + L.bins) + rec;
+            node += 1u << m.lf;
+            rec += (b.n + 127u) & ~(size_t)127u;
+        }
+    }
 }
 
-__global__ void multi_top_kernel(const KdMultiMap *maps) {
-    const KdMultiMap &m = maps[blockIdx.x];
-    top_box((uint32_t)min(m.depth, 10), m.cell_lo, m.cell_hi);
+template <class Maps>
+cudaError_t launch_build(const Maps &maps, const KdMap *host, int count, uint32_t subs, uint32_t *hist,
+                         uint32_t *box, uint4 *thr, uint2 *tile_cnt, cudaStream_t s) {
+    for (int l = 0; l < host[0].lf; ++l) {
+        // the maps split at this level come first
+        uint32_t t = 0;
+        for (int i = 0; i < count && host[i].lf > l; ++i) t = host[i].tile0 + tiles_of(host[i].n);
+        kd_hist_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, box, hist);
+        kd_count_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, hist, thr, tile_cnt);
+        kd_split_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, thr, tile_cnt, box);
+        note_launches(3);
+    }
+    const int smem = (int)sizeof(SubScratch);
+    cudaError_t e = cudaFuncSetAttribute(kd_finish_kernel<Maps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kd_finish_kernel<Maps><<<subs, kSubThreads, smem, s>>>(maps);
+    note_launch();
+    return cudaGetLastError();
 }
+
 }  // namespace
 
 int tree_depth(uint32_t n, int leaf_shift) {
@@ -475,101 +782,47 @@ int tree_depth(uint32_t n, int leaf_shift) {
 
 size_t tree_nodes(uint32_t n, int leaf_shift) { return (size_t)2 << tree_depth(n, leaf_shift); }
 
-// The first level finished per subtree in shared memory: nodes of at most
-// kSubtreeMax records.
-int first_finish_level(int D, uint32_t leaf) {
-    int lf = D;
-    while (lf > 0 && ((uint64_t)leaf << (D - (lf - 1))) <= (uint64_t)kSubtreeMax) --lf;
-    return lf;
+size_t kd_scratch_bytes(const uint32_t *n, const int *leaf_shift, int maps) {
+    return layout_of(n, leaf_shift, maps).total;
 }
 
-cudaError_t build_tree(const KdBuildArgs &a, cudaStream_t s) {
-    const uint32_t n = a.n;
-    if (n == 0) return cudaSuccess;
-    const int D = tree_depth(n, a.leaf_shift);
-    const uint32_t blocks = (n + 255) / 256;
-    // Top-down median splits; the current order ping-pongs between the two
-    // (keys, vals) buffer pairs of the sort.
-    uint64_t *ka = a.keys, *kb = a.keys_tmp;
-    uint32_t *va = a.vals, *vb = a.vals_tmp;
-    cudaError_t e;
-    if (D == 0) {
-        iota_kernel<<<blocks, 256, 0, s>>>(va, n); note_launch();
-    } else {
-        root_cell_kernel<<<1, 1, 0, s>>>(a.lo, a.hi, a.box_dev, a.node_lo, a.node_hi); note_launch();
-    }
-    // levels [lf, D) are finished per subtree in shared memory
-    const uint32_t leaf = 32u << a.leaf_shift;
-    const int lf = first_finish_level(D, leaf);
-    if (lf == 0 && D > 0) {
-        iota_kernel<<<blocks, 256, 0, s>>>(va, n);
-        note_launch();
-    }
-    for (int l = 0; l < lf; ++l) {
-        const uint32_t span = (32u << a.leaf_shift) << (D - l);
-        const uint32_t nodes = (n + span - 1) / span;
-        split_key_kernel<<<blocks, 256, 0, s>>>(a.pos_in, l == 0 ? nullptr : va, n, l, span,
-                                                a.node_lo, a.node_hi, ka, va); note_launch();
-        int node_bits = 0;
-        while ((1u << node_bits) < nodes) ++node_bits;
-        uint64_t *ko = nullptr;
-        uint32_t *vo = nullptr;
-        // the records are grouped by node already (a node is a fixed range of
-        // positions, a whole number of sort tiles at these levels): sort each
-        // node's range by its 16-bit coordinate alone
-        e = span % kSortTile == 0
-                ? radix_sort_pairs_u64(ka, va, kb, vb, a.n_dev, n, 0, 16, a.hist, s, &ko, &vo, span / kSortTile)
-                : radix_sort_pairs_u64(ka, va, kb, vb, a.n_dev, n, 0, 16 + node_bits, a.hist, s, &ko, &vo);
-        if (e != cudaSuccess) return e;
-        if (vo != va) {
-            uint64_t *tk = ka; ka = kb; kb = tk;
-            uint32_t *tv = va; va = vb; vb = tv;
-        }
-        split_cell_kernel<<<(nodes + 255) / 256, 256, 0, s>>>(a.pos_in, va, n, l, span, nodes,
-                                                               a.node_lo, a.node_hi); note_launch();
-    }
-    return build_tree_finish(a, va, s);
+namespace {
+Layout layout_of_args(const KdBuildArgs *a, int maps) {
+    uint32_t n[2] = {a[0].n, maps > 1 ? a[1].n : 0u};
+    int ls[2] = {a[0].leaf_shift, maps > 1 ? a[1].leaf_shift : 0};
+    return layout_of(n, ls, maps);
+}
+}  // namespace
+
+uint32_t *kd_root_box_words(const KdBuildArgs &a, void *scratch) {
+    const Layout L = layout_of_args(&a, 1);
+    return L.nodes ? (uint32_t *)((unsigned char *)scratch + L.box) + 8 : nullptr;
 }
 
-cudaError_t build_tree_finish(const KdBuildArgs &a, uint32_t *va, cudaStream_t s) {
-    const uint32_t n = a.n;
-    if (n == 0) return cudaSuccess;
-    const int D = tree_depth(n, a.leaf_shift);
-    const uint32_t blocks = (n + 255) / 256;
-    const uint32_t leaf = 32u << a.leaf_shift;
-    const int lf = first_finish_level(D, leaf);
-    cudaError_t e;
-    if (lf < D) {
-        const uint32_t span = leaf << (D - lf);
-        const uint32_t nodes = (n + span - 1) / span;
-        const int smem = (int)sizeof(SubtreeScratch);
-        e = cudaFuncSetAttribute(subtree_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        subtree_finish_kernel<<<nodes, kSubtreeThreads, smem, s>>>(a.pos_in, va, n, lf, D, span, a.node_lo,
-                                                                   a.node_hi);
-        note_launch();
-    }
-    permute_kernel<<<blocks, 256, 0, s>>>(va, n, a.pos_in, a.pow_in, a.pos_out, a.pow_out, a.dir_out);
-    note_launch();
-    const uint32_t first_leaf = 1u << D;
-    leaf_box_kernel<<<(first_leaf * 32 + 255) / 256, 256, 0, s>>>(a.pos_out, n, first_leaf, first_leaf,
-                                                                 a.leaf_shift, a.node_lo, a.node_hi);
-    note_launch();
-    // Wide levels one launch each; the top 10 levels in a single CTA.
-    int l = D - 1;
-    for (; l >= 10; --l) {
-        uint32_t first = 1u << l;
-        inner_box_kernel<<<(first + 255) / 256, 256, 0, s>>>(first, first, a.node_lo, a.node_hi); note_launch();
-    }
-    if (l >= 0) {
-        top_box_kernel<<<1, 1024, 0, s>>>((uint32_t)(l + 1), a.node_lo, a.node_hi);
-        note_launch();
-    }
-    if (a.order_out) {
-        e = cudaMemcpyAsync(a.order_out, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s);
+cudaError_t kd_clear_scratch(const KdBuildArgs &a, void *scratch, cudaStream_t s) {
+    const Layout L = layout_of_args(&a, 1);
+    return L.nodes ? cudaMemsetAsync(scratch, 0, L.clear, s) : cudaSuccess;
+}
+
+cudaError_t build_trees(const KdBuildArgs *a, int maps, void *scratch, cudaStream_t s) {
+    if (maps < 1 || maps > 2 || (maps == 2 && a[0].root_boxed)) return cudaErrorInvalidValue;
+    int idx[2], count = 0;  // the map with the most split levels first
+    for (int i = 0; i < maps; ++i)
+        if (a[i].n > 0) idx[count++] = i;
+    if (count == 0) return cudaSuccess;
+    if (count == 2 && finish_level_of(a[1]) > finish_level_of(a[0])) std::swap(idx[0], idx[1]);
+    const Layout L = layout_of_args(a, maps);
+    if (L.nodes && !a[0].root_boxed) {
+        cudaError_t e = cudaMemsetAsync(scratch, 0, L.clear, s);
         if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    Maps2 m;
+    memset(&m, 0, sizeof(m));
+    m.n = count;
+    describe(a, idx, count, L, scratch, m.m);
+    unsigned char *base = (unsigned char *)scratch;
+    return launch_build(m, m.m, count, L.subs, (uint32_t *)(base + L.hist), (uint32_t *)(base + L.box),
+                        (uint4 *)(base + L.thr), (uint2 *)(base + L.tile_cnt), s);
 }
 
 namespace {
@@ -582,201 +835,69 @@ cudaError_t kd_alloc(T **p, size_t count) {
 
 cudaError_t kd_multi_create(const std::vector<KdBuildArgs> &args, KdMulti *k) {
     *k = KdMulti();
-    std::vector<int> idx;
-    for (int i = 0; i < (int)args.size(); ++i)
+    std::vector<int> idx, shift;  // maps with records, those with the most split levels first
+    std::vector<uint32_t> n;
+    for (int i = 0; i < (int)args.size(); ++i) {
+        n.push_back(args[i].n);
+        shift.push_back(args[i].leaf_shift);
         if (args[i].n > 0) idx.push_back(i);
-    auto lf_of = [&](int i) {
-        const int D = tree_depth(args[i].n, args[i].leaf_shift);
-        return first_finish_level(D, 32u << args[i].leaf_shift);
-    };
-    std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return lf_of(a) > lf_of(b); });
-    uint32_t tiles = 0;
-    for (int i : idx) {
-        const KdBuildArgs &a = args[i];
-        KdMultiMap m;
-        memset(&m, 0, sizeof(m));
-        m.pos = a.pos_in;
-        m.cell_lo = a.node_lo;
-        m.cell_hi = a.node_hi;
-        m.root_lo = make_float4(a.lo.x, a.lo.y, a.lo.z, 0.0f);
-        m.root_hi = make_float4(a.hi.x, a.hi.y, a.hi.z, 0.0f);
-        m.n = a.n;
-        m.base = tiles * kSortTile;
-        m.depth = tree_depth(a.n, a.leaf_shift);
-        m.lf = lf_of(i);
-        m.leaf_shift = a.leaf_shift;
-        m.pad_pos = const_cast<float4 *>(a.pos_in);
-        m.pad_pow = const_cast<float4 *>(a.pow_in);
-        m.pow = a.pow_in;
-        m.pos_out = a.pos_out;
-        m.pow_out = a.pow_out;
-        m.dir_out = a.dir_out;
-        m.pad_count = a.pad_count;
-        if (a.pad_count) k->pad = true;
-        tiles += (a.n + kSortTile - 1) / kSortTile;
-        k->levels = std::max(k->levels, m.lf);
-        k->maps.push_back(m);
-        k->index.push_back(i);
     }
-    k->nmaps = (int)k->maps.size();
-    k->total = tiles * kSortTile;
-    const int L = std::max(k->levels, 1);
-    std::vector<uint32_t> tile_map(std::max<uint32_t>(tiles, 1), 0);
-    std::vector<uint2> seg((size_t)L * std::max<uint32_t>(tiles, 1), make_uint2(0, 1));
-    std::vector<uint32_t> prefix((size_t)L * (k->nmaps + 1), 0);
-    std::vector<uint32_t> level_n(L, 0);
-    for (int mi = 0; mi < k->nmaps; ++mi) {
-        const KdMultiMap &m = k->maps[mi];
-        const uint32_t t0 = m.base / kSortTile, nt = (m.n + kSortTile - 1) / kSortTile;
-        for (uint32_t t = 0; t < nt; ++t) tile_map[t0 + t] = (uint32_t)mi;
-    }
-    k->level_tiles.assign(L, 0);
-    k->level_nodes.assign(L, 0);
-    k->level_maps.assign(L, 0);
-    for (int l = 0; l < k->levels; ++l) {
-        uint32_t nodes = 0;
-        for (int mi = 0; mi < k->nmaps; ++mi) {
-            const KdMultiMap &m = k->maps[mi];
-            prefix[(size_t)l * (k->nmaps + 1) + mi] = nodes;
-            if (l >= m.lf) continue;  // maps sorted by lf: the rest are finished
-            const uint32_t span = (32u << m.leaf_shift) << (m.depth - l);
-            const uint32_t t0 = m.base / kSortTile, nt = (m.n + kSortTile - 1) / kSortTile;
-            const uint32_t st = span / kSortTile;  // whole tiles at the sorted levels
-            for (uint32_t t = 0; t < nt; ++t) {
-                const uint32_t first = t / st * st;
-                seg[(size_t)l * tiles + t0 + t] = make_uint2(t0 + first, std::min(st, nt - first));
-            }
-            nodes += (m.n + span - 1) / span;
-            k->level_tiles[l] = t0 + nt;
-            k->level_maps[l] = (uint32_t)(mi + 1);
-        }
-        prefix[(size_t)l * (k->nmaps + 1) + k->nmaps] = nodes;
-        k->level_nodes[l] = nodes;
-        level_n[l] = k->level_tiles[l] * kSortTile;
-    }
-    // the finish tables: subtrees, leaf slots, inner nodes of levels 10 ..
-    const int nm1 = k->nmaps + 1;
-    for (const KdMultiMap &m : k->maps) k->max_depth = std::max(k->max_depth, m.depth);
-    const int inner_levels = std::max(k->max_depth - 10, 0);
-    std::vector<uint32_t> fin((size_t)(2 + inner_levels) * nm1, 0);
-    k->inner_nodes.assign(inner_levels, 0);
-    uint32_t subs = 0, leaves = 0;
-    std::vector<uint32_t> inner(inner_levels, 0);
-    for (int mi = 0; mi < k->nmaps; ++mi) {
-        const KdMultiMap &m = k->maps[mi];
-        fin[mi] = subs;
-        fin[nm1 + mi] = leaves;
-        if (m.lf < m.depth) {
-            const uint32_t span0 = (32u << m.leaf_shift) << (m.depth - m.lf);
-            subs += (m.n + span0 - 1) / span0;
-        }
-        leaves += 1u << m.depth;
-        for (int l = 10; l < m.depth; ++l) {
-            fin[(size_t)(2 + l - 10) * nm1 + mi] = inner[l - 10];
-            inner[l - 10] += 1u << l;
-        }
-        for (int l = std::max(m.depth, 10); l < k->max_depth; ++l) fin[(size_t)(2 + l - 10) * nm1 + mi] = inner[l - 10];
-    }
-    fin[k->nmaps] = subs;
-    fin[nm1 + k->nmaps] = leaves;
-    for (int l = 0; l < inner_levels; ++l) {
-        fin[(size_t)(2 + l) * nm1 + k->nmaps] = inner[l];
-        k->inner_nodes[l] = inner[l];
-    }
-    k->subtrees = subs;
-    k->leaves = leaves;
+    std::stable_sort(idx.begin(), idx.end(),
+                     [&](int x, int y) { return finish_level_of(args[x]) > finish_level_of(args[y]); });
+    const Layout L = layout_of(n.data(), shift.data(), (int)n.size());
     cudaError_t e;
 #define KM_TRY(x) do { e = (x); if (e != cudaSuccess) { kd_multi_free(*k); return e; } } while (0)
-    KM_TRY(kd_alloc(&k->fin_prefix, fin.size()));
-    KM_TRY(cudaMemcpy(k->fin_prefix, fin.data(), sizeof(uint32_t) * fin.size(), cudaMemcpyHostToDevice));
+    KM_TRY(cudaMalloc(&k->scratch, std::max<size_t>(L.total, 256)));
+    k->nmaps = (int)idx.size();
+    k->maps.resize(k->nmaps);
+    describe(args.data(), idx.data(), k->nmaps, L, k->scratch, k->maps.data());
+    k->tiles = L.tiles;
+    k->subs = L.subs;
+    k->clear_bytes = L.nodes ? L.clear : 0;
+    unsigned char *base = (unsigned char *)k->scratch;
+    k->hist = (uint32_t *)(base + L.hist);
+    k->box = (uint32_t *)(base + L.box);
+    k->thr = (uint4 *)(base + L.thr);
+    k->tile_cnt = (uint2 *)(base + L.tile_cnt);
+    std::vector<uint32_t> tile_map(std::max<uint32_t>(L.tiles, 1), 0), sub_first(k->nmaps + 1, 0);
+    for (int i = 0; i < k->nmaps; ++i) {
+        const KdMap &m = k->maps[i];
+        for (uint32_t t = 0; t < tiles_of(m.n); ++t) tile_map[m.tile0 + t] = (uint32_t)i;
+        sub_first[i] = m.sub0;
+        if (m.pad_count) k->pad = true;
+    }
+    sub_first[k->nmaps] = L.subs;
     KM_TRY(kd_alloc(&k->desc, k->nmaps));
     KM_TRY(kd_alloc(&k->tile_map, tile_map.size()));
-    KM_TRY(kd_alloc(&k->seg_tab, seg.size()));
-    KM_TRY(kd_alloc(&k->node_prefix, prefix.size()));
-    KM_TRY(kd_alloc(&k->level_n, level_n.size()));
-    KM_TRY(kd_alloc(&k->keys, k->total));
-    KM_TRY(kd_alloc(&k->keys_tmp, k->total));
-    KM_TRY(kd_alloc(&k->vals, k->total));
-    KM_TRY(kd_alloc(&k->vals_tmp, k->total));
-    KM_TRY(kd_alloc(&k->hist, radix_sort_hist_words(k->total)));
-    if (k->nmaps)
-        KM_TRY(cudaMemcpy(k->desc, k->maps.data(), sizeof(KdMultiMap) * k->nmaps, cudaMemcpyHostToDevice));
+    KM_TRY(kd_alloc(&k->sub_first, sub_first.size()));
+    if (k->nmaps) KM_TRY(cudaMemcpy(k->desc, k->maps.data(), sizeof(KdMap) * k->nmaps, cudaMemcpyHostToDevice));
     KM_TRY(cudaMemcpy(k->tile_map, tile_map.data(), sizeof(uint32_t) * tile_map.size(), cudaMemcpyHostToDevice));
-    KM_TRY(cudaMemcpy(k->seg_tab, seg.data(), sizeof(uint2) * seg.size(), cudaMemcpyHostToDevice));
-    KM_TRY(cudaMemcpy(k->node_prefix, prefix.data(), sizeof(uint32_t) * prefix.size(), cudaMemcpyHostToDevice));
-    KM_TRY(cudaMemcpy(k->level_n, level_n.data(), sizeof(uint32_t) * level_n.size(), cudaMemcpyHostToDevice));
+    KM_TRY(cudaMemcpy(k->sub_first, sub_first.data(), sizeof(uint32_t) * sub_first.size(), cudaMemcpyHostToDevice));
 #undef KM_TRY
     return cudaSuccess;
 }
 
 void kd_multi_free(KdMulti &k) {
-    cudaFree(k.desc); cudaFree(k.tile_map); cudaFree(k.seg_tab); cudaFree(k.node_prefix); cudaFree(k.level_n);
-    cudaFree(k.keys); cudaFree(k.keys_tmp); cudaFree(k.vals); cudaFree(k.vals_tmp); cudaFree(k.hist);
-    cudaFree(k.fin_prefix);
+    cudaFree(k.desc); cudaFree(k.tile_map); cudaFree(k.sub_first); cudaFree(k.scratch);
     k = KdMulti();
 }
 
-cudaError_t kd_multi_levels(KdMulti &k, cudaStream_t s, uint32_t **order) {
-    uint64_t *ka = k.keys, *kb = k.keys_tmp;
-    uint32_t *va = k.vals, *vb = k.vals_tmp;
-    *order = va;
+cudaError_t kd_multi_build(KdMulti &k, cudaStream_t s) {
     if (k.nmaps == 0) return cudaSuccess;
+    MapsN m;
+    m.m = k.desc;
+    m.tile_map = k.tile_map;
+    m.sub_first = k.sub_first;
+    m.n = k.nmaps;
+    if (k.clear_bytes) {
+        cudaError_t e = cudaMemsetAsync(k.scratch, 0, k.clear_bytes, s);
+        if (e != cudaSuccess) return e;
+    }
     if (k.pad) {
-        multi_pad_kernel<<<(k.total + 255) / 256, 256, 0, s>>>(k.desc, k.tile_map, k.total);
+        kd_pad_kernel<MapsN><<<k.tiles, kTileThreads, 0, s>>>(m);
         note_launch();
     }
-    multi_init_kernel<<<(k.total + 255) / 256, 256, 0, s>>>(k.desc, k.tile_map, k.total, va);
-    note_launch();
-    multi_root_kernel<<<(k.nmaps + 127) / 128, 128, 0, s>>>(k.desc, k.nmaps);
-    note_launch();
-    const uint32_t tiles = k.total / kSortTile;
-    for (int l = 0; l < k.levels; ++l) {
-        const uint32_t n = k.level_tiles[l] * kSortTile;
-        split_key_multi_kernel<<<(n + 255) / 256, 256, 0, s>>>(k.desc, k.tile_map, n, l, va, ka);
-        note_launch();
-        uint64_t *ko = nullptr;
-        uint32_t *vo = nullptr;
-        cudaError_t e = radix_sort_pairs_u64(ka, va, kb, vb, k.level_n + l, n, 0, 16, k.hist, s, &ko, &vo, 0,
-                                             k.seg_tab + (size_t)l * tiles);
-        if (e != cudaSuccess) return e;
-        if (vo != va) {
-            uint64_t *tk = ka; ka = kb; kb = tk;
-            uint32_t *tv = va; va = vb; vb = tv;
-        }
-        split_cell_multi_kernel<<<(k.level_nodes[l] + 255) / 256, 256, 0, s>>>(
-            k.desc, (int)k.level_maps[l], k.node_prefix + (size_t)l * (k.nmaps + 1), l, va);
-        note_launch();
-    }
-    *order = va;
-    return cudaGetLastError();
-}
-
-cudaError_t kd_multi_finish(KdMulti &k, uint32_t *order, cudaStream_t s) {
-    if (k.nmaps == 0) return cudaSuccess;
-    const int nm1 = k.nmaps + 1;
-    cudaError_t e;
-    if (k.subtrees > 0) {
-        const int smem = (int)sizeof(SubtreeScratch);
-        e = cudaFuncSetAttribute(multi_subtree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        multi_subtree_kernel<<<k.subtrees, kSubtreeThreads, smem, s>>>(k.desc, k.nmaps, k.fin_prefix, order);
-        note_launch();
-    }
-    multi_permute_kernel<<<(k.total + 255) / 256, 256, 0, s>>>(k.desc, k.tile_map, k.total, order);
-    note_launch();
-    multi_leaf_kernel<<<(uint32_t)(((uint64_t)k.leaves * 32 + 255) / 256), 256, 0, s>>>(k.desc, k.nmaps,
-                                                                                          k.fin_prefix + nm1);
-    note_launch();
-    for (int l = k.max_depth - 1; l >= 10; --l) {
-        const uint32_t cnt = k.inner_nodes[l - 10];
-        if (cnt == 0) continue;
-        multi_inner_kernel<<<(cnt + 255) / 256, 256, 0, s>>>(k.desc, k.nmaps, k.fin_prefix + (size_t)(2 + l - 10) * nm1,
-                                                             l);
-        note_launch();
-    }
-    multi_top_kernel<<<k.nmaps, 1024, 0, s>>>(k.desc);
-    note_launch();
-    return cudaGetLastError();
+    return launch_build(m, k.maps.data(), k.nmaps, k.subs, k.hist, k.box, k.thr, k.tile_cnt, s);
 }
 
 }  // namespace pm

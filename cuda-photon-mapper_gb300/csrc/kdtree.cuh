@@ -13,74 +13,81 @@ int tree_depth(uint32_t n, int leaf_shift = 0);
 size_t tree_nodes(uint32_t n, int leaf_shift = 0);
 
 struct KdBuildArgs {
-    uint32_t n;                 // records
-    const uint32_t *n_dev;      // the same count in device memory
-    float3 lo, hi;              // root cell (the scene box)
-    const float *box_dev;       // nullable: root cell read from device memory (6 floats)
-    const float4 *pos_in, *pow_in;   // records in index order (pow_in nullable)
-    float4 *pos_out, *pow_out;       // records in tree order (pow_out nullable)
+    uint32_t n = 0;                  // records
+    float3 lo, hi;                   // root cell (the scene box)
+    bool root_boxed = false;         // the root cell is the box already in the node words
+                                     // (kd_root_box_words): lo and hi are not read
+    const float4 *pos_in = nullptr, *pow_in = nullptr;  // records in index order, pos.w the index (pow_in nullable)
+    float4 *pos_out = nullptr, *pow_out = nullptr;      // records in tree order (pow_out with pow_in)
     float4 *dir_out = nullptr;       // nullable: decoded directions (xyz) in tree order
-    float4 *node_lo, *node_hi;       // tree_nodes(n) boxes
-    uint64_t *keys, *keys_tmp;       // n each
-    uint32_t *vals, *vals_tmp;       // n each
-    uint32_t *hist;                  // radix_sort_hist_words(n)
-    uint32_t *order_out;             // nullable: tree position -> record index
+    float4 *node_lo = nullptr, *node_hi = nullptr;      // tree_nodes(n) boxes
     int leaf_shift = 0;              // leaves of 32 << leaf_shift records
-    // multi build only (nullable): the records from *pad_count to n are set
-    // to infinity (position) and zero (power) before the build
+    // plans only (nullable): the records from *pad_count to n are set to
+    // infinity (position) and zero (power) before the build
     const uint32_t *pad_count = nullptr;
 };
 
-cudaError_t build_tree(const KdBuildArgs &a, cudaStream_t s);
-// The part of build_tree below the radix-sorted levels -- the subtree
-// finish, the permutation into tree order and the boxes -- for a tree whose
-// record order after those levels is order[0..a.n).
-cudaError_t build_tree_finish(const KdBuildArgs &a, uint32_t *order, cudaStream_t s);
+// One map of a build as the kernels read it.
+struct KdMap {
+    const float4 *pos, *pow;               // records in index order
+    float4 *pos_out, *pow_out, *dir_out;   // tree order
+    float4 *lo, *hi;                       // node boxes
+    float4 *tmp;                           // n records: the other buffer of the split levels
+    uint16_t *bins;                        // n: each record's bin at the current level
+    uint32_t *done;                        // finished subtrees (zero between builds)
+    const uint32_t *pad_count;             // nullable
+    float3 root_lo, root_hi;
+    uint32_t n, tile0, sub0, node0;        // first tile, subtree and node words of this map in the launch
+    int depth, lf, leaf_shift, root_boxed;
+};
 
-// Several trees built together (a batch's maps): the radix-sorted levels of
-// every map in shared launches over one pooled order, then each map's
-// finish (build_tree_finish). Each tree comes out as build_tree makes it.
-struct KdMultiMap {           // one map, device copy
-    const float4 *pos;        // records in index order
-    float4 *pad_pos, *pad_pow;     // the same arrays, written by the padding
-    const float4 *pow;
-    float4 *pos_out, *pow_out, *dir_out;  // tree order
-    const uint32_t *pad_count;     // nullable
-    float4 *cell_lo, *cell_hi;
-    float4 root_lo, root_hi;  // the root cell
-    uint32_t n;               // records
-    uint32_t base;            // first pooled position (a multiple of the sort tile)
-    int depth, lf, leaf_shift;
-};
+// Scratch of build_trees over these maps (one or two, built in shared
+// launches), in bytes.
+size_t kd_scratch_bytes(const uint32_t *n, const int *leaf_shift, int maps);
+// Builds the trees of one or two maps. scratch: kd_scratch_bytes, 256-byte
+// aligned.
+cudaError_t build_trees(const KdBuildArgs *a, int maps, void *scratch, cudaStream_t s);
+// A build of one map with root_boxed: the caller zeroes the scratch's words
+// (kd_clear_scratch) and fills the root's box -- ~kd_flip of the minimum and
+// kd_flip of the maximum per axis, combined with atomicMax, zero: no point
+// (null: the tree needs no root box) -- before build_trees, which then
+// leaves the clearing out.
+uint32_t *kd_root_box_words(const KdBuildArgs &a, void *scratch);
+cudaError_t kd_clear_scratch(const KdBuildArgs &a, void *scratch, cudaStream_t s);
+
+// Order-preserving words of a coordinate: kd_flip grows with x; a box's
+// minimum is kept as the complement so that both sides grow under atomicMax
+// from zero.
+__device__ __forceinline__ uint32_t kd_flip(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return u ^ ((uint32_t)((int)u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float kd_unflip(uint32_t f) {
+    return __uint_as_float(f ^ ((f & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+
+// Several trees built together (a batch's maps): one plan, shared launches.
+// Each tree comes out as build_trees makes it.
 struct KdMulti {
-    int nmaps = 0, levels = 0;          // levels: the most radix-sorted levels of any map
-    std::vector<KdMultiMap> maps;       // in build order: the most sorted levels first
-    std::vector<int> index;             // build order -> the caller's map index
-    KdMultiMap *desc = nullptr;
-    uint32_t *tile_map = nullptr;       // per pooled tile: its map (build order)
-    uint2 *seg_tab = nullptr;           // per level and pooled tile: (node's first tile, node's tiles)
-    uint32_t *node_prefix = nullptr;    // per level: nmaps + 1 scanned node counts of the sorted maps
-    uint32_t *level_n = nullptr;        // per level: pooled positions of the maps sorted at that level
-    std::vector<uint32_t> level_tiles, level_nodes, level_maps;
-    // the finish of every map at once: scanned per-map counts of subtrees,
-    // leaf slots and (per level from 10 up) inner nodes
-    uint32_t *fin_prefix = nullptr;     // subtrees, leaves, then one row per inner level
-    uint32_t subtrees = 0, leaves = 0;
-    int max_depth = 0;
-    std::vector<uint32_t> inner_nodes;  // per level 10 .. max_depth - 1
+    int nmaps = 0;
+    std::vector<KdMap> maps;            // the most split levels first
+    KdMap *desc = nullptr;
+    uint32_t *tile_map = nullptr;       // per tile: its map
+    uint32_t *sub_first = nullptr;      // per map: its first subtree (+ the total)
+    uint32_t tiles = 0, subs = 0;
     bool pad = false;                   // some map pads its records
-    uint32_t total = 0;                 // pooled positions
-    uint64_t *keys = nullptr, *keys_tmp = nullptr;
-    uint32_t *vals = nullptr, *vals_tmp = nullptr, *hist = nullptr;
+    void *scratch = nullptr;
+    uint32_t *hist = nullptr;           // into scratch
+    uint32_t *box = nullptr;
+    uint4 *thr = nullptr;
+    uint2 *tile_cnt = nullptr;
+    size_t clear_bytes = 0;             // of scratch, zeroed by each build
 };
-// Plans the build of the maps args[i] (n, pos_in, node_lo/hi, leaf_shift, lo/hi) and allocates
-// its tables and pooled scratch. Maps with no records are left out.
+// Plans the build of the maps args[i] and allocates its tables and scratch.
+// Maps with no records are left out.
 cudaError_t kd_multi_create(const std::vector<KdBuildArgs> &args, KdMulti *k);
 void kd_multi_free(KdMulti &k);
-// The padding and the shared levels of every map; *order receives the
-// pooled order (map i of the build order at *order + maps[i].base).
-cudaError_t kd_multi_levels(KdMulti &k, cudaStream_t s, uint32_t **order);
-// Every map's finish (build_tree_finish) in shared launches.
-cudaError_t kd_multi_finish(KdMulti &k, uint32_t *order, cudaStream_t s);
+// The padding and the trees of every map.
+cudaError_t kd_multi_build(KdMulti &k, cudaStream_t s);
 
 }  // namespace pm

@@ -56,9 +56,8 @@ struct PhysicalState {
         int leaf_shift = 0;
         bool built = false;
     } map[2];
-    uint64_t *keys = nullptr, *keys_tmp = nullptr;
-    uint32_t *vals = nullptr, *vals_tmp = nullptr, *hist = nullptr;
-    uint32_t sort_cap = 0;
+    void *kd_scratch = nullptr;  // tree builds
+    size_t kd_bytes = 0;
     unsigned long long *gctr = nullptr;
     cudaEvent_t ev[8] = {};  // emit, build, render, k-NN estimates within the render: start/stop
     pm_frame_stats stats;

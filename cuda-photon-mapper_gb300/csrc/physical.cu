@@ -39,14 +39,35 @@ void free_state(PhysicalState *st) {
         cudaFree(m.pos); cudaFree(m.pow); cudaFree(m.tpos); cudaFree(m.tpow); cudaFree(m.tdir);
         cudaFree(m.lo); cudaFree(m.hi);
     }
-    cudaFree(st->keys); cudaFree(st->keys_tmp); cudaFree(st->vals); cudaFree(st->vals_tmp);
-    cudaFree(st->hist);
+    cudaFree(st->kd_scratch);
     cudaFree(st->gctr);
     for (auto &e : st->ev)
         if (e) cudaEventDestroy(e);
     delete st;
 }
 
+// Both trees in shared launches while that saves launches worth saving: at
+// 4M records a split level takes about ten times a launch's latency, and
+// larger maps share the scratch instead.
+bool kd_together(uint32_t n0, uint32_t n1) { return (uint64_t)n0 + n1 <= (1u << 22); }
+
+// Build scratch for the maps' capacities (grown, never shrunk). A map holds
+// any number of records up to its capacity, and the scratch grows with it.
+cudaError_t kd_reserve(PhysicalState *st) {
+    const uint32_t n[2] = {st->map[0].cap, st->map[1].cap};
+    const int ls[2] = {st->map[0].leaf_shift, st->map[1].leaf_shift};
+    size_t bytes = std::max(kd_scratch_bytes(n, ls, 1), kd_scratch_bytes(n + 1, ls + 1, 1));
+    // the two built together: any pair of sizes kd_together admits
+    const uint32_t half[2] = {std::min(n[0], 1u << 22), std::min(n[1], 1u << 22)};
+    bytes = std::max(bytes, kd_scratch_bytes(half, ls, 2));
+    if (bytes <= st->kd_bytes) return cudaSuccess;
+    cudaFree(st->kd_scratch);
+    st->kd_scratch = nullptr;
+    st->kd_bytes = 0;
+    cudaError_t e = cudaMalloc(&st->kd_scratch, bytes);
+    if (e == cudaSuccess) st->kd_bytes = bytes;
+    return e;
+}
 
 }  // namespace
 
@@ -110,12 +131,7 @@ pm_status pm_set_scene(pm_ctx *ctx, const pm_scene *scene, const pm_config *cfg)
         PM_TRY(dalloc(&mp.lo, tree_nodes(mp.cap)));
         PM_TRY(dalloc(&mp.hi, tree_nodes(mp.cap)));
     }
-    PM_TRY(dalloc(&st->keys, tmax));
-    PM_TRY(dalloc(&st->keys_tmp, tmax));
-    PM_TRY(dalloc(&st->vals, tmax));
-    PM_TRY(dalloc(&st->vals_tmp, tmax));
-    PM_TRY(dalloc(&st->hist, radix_sort_hist_words(std::max<uint32_t>(tmax, 1))));
-    st->sort_cap = tmax;
+    PM_TRY(kd_reserve(st));
     PM_TRY(dalloc(&st->gctr, 2));
     if (scene->het_res > 0) {
         const size_t nv = (size_t)scene->het_res * scene->het_res * scene->het_res;
@@ -230,14 +246,12 @@ pm_status pm_build(pm_ctx *ctx, cudaStream_t stream) {
     DeviceGuard g(ctx->device);
     cudaError_t e;
     PM_TRY(cudaEventRecord(st->ev[2], stream));
+    KdBuildArgs args[2];
     for (int m = 0; m < 2; ++m) {
         auto &mp = st->map[m];
-        if (mp.n == 0) { mp.built = true; continue; }
-        if (mp.depth > 29) return fail(ctx, PM_ERR_LIMIT, "photon map too large for the tree");
-        KdBuildArgs a;
-        a.box_dev = nullptr;
+        if (mp.n > 0 && mp.depth > 29) return fail(ctx, PM_ERR_LIMIT, "photon map too large for the tree");
+        KdBuildArgs &a = args[m];
         a.n = mp.n;
-        a.n_dev = st->words + 4 + 2 * m;
         a.lo = make_float3(st->scene.box_min[0], st->scene.box_min[1], st->scene.box_min[2]);
         a.hi = make_float3(st->scene.box_max[0], st->scene.box_max[1], st->scene.box_max[2]);
         a.pos_in = mp.pos;
@@ -247,14 +261,14 @@ pm_status pm_build(pm_ctx *ctx, cudaStream_t stream) {
         a.dir_out = mp.tdir;
         a.node_lo = mp.lo;
         a.node_hi = mp.hi;
-        a.keys = st->keys; a.keys_tmp = st->keys_tmp;
-        a.vals = st->vals; a.vals_tmp = st->vals_tmp;
-        a.hist = st->hist;
-        a.order_out = nullptr;
         a.leaf_shift = mp.leaf_shift;
-        PM_TRY(build_tree(a, stream));
-        mp.built = true;
     }
+    if (kd_together(args[0].n, args[1].n)) {
+        PM_TRY(build_trees(args, 2, st->kd_scratch, stream));
+    } else {
+        for (int m = 0; m < 2; ++m) PM_TRY(build_trees(args + m, 1, st->kd_scratch, stream));
+    }
+    for (auto &mp : st->map) mp.built = true;
     PM_TRY(cudaEventRecord(st->ev[3], stream));
     PM_TRY(cudaEventSynchronize(st->ev[3]));
     float ms = 0.f;
@@ -433,14 +447,7 @@ pm_status pm_set_photons(pm_ctx *ctx, int map, const float4 *pos, const float4 *
         PM_TRY(dalloc(&mp.tpos, n)); PM_TRY(dalloc(&mp.tpow, n)); PM_TRY(dalloc(&mp.tdir, n));
         PM_TRY(dalloc(&mp.lo, tree_nodes(n))); PM_TRY(dalloc(&mp.hi, tree_nodes(n)));
         mp.cap = n;
-        if (n > st->sort_cap) {
-            cudaFree(st->keys); cudaFree(st->keys_tmp); cudaFree(st->vals); cudaFree(st->vals_tmp);
-            cudaFree(st->hist);
-            PM_TRY(dalloc(&st->keys, n)); PM_TRY(dalloc(&st->keys_tmp, n));
-            PM_TRY(dalloc(&st->vals, n)); PM_TRY(dalloc(&st->vals_tmp, n));
-            PM_TRY(dalloc(&st->hist, radix_sort_hist_words(n)));
-            st->sort_cap = n;
-        }
+        PM_TRY(kd_reserve(st));
     }
     std::vector<float4> tmp(pos, pos + n);
     for (uint32_t i = 0; i < n; ++i) memcpy(&tmp[i].w, &i, 4);
