@@ -23,6 +23,7 @@
 #include "radix_sort.cuh"
 
 #include <algorithm>
+#include <cstddef>
 
 namespace pm {
 namespace {
@@ -174,7 +175,13 @@ __device__ bool step_path(const PScene &S, const TraceParams &P, Path &p, const 
 // refilling lanes rarely waits for the counter; every block a warp takes is
 // traced in full (the ids stay a gap-free prefix, which the record extents
 // need), and the counting pass stops requesting blocks once both maps are
-// full.
+// full. The records of finished paths are counted in registers and added to
+// the maps' counters once per block; the sums those atomics return, looked
+// at when the warp takes its next block, say whether the maps are full. One
+// addition per finished path instead puts three billion atomics a second on
+// two addresses, which is about what one L2 sector serves: it, not the
+// tracing, bounded scenes of few spheres (preset 2, 8.5M paths: 3.51 -> 1.72
+// ms; preset 1, 1.1M paths: 0.54 -> 0.38 ms).
 constexpr uint32_t kIdBlock = 32;
 
 // The persistent per-warp loop of one scene: keep 32 live paths, refill
@@ -194,6 +201,8 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
     bool live = false;
     // warp-uniform pool [pool, pool_end); lane 0 holds the prefetched block
     uint32_t pool = 0, pool_end = 0, pending = 0;
+    uint32_t done_s = 0, done_v = 0;  // counting pass: this lane's records not yet added
+    uint32_t seen_s = 0, seen_v = 0;  // lane 0: the counters after the warp's last addition
     bool has_pending = cap > 0;
     if (has_pending && lane == 0) pending = atomicAdd(P.path_counter, kIdBlock);
     for (;;) {
@@ -209,11 +218,15 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
                 took = true;
                 bool more = nb < cap && cap - nb > kIdBlock;
                 if (more && !P.store) {
-                    int full = 0;
-                    if (lane == 0)
-                        full = *((volatile uint32_t *)P.stored_s) >= P.target_s &&
-                               *((volatile uint32_t *)P.stored_v) >= P.target_v;
+                    const int full = seen_s >= P.target_s && seen_v >= P.target_v;
                     more = __shfl_sync(0xffffffffu, full, 0) == 0;
+                    const uint32_t ns = __reduce_add_sync(0xffffffffu, done_s);
+                    const uint32_t nv = __reduce_add_sync(0xffffffffu, done_v);
+                    done_s = done_v = 0;
+                    if (lane == 0) {
+                        seen_s = atomicAdd(P.stored_s, ns) + ns;
+                        seen_v = atomicAdd(P.stored_v, nv) + nv;
+                    }
                 }
                 if (more) {
                     if (lane == 0) pending = atomicAdd(P.path_counter, kIdBlock);
@@ -259,8 +272,8 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
                     uint32_t nv = min(p.nv, (uint32_t)P.max_bounces);
                     P.cnt_s[p.id] = ns;
                     P.cnt_v[p.id] = nv;
-                    if (ns) atomicAdd(P.stored_s, ns);
-                    if (nv) atomicAdd(P.stored_v, nv);
+                    done_s += ns;
+                    done_v += nv;
                 }
                 live = false;
             }
@@ -268,7 +281,18 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
     }
 }
 
-__global__ void __launch_bounds__(128) trace_kernel(PScene S, TraceParams P) { trace_loop(S, P); }
+// The scene is read from shared memory: the lanes' materials and normals
+// sit at different objects, which the constant bank serves one at a time
+// (preset 3, 87.6M paths: 57.8 -> 56.1 ms). 8 blocks per SM: 64 registers.
+__global__ void __launch_bounds__(128, 8) trace_kernel(const __grid_constant__ PScene S,
+                                                       const __grid_constant__ TraceParams P) {
+    __shared__ PScene sS;
+    const uint32_t *a = reinterpret_cast<const uint32_t *>(&S);
+    uint32_t *b = reinterpret_cast<uint32_t *>(&sS);
+    for (int i = threadIdx.x; i < (int)(offsetof(PScene, cell_mask) / 4); i += blockDim.x) b[i] = a[i];
+    __syncthreads();
+    trace_loop(sS, P);
+}
 
 // Many scenes in one persistent launch: every block walks the scene list
 // (starting at a different scene per block, so scenes are worked on side
