@@ -130,42 +130,79 @@ __global__ void __launch_bounds__(kSortThreads) hist_kernel(const uint32_t *keys
     hist[count_at(threadIdx.x, blockIdx.x, ntiles, seg_tab)] = h[threadIdx.x];
 }
 
+// A warp ranks its own 512 consecutive items of the tile against its own
+// digit counters (no block barrier inside); one pass over the warps' counters
+// and a scan of the digits turn the ranks into places in the tile's sorted
+// order, which is staged in shared memory, so that each digit's run leaves in
+// consecutive writes. Bound by those writes: a run averages 64 bytes.
+// Measured per pass: 41M pairs 396 us, 5 tiles 10 us (ranking 256 items at a
+// time with four block barriers each and writing them unstaged: 528 us,
+// 30 us; this ranking written unstaged: 732 us for 41M).
 __global__ void __launch_bounds__(kSortThreads) scatter_kernel(
     const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
     const uint32_t *n_dev, int shift, const uint32_t *offs, uint32_t ntiles,
     const uint2 *seg_tab) {
     constexpr int kWarps = kSortThreads / 32;
-    __shared__ uint32_t run[256];
     __shared__ uint32_t wcnt[kWarps][256];
-    const int warp = threadIdx.x >> 5;
+    __shared__ uint32_t sk[kSortTile], sv[kSortTile];
+    __shared__ uint32_t gofs[256], warp_sums[32], total;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n = *n_dev;
-    const uint32_t base = blockIdx.x * kSortTile;
-    run[threadIdx.x] = offs[count_at(threadIdx.x, blockIdx.x, ntiles, seg_tab)];
+    if (blockIdx.x * kSortTile >= n) return;
+    const uint32_t base = blockIdx.x * kSortTile + (uint32_t)warp * (32u * kSortItems) + (uint32_t)lane;
+    uint32_t k[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) k[r] = base + 32u * r < n ? keys_in[base + 32u * r] : 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wcnt[warp][32 * i + lane] = 0u;
+    __syncwarp();
+#pragma unroll
     for (int r = 0; r < kSortItems; ++r) {
-        const uint32_t idx = base + r * kSortThreads + threadIdx.x;
-        if (base + r * kSortThreads >= n) break;  // uniform across the block
+        const bool valid = base + 32u * r < n;
+        const uint32_t d = valid ? ((k[r] >> shift) & 255u) : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = valid ? wcnt[warp][d] : 0u;
+        rank[r] = before + __popc(peers & lanemask_lt());
+        __syncwarp();
+        if (valid && (peers & lanemask_lt()) == 0u) wcnt[warp][d] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    {
+        // digit threadIdx.x: its items in the tile, its place among the
+        // digits, the warps in order, and what takes a place to the output
+        uint32_t c[kWarps], sum = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) wcnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        const bool valid = idx < n;
-        uint32_t k = valid ? keys_in[idx] : 0u;
-        uint32_t d = valid ? ((k >> shift) & 255u) : 256u;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        uint32_t rank = __popc(peers & lanemask_lt());
-        if (valid && rank == 0) wcnt[warp][d] = __popc(peers);
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = run[d] + rank;
-            for (int w = 0; w < warp; ++w) pos += wcnt[w][d];
-            keys_out[pos] = k;
-            vals_out[pos] = vals_in[idx];
+        for (int w = 0; w < kWarps; ++w) {
+            c[w] = wcnt[w][threadIdx.x];
+            sum += c[w];
         }
-        __syncthreads();
-        uint32_t add = 0;
+        uint32_t run = block_exclusive_scan(sum, warp_sums, &total);
+        gofs[threadIdx.x] = offs[count_at(threadIdx.x, blockIdx.x, ntiles, seg_tab)] - run;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) add += wcnt[w][threadIdx.x];
-        run[threadIdx.x] += add;
-        __syncthreads();
+        for (int w = 0; w < kWarps; ++w) {
+            wcnt[w][threadIdx.x] = run;
+            run += c[w];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r)
+        if (base + 32u * r < n) {
+            const uint32_t at = wcnt[warp][(k[r] >> shift) & 255u] + rank[r];
+            sk[at] = k[r];
+            sv[at] = vals_in[base + 32u * r];
+        }
+    __syncthreads();
+    const uint32_t cnt = min((uint32_t)kSortTile, n - blockIdx.x * kSortTile);
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const uint32_t t = (uint32_t)r * kSortThreads + threadIdx.x;
+        if (t < cnt) {
+            const uint32_t key = sk[t], at = gofs[(key >> shift) & 255u] + t;
+            keys_out[at] = key;
+            vals_out[at] = sv[t];
+        }
     }
 }
 
