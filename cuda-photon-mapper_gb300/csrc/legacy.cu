@@ -10,6 +10,7 @@
 // ahead, and grid accumulation is a deterministic sort + ordered sum.
 #include "launch_count.cuh"
 #include "legacy.cuh"
+#include "legacy_voxel.cuh"
 #include "pm_vec.cuh"
 #include "radix_sort.cuh"
 
@@ -24,8 +25,11 @@ struct Scene {
     float sph[2][4];  // the two traced spheres (nrObjects = {2,5}, :61)
 };
 
-__constant__ int c_plane_axis[5] = {0, 1, 0, 1, 2};              // planes[] (:66-72)
-__constant__ float c_plane_off[5] = {1.5f, -1.5f, -1.5f, 1.5f, 6.0f};
+// planes[] (:66-72), folded into the unrolled loop over them
+__device__ __forceinline__ int plane_axis(int i) { return i == 4 ? 2 : i & 1; }
+__device__ __forceinline__ float plane_off(int i) {
+    return i == 4 ? 6.0f : (i == 0 || i == 3 ? 1.5f : -1.5f);
+}
 __constant__ float c_vox_dim[3] = {0.09375f, 0.09375f, 0.1875f};  // getVoxelDim (:426-437)
 
 __device__ __forceinline__ v3 light_pos() { return mk3(0.0f, 1.4f, 3.5f); }  // Light (:64)
@@ -49,18 +53,18 @@ __device__ void trace(const Scene &sc, v3 r, v3 o, Hit &h) {
         v3 s = mk3(sc.sph[i][0], sc.sph[i][1], sc.sph[i][2]) - o;
         float rad = sc.sph[i][3];
         float A = dot(r, r);
-        float B = (float)(-2.0 * (double)dot(s, r));
+        float B = -2.0f * dot(s, r);  // a power of two: exact, as in double
         float C = dot(s, s) - rad * rad;
         float D = B * B - (4.0f * A) * C;
         if (D > 0.0f) {
-            float sign = ((double)C < -0.00001) ? 1.0f : -1.0f;
+            float sign = C < -0.00001f ? 1.0f : -1.0f;  // no float lies between the constant and its double
             consider(h, (-B + sign * sqrtf(D)) / (2.0f * A), 0, i);
         }
     }
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-        float ra = axis_of(r, c_plane_axis[i]);
-        if (ra != 0.0f) consider(h, (c_plane_off[i] - axis_of(o, c_plane_axis[i])) / ra, 1, i);
+        float ra = axis_of(r, plane_axis(i));
+        if (ra != 0.0f) consider(h, (plane_off(i) - axis_of(o, plane_axis(i))) / ra, 1, i);
     }
 }
 
@@ -68,7 +72,7 @@ __device__ void trace(const Scene &sc, v3 r, v3 o, Hit &h) {
 __device__ v3 normal_at(const Scene &sc, int type, int idx, v3 p, v3 from) {
     if (type == 0) return normalize(p - mk3(sc.sph[idx][0], sc.sph[idx][1], sc.sph[idx][2]));
     v3 n = mk3(0.0f, 0.0f, 0.0f);
-    set_axis(n, c_plane_axis[idx], axis_of(from, c_plane_axis[idx]) - c_plane_off[idx]);
+    set_axis(n, plane_axis(idx), axis_of(from, plane_axis(idx)) - plane_off(idx));
     return normalize(n);
 }
 
@@ -126,17 +130,15 @@ struct I3 {
 
 __device__ __forceinline__ I3 voxel_of(v3 p) {  // getVoxelCoordinates (:254-261)
     I3 v;
-    v.x = d2i_sat((((double)p.x + 1.5) / 3.0) * 32.0);
-    v.y = d2i_sat((((double)p.y + 1.5) / 3.0) * 32.0);
-    v.z = d2i_sat(((double)p.z / 6.0) * 32.0);
+    v.x = legacy_voxel_xy(p.x);
+    v.y = legacy_voxel_xy(p.y);
+    v.z = legacy_voxel_z(p.z);
     return v;
 }
 
 __device__ __forceinline__ v3 voxel_center(v3 p) {  // centerPoint + getWorldCoordinates (:263-268, 392-400)
     I3 v = voxel_of(p);
-    v3 c = mk3((float)((double)((float)v.x / 32.0f) * 3.0 - 1.5),
-               (float)((double)((float)v.y / 32.0f) * 3.0 - 1.5),
-               (float)((double)((float)v.z / 32.0f) * 6.0));
+    v3 c = mk3(legacy_world_xy(v.x), legacy_world_xy(v.y), legacy_world_z(v.z));
     return c + mk3(0.046875f, 0.046875f, 0.09375f);
 }
 
@@ -172,7 +174,9 @@ __device__ v3 integrate_slab(const float4 *__restrict__ g, v3 e, I3 wp, int type
 }
 
 __device__ __forceinline__ v3 lerp3(v3 a, v3 b, float t) {  // interpolate3f (:421-423)
-    return a * (float)(1.0 - (double)t) + b * t;
+    // 1 - t rounds to the same float as through double: the double is exact
+    // unless t is below 2^-29, where both give 1
+    return a * (1.0f - t) + b * t;
 }
 
 __device__ __forceinline__ float alpha_of(v3 p, v3 a, v3 b, int ax) {  // getAlpha (:404-418)
@@ -186,8 +190,16 @@ __device__ v3 integrate_volume(const float4 *__restrict__ g, I3 wp) {
     int x0 = lo_edge(wp.x, 1), y0 = lo_edge(wp.y, 1), z0 = lo_edge(wp.z, 1);
     int x1 = hi_edge(wp.x, G - 1), y1 = hi_edge(wp.y, G - 1), z1 = hi_edge(wp.z, G - 1);
     for (int i = x0; i < x1; ++i)
-        for (int j = y0; j < y1; ++j)
-            for (int k = z0; k < z1; ++k) acc = acc + grid_at(g, i, j, k);
+        for (int j = y0; j < y1; ++j) {
+            // a row of the window is at most six voxels: all its loads together
+            v3 g6[6];
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (z0 + k < z1) g6[k] = grid_at(g, i, j, z0 + k);
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                if (z0 + k < z1) acc = acc + g6[k];
+        }
     return acc;
 }
 
@@ -275,54 +287,93 @@ __device__ v3 interpolate_slab(const float4 *__restrict__ slab, v3 p, int type, 
 
 // ---- emission --------------------------------------------------------------
 
+// A photon's path is traced by kPhotonLanes lanes together: the path is the
+// same on each of them, a wall's splat window of up to 36 cells takes a cell
+// per lane. 8 lanes: the path's arithmetic is repeated eight times, the
+// window's is spread over them. The writing launch takes 61 us, the counting
+// one, which needs no windows, 37 us (a thread per photon, which walks a
+// bounce's 72 cells one by one: 121 us each).
+constexpr int kPhotonLanes = 8;
+__device__ __forceinline__ int photon_lane() { return (int)(threadIdx.x & (kPhotonLanes - 1)); }
+__device__ __forceinline__ unsigned photon_mask() {
+    return ((1u << kPhotonLanes) - 1u) << (threadIdx.x & (31u & ~(kPhotonLanes - 1u)));
+}
+
 // Records a photon's grid deposits in the order the reference applies them.
-// The counting pass only counts; the writing pass stores (voxel, value)
-// at this photon's offset.
+// The counting pass (kWrite false) only counts; the writing pass stores
+// (voxel, value) at this photon's offset.
+template <bool kWrite>
 struct Deposits {
     uint32_t *keys, *idx;
     float4 *vals;
+    const float *inv;  // 1 / sqrt(i), i < kInvN
     uint32_t off, n;
+    __device__ __forceinline__ void store(uint32_t at, int vox, v3 e) {
+        keys[at] = (uint32_t)vox;
+        idx[at] = at;
+        vals[at] = make_float4(e.x, e.y, e.z, 0.0f);
+    }
+    // One deposit (the same on every lane).
     __device__ __forceinline__ void put(int vox, v3 e) {
-        if (keys) {
-            uint32_t at = off + n;
-            keys[at] = (uint32_t)vox;
-            idx[at] = at;
-            vals[at] = make_float4(e.x, e.y, e.z, 0.0f);
-        }
+        if (kWrite && photon_lane() == 0) store(off + n, vox, e);
         ++n;
+    }
+    // One deposit on each lane with `on`, in lane order.
+    __device__ __forceinline__ void put_lanes(bool on, int vox, v3 e) {
+        const unsigned m = __ballot_sync(photon_mask(), on);
+        if (on) store(off + n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u)), vox, e);
+        n += __popc(m);
     }
 };
 
-__device__ __forceinline__ I3 clamp_voxel(I3 v) {
-    v.x = v.x < G ? v.x : G - 1; v.x = v.x < 0 ? 0 : v.x;
-    v.y = v.y < G ? v.y : G - 1; v.y = v.y < 0 ? 0 : v.y;
-    v.z = v.z < G ? v.z : G - 1; v.z = v.z < 0 ? 0 : v.z;
+// Squared distances of a splat: two axes up to 3 cells, one up to 31.
+constexpr int kInvN = 31 * 31 + 3 * 3 + 3 * 3 + 1;
+
+// The voxel of p clamped to the grid. A coordinate beyond the fast range
+// lies outside the grid: above it only a positive one clamps to the last
+// voxel, NaN converts to 0 (a shadow photon that hits nothing is there).
+__device__ __forceinline__ int clamped(float x, int v) {
+    const int far = x >= kLegacyFastRange ? G - 1 : 0;
+    return fabsf(x) < kLegacyFastRange ? min(max(v, 0), G - 1) : far;
+}
+__device__ __forceinline__ I3 clamped_voxel(v3 p) {
+    const float r = kLegacyFastRange;
+    I3 v;
+    v.x = clamped(p.x, legacy_voxel_xy(fabsf(p.x) < r ? p.x : 0.0f));
+    v.y = clamped(p.y, legacy_voxel_xy(fabsf(p.y) < r ? p.y : 0.0f));
+    v.z = clamped(p.z, legacy_voxel_z(fabsf(p.z) < r ? p.z : 0.0f));
     return v;
 }
 
-__device__ __forceinline__ void splat_one(Deposits &d, v3 e, I3 c, int i, int j, int k) {  // :1059-1071
-    if (c.x == i && c.y == j && c.z == k) return;
-    int dx = c.x - i, dy = c.y - j, dz = c.z - k;
-    float dist = sqrtf((float)(dx * dx + dy * dy + dz * dz));
-    d.put(vox_index(i, j, k), div_scalar(e * 0.05f, dist));
-}
-
-// storePhoton + splatEnergy (:1074-1144, 1164-1183).
-__device__ void store_surface(Deposits &d, int type, int id, v3 loc, v3 e) {
-    I3 c = clamp_voxel(voxel_of(loc));
+// storePhoton + splatEnergy (:1074-1144, 1164-1183): the window's cells in
+// the reference's row order, a cell per lane. A cell's value is the energy's
+// twentieth over its distance (:1059-1071), whose reciprocal depends only on
+// the squared distance in cells and is read from a table.
+template <bool kWrite>
+__device__ __forceinline__ void store_surface(Deposits<kWrite> &d, int type, int id, v3 loc, v3 e) {
+    I3 c = clamped_voxel(loc);
     if (type != 0) d.put(vox_index(c.x, c.y, c.z), e);
-    if (type != 1) return;
-    int x0 = lo_edge(c.x, 0), y0 = lo_edge(c.y, 0), z0 = lo_edge(c.z, 0);
-    int x1 = hi_edge(c.x, G), y1 = hi_edge(c.y, G), z1 = hi_edge(c.z, G);
-    if (id == 0 || id == 2) {
-        int i = id == 0 ? G - 1 : 0;
-        for (int j = y0; j < y1; ++j) for (int k = z0; k < z1; ++k) splat_one(d, e, c, i, j, k);
-    } else if (id == 1 || id == 3) {
-        int j = id == 1 ? 0 : G - 1;
-        for (int i = x0; i < x1; ++i) for (int k = z0; k < z1; ++k) splat_one(d, e, c, i, j, k);
-    } else if (id == 4) {
-        int k = G - 1;
-        for (int i = x0; i < x1; ++i) for (int j = y0; j < y1; ++j) splat_one(d, e, c, i, j, k);
+    if (type != 1 || id < 0 || id > 4) return;
+    // the wall's fixed coordinate and its two free ones, outer a, inner b
+    const bool on_x = id == 0 || id == 2, on_y = id == 1 || id == 3;
+    const int fixed = id == 1 || id == 2 ? 0 : G - 1;
+    const int ca = on_x ? c.y : c.x, cb = on_x || on_y ? c.z : c.y, cf = on_x ? c.x : (on_y ? c.y : c.z);
+    const int a0 = lo_edge(ca, 0), a1 = hi_edge(ca, G), b0 = lo_edge(cb, 0), b1 = hi_edge(cb, G);
+    const int nb = b1 - b0, cells = (a1 - a0) * nb;  // 3 to 6 a side
+    if (!kWrite) {
+        d.n += (uint32_t)(cells - (cf == fixed ? 1 : 0));  // the photon's own cell is left out
+        return;
+    }
+    const v3 e20 = e * 0.05f;
+    const int rcp = 65536 / nb + 1;  // t / nb for t < 64
+    const int df = cf - fixed;
+    for (int base = 0; base < cells; base += kPhotonLanes) {
+        const int t = base + photon_lane();
+        const int row = (t * rcp) >> 16, a = a0 + row, b = b0 + (t - row * nb);
+        const int i = on_x ? fixed : a, j = on_y ? fixed : (on_x ? a : b), k = on_x || on_y ? b : fixed;
+        const int da = ca - a, db = cb - b, d2 = da * da + db * db + df * df;
+        const bool on = t < cells && d2 > 0;
+        d.put_lanes(on, vox_index(i, j, k), e20 * (on ? d.inv[d2] : 0.0f));
     }
 }
 
@@ -363,8 +414,9 @@ struct Mwc {
 
 // emitPhotons (:1215-1375) for photon `index`; the medium steps draw from
 // the generator positioned at this photon's first draw.
+template <bool kWrite>
 __device__ void emit_one(const Scene &sc, const float4 *__restrict__ table, int index, bool media,
-                         Mwc rng, Deposits &d) {
+                         Mwc rng, Deposits<kWrite> &d) {
     int bounces = 1;
     v3 rgb = mk3(10.0f, 10.0f, 10.0f);
     float4 t = table[index];
@@ -377,7 +429,7 @@ __device__ void emit_one(const Scene &sc, const float4 *__restrict__ table, int 
         for (int i = 0; i < 3; ++i) {
             rgb = sub_scalar(rgb, 1.0f);
             c.point = ray * 1.0f + prev;
-            I3 v = clamp_voxel(voxel_of(c.point));
+            I3 v = clamped_voxel(c.point);
             d.put(vox_index(v.x, v.y, v.z), rgb * 0.00005f);
             float4 q = table[i];
             v3 rnd;
@@ -429,93 +481,142 @@ __device__ void emit_one(const Scene &sc, const float4 *__restrict__ table, int 
     }
 }
 
-__global__ void __launch_bounds__(256) emit_kernel(Scene sc, const float4 *__restrict__ table,
-                                                   bool media, uint32_t z0, uint32_t w0,
-                                                   uint32_t *counts, const uint32_t *offsets,
-                                                   uint32_t *keys, uint32_t *idx, float4 *vals) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kLegacyPhotons) return;
+// base^(9 * 2^i) of both generator halves: photon p's medium loop starts
+// 9p draws after the emission's first, p below 2^14.
+constexpr int kJumpBits = 16;
+static_assert(kLegacyPhotons <= 1 << kJumpBits && kJumpBits % kPhotonLanes == 0, "jump powers cover every photon");
+struct JumpTable {
+    uint32_t z[kJumpBits], w[kJumpBits];
+};
+
+// The generator 9p draws on: each lane of the photon multiplies the powers
+// of its share of p's bits, three butterfly steps the rest.
+__device__ __forceinline__ Mwc jump_photon(const JumpTable &J, uint32_t z0, uint32_t w0, int p) {
+    uint32_t z = 1u, w = 1u;
+#pragma unroll
+    for (int i = 0; i < kJumpBits / kPhotonLanes; ++i) {
+        const int bit = i * kPhotonLanes + photon_lane();
+        if ((p >> bit) & 1) {
+            z = mulmod(z, J.z[bit], kMwcMz);
+            w = mulmod(w, J.w[bit], kMwcMw);
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < kPhotonLanes; o <<= 1) {
+        z = mulmod(z, __shfl_xor_sync(photon_mask(), z, o), kMwcMz);
+        w = mulmod(w, __shfl_xor_sync(photon_mask(), w, o), kMwcMw);
+    }
+    Mwc r;
+    r.z = mulmod(z, z0, kMwcMz);
+    r.w = mulmod(w, w0, kMwcMw);
+    return r;
+}
+
+// Bound by the latency of a photon's serial bounces and their arithmetic.
+template <bool kWrite>
+__global__ void __launch_bounds__(256) emit_kernel(Scene sc, const float4 *__restrict__ table, bool media,
+                                                   uint32_t z0, uint32_t w0, JumpTable jump, uint32_t *counts,
+                                                   const uint32_t *offsets, uint32_t *keys, uint32_t *idx,
+                                                   float4 *vals) {
+    __shared__ float inv[kWrite ? kInvN : 1];
+    if (kWrite) {
+        for (int i = threadIdx.x; i < kInvN; i += blockDim.x) inv[i] = 1.0f / sqrtf((float)i);
+        __syncthreads();
+    }
+    const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kPhotonLanes);
+    if (p >= kLegacyPhotons) return;  // whole photons
     Mwc rng;
     rng.z = z0;
     rng.w = w0;
-    if (media) {  // each photon's medium loop takes 9 draws, photons in index order
-        rng.z = mwc_jump(z0, kMwcAz, kMwcMz, 9ull * (uint64_t)p);
-        rng.w = mwc_jump(w0, kMwcAw, kMwcMw, 9ull * (uint64_t)p);
-    }
-    Deposits d;
-    d.keys = offsets ? keys : nullptr;
+    if (kWrite && media) rng = jump_photon(jump, z0, w0, p);  // the draws do not change the count
+    Deposits<kWrite> d;
+    d.keys = keys;
     d.idx = idx;
     d.vals = vals;
-    d.off = offsets ? offsets[p] : 0u;
+    d.inv = inv;
+    d.off = kWrite ? offsets[p] : 0u;
     d.n = 0;
     emit_one(sc, table, p, media, rng, d);
-    if (!offsets) counts[p] = d.n;
+    if (!kWrite && photon_lane() == 0) counts[p] = d.n;
 }
 
 // Deposit values in sorted order (one parallel gather), so that each
-// voxel's sum below streams a contiguous range.
-__global__ void gather_deposits_kernel(const uint32_t *__restrict__ sidx,
-                                       const float4 *__restrict__ vals, const uint32_t *total,
-                                       float4 *sorted) {
+// voxel's sum below streams a contiguous range, and each voxel's first
+// deposit (start[v] = the deposits below voxel v).
+__global__ void gather_deposits_kernel(const uint32_t *__restrict__ skeys, const uint32_t *__restrict__ sidx,
+                                       const float4 *__restrict__ vals, const uint32_t *total, float4 *sorted,
+                                       uint32_t *start) {
     const uint32_t n = *total;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (uint32_t j = first; j < n; j += step) {
         sorted[j] = vals[sidx[j]];
-}
-
-__device__ __forceinline__ uint32_t first_at_least(const uint32_t *__restrict__ keys, uint32_t n,
-                                                   uint32_t v) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (keys[mid] < v) lo = mid + 1; else hi = mid;
+        const uint32_t v = skeys[j];
+        for (uint32_t u = j ? skeys[j - 1] + 1u : 0u; u <= v; ++u) start[u] = j;
+        if (j == n - 1)
+            for (uint32_t u = v + 1u; u <= (uint32_t)kLegacyVoxels; ++u) start[u] = n;
     }
-    return lo;
+    if (n == 0)
+        for (uint32_t u = first; u <= (uint32_t)kLegacyVoxels; u += step) start[u] = 0u;
 }
 
 // Sums each voxel's deposits in photon order and writes both grid layouts;
-// one warp per voxel. The lanes load 32 consecutive deposits at a time
-// (coalesced, the next 32 already in flight) and the warp adds them in
-// order through shuffles: exactly the serial additions, bound by the add
-// chain instead of one thread's load latency.
-__global__ void __launch_bounds__(256) reduce_kernel(const uint32_t *__restrict__ skeys,
-                                                     const float4 *__restrict__ sorted,
-                                                     const uint32_t *total, float *grid3,
-                                                     float4 *grid4) {
-    const int v = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
+// one warp per voxel. The warp loads 128 consecutive deposits at a time
+// (coalesced, the next 128 already in flight) and turns them into three rows
+// in shared memory; lanes 0, 1 and 2 add a component each, four deposits
+// per load: exactly the serial additions, bound by the chain of them in the
+// voxels beside the light. 33 us a frame; broadcasting each deposit through
+// three shuffles took 84 us, and 113 us with each voxel's range searched
+// for instead of read.
+constexpr int kSumWarps = 4;
+constexpr int kSumItems = 128;
+__global__ void __launch_bounds__(kSumWarps * 32) reduce_kernel(const uint32_t *__restrict__ start,
+                                                                const float4 *__restrict__ sorted, float *grid3,
+                                                                float4 *grid4) {
+    __shared__ __align__(16) float row[kSumWarps][3][kSumItems + 4];  // rows a bank apart
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int v = blockIdx.x * kSumWarps + wib;
     if (v >= kLegacyVoxels) return;
-    const uint32_t n = *total;
-    const uint32_t lo = first_at_least(skeys, n, (uint32_t)v);
-    const uint32_t hi = first_at_least(skeys, n, (uint32_t)v + 1u);
-    float ax = 0.0f, ay = 0.0f, az = 0.0f;
+    const uint32_t lo = start[v], hi = start[v + 1];
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 e = lo + lane < hi ? __ldg(&sorted[lo + lane]) : zero;
-    for (uint32_t base = lo; base < hi; base += 32) {
-        const uint32_t nb = base + 32;
-        const float4 next = nb + lane < hi ? __ldg(&sorted[nb + lane]) : zero;
-        const uint32_t cnt = min(32u, hi - base);
-        if (cnt == 32) {
+    float4 e[kSumItems / 32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                ax = ax + __shfl_sync(0xffffffffu, e.x, i);
-                ay = ay + __shfl_sync(0xffffffffu, e.y, i);
-                az = az + __shfl_sync(0xffffffffu, e.z, i);
-            }
-        } else {
-            for (uint32_t i = 0; i < cnt; ++i) {
-                ax = ax + __shfl_sync(0xffffffffu, e.x, i);
-                ay = ay + __shfl_sync(0xffffffffu, e.y, i);
-                az = az + __shfl_sync(0xffffffffu, e.z, i);
+    for (int i = 0; i < kSumItems / 32; ++i) {
+        const uint32_t at = lo + 32u * i + lane;
+        e[i] = at < hi ? __ldg(&sorted[at]) : zero;
+    }
+    float acc = 0.0f;
+    for (uint32_t base = lo; base < hi; base += kSumItems) {
+#pragma unroll
+        for (int i = 0; i < kSumItems / 32; ++i) {
+            row[wib][0][32 * i + lane] = e[i].x;
+            row[wib][1][32 * i + lane] = e[i].y;
+            row[wib][2][32 * i + lane] = e[i].z;
+        }
+#pragma unroll
+        for (int i = 0; i < kSumItems / 32; ++i) {
+            const uint32_t at = base + kSumItems + 32u * i + lane;
+            e[i] = at < hi ? __ldg(&sorted[at]) : zero;
+        }
+        __syncwarp();
+        if (lane < 3) {
+            const float4 *r = reinterpret_cast<const float4 *>(row[wib][lane]);
+            const int cnt = (int)min((uint32_t)kSumItems, hi - base);
+            if (cnt == kSumItems) {
+#pragma unroll
+                for (int i = 0; i < kSumItems / 4; ++i) {
+                    const float4 q = r[i];
+                    acc = ((acc + q.x) + q.y) + q.z;
+                    acc = acc + q.w;
+                }
+            } else {
+                for (int i = 0; i < cnt; ++i) acc = acc + row[wib][lane][i];
             }
         }
-        e = next;
+        __syncwarp();
     }
-    if (lane == 0) {
-        grid3[3 * v + 0] = ax;
-        grid3[3 * v + 1] = ay;
-        grid3[3 * v + 2] = az;
-        grid4[v] = make_float4(ax, ay, az, 0.0f);
-    }
+    if (lane < 3) grid3[3 * v + lane] = acc;
+    const float ay = __shfl_sync(0xffffffffu, acc, 1), az = __shfl_sync(0xffffffffu, acc, 2);
+    if (lane == 0) grid4[v] = make_float4(acc, ay, az, 0.0f);
 }
 
 // init_random_numbers_kernel (:1483-1498): entry i holds draws 3i..3i+2
@@ -539,13 +640,17 @@ __global__ void grid_from_host_kernel(const float *grid3, float4 *grid4) {
 
 // ---- render ----------------------------------------------------------------
 
-// computePixelColor (:926-1017).
+// computePixelColor (:926-1017). The voxels of its up to ten march points and
+// five interpolation corners are found in single precision
+// (legacy_voxel.cuh): a 512 x 512 frame takes 38 us; in double precision,
+// three divisions each, it took 366 us, bound by the double-precision units.
 __device__ v3 shade_pixel(const Scene &sc, const float4 *__restrict__ vol,
                           const float4 *__restrict__ slab, float x, float y, bool interp, bool media) {
     v3 rgb = mk3(0.0f, 0.0f, 0.0f);
     v3 origin = mk3(0.0f, 0.0f, 0.0f);
     Chain c;
-    c.ray = mk3((float)((double)(x / 512.0f) - 0.5), (float)(-((double)(y / 512.0f) - 0.5)), 1.0f);
+    // one rounding, in the difference: the double that held it was exact
+    c.ray = mk3(x / 512.0f - 0.5f, -(y / 512.0f - 0.5f), 1.0f);
     c.h.hit = false;
     c.h.type = 0;
     c.h.idx = 0;
@@ -581,8 +686,7 @@ __global__ void __launch_bounds__(256) render_kernel(Scene sc, const float4 *__r
         rgb_out[3 * index + 1] = c.y;
         rgb_out[3 * index + 2] = c.z;
     }
-    out[index] = make_uchar4(to_u8_sat((double)c.x * 255.0), to_u8_sat((double)c.y * 255.0),
-                             to_u8_sat((double)c.z * 255.0), 0);
+    out[index] = make_uchar4(unit_to_u8(c.x), unit_to_u8(c.y), unit_to_u8(c.z), 0);
 }
 
 Scene make_scene(float anim_time) {
@@ -620,6 +724,7 @@ cudaError_t legacy_alloc(LegacyState &st) {
     PM_ALLOC(st.counts, sizeof(uint32_t) * kLegacyPhotons);
     PM_ALLOC(st.offsets, sizeof(uint32_t) * kLegacyPhotons);
     PM_ALLOC(st.total, sizeof(uint32_t));
+    PM_ALLOC(st.start, sizeof(uint32_t) * (kLegacyVoxels + 1));
     PM_ALLOC(st.keys, sizeof(uint32_t) * kLegacyMaxDeposits);
     PM_ALLOC(st.keys_tmp, sizeof(uint32_t) * kLegacyMaxDeposits);
     PM_ALLOC(st.idx, sizeof(uint32_t) * kLegacyMaxDeposits);
@@ -640,7 +745,7 @@ cudaError_t legacy_alloc(LegacyState &st) {
 void legacy_free(LegacyState &st) {
     cudaFree(st.table); cudaFree(st.grid3); cudaFree(st.grid4); cudaFree(st.counts);
     cudaFree(st.vol_win); cudaFree(st.slab_win);
-    cudaFree(st.offsets); cudaFree(st.total); cudaFree(st.keys); cudaFree(st.keys_tmp);
+    cudaFree(st.offsets); cudaFree(st.total); cudaFree(st.start); cudaFree(st.keys); cudaFree(st.keys_tmp);
     cudaFree(st.idx); cudaFree(st.idx_tmp); cudaFree(st.dep); cudaFree(st.sdep); cudaFree(st.hist);
     st = LegacyState();
 }
@@ -659,20 +764,25 @@ cudaError_t legacy_emit(LegacyState &st, float anim_time, int flags, cudaStream_
     bool media = (flags & kLegacyMedia) != 0;
     uint32_t z0 = mwc_jump_host(kMwcSeedZ, kMwcAz, kMwcMz, st.rng_draws);
     uint32_t w0 = mwc_jump_host(kMwcSeedW, kMwcAw, kMwcMw, st.rng_draws);
-    const int blocks = (kLegacyPhotons + 255) / 256;
-    emit_kernel<<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, st.counts, nullptr, nullptr,
-                                       nullptr, nullptr); note_launch();
+    JumpTable jump;
+    for (int i = 0; i < kJumpBits; ++i) {
+        jump.z[i] = mwc_jump_host(1u, kMwcAz, kMwcMz, 9ull << i);
+        jump.w[i] = mwc_jump_host(1u, kMwcAw, kMwcMw, 9ull << i);
+    }
+    const int blocks = (kLegacyPhotons * kPhotonLanes + 255) / 256;
+    emit_kernel<false><<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, jump, st.counts, nullptr, nullptr,
+                                              nullptr, nullptr); note_launch();
     cudaError_t e = exclusive_scan_u32(st.counts, st.offsets, kLegacyPhotons, st.total, s);
     if (e != cudaSuccess) return e;
-    emit_kernel<<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, st.counts, st.offsets, st.keys,
-                                       st.idx, st.dep); note_launch();
+    emit_kernel<true><<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, jump, st.counts, st.offsets, st.keys,
+                                             st.idx, st.dep); note_launch();
     uint32_t *sk = nullptr, *si = nullptr;
     e = radix_sort_pairs_u32(st.keys, st.idx, st.keys_tmp, st.idx_tmp, st.total, kLegacyMaxDeposits,
                              0, 16, st.hist, s, &sk, &si);
     if (e != cudaSuccess) return e;
-    gather_deposits_kernel<<<512, 256, 0, s>>>(si, st.dep, st.total, st.sdep); note_launch();
-    reduce_kernel<<<(kLegacyVoxels * 32 + 255) / 256, 256, 0, s>>>(sk, st.sdep, st.total, st.grid3,
-                                                                  st.grid4); note_launch();
+    gather_deposits_kernel<<<512, 256, 0, s>>>(sk, si, st.dep, st.total, st.sdep, st.start); note_launch();
+    reduce_kernel<<<(kLegacyVoxels + kSumWarps - 1) / kSumWarps, kSumWarps * 32, 0, s>>>(st.start, st.sdep, st.grid3,
+                                                                                        st.grid4); note_launch();
     if (media) st.rng_draws += 9ull * kLegacyPhotons;
     return cudaGetLastError();
 }

@@ -34,6 +34,7 @@ struct LegacyState {
     uint32_t *counts = nullptr;   // deposits per photon
     uint32_t *offsets = nullptr;  // exclusive scan of counts
     uint32_t *total = nullptr;    // total deposits (device scalar)
+    uint32_t *start = nullptr;    // per voxel: its first sorted deposit (+ the total)
     uint32_t *keys = nullptr, *keys_tmp = nullptr;
     uint32_t *idx = nullptr, *idx_tmp = nullptr;
     float4 *dep = nullptr;        // deposit values in photon order
