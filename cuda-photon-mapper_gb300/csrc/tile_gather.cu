@@ -4,19 +4,16 @@
 // A warp takes 1 to 4 consecutive groups of 32 queries of the (map, Morton
 // code) order. The k-th-neighbour distance d(x) (capped at the gather radius) is
 // 1-Lipschitz in the query position, so exact distances d_j at points x_j
-// bound it everywhere:
-//     max_j (d_j - |x - x_j|)  <=  d(x)  <=  min_j (d_j + |x - x_j|).
-// The warp's first group is bounded by one anchor (an exact list search at
-// one of its queries, done by a separate launch before), every later group
-// by the exact results of the group before it. A group's records are
-// collected once from the kd-tree -- every record within the largest upper
-// bound of the group's bounding box -- into shared memory, and each query
-// selects its k nearest from that set: records closer than its lower bound
-// are in, records beyond its upper bound are out, and only the band between
-// the bounds is ranked (the previous query of the group tightens both
-// bounds the same way).
+// bound it everywhere: d(x) <= min_j (d_j + |x - x_j|). The warp's first group
+// is bounded by one anchor (an exact list search at one of its queries, done
+// by a separate launch before), every later group by the exact results of the
+// group before it. A group's records are found once in the kd-tree -- every
+// record within the largest upper bound of the group's bounding box -- and
+// held in registers, kSlots positions to a lane. A query computes its squared
+// distances to all of them and searches for the threshold that exactly k of
+// them lie at or below (select_k), starting from its predecessor's.
 //
-// A group whose set does not fit in shared memory is processed in segments:
+// A group whose set does not fit the registers is processed in segments:
 // halves, down to single queries, each finished segment tightening the
 // bounds of the queries after it. A single query whose set still does not
 // fit, queries of the other map in a mixed group, and any result that
@@ -24,6 +21,14 @@
 // after the pass. The selected set is exactly the list search's (ties
 // broken by photon index) and the estimate's sum is order-independent
 // (knn_core.cuh), so every value is bit-identical to the list search's.
+//
+// Bound by instruction issue; the selected records' flux comes from L1 and
+// L2. Candidates in registers instead of shared memory make a query's
+// distances and counts straight-line code without loads, need no lists of
+// the certain and the doubtful candidates, and leave most of the L1 to the
+// flux. Estimate pass (GB300; candidates in shared memory, scanned, the band
+// between two bounds ranked, before): preset 2 113.0 -> 76.0 ms, preset 3
+// 45.4 -> 34.5 ms, preset 1 16.9 -> 12.0 ms.
 #include <algorithm>
 
 #include "cache.cuh"
@@ -39,14 +44,12 @@ using namespace wknn;
 
 constexpr int kTileWarps = 4;
 constexpr int kAnchorAt = 15;                // the anchor: query 15 of a warp's chunk
-// Residency before capacity: 7 blocks of 4 warps per SM (the registers capped
-// at 72, a few spilled) with candidate sets of 272 records measured faster
-// than 5 blocks with 400 (more groups halve, but more warps hide the
-// latency of every phase).
-constexpr int kTileBlocks = 7;
-constexpr int kTileCap = 272;                // candidate records per warp (fits 7 blocks' shared memory)
-constexpr int kScanSlots = 2;   // candidates per lane per step of the selection scan
-constexpr int kPickSlots = 1;   // band entries per lane per step of the final selection
+// Blocks of 4 warps per SM (registers capped at 64) and candidates per lane.
+// Presets 2 / 3: 8 blocks and 8 slots 76.0 / 34.5 ms, 7 blocks 79.1 / 35.2,
+// 6 blocks 82.8 / 36.2; 10 slots at 6 blocks 81.3 / 36.7.
+constexpr int kTileBlocks = 8;
+constexpr int kSlots = 8;
+constexpr int kTileCap = 32 * kSlots;        // candidate records per warp
 constexpr float kRel = 2e-4f;                // relative and absolute margins of the distance bounds
 constexpr float kAbs = 1e-6f;
 
@@ -54,17 +57,14 @@ constexpr float kAbs = 1e-6f;
 enum TileStat { kStTiled, kStList, kStShrunk, kStViolations, kStGroups, kStCandidates, kStHalvings, kStCount };
 
 struct TileScratch {
-    float4 cpos[kTileCap];   // candidate positions (+ photon index bits)
-    uint32_t cat[kTileCap];  // their tree positions
+    uint32_t cat[kTileCap];  // tree positions of the candidates
     union {
         uint32_t stack[kStackCap];  // the collection's node stack
-        struct {
-            float bd2[kTileCap];       // band: squared distances
-            uint16_t bslot[kTileCap];  // band: candidate slots
-            uint16_t sel[128];         // the k selected candidates
-            uint64_t win[32];          // ranking window keys
-        } b;
+        uint32_t sel[128];          // tree positions of the k selected candidates
     };
+    float4 qx[32];           // the group's queries: position, upper bound of the k-th distance
+    float4 qd[32];           // weight direction, query index bits
+    float4 known[32];        // exact distances that bound the group: point, distance
     unsigned long long st[kStCount];  // counters, lane 0
 };
 
@@ -124,16 +124,6 @@ struct Query {
     uint32_t out;  // query index (destination)
 };
 
-__device__ __forceinline__ Query shfl_query(const Query &q, int j) {
-    Query r;
-    r.x = mk3(__shfl_sync(kFull, q.x.x, j), __shfl_sync(kFull, q.x.y, j), __shfl_sync(kFull, q.x.z, j));
-    r.dirv = mk3(__shfl_sync(kFull, q.dirv.x, j), __shfl_sync(kFull, q.dirv.y, j),
-                 __shfl_sync(kFull, q.dirv.z, j));
-    r.map = __shfl_sync(kFull, q.map, j);
-    r.out = __shfl_sync(kFull, q.out, j);
-    return r;
-}
-
 // One query of the list: position, the weight direction and its map.
 __device__ __forceinline__ Query load_query(const PScene &Sc, const float4 *qa, const float4 *qd,
                                             uint32_t i) {
@@ -148,15 +138,23 @@ __device__ __forceinline__ Query load_query(const PScene &Sc, const float4 *qa, 
     return q;
 }
 
+// Minimum and maximum of a float over the warp (NaN only when all are).
 __device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(kFull, v, o));
-    return v;
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 __device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
-    return v;
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+// The hardware's approximate square root, for distances that only bound or
+// steer (the bounds' margins are far above its error).
+__device__ __forceinline__ float approx_sqrt(float v) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 __device__ __forceinline__ float gap(float lo, float hi, float v) {
@@ -186,22 +184,23 @@ __device__ __forceinline__ void write_estimate(float4 *out, uint32_t i, v3 e, in
     if ((threadIdx.x & 31) == 0) out[i] = make_float4(e.x, e.y, e.z, raw ? r2out : 0.0f);
 }
 
-// Queues the lanes of `mask` for the list-search launch.
-__device__ __forceinline__ void defer(const Query &q, unsigned mask) {
+// Queues the queries (their indices on the lanes) of `mask` for the
+// list-search launch.
+__device__ __forceinline__ void defer(uint32_t out, unsigned mask) {
     const int lane = threadIdx.x & 31;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(targs().defer_n, (uint32_t)__popc(mask));
     base = __shfl_sync(kFull, base, 0);
     if ((mask >> lane) & 1u) {
         const uint32_t at = base + __popc(mask & ((1u << lane) - 1u));
-        targs().defer[at] = q.out;
+        targs().defer[at] = out;
         if (targs().defer_sc) targs().defer_sc[at] = targs().scene;
     }
     count(kStList, (unsigned long long)__popc(mask));
 }
 
-// Every record of map `mid` within sqrt(rho2) of the box [lo, hi] into
-// cpos/cat. Returns the count, or -1 when more than kTileCap qualify.
+// The tree positions of every record of map `mid` within sqrt(rho2) of the
+// box [lo, hi] into cat. Returns the count, or -1 when more than kTileCap qualify.
 __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
     TileScratch &ts = scratch();
     const MapView &m = targs().map[mid];
@@ -222,20 +221,15 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
             for (int c = 0; c < chunks; ++c) {
                 const uint32_t r = ((node - first_leaf) << (5 + m.leaf_shift)) + ((uint32_t)c << 5) + lane;
                 bool in = false;
-                float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (r < m.n) {
-                    p = __ldg(&m.pos[r]);
+                    const float4 p = __ldg(&m.pos[r]);
                     const float gx = gap(lo.x, hi.x, p.x), gy = gap(lo.y, hi.y, p.y),
                                 gz = gap(lo.z, hi.z, p.z);
                     in = gx * gx + gy * gy + gz * gz <= rho2;
                 }
                 const unsigned mk = __ballot_sync(kFull, in);
                 if (n + __popc(mk) > kTileCap) return -1;
-                if (in) {
-                    const int at = n + __popc(mk & lt);
-                    ts.cpos[at] = p;
-                    ts.cat[at] = r;
-                }
+                if (in) ts.cat[n + __popc(mk & lt)] = r;
                 n += __popc(mk);
             }
         } else {
@@ -262,268 +256,195 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
     return n;
 }
 
-// The need-th smallest key (1-based) among the band entries bd2/bslot[0..B),
-// all with lo2 <= d2 <= hi2. The window of squared distances holding it is
-// narrowed (interpolating in r^3, else halving the float bit range) until at
-// most 32 entries remain, which are ranked by full key.
-__device__ __noinline__ uint64_t band_select(int B, int need, float lo2, float hi2) {
-    TileScratch &ts = scratch();
-    const int lane = threadIdx.x & 31;
-    uint32_t blo = __float_as_uint(lo2), bhi = __float_as_uint(hi2) + 1u;  // [blo, bhi)
-    int below = 0, inwin = B;
-    bool interp = true;
-    while (inwin > 32 && bhi - blo > 1u) {
-        uint32_t t;
-        if (interp) {
-            const float rl = sqrtf(__uint_as_float(blo)), rh = sqrtf(__uint_as_float(bhi - 1u));
-            const float f = ((float)(need - below) - 0.5f) / (float)inwin;
-            const float vl = rl * rl * rl, vh = rh * rh * rh;
-            const float rt = cbrtf(vl + f * (vh - vl));
-            t = __float_as_uint(rt * rt);
-        } else {
-            t = blo + ((bhi - blo) >> 1);
-        }
-        t = min(max(t, blo + 1u), bhi - 1u);
-        int c = 0;
-        for (int e = lane; e < B; e += 32) {
-            const uint32_t b = __float_as_uint(ts.b.bd2[e]);
-            c += (b >= blo && b < t) ? 1 : 0;
-        }
+// The k nearest of the warp's candidates, d2[s] their squared distances (bits;
+// slots without a candidate above every other). A threshold with exactly k
+// candidates at or below it is searched for: a count costs a compare and an
+// addition per slot and one warp sum, the next threshold scales the last by
+// the density it found (r^3 in the medium, r^2 on surfaces), and the last one
+// or two candidates are stepped over one by one. Where the k-th distance
+// occurs more than once the photon index decides. `t`: the first guess, at
+// most capb (the squared gather radius), the search's upper end. Returns the
+// mask of this lane's selected slots; *found: how many (k, or all within the
+// cap when fewer).
+__device__ __forceinline__ uint32_t select_k(const uint32_t (&d2)[kSlots], int n, uint32_t t, uint32_t capb, int k,
+                                             float expo, const MapView &m, int *found) {
+    int lo = -1, hi = (int)capb + 1;  // at or below lo: fewer than k; hi: more than k, or past the cap
+    uint32_t mask;
+    int c;
+    for (int it = 0;; ++it) {
+        c = 0;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) c += d2[s] <= t ? 1 : 0;
         c = (int)__reduce_add_sync(kFull, (uint32_t)c);
-        const int before = inwin;
-        if (below + c >= need) {
-            bhi = t;
-            inwin = c;
-        } else {
-            below += c;
-            blo = t;
-            inwin -= c;
-        }
-        interp = 4 * inwin <= 3 * before;  // interpolation pays while it cuts a quarter
-    }
-    const int want = need - below;  // 1-based rank inside the window
-    const unsigned lt = (1u << lane) - 1u;
-    if (inwin <= 32) {
-        int n = 0;
-        for (int base = 0; base < B; base += 32) {
-            const int e = base + lane;
-            bool in = false;
-            uint64_t key = 0;
-            if (e < B) {
-                const uint32_t b = __float_as_uint(ts.b.bd2[e]);
-                in = b >= blo && b < bhi;
-                if (in) key = make_key(ts.b.bd2[e], __float_as_uint(ts.cpos[ts.b.bslot[e]].w));
+        if (c == k || (c < k && t == capb)) break;
+        if (c < k) lo = (int)t; else hi = (int)t;
+        if (hi - lo == 1) break;  // hi's distance occurs several times
+        uint32_t nt = t;
+        if (c < k && k - c <= 2) {
+            for (int i = c; i < k; ++i) {
+                uint32_t v = 0x7f800000u;
+#pragma unroll
+                for (int s = 0; s < kSlots; ++s) v = min(v, d2[s] > nt ? d2[s] : 0x7f800000u);
+                nt = __reduce_min_sync(kFull, v);
             }
-            const unsigned mk = __ballot_sync(kFull, in);
-            if (in) ts.b.win[n + __popc(mk & lt)] = key;
-            n += __popc(mk);
+            nt = min(nt, capb);
+        } else if (c > k && c - k <= 2) {
+            for (int i = k; i < c; ++i) {
+                uint32_t v = 0u;
+#pragma unroll
+                for (int s = 0; s < kSlots; ++s) v = max(v, d2[s] <= nt ? d2[s] : 0u);
+                nt = __reduce_max_sync(kFull, v) - 1u;
+            }
+        } else if (it < 6) {
+            nt = min(__float_as_uint(__uint_as_float(t) * __powf(__fdividef((float)k, (float)max(c, 1)), expo)), capb);
+        } else {
+            nt = 0u;  // halve
         }
-        __syncwarp();
-        const uint64_t mine = lane < n ? ts.b.win[lane] : ~0ull;
-        int rank = 0;
-        for (int f = 0; f < n; ++f) rank += ts.b.win[f] < mine ? 1 : 0;
-        const unsigned hit = __ballot_sync(kFull, lane < n && rank == want - 1);
-        const uint64_t kth = __shfl_sync(kFull, mine, __ffs(hit) - 1);
-        __syncwarp();
-        return kth;
+        if ((int)nt <= lo || (int)nt >= hi) nt = (uint32_t)(lo + ((hi - lo) >> 1));
+        t = nt;
     }
-    // more than 32 entries at one squared distance: rank by photon index
-    const float v = __uint_as_float(blo);
-    uint64_t lo_i = 0, hi_i = 0xffffffffull;  // the index is in [lo_i, hi_i]
-    while (lo_i < hi_i) {
-        const uint64_t mid = (lo_i + hi_i) >> 1;
-        int c = 0;
-        for (int e = lane; e < B; e += 32)
-            if (ts.b.bd2[e] == v && __float_as_uint(ts.cpos[ts.b.bslot[e]].w) <= (uint32_t)mid) ++c;
-        c = (int)__reduce_add_sync(kFull, (uint32_t)c);
-        if (c >= want) hi_i = mid; else lo_i = mid + 1;
+    *found = min(c, k);
+    mask = 0u;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) mask |= d2[s] <= t ? 1u << s : 0u;
+    if (hi - lo == 1 && c != k && !(c < k && t == capb)) {
+        // those nearer than hi, then those at hi by photon index
+        const uint32_t v = (uint32_t)hi;
+        const int lane = threadIdx.x & 31;
+        uint32_t id[kSlots];
+        int less = 0;
+        mask = 0u;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            id[s] = 0xffffffffu;
+            if (d2[s] == v) id[s] = __float_as_uint(__ldg(&m.pos[scratch().cat[32 * s + lane]]).w);
+            less += d2[s] < v ? 1 : 0;
+            mask |= d2[s] < v ? 1u << s : 0u;
+        }
+        less = (int)__reduce_add_sync(kFull, (uint32_t)less);
+        for (int i = less; i < k; ++i) {
+            uint32_t w = 0xffffffffu;
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s) w = min(w, id[s]);
+            w = __reduce_min_sync(kFull, w);
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s)
+                if (id[s] == w) {
+                    mask |= 1u << s;
+                    id[s] = 0xffffffffu;
+                }
+        }
+        *found = k;
     }
-    return make_key(v, (uint32_t)lo_i);
+    return mask;
 }
 
-struct Pick {
-    int found;     // records selected (k, or all within the cap when fewer)
-    bool ok;       // false: the bounds contradicted the candidates
-    uint64_t kth;  // the k-th key when found == k
-};
-
-// Selects the k nearest candidates of q into sel[0..found) given bounds
-// lo2 <= (k-th squared distance) <= hi2 (hi2 <= r2cap).
-__device__ __forceinline__ Pick pick_k(int n, v3 q, float lo2, float hi2) {
-    TileScratch &ts = scratch();
-    const int lane = threadIdx.x & 31;
-    const int k = targs().k;
-    const uint64_t cap = targs().cap;
-    const unsigned lt = (1u << lane) - 1u;
-    int n_in = 0, B = 0;
-    // kScanSlots slots per lane and step: their loads and distances are
-    // independent; the ballots and stores keep slot order
-    for (int base = 0; base < n; base += 32 * kScanSlots) {
-        bool in[kScanSlots], band[kScanSlots];
-        float d2[kScanSlots];
-        unsigned mi[kScanSlots], mb[kScanSlots];
-#pragma unroll
-        for (int u = 0; u < kScanSlots; ++u) {
-            const int c = base + 32 * u + lane;
-            in[u] = band[u] = false;
-            d2[u] = 0.0f;
-            if (c < n) {
-                const float4 p = ts.cpos[c];
-                const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-                d2[u] = dx * dx + dy * dy + dz * dz;
-                in[u] = d2[u] < lo2;
-                band[u] = !in[u] && d2[u] <= hi2 && make_key(d2[u], __float_as_uint(p.w)) < cap;
-            }
-        }
-        int tin = 0;
-#pragma unroll
-        for (int u = 0; u < kScanSlots; ++u) {
-            mi[u] = __ballot_sync(kFull, in[u]);
-            mb[u] = __ballot_sync(kFull, band[u]);
-            tin += __popc(mi[u]);
-        }
-        if (n_in + tin >= k) {  // the lower bound was too high
-            __syncwarp();
-            return Pick{0, false, 0};
-        }
-#pragma unroll
-        for (int u = 0; u < kScanSlots; ++u) {
-            const int c = base + 32 * u + lane;
-            if (in[u]) ts.b.sel[n_in + __popc(mi[u] & lt)] = (uint16_t)c;
-            if (band[u]) {
-                const int at = B + __popc(mb[u] & lt);
-                ts.b.bd2[at] = d2[u];
-                ts.b.bslot[at] = (uint16_t)c;
-            }
-            n_in += __popc(mi[u]);
-            B += __popc(mb[u]);
-        }
-    }
-    __syncwarp();
-    const int need = k - n_in;
-    if (B < need) {
-        if (hi2 < targs().r2cap) return Pick{0, false, 0};  // the upper bound was too low
-        for (int e = lane; e < B; e += 32) ts.b.sel[n_in + e] = ts.b.bslot[e];
-        __syncwarp();
-        return Pick{n_in + B, true, cap};
-    }
-    const uint64_t kth = band_select(B, need, lo2, hi2);
-    int sel = n_in;
-    for (int base = 0; base < B; base += 32 * kPickSlots) {
-        bool sl[kPickSlots];
-        uint16_t slot[kPickSlots];
-#pragma unroll
-        for (int u = 0; u < kPickSlots; ++u) {
-            const int e = base + 32 * u + lane;
-            sl[u] = false;
-            slot[u] = 0;
-            if (e < B) {
-                slot[u] = ts.b.bslot[e];
-                sl[u] = make_key(ts.b.bd2[e], __float_as_uint(ts.cpos[slot[u]].w)) <= kth;
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kPickSlots; ++u) {
-            const unsigned ms = __ballot_sync(kFull, sl[u]);
-            if (sl[u]) ts.b.sel[sel + __popc(ms & lt)] = slot[u];
-            sel += __popc(ms);
-        }
-    }
-    __syncwarp();
-    return Pick{sel, true, kth};
-}
-
-// The lanes of `mask` (queries of one map, lane order = spatial order) from
-// one shared candidate set; lb / ub: each lane's bounds on its capped k-th
-// distance. Returns false when the set does not fit; otherwise sets d_lane
-// to the capped k-th distance of the lane's query (-1 if it was deferred).
+// The queries of `mask` (one map, lane order = spatial order; this lane's at
+// x, bounded by ub) from one shared candidate set. Returns false when the
+// set does not fit; otherwise sets d_lane to the capped k-th distance of the
+// lane's query (-1 if it was deferred).
 template <int S>
-__device__ __noinline__ bool tile_queries(Query q, unsigned mask, float lb, float ub, float *d_lane) {
+__device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask, float *d_lane) {
     TileScratch &ts = scratch();
     const int lane = threadIdx.x & 31;
     const int k = targs().k;
-    const int mid = __shfl_sync(kFull, q.map, __ffs(mask) - 1);
     const MapView &m = targs().map[mid];
     const bool member = (mask >> lane) & 1u;
     const float inf = __int_as_float(0x7f800000);
-    const v3 lo = mk3(warp_min(member ? q.x.x : inf), warp_min(member ? q.x.y : inf),
-                      warp_min(member ? q.x.z : inf));
-    const v3 hi = mk3(warp_max(member ? q.x.x : -inf), warp_max(member ? q.x.y : -inf),
-                      warp_max(member ? q.x.z : -inf));
+    const v3 lo = mk3(warp_min(member ? x.x : inf), warp_min(member ? x.y : inf), warp_min(member ? x.z : inf));
+    const v3 hi = mk3(warp_max(member ? x.x : -inf), warp_max(member ? x.y : -inf), warp_max(member ? x.z : -inf));
     const float rho = warp_max(member ? ub : 0.0f);
     const int n = collect(mid, lo, hi, rho * rho);
     if (n < 0) return false;
     count(kStGroups);
     count(kStCandidates, (unsigned long long)n);
+    // the candidates, kSlots to a lane
+    float px[kSlots], py[kSlots], pz[kSlots];
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) {
+        px[s] = py[s] = pz[s] = inf;
+        if (32 * s + lane < n) {
+            const float4 p = __ldg(&m.pos[ts.cat[32 * s + lane]]);
+            px[s] = p.x;
+            py[s] = p.y;
+            pz[s] = p.z;
+        }
+    }
     const float r2cap = targs().r2cap, rcap = targs().rcap;
-    float prev_r = -1.0f;
-    v3 xp = mk3(0.f, 0.f, 0.f);
+    const uint32_t capb = __float_as_uint(r2cap);
+    const float expo = mid == 0 ? 1.0f : 0.6666667f;
+    const unsigned lt = (1u << lane) - 1u;
+    uint32_t guess = 0u;
     for (unsigned mm = mask; mm; mm &= mm - 1) {
         const int j = __ffs(mm) - 1;
-        const Query qj = shfl_query(q, j);
-        float lo_r = __shfl_sync(kFull, lb, j), hi_r = __shfl_sync(kFull, ub, j);
-        const float ubj = hi_r;
-        if (prev_r >= 0.0f) {
-            const v3 dv = qj.x - xp;
-            const float dl = sqrtf(dot(dv, dv));
-            lo_r = fmaxf(lo_r, (prev_r - dl) * (1.0f - kRel) - kAbs);
-            hi_r = fminf(hi_r, (prev_r + dl) * (1.0f + kRel) + kAbs);
+        const float4 q = ts.qx[j];
+        uint32_t d2[kSlots];
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            const float dx = px[s] - q.x, dy = py[s] - q.y, dz = pz[s] - q.z;
+            d2[s] = __float_as_uint(dx * dx + dy * dy + dz * dz);
         }
-        float lo2 = fmaxf(lo_r, 0.0f) * fmaxf(lo_r, 0.0f);
-        float hi2 = fminf(hi_r * hi_r, r2cap);
-        Pick pk;
-        for (;;) {
-            pk = pick_k(n, qj.x, lo2, hi2);
-            if (pk.ok) break;
-            lo2 = 0.0f;  // inconsistent bounds: select over the whole set
-            hi2 = r2cap;
-        }
+        if (guess == 0u) guess = __float_as_uint(q.w * q.w);
+        int found;
+        const uint32_t sm = select_k(d2, n, min(guess, capb), capb, k, expo, m, &found);
+        uint32_t far = 0u;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) far = max(far, (sm >> s) & 1u ? d2[s] : 0u);
+        far = __reduce_max_sync(kFull, far);
         // the set holds every record within the upper bound; a result
         // beyond it would mean the bound failed: defer to the list search
-        const float kd2 = pk.found == k ? key_d2(pk.kth) : r2cap;
-        if ((pk.found == k && kd2 > ubj * ubj) || (pk.found < k && ubj < rcap)) {
+        const float kd2 = found == k ? __uint_as_float(far) : r2cap;
+        if ((found == k && kd2 > q.w * q.w) || (found < k && q.w < rcap)) {
             count(kStViolations);
-            defer(q, 1u << j);
+            defer(__float_as_uint(ts.qd[j].w), 1u);
             if (lane == j) *d_lane = -1.0f;
-            prev_r = -1.0f;
+            guess = 0u;
             continue;
         }
+        guess = __float_as_uint(kd2);
+        int at = 0;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            const bool in = (sm >> s) & 1u;
+            const unsigned b = __ballot_sync(kFull, in);
+            if (in) ts.sel[at + __popc(b & lt)] = ts.cat[32 * s + lane];
+            at += __popc(b);
+        }
+        __syncwarp();
+        const float4 qd = ts.qd[j];
+        const v3 dirv = mk3(qd.x, qd.y, qd.z);
         float tx[S], ty[S], tz[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             tx[s] = ty[s] = tz[s] = 0.0f;
             const int e = lane + 32 * s;
-            if (e < pk.found) {
-                const v3 t = flux_term(m, ts.cat[ts.b.sel[e]], mid, qj.dirv, targs().g);
+            if (e < found) {
+                const v3 t = flux_term(m, ts.sel[e], mid, dirv, targs().g);
                 tx[s] = t.x;
                 ty[s] = t.y;
                 tz[s] = t.z;
             }
         }
         const v3 e = mk3(warp_fixed_sum<S>(tx), warp_fixed_sum<S>(ty), warp_fixed_sum<S>(tz));
-        write_estimate(targs().out, qj.out, e, pk.found, kd2, mid == 0, targs().raw);
+        write_estimate(targs().out, __float_as_uint(qd.w), e, found, kd2, mid == 0, targs().raw);
         __syncwarp();
-        const float dj = pk.found == k ? sqrtf(kd2) : rcap;
-        if (lane == j) *d_lane = dj;
-        prev_r = dj;
-        xp = qj.x;
+        if (lane == j) *d_lane = found == k ? sqrtf(kd2) : rcap;
         count(kStTiled);
     }
     return true;
 }
 
-// Bounds for the single query of lane j whose set within its upper bound
-// does not fit: the radius is bisected (in r^3) between the bounds. A
+// The upper bound for the single query of lane j (at x) whose set within its
+// bound *ub does not fit: the radius is bisected (in r^3) below the bound. A
 // collection that overflows holds more than kTileCap >= k records, so its
-// radius is an upper bound; one with fewer than k records (and below the
-// cap) is a lower bound; one in between holds the k nearest. Returns
-// false when no such radius turns up.
-__device__ __noinline__ bool shrink_single(Query q, int j, float *lb, float *ub) {
+// radius is an upper bound; one with fewer than k (and below the cap) is a
+// lower bound; one in between holds the k nearest. Returns false when no
+// such radius turns up.
+__device__ __noinline__ bool shrink_single(int mid, int j, float *ub) {
     const int k = targs().k;
-    const int mid = __shfl_sync(kFull, q.map, j);
-    const v3 x = mk3(__shfl_sync(kFull, q.x.x, j), __shfl_sync(kFull, q.x.y, j),
-                     __shfl_sync(kFull, q.x.z, j));
-    float lo = __shfl_sync(kFull, *lb, j), hi = fminf(__shfl_sync(kFull, *ub, j), targs().rcap);
+    const float4 q = scratch().qx[j];
+    const v3 x = mk3(q.x, q.y, q.z);
+    float lo = 0.0f, hi = fminf(q.w, targs().rcap);
     for (int it = 0; it < 24; ++it) {
         const float r = cbrtf(0.5f * (lo * lo * lo + hi * hi * hi));
         const int n = collect(mid, x, x, r * r);
@@ -532,31 +453,25 @@ __device__ __noinline__ bool shrink_single(Query q, int j, float *lb, float *ub)
         } else if (n < k && r < targs().rcap) {
             lo = r;
         } else {
-            if ((threadIdx.x & 31) == j) {
-                *ub = r * (1.0f + kRel) + kAbs;
-                *lb = fmaxf(*lb, lo * (1.0f - kRel) - kAbs);
-            }
+            *ub = r * (1.0f + kRel) + kAbs;
             return true;
         }
     }
     return false;
 }
 
-// Tightens each lane's bounds with the exact distances of the lanes in
-// `mask` (d_lane >= 0).
-__device__ __forceinline__ void tighten(const Query &q, unsigned mask, float d_lane, float *lb, float *ub) {
-    for (unsigned mm = mask; mm; mm &= mm - 1) {
-        const int j = __ffs(mm) - 1;
-        const float dj = __shfl_sync(kFull, d_lane, j);
-        const float jx = __shfl_sync(kFull, q.x.x, j), jy = __shfl_sync(kFull, q.x.y, j),
-                    jz = __shfl_sync(kFull, q.x.z, j);
-        if (dj >= 0.0f) {
-            const float dx = q.x.x - jx, dy = q.x.y - jy, dz = q.x.z - jz;
-            const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
-            *ub = fminf(*ub, (dj + dist) * (1.0f + kRel) + kAbs);
-            *lb = fmaxf(*lb, (dj - dist) * (1.0f - kRel) - kAbs);
-        }
+// The least of ub and what the exact distances of known[0..n) allow at x
+// (entries with a negative distance say nothing).
+__device__ __forceinline__ float bound_by(const float4 *known, int n, v3 x, float ub) {
+    float u = 3.0e38f;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+        const float4 o = known[j];
+        const float dx = x.x - o.x, dy = x.y - o.y, dz = x.z - o.z;
+        const float v = o.w + approx_sqrt(dx * dx + dy * dy + dz * dz);
+        u = fminf(u, o.w >= 0.0f ? v : u);
     }
+    return fminf(ub, u * (1.0f + kRel) + kAbs);
 }
 
 // One chunk (groups of 32 consecutive queries of the sorted order, from
@@ -566,23 +481,17 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
                                            const float4 *qa, const float4 *qd, const uint32_t *order,
                                            uint32_t n, uint32_t chunk, float anchor, int groups,
                                            float r2cap, bool raw, float4 *out) {
+    TileScratch &ts = scratch();
     const int lane = threadIdx.x & 31;
     const float rcap = sqrtf(r2cap);
     const uint32_t wfirst = chunk * (uint32_t)(32 * groups);
-    // exact distances known so far (lane j: one point; kd < 0: none): the
-    // anchor, later the previous group
-    float kx = 0.f, ky = 0.f, kz = 0.f, kd = -1.0f;
-    int wkind;
+    // exact distances known so far: the anchor, later the previous group
+    int nknown = 1, wkind;
     {
         const uint32_t ai = order[wfirst + min((uint32_t)kAnchorAt, n - 1 - wfirst)];
         const float4 a = qa[ai];
         wkind = __float_as_int(a.w) != kNone ? 0 : 1;
-        if (lane == 0) {
-            kx = a.x;
-            ky = a.y;
-            kz = a.z;
-            kd = anchor;
-        }
+        if (lane == 0) ts.known[0] = make_float4(a.x, a.y, a.z, anchor);
     }
     for (int g = 0; g < groups; ++g) {
         const uint32_t first = wfirst + (uint32_t)(32 * g);
@@ -599,24 +508,18 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
         const uint32_t mn = gkind == 0 ? surf.n : vol.n;
         float dnew = -1.0f;
         if (gkind != wkind) {
-            kd = -1.0f;
+            nknown = 0;
             wkind = gkind;
         }
+        __syncwarp();
         if (mn == 0) {
             // an empty map: nothing found
             if ((members >> lane) & 1u) out[q.out] = make_float4(0.f, 0.f, 0.f, raw ? -1.0f : 0.0f);
         } else {
-            float ub = rcap, lb = 0.0f;
-            for (int j = 0; j < 32; ++j) {
-                const float jx = __shfl_sync(kFull, kx, j), jy = __shfl_sync(kFull, ky, j);
-                const float jz = __shfl_sync(kFull, kz, j), jd = __shfl_sync(kFull, kd, j);
-                if (jd >= 0.0f) {
-                    const float dx = q.x.x - jx, dy = q.x.y - jy, dz = q.x.z - jz;
-                    const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
-                    ub = fminf(ub, (jd + dist) * (1.0f + kRel) + kAbs);
-                    lb = fmaxf(lb, (jd - dist) * (1.0f - kRel) - kAbs);
-                }
-            }
+            float ub = bound_by(ts.known, nknown, q.x, rcap);
+            ts.qx[lane] = make_float4(q.x.x, q.x.y, q.x.z, ub);
+            ts.qd[lane] = make_float4(q.dirv.x, q.dirv.y, q.dirv.z, __uint_as_float(q.out));
+            __syncwarp();
             // segments of the members in spatial order: the whole group,
             // then halves of a segment whose set does not fit, down to
             // single queries (growing again after a fit); each finished
@@ -625,31 +528,47 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
             int sz = 32;
             while (rem) {
                 const unsigned seg = __popc(rem) <= sz ? rem : rem & ((1u << __fns(rem, 0, sz + 1)) - 1u);
-                if (tile_queries<S>(q, seg, lb, ub, &dnew)) {
-                    rem &= ~seg;
-                    if (rem) tighten(q, seg, dnew, &lb, &ub);
-                    sz = min(2 * sz, 32);
-                } else if (__popc(seg) > 1) {
+                const int j = __ffs(seg) - 1;
+                bool done = tile_queries<S>(q.x, ub, gkind, seg, &dnew);
+                if (!done && __popc(seg) > 1) {
                     count(kStHalvings);
                     sz = __popc(seg) >> 1;
-                } else if (shrink_single(q, __ffs(seg) - 1, &lb, &ub) &&
-                           tile_queries<S>(q, seg, lb, ub, &dnew)) {
-                    count(kStShrunk);
-                    rem &= ~seg;
-                    if (rem) tighten(q, seg, dnew, &lb, &ub);
+                    continue;
+                }
+                if (done) {
+                    sz = min(2 * sz, 32);
                 } else {
-                    defer(q, seg);
-                    rem &= ~seg;
+                    float u = 0.0f;
+                    if (shrink_single(gkind, j, &u)) {
+                        __syncwarp();
+                        if (lane == j) {
+                            ub = u;
+                            ts.qx[j].w = u;
+                        }
+                        __syncwarp();
+                        done = tile_queries<S>(q.x, ub, gkind, seg, &dnew);
+                    }
+                    if (done) count(kStShrunk);
+                    else defer(q.out, seg);
+                }
+                rem &= ~seg;
+                if (rem && done) {
+                    // the segment's exact distances, through the known list
+                    const unsigned in = (seg >> lane) & 1u;
+                    if (in) ts.known[__popc(seg & ((1u << lane) - 1u))] = make_float4(q.x.x, q.x.y, q.x.z, dnew);
+                    __syncwarp();
+                    ub = bound_by(ts.known, __popc(seg), q.x, ub);
+                    ts.qx[lane].w = ub;
+                    __syncwarp();
                 }
             }
         }
         const unsigned odd = valid & ~members;
-        if (odd) defer(q, odd);
+        if (odd) defer(q.out, odd);
         // this group's exact distances bound the next group
-        kx = q.x.x;
-        ky = q.x.y;
-        kz = q.x.z;
-        kd = ((members >> lane) & 1u) ? dnew : -1.0f;
+        ts.known[lane] = make_float4(q.x.x, q.x.y, q.x.z, ((members >> lane) & 1u) ? dnew : -1.0f);
+        nknown = 32;
+        __syncwarp();
     }
 }
 
