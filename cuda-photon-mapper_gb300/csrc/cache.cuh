@@ -106,7 +106,7 @@ cudaError_t render_composite(const PScene &S, const uint32_t *off, const float4 
                              const float4 *qd, const float4 *raw, uint32_t npix, float exposure,
                              float4 *rad, uchar4 *rgba, cudaStream_t s);
 // keys[i] = (1 for a volume query, 0 for a diffuse one) << 30 | the 30-bit
-// Morton code of query sel[i]'s (or query i's, sel null) position in the
+// (map, Morton code) of query sel[i] -- or (map, Hilbert code) of query i, sel null -- in the
 // grid box; vals[i] = i.
 cudaError_t cache_sample_keys(const CacheGrid &g, const float4 *qa, const uint32_t *sel, uint32_t n,
                               uint32_t *keys, uint32_t *vals, cudaStream_t s);
