@@ -20,7 +20,7 @@
 //      arena sized at creation (a scene's query count depends only on its
 //      geometry and camera; each scene's pixel words and query slots are
 //      tile-aligned segments of two pools): one count launch, segmented
-//      scans, one write launch, one segmented (map, Morton) sort; then one
+//      scans, one write launch, one segmented (map, Hilbert) sort; then one
 //      persistent shared-candidate estimate pass over all of them per
 //      k-list width and one exact composite launch, every count the
 //      launches need kept on the device. The frame's launch count does not
@@ -229,7 +229,6 @@ struct pm_batch {
         uint32_t *scan_tmp = nullptr;
         float4 *qa = nullptr, *qd = nullptr, *val = nullptr;
         uint32_t *key = nullptr, *ord = nullptr, *key_tmp = nullptr, *ord_tmp = nullptr, *hist = nullptr;
-        float *anchor_d = nullptr;
         uint32_t *defer_n = nullptr;
         size_t pix_cap = 0, q_cap = 0;
     } q;
@@ -246,7 +245,6 @@ struct pm_batch {
         uint32_t *ord = nullptr, *off = nullptr;
         uint32_t *cnt = nullptr, *scnt = nullptr, *soff = nullptr, *slist = nullptr;  // pixel pool
         uint32_t *defer = nullptr, *defer_sc = nullptr, *defer_n = nullptr;
-        float *anchor_d = nullptr;
         TileScene *desc = nullptr;
         std::vector<size_t> q_off, p_off;  // per scene: first query slot, first pixel word
         size_t q_total = 0, p_total = 0;
@@ -263,6 +261,7 @@ struct pm_batch {
         uint32_t list_blocks = 0;
         int class_first[5] = {}, class_n[5] = {};
         uint32_t class_chunks[5] = {};
+        int class_groups[5] = {};
         bool on = false;
     } ar;
     std::vector<uint32_t> nsurf;  // diffuse queries per scene
@@ -322,11 +321,11 @@ void free_batch(pm_batch *b) {
     auto &q = b->q;
     cudaFree(q.cnt); cudaFree(q.off); cudaFree(q.scnt); cudaFree(q.soff); cudaFree(q.slist);
     cudaFree(q.scan_tmp); cudaFree(q.qa); cudaFree(q.qd); cudaFree(q.val); cudaFree(q.key);
-    cudaFree(q.ord); cudaFree(q.key_tmp); cudaFree(q.ord_tmp); cudaFree(q.hist); cudaFree(q.anchor_d);
+    cudaFree(q.ord); cudaFree(q.key_tmp); cudaFree(q.ord_tmp); cudaFree(q.hist);
     cudaFree(q.defer_n);
     auto &ar = b->ar;
     cudaFree(ar.qa); cudaFree(ar.qd); cudaFree(ar.val); cudaFree(ar.ord); cudaFree(ar.off);
-    cudaFree(ar.defer); cudaFree(ar.defer_sc); cudaFree(ar.defer_n); cudaFree(ar.anchor_d);
+    cudaFree(ar.defer); cudaFree(ar.defer_sc); cudaFree(ar.defer_n);
     cudaFree(ar.desc);
     cudaFree(ar.cnt); cudaFree(ar.scnt); cudaFree(ar.soff); cudaFree(ar.slist);
     seg_runs_free(ar.q_runs);
@@ -466,8 +465,8 @@ cudaError_t enqueue_query_scene(pm_batch *b, int s, cudaStream_t st) {
         uint32_t *ok_keys = nullptr, *ok_vals = nullptr;
         Q_TRY(radix_sort_pairs_u32(q.key, q.ord, q.key_tmp, q.ord_tmp, q.off + npix, nq, 0, 31, q.hist, st,
                                    &ok_keys, &ok_vals));
-        const TileBuffers buf{q.anchor_d, ok_vals == q.ord ? q.ord_tmp : q.ord, q.defer_n, nullptr};
-        Q_TRY(knn_values_tiles(d.sc, d.surf, d.vol, q.qa, q.qd, ok_vals, nq, q.off + npix, 4, c.k, c.radius,
+        const TileBuffers buf{ok_vals == q.ord ? q.ord_tmp : q.ord, q.defer_n, nullptr};
+        Q_TRY(knn_values_tiles(d.sc, d.surf, d.vol, q.qa, q.qd, ok_vals, nq, q.off + npix, c.k, c.radius,
                                true, q.val, buf, b->sm_count, st));
     }
     Q_TRY(render_composite(d.sc, q.off, q.qa, q.qd, q.val, npix, c.exposure, d.rad, d.rgba, st));
@@ -475,7 +474,6 @@ cudaError_t enqueue_query_scene(pm_batch *b, int s, cudaStream_t st) {
     return cudaSuccess;
 }
 
-constexpr int kTileGroups = 4;  // groups of 32 queries per chunk of the estimate pass
 
 // The sort box of scene s's queries: the scene box with a 1 % margin.
 CacheGrid sort_box(const pm_batch *b, int s) {
@@ -548,8 +546,15 @@ cudaError_t upload_tile_scenes(pm_batch *b) {
     for (int c = 1; c <= 4; ++c) {
         ar.class_first[c] = (int)d.size();
         uint32_t chunks = 0;
+        auto in_class = [&](int s) {
+            return b->tune[s].query_list && b->nq[s] > 0 && slots_for_k(b->cfgs[s].k) == c;
+        };
+        uint64_t queries = 0;
+        for (int s = 0; s < b->n; ++s)
+            if (in_class(s)) queries += b->nq[s];
+        ar.class_groups[c] = tile_groups(queries, b->sm_count);
         for (int s = 0; s < b->n; ++s) {
-            if (!b->tune[s].query_list || b->nq[s] == 0 || slots_for_k(b->cfgs[s].k) != c) continue;
+            if (!in_class(s)) continue;
             const BatchRenderScene r = render_desc(b, s);
             TileScene t;
             t.sc = b->scenes_dev + s;
@@ -563,7 +568,7 @@ cudaError_t upload_tile_scenes(pm_batch *b) {
             t.chunk_begin = chunks;
             t.k = b->cfgs[s].k;
             t.r2cap = b->cfgs[s].radius * b->cfgs[s].radius;
-            chunks += tile_chunks(t.n, kTileGroups);
+            chunks += tile_chunks(t.n, ar.class_groups[c]);
             d.push_back(t);
         }
         ar.class_n[c] = (int)d.size() - ar.class_first[c];
@@ -575,7 +580,7 @@ cudaError_t upload_tile_scenes(pm_batch *b) {
 
 // The query lists of every query-list scene into the arena: per-pixel
 // counts, their scans restarted at each scene, the records, the gather
-// counters, then each scene's (map, Morton) order by one segmented sort
+// counters, then each scene's (map, Hilbert) order by one segmented sort
 // (the sort keys and their second buffer live in the value array, the
 // second index buffer in the deferred-query list: both are free until the
 // estimate pass).
@@ -613,8 +618,8 @@ cudaError_t enqueue_arena_estimates(pm_batch *b, cudaStream_t st) {
     cudaError_t e;
     for (int c = 1; c <= 4; ++c) {
         if (ar.class_n[c] == 0) continue;
-        const TileBuffers buf{ar.anchor_d, ar.defer, ar.defer_n, nullptr};
-        e = knn_values_tiles_multi(ar.desc + ar.class_first[c], ar.class_n[c], ar.class_chunks[c], kTileGroups, c,
+        const TileBuffers buf{ar.defer, ar.defer_n, nullptr};
+        e = knn_values_tiles_multi(ar.desc + ar.class_first[c], ar.class_n[c], ar.class_chunks[c], ar.class_groups[c], c,
                                    true, buf, ar.defer_sc, b->sm_count, st);
         if (e != cudaSuccess) return e;
     }
@@ -698,18 +703,15 @@ cudaError_t size_query_buffers(pm_batch *b) {
     Z_TRY(dalloc(&q.key_tmp, max_q));
     Z_TRY(dalloc(&q.ord_tmp, max_q));
     Z_TRY(dalloc(&q.hist, radix_sort_hist_words((uint32_t)max_q)));
-    Z_TRY(dalloc(&q.anchor_d, tile_chunks((uint32_t)max_q, 4)));
     Z_TRY(dalloc(&q.defer_n, 2));  // deferred count, chunk counter
     q.q_cap = max_q;
     // the arena: every scene's pixel words and query slots, each a
     // segment of whole sort tiles
     auto &ar = b->ar;
-    size_t max_chunks = 1;
     std::vector<size_t> q_items(b->n), p_items(b->n);
     for (int s = 0; s < b->n; ++s) {
         q_items[s] = b->nq[s];
         p_items[s] = (size_t)b->cfgs[s].width * b->cfgs[s].height + 1;
-        max_chunks += tile_chunks(b->nq[s], kTileGroups);
     }
     Z_TRY(seg_runs_build(q_items, &ar.q_runs, &ar.q_off, &ar.q_total));
     Z_TRY(seg_runs_build(p_items, &ar.p_runs, &ar.p_off, &ar.p_total));
@@ -730,7 +732,6 @@ cudaError_t size_query_buffers(pm_batch *b) {
     Z_TRY(dalloc(&ar.defer, q_total));
     Z_TRY(dalloc(&ar.defer_sc, q_total));
     Z_TRY(dalloc(&ar.defer_n, 2));
-    Z_TRY(dalloc(&ar.anchor_d, max_chunks));
     Z_TRY(dalloc(&ar.desc, (size_t)b->n));
     Z_TRY(dalloc(&ar.lists, (size_t)b->n));
     Z_TRY(dalloc(&ar.list_ids, (size_t)b->n));

@@ -383,8 +383,17 @@ __device__ __forceinline__ float scale_pow2(float f, int n) {
 // 2^n as a float, n in [-126, 127].
 __device__ __forceinline__ float pow2f(int n) { return __uint_as_float((uint32_t)(n + 127) << 23); }
 
+// The integer sum and E: the value is sum * 2^(E - 182).
+struct FixedSum {
+    uint64_t sum;
+    int emax;
+};
+__device__ __forceinline__ float fixed_value(const FixedSum &f) {
+    return scale_pow2(__ull2float_rn(f.sum), f.emax - 182);
+}
+
 template <int T>
-__device__ __forceinline__ float warp_fixed_sum(const float (&t)[T]) {
+__device__ __forceinline__ FixedSum warp_fixed_parts(const float (&t)[T]) {
     uint32_t emax = 1;
 #pragma unroll
     for (int i = 0; i < T; ++i) emax = max(emax, __float_as_uint(t[i]) >> 23);
@@ -405,7 +414,15 @@ __device__ __forceinline__ float warp_fixed_sum(const float (&t)[T]) {
     const uint64_t a0 = __reduce_add_sync(kFull, (uint32_t)(acc & 0xfffffu));
     const uint64_t a1 = __reduce_add_sync(kFull, (uint32_t)((acc >> 20) & 0xfffffu));
     const uint64_t a2 = __reduce_add_sync(kFull, (uint32_t)(acc >> 40));
-    return scale_pow2(__ull2float_rn(a0 + (a1 << 20) + (a2 << 40)), (int)emax - 182);
+    FixedSum f;
+    f.sum = a0 + (a1 << 20) + (a2 << 40);
+    f.emax = (int)emax;
+    return f;
+}
+
+template <int T>
+__device__ __forceinline__ float warp_fixed_sum(const float (&t)[T]) {
+    return fixed_value(warp_fixed_parts<T>(t));
 }
 
 // One record's contribution to an estimate's numerator: its flux times the

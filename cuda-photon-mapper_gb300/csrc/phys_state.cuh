@@ -19,7 +19,7 @@ struct QueryList {
     uint32_t qcap = 0, nq = 0, nsurf = 0;
     uint64_t gen = 0;                           // scene generation the list was built for
     int flags = -1;                             // bit 0: volume queries, bit 1: diffuse
-    // spatial order: (map, Morton code) sort of the queries
+    // spatial order: (map, Hilbert code) sort of the queries
     uint32_t *key = nullptr, *ord = nullptr, *key_tmp = nullptr, *ord_tmp = nullptr;
     uint32_t *hist = nullptr, *n_dev = nullptr;
     uint32_t *order = nullptr;                  // points at the sorted query indices
@@ -28,9 +28,7 @@ struct QueryList {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float ms_build = 0.0f;
     unsigned long long *gather_stats = nullptr;  // counters of the last estimate pass
-    float *anchor_d = nullptr;                   // per warp chunk of the estimate pass
     uint32_t *defer_n = nullptr;
-    uint32_t anchor_cap = 0;
 };
 
 struct PhysicalState {
@@ -89,7 +87,7 @@ inline MapView view_of(const PhysicalState::Map &m) {
 // only when the scene changed since); synchronises the stream once to size
 // the list. Resets the spatial order.
 cudaError_t query_list_build(PhysicalState *st, bool force, cudaStream_t s);
-// Sorts the list by (map, Morton code of the position in the scene box)
+// Sorts the list by (map, Hilbert code of the position in the scene box)
 // into ql.order, unless already sorted.
 cudaError_t query_list_sort(PhysicalState *st, cudaStream_t s);
 void query_list_free(QueryList &ql);
@@ -97,17 +95,15 @@ void query_list_free(QueryList &ql);
 // into ql.val: the list in spatial order, warm-started runs of queries.
 cudaError_t knn_values_raw(PhysicalState *st, cudaStream_t s);
 constexpr int kGatherStats = 7;
-// Scratch of knn_values_tiles: anchor_d[tile_chunks(n, groups)], defer[n],
-// two defer_n words (deferred count, chunk counter); stats: kGatherStats
-// counters added (nullable).
+// Scratch of knn_values_tiles: defer[n], two defer_n words (deferred count,
+// chunk counter); stats: kGatherStats counters added (nullable).
 struct TileBuffers {
-    float *anchor_d;
     uint32_t *defer;
     uint32_t *defer_n;
     unsigned long long *stats;
 };
 // One scene of an estimate pass over many scenes (device memory): its
-// scene, maps, query records and values, its queries in (map, Morton)
+// scene, maps, query records and values, its queries in (map, Hilbert)
 // order, their count, the first of its chunks in the launch's numbering,
 // k and the squared gather radius.
 struct TileScene {
@@ -121,29 +117,30 @@ struct TileScene {
     int k;
     float r2cap;
 };
-// knn_values_tiles over the scenes of `scenes` (nsc descriptors, chunks
-// numbered scene after scene, total_chunks in all), all with k <= 32 *
-// slots, in three launches (anchors, one persistent shared-candidate launch,
-// deferred queries). buf.anchor_d holds total_chunks words, buf.defer and
-// defer_sc the largest possible number of deferred queries.
+// knn_values_tiles over the scenes of `scenes` (nsc descriptors, chunks of
+// `groups` groups numbered scene after scene, total_chunks in all), all with
+// k <= 32 * slots, in two launches (one persistent shared-candidate launch,
+// deferred queries). buf.defer and defer_sc hold the largest possible number
+// of deferred queries.
 cudaError_t knn_values_tiles_multi(const TileScene *scenes, int nsc, uint32_t total_chunks, int groups,
                                    int slots, bool raw, const TileBuffers &buf, uint32_t *defer_sc,
                                    int sm_count, cudaStream_t s);
-// Warps of an estimate pass over n queries, `groups` groups of 32 per warp.
+// Groups of 32 queries a warp takes at once in an estimate pass over n
+// queries in all, and the chunks that makes of n queries.
+int tile_groups(uint64_t n, int sm_count);
 uint32_t tile_chunks(uint32_t n, int groups);
 // k-NN estimates of the queries in spatial order (order[0..n) indexes qa/qd
 // and val; with n_dev, the first min(n, *n_dev): n is then a capacity and
 // the launch sizes do not depend on the count), one shared candidate set
-// per group of 32 neighbours, `groups`
-// (1-4) consecutive groups per warp of which the later ones are bounded by
-// the earlier (tile_gather.cu; use 1 when the groups are not neighbours): diffuse queries e / (pi r^2) / pi from the surface map,
+// per group of 32 neighbours, of which a warp takes several in a row
+// (tile_gather.cu): diffuse queries e / (pi r^2) / pi from the surface map,
 // volume queries e / (4/3 pi r^3) with the phase function toward wo from
 // the volume map; with raw set, the flux sum e and r^2 (-1 when nothing
 // was found) instead.
 cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView &vol,
                              const float4 *qa, const float4 *qd, const uint32_t *order, uint32_t n,
-                             const uint32_t *n_dev, int groups, int k, float radius, bool raw,
-                             float4 *val, const TileBuffers &buf, int sm_count, cudaStream_t s);
+                             const uint32_t *n_dev, int k, float radius, bool raw, float4 *val,
+                             const TileBuffers &buf, int sm_count, cudaStream_t s);
 
 // The render parameters pm_render passes for the installed configuration.
 inline RenderParams render_params(const PhysicalState *st) {

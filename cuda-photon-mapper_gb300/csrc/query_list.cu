@@ -1,5 +1,5 @@
 // query_list.cu -- the frame's radiance queries: build (count, scan, write
-// per pixel) and spatial order (map, Morton code), shared by the k-NN render
+// per pixel) and spatial order (map, Hilbert code), shared by the k-NN render
 // (pm_render) and the learned radiance cache.
 #include "cache.cuh"
 #include "phys_state.cuh"
@@ -24,7 +24,7 @@ void query_list_free(QueryList &ql) {
     cudaFree(ql.scan_tmp); cudaFree(ql.qa); cudaFree(ql.qd); cudaFree(ql.val);
     cudaFree(ql.key); cudaFree(ql.ord); cudaFree(ql.key_tmp); cudaFree(ql.ord_tmp);
     cudaFree(ql.hist); cudaFree(ql.n_dev); cudaFree(ql.gather_stats);
-    cudaFree(ql.anchor_d); cudaFree(ql.defer_n);
+    cudaFree(ql.defer_n);
     if (ql.ev0) cudaEventDestroy(ql.ev0);
     if (ql.ev1) cudaEventDestroy(ql.ev1);
     ql = QueryList();
@@ -133,19 +133,11 @@ cudaError_t knn_values_raw(PhysicalState *st, cudaStream_t s) {
         QL_TRY(dalloc(&ql.gather_stats, kGatherStats));
         QL_TRY(dalloc(&ql.defer_n, 2));  // deferred count, chunk counter
     }
-    if (tile_chunks(ql.nq, 4) > ql.anchor_cap) {
-        cudaFree(ql.anchor_d);
-        ql.anchor_d = nullptr;
-        ql.anchor_cap = 0;
-        QL_TRY(dalloc(&ql.anchor_d, tile_chunks(ql.qcap, 4)));
-        ql.anchor_cap = tile_chunks(ql.qcap, 4);
-    }
     QL_TRY(cudaMemsetAsync(ql.gather_stats, 0, sizeof(unsigned long long) * kGatherStats, s));
     // the sort's other index array is free again: the deferred-query list
-    const TileBuffers buf{ql.anchor_d, ql.order == ql.ord ? ql.ord_tmp : ql.ord, ql.defer_n, ql.gather_stats};
+    const TileBuffers buf{ql.order == ql.ord ? ql.ord_tmp : ql.ord, ql.defer_n, ql.gather_stats};
     QL_TRY(knn_values_tiles(st->dscene, view_of(st->map[0]), view_of(st->map[1]), ql.qa, ql.qd, ql.order,
-                            ql.nq, nullptr, 4, st->cfg.k, st->cfg.radius, true, ql.val, buf, st->sm_count,
-                            s));
+                            ql.nq, nullptr, st->cfg.k, st->cfg.radius, true, ql.val, buf, st->sm_count, s));
 #undef QL_TRY
     return cudaSuccess;
 }

@@ -1,34 +1,40 @@
 // tile_gather.cu -- k-NN radiance estimates of a query list in spatial
 // order, one candidate set per group of neighbouring queries.
 //
-// A warp takes 1 to 4 consecutive groups of 32 queries of the (map, Morton
-// code) order. The k-th-neighbour distance d(x) (capped at the gather radius) is
-// 1-Lipschitz in the query position, so exact distances d_j at points x_j
-// bound it everywhere: d(x) <= min_j (d_j + |x - x_j|). The warp's first group
-// is bounded by one anchor (an exact list search at one of its queries, done
-// by a separate launch before), every later group by the exact results of the
-// group before it. A group's records are found once in the kd-tree -- every
-// record within the largest upper bound of the group's bounding box -- and
-// held in registers, kSlots positions to a lane. A query computes its squared
-// distances to all of them and searches for the threshold that exactly k of
-// them lie at or below (select_k), starting from its predecessor's.
+// A warp takes chunks of 1, 2 or 4 consecutive groups of 32 queries of the
+// (map, Hilbert code) order. The k-th-neighbour distance d(x) (capped at the
+// gather radius) is 1-Lipschitz in the query position, so exact distances d_j
+// at points x_j bound it everywhere: d(x) <= min_j (d_j + |x - x_j|). A
+// chunk's first group is bounded by its middle query, which is answered by
+// itself first (single_bound, alone), every later group by the exact results
+// of the group before it. A group's records are found once in the kd-tree --
+// every record within the largest upper bound of the group's bounding box --
+// and held in registers, kSlots positions to a lane. A query computes its
+// squared distances to all of them and searches for the threshold that
+// exactly k of them lie at or below (select_k), starting from its
+// predecessor's.
 //
-// A group whose set does not fit the registers is processed in segments:
-// halves, down to single queries, each finished segment tightening the
-// bounds of the queries after it. A single query whose set still does not
-// fit, queries of the other map in a mixed group, and any result that
-// contradicts its own upper bound, are deferred to a list-search launch
-// after the pass. The selected set is exactly the list search's (ties
-// broken by photon index) and the estimate's sum is order-independent
-// (knn_core.cuh), so every value is bit-identical to the list search's.
+// A group whose set does not fit the registers, or is not expected to
+// (expected), is processed in segments: halves, down to single queries, each
+// finished segment tightening the bounds of the queries after it. A single
+// query whose set does not fit finds a radius of its own. Queries of the
+// other map in a mixed group, and any result that contradicts its own upper
+// bound, are deferred to a list-search launch after the pass. The selected
+// set is exactly the list search's (ties broken by photon index) and the
+// estimate's sum is order-independent (knn_core.cuh), so every value is
+// bit-identical to the list search's.
 //
-// Bound by instruction issue; the selected records' flux comes from L1 and
-// L2. Candidates in registers instead of shared memory make a query's
-// distances and counts straight-line code without loads, need no lists of
-// the certain and the doubtful candidates, and leave most of the L1 to the
-// flux. Estimate pass (GB300; candidates in shared memory, scanned, the band
-// between two bounds ranked, before): preset 2 113.0 -> 76.0 ms, preset 3
-// 45.4 -> 34.5 ms, preset 1 16.9 -> 12.0 ms.
+// Bound by instruction issue (75 % of the slots with 7 warps a scheduler);
+// the selected records' flux comes from L1 and L2. Candidates in registers
+// instead of shared memory make a query's distances and counts straight-line
+// code without loads, need no lists of the certain and the doubtful
+// candidates, and leave most of the L1 to the flux. Estimate pass (GB300,
+// presets 1 / 2 / 3): candidates in shared memory, scanned, the band between
+// two bounds ranked, 16.9 / 113.0 / 45.4 ms; in registers 12.0 / 76.0 / 34.5;
+// Hilbert instead of Morton order, a lane per channel for the last rounding
+// 10.0 / 64.0 / 29.9; expected set sizes instead of failed collections 9.8 /
+// 62.6 / 29.7; no separate anchor launch, 10 candidates per lane 10.0 / 59.8 /
+// 25.9.
 #include <algorithm>
 
 #include "cache.cuh"
@@ -43,12 +49,14 @@ namespace {
 using namespace wknn;
 
 constexpr int kTileWarps = 4;
-constexpr int kAnchorAt = 15;                // the anchor: query 15 of a warp's chunk
-// Blocks of 4 warps per SM (registers capped at 64) and candidates per lane.
-// Presets 2 / 3: 8 blocks and 8 slots 76.0 / 34.5 ms, 7 blocks 79.1 / 35.2,
-// 6 blocks 82.8 / 36.2; 10 slots at 6 blocks 81.3 / 36.7.
-constexpr int kTileBlocks = 8;
-constexpr int kSlots = 8;
+// Blocks of 4 warps per SM (registers capped at 72) and candidates per lane:
+// more candidates let a set serve more queries, more warps hide latency.
+// Presets 1 / 2 / 3 (ms): 7 blocks with 8 slots 11.7 / 65.3 / 27.9, 9 slots
+// 10.9 / 63.5 / 27.2, 10 slots 10.0 / 59.8 / 25.9, 11 slots 10.6 / 60.2 /
+// 26.2, 12 slots 10.3 / 68.7 / 29.0; 8 blocks with 9 slots 10.7 / 59.7 / 26.3,
+// 6 blocks with 10 slots 10.4 / 64.0 / 26.8.
+constexpr int kTileBlocks = 7;
+constexpr int kSlots = 10;
 constexpr int kTileCap = 32 * kSlots;        // candidate records per warp
 constexpr float kRel = 2e-4f;                // relative and absolute margins of the distance bounds
 constexpr float kAbs = 1e-6f;
@@ -57,7 +65,7 @@ constexpr float kAbs = 1e-6f;
 enum TileStat { kStTiled, kStList, kStShrunk, kStViolations, kStGroups, kStCandidates, kStHalvings, kStCount };
 
 struct TileScratch {
-    uint32_t cat[kTileCap];  // tree positions of the candidates
+    uint32_t cat[kTileCap + kTileCap / kSlots];  // tree positions of the candidates (cat_at)
     union {
         uint32_t stack[kStackCap];  // the collection's node stack
         uint32_t sel[128];          // tree positions of the k selected candidates
@@ -67,6 +75,10 @@ struct TileScratch {
     float4 known[32];        // exact distances that bound the group: point, distance
     unsigned long long st[kStCount];  // counters, lane 0
 };
+
+// Place of candidate c in cat: a lane's kSlots consecutive candidates, lanes
+// an odd number of words apart.
+__device__ __forceinline__ int cat_at(int c) { return c + c / kSlots; }
 
 // The parameters of the scene a warp is working on (per warp: in a launch
 // over many scenes the warps of one block may serve different scenes).
@@ -168,20 +180,35 @@ __device__ __forceinline__ void count(int i, unsigned long long v = 1) {
 // Writes one estimate (lane 0): the flux sum and squared radius (raw; -1
 // when nothing was found), or the normalised radiance estimate (the
 // render's own expressions).
+__device__ __forceinline__ float estimate_scale(float r2, bool surface) {
+    return surface ? (1.0f / (3.14159265f * r2)) * 0.318309886f : 1.0f / (4.18879020f * r2 * sqrtf(r2));
+}
 __device__ __forceinline__ void write_estimate(float4 *out, uint32_t i, v3 e, int found, float r2,
                                                bool surface, bool raw) {
     float r2out = -1.0f;
     if (found > 0) {
         r2out = r2;
-        if (!raw) {
-            const float sc = surface ? (1.0f / (3.14159265f * r2)) * 0.318309886f
-                                     : 1.0f / (4.18879020f * r2 * sqrtf(r2));
-            e = e * sc;
-        }
+        if (!raw) e = e * estimate_scale(r2, surface);
     } else {
         e = mk3(0.f, 0.f, 0.f);
     }
     if ((threadIdx.x & 31) == 0) out[i] = make_float4(e.x, e.y, e.z, raw ? r2out : 0.0f);
+}
+
+// The same from the integer sums of the three channels: lanes 0, 1 and 2
+// round one channel each (one pass through the 64-bit conversion instead of
+// three), lane 3 has the squared radius.
+__device__ __forceinline__ void write_sums(float4 *out, uint32_t i, const FixedSum &x, const FixedSum &y,
+                                           const FixedSum &z, int found, float r2, bool surface, bool raw) {
+    const int lane = threadIdx.x & 31;
+    FixedSum f;
+    f.sum = lane == 0 ? x.sum : (lane == 1 ? y.sum : z.sum);
+    f.emax = lane == 0 ? x.emax : (lane == 1 ? y.emax : z.emax);
+    float v = fixed_value(f);
+    if (!raw) v = v * estimate_scale(r2, surface);
+    if (found == 0) v = 0.0f;
+    if (lane == 3) v = raw ? (found > 0 ? r2 : -1.0f) : 0.0f;
+    if (lane < 4) reinterpret_cast<float *>(out + i)[lane] = v;
 }
 
 // Queues the queries (their indices on the lanes) of `mask` for the
@@ -229,7 +256,7 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
                 }
                 const unsigned mk = __ballot_sync(kFull, in);
                 if (n + __popc(mk) > kTileCap) return -1;
-                if (in) ts.cat[n + __popc(mk & lt)] = r;
+                if (in) ts.cat[cat_at(n + __popc(mk & lt))] = r;
                 n += __popc(mk);
             }
         } else {
@@ -262,21 +289,23 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
 // addition per slot and one warp sum, the next threshold scales the last by
 // the density it found (r^3 in the medium, r^2 on surfaces), and the last one
 // or two candidates are stepped over one by one. Where the k-th distance
-// occurs more than once the photon index decides. `t`: the first guess, at
-// most capb (the squared gather radius), the search's upper end. Returns the
-// mask of this lane's selected slots; *found: how many (k, or all within the
-// cap when fewer).
-__device__ __forceinline__ uint32_t select_k(const uint32_t (&d2)[kSlots], int n, uint32_t t, uint32_t capb, int k,
-                                             float expo, const MapView &m, int *found) {
+// occurs more than once the photon index decides, and those left out get an
+// infinite distance. t: the first guess, at most capb (the squared gather
+// radius), the search's upper end; on return the threshold, with *own the
+// candidates of this lane at or below it. Returns how many there are: k, or
+// all within the cap when fewer.
+__device__ __forceinline__ int select_k(uint32_t (&d2)[kSlots], uint32_t &t, uint32_t capb, int k, float expo,
+                                        const MapView &m, int *own) {
     int lo = -1, hi = (int)capb + 1;  // at or below lo: fewer than k; hi: more than k, or past the cap
-    uint32_t mask;
-    int c;
     for (int it = 0;; ++it) {
-        c = 0;
+        int mine = 0;
 #pragma unroll
-        for (int s = 0; s < kSlots; ++s) c += d2[s] <= t ? 1 : 0;
-        c = (int)__reduce_add_sync(kFull, (uint32_t)c);
-        if (c == k || (c < k && t == capb)) break;
+        for (int s = 0; s < kSlots; ++s) mine += d2[s] <= t ? 1 : 0;
+        const int c = (int)__reduce_add_sync(kFull, (uint32_t)mine);
+        if (c == k || (c < k && t == capb)) {
+            *own = mine;
+            return c;
+        }
         if (c < k) lo = (int)t; else hi = (int)t;
         if (hi - lo == 1) break;  // hi's distance occurs several times
         uint32_t nt = t;
@@ -303,40 +332,38 @@ __device__ __forceinline__ uint32_t select_k(const uint32_t (&d2)[kSlots], int n
         if ((int)nt <= lo || (int)nt >= hi) nt = (uint32_t)(lo + ((hi - lo) >> 1));
         t = nt;
     }
-    *found = min(c, k);
-    mask = 0u;
+    // those nearer than hi, then those at hi by photon index
+    t = (uint32_t)hi;
+    const int lane = threadIdx.x & 31;
+    uint32_t id[kSlots];
+    int less = 0;
 #pragma unroll
-    for (int s = 0; s < kSlots; ++s) mask |= d2[s] <= t ? 1u << s : 0u;
-    if (hi - lo == 1 && c != k && !(c < k && t == capb)) {
-        // those nearer than hi, then those at hi by photon index
-        const uint32_t v = (uint32_t)hi;
-        const int lane = threadIdx.x & 31;
-        uint32_t id[kSlots];
-        int less = 0;
-        mask = 0u;
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s) {
-            id[s] = 0xffffffffu;
-            if (d2[s] == v) id[s] = __float_as_uint(__ldg(&m.pos[scratch().cat[32 * s + lane]]).w);
-            less += d2[s] < v ? 1 : 0;
-            mask |= d2[s] < v ? 1u << s : 0u;
+    for (int s = 0; s < kSlots; ++s) {
+        id[s] = 0xffffffffu;
+        if (d2[s] == t) {
+            id[s] = __float_as_uint(__ldg(&m.pos[scratch().cat[cat_at(kSlots * lane + s)]]).w);
+            d2[s] = 0x7f800000u;
         }
-        less = (int)__reduce_add_sync(kFull, (uint32_t)less);
-        for (int i = less; i < k; ++i) {
-            uint32_t w = 0xffffffffu;
-#pragma unroll
-            for (int s = 0; s < kSlots; ++s) w = min(w, id[s]);
-            w = __reduce_min_sync(kFull, w);
-#pragma unroll
-            for (int s = 0; s < kSlots; ++s)
-                if (id[s] == w) {
-                    mask |= 1u << s;
-                    id[s] = 0xffffffffu;
-                }
-        }
-        *found = k;
+        less += d2[s] < t ? 1 : 0;
     }
-    return mask;
+    less = (int)__reduce_add_sync(kFull, (uint32_t)less);
+    for (int i = less; i < k; ++i) {
+        uint32_t w = 0xffffffffu;
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) w = min(w, id[s]);
+        w = __reduce_min_sync(kFull, w);
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s)
+            if (id[s] == w) {
+                d2[s] = t;
+                id[s] = 0xffffffffu;
+            }
+    }
+    int mine = 0;
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) mine += d2[s] <= t ? 1 : 0;
+    *own = mine;
+    return k;
 }
 
 // The queries of `mask` (one map, lane order = spatial order; this lane's at
@@ -358,13 +385,13 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
     if (n < 0) return false;
     count(kStGroups);
     count(kStCandidates, (unsigned long long)n);
-    // the candidates, kSlots to a lane
+    // the candidates, kSlots consecutive ones (neighbours in the tree) to a lane
     float px[kSlots], py[kSlots], pz[kSlots];
 #pragma unroll
     for (int s = 0; s < kSlots; ++s) {
         px[s] = py[s] = pz[s] = inf;
-        if (32 * s + lane < n) {
-            const float4 p = __ldg(&m.pos[ts.cat[32 * s + lane]]);
+        if (kSlots * lane + s < n) {
+            const float4 p = __ldg(&m.pos[ts.cat[cat_at(kSlots * lane + s)]]);
             px[s] = p.x;
             py[s] = p.y;
             pz[s] = p.z;
@@ -373,7 +400,6 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
     const float r2cap = targs().r2cap, rcap = targs().rcap;
     const uint32_t capb = __float_as_uint(r2cap);
     const float expo = mid == 0 ? 1.0f : 0.6666667f;
-    const unsigned lt = (1u << lane) - 1u;
     uint32_t guess = 0u;
     for (unsigned mm = mask; mm; mm &= mm - 1) {
         const int j = __ffs(mm) - 1;
@@ -385,12 +411,27 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
             d2[s] = __float_as_uint(dx * dx + dy * dy + dz * dz);
         }
         if (guess == 0u) guess = __float_as_uint(q.w * q.w);
-        int found;
-        const uint32_t sm = select_k(d2, n, min(guess, capb), capb, k, expo, m, &found);
+        uint32_t t = min(guess, capb);
+        int own;
+        const int found = select_k(d2, t, capb, k, expo, m, &own);
+        // the selected ones' tree positions, in candidate order, and the
+        // largest distance among them
+        int at = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, at, o);
+            if (lane >= o) at += v;
+        }
+        at -= own;
         uint32_t far = 0u;
 #pragma unroll
-        for (int s = 0; s < kSlots; ++s) far = max(far, (sm >> s) & 1u ? d2[s] : 0u);
+        for (int s = 0; s < kSlots; ++s)
+            if (d2[s] <= t) {
+                far = max(far, d2[s]);
+                ts.sel[at++] = ts.cat[cat_at(kSlots * lane + s)];
+            }
         far = __reduce_max_sync(kFull, far);
+        __syncwarp();
         // the set holds every record within the upper bound; a result
         // beyond it would mean the bound failed: defer to the list search
         const float kd2 = found == k ? __uint_as_float(far) : r2cap;
@@ -399,18 +440,10 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
             defer(__float_as_uint(ts.qd[j].w), 1u);
             if (lane == j) *d_lane = -1.0f;
             guess = 0u;
+            __syncwarp();
             continue;
         }
         guess = __float_as_uint(kd2);
-        int at = 0;
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s) {
-            const bool in = (sm >> s) & 1u;
-            const unsigned b = __ballot_sync(kFull, in);
-            if (in) ts.sel[at + __popc(b & lt)] = ts.cat[32 * s + lane];
-            at += __popc(b);
-        }
-        __syncwarp();
         const float4 qd = ts.qd[j];
         const v3 dirv = mk3(qd.x, qd.y, qd.z);
         float tx[S], ty[S], tz[S];
@@ -425,8 +458,8 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
                 tz[s] = t.z;
             }
         }
-        const v3 e = mk3(warp_fixed_sum<S>(tx), warp_fixed_sum<S>(ty), warp_fixed_sum<S>(tz));
-        write_estimate(targs().out, __float_as_uint(qd.w), e, found, kd2, mid == 0, targs().raw);
+        const FixedSum fx = warp_fixed_parts<S>(tx), fy = warp_fixed_parts<S>(ty), fz = warp_fixed_parts<S>(tz);
+        write_sums(targs().out, __float_as_uint(qd.w), fx, fy, fz, found, kd2, mid == 0, targs().raw);
         __syncwarp();
         if (lane == j) *d_lane = found == k ? sqrtf(kd2) : rcap;
         count(kStTiled);
@@ -434,30 +467,57 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
     return true;
 }
 
-// The upper bound for the single query of lane j (at x) whose set within its
-// bound *ub does not fit: the radius is bisected (in r^3) below the bound. A
-// collection that overflows holds more than kTileCap >= k records, so its
-// radius is an upper bound; one with fewer than k (and below the cap) is a
-// lower bound; one in between holds the k nearest. Returns false when no
-// such radius turns up.
-__device__ __noinline__ bool shrink_single(int mid, int j, float *ub) {
-    const int k = targs().k;
+// A radius around query j of the group that at least k and at most kTileCap
+// records of map `mid` lie within (or the gather radius, when fewer do), at
+// most `hi`; -1 when none turns up. The first radius is that of k records at
+// the density of the leaf nearest to the query (volume for the medium, area
+// for surfaces); it then grows by the density found and, between a radius
+// that overflows and one with too few, is bisected in r^3.
+__device__ __noinline__ float single_bound(int mid, int j, float hi) {
+    const int k = targs().k, lane = threadIdx.x & 31;
+    const MapView &m = targs().map[mid];
     const float4 q = scratch().qx[j];
     const v3 x = mk3(q.x, q.y, q.z);
-    float lo = 0.0f, hi = fminf(q.w, targs().rcap);
-    for (int it = 0; it < 24; ++it) {
-        const float r = cbrtf(0.5f * (lo * lo * lo + hi * hi * hi));
+    const float rcap = targs().rcap;
+    uint32_t node = 1u;
+    float dist = 0.0f;
+    for (int dn = 0; dn < m.depth;) {
+        int w = (m.depth - dn) % 5;
+        if (w == 0) w = 5;
+        const uint32_t child = (node << w) + lane;
+        uint32_t d = 0xffffffffu;
+        if (lane < (1 << w)) d = __float_as_uint(box_d2(__ldg(&m.lo[child]), __ldg(&m.hi[child]), x));
+        const uint32_t best = __reduce_min_sync(kFull, d);
+        const unsigned at = __ballot_sync(kFull, d == best);
+        node = (node << w) + (uint32_t)(__ffs(at) - 1);
+        dist = __uint_as_float(best);
+        dn += w;
+    }
+    const float4 bl = __ldg(&m.lo[node]), bh = __ldg(&m.hi[node]);
+    const float ex = bh.x - bl.x, ey = bh.y - bl.y, ez = bh.z - bl.z;
+    const float f = (float)k / (float)(32 << m.leaf_shift);
+    const float area = fmaxf(ex * ey, fmaxf(ey * ez, ez * ex));
+    float r = mid == 0 ? approx_sqrt(f * area * 0.31830989f) : cbrtf(f * ex * ey * ez * 0.23873241f);
+    r = 1.1f * r + approx_sqrt(dist);
+    hi = fminf(hi, rcap);
+    r = r > 0.0f ? fminf(r, hi) : hi;  // and NaN
+    float lo = 0.0f;
+    bool over = false;
+    for (int it = 0; it < 32; ++it) {
         const int n = collect(mid, x, x, r * r);
         if (n < 0) {
             hi = r;
-        } else if (n < k && r < targs().rcap) {
+            over = true;
+        } else if (n < k && r < rcap) {
             lo = r;
         } else {
-            *ub = r * (1.0f + kRel) + kAbs;
-            return true;
+            return r;
         }
+        if (over) r = lo > 0.0f ? cbrtf(0.5f * (lo * lo * lo + hi * hi * hi)) : 0.75f * hi;
+        else r = fminf(lo * fminf(fmaxf(__powf(__fdividef(1.4f * (float)k, (float)max(n, 1)), mid == 0 ? 0.5f : 0.3333333f), 1.05f), 2.0f), hi);
+        if (!(r > lo)) return -1.0f;
     }
-    return false;
+    return -1.0f;
 }
 
 // The least of ub and what the exact distances of known[0..n) allow at x
@@ -474,25 +534,55 @@ __device__ __forceinline__ float bound_by(const float4 *known, int n, v3 x, floa
     return fminf(ub, u * (1.0f + kRel) + kAbs);
 }
 
+// Query j of the group by itself, its bound found first (below ub); false:
+// to be deferred.
+template <int S>
+__device__ __noinline__ bool alone(v3 x, float ub, int mid, int j, float *d_lane) {
+    const float r = single_bound(mid, j, __shfl_sync(kFull, ub, j));
+    if (!(r >= 0.0f)) return false;
+    const float u = fminf(r * (1.0f + kRel) + kAbs, targs().rcap);
+    __syncwarp();
+    if ((threadIdx.x & 31) == j) scratch().qx[j].w = u;
+    __syncwarp();
+    return tile_queries<S>(x, u, mid, 1u << j, d_lane);
+}
+
+// The records expected in the candidate set of the queries of `mask`: the
+// volume within the largest bound of their box (for a surface map the area
+// of its two longer sides) at the density of k records per ball of the mean
+// known distance; 0 when that says nothing (nothing known, or the gather
+// radius binds).
+__device__ __forceinline__ float expected(v3 x, float ub, int mid, unsigned mask, float mean) {
+    if (!(mean > 0.0f) || mean >= targs().rcap) return 0.0f;
+    const bool member = (mask >> (threadIdx.x & 31)) & 1u;
+    const float inf = __int_as_float(0x7f800000);
+    const float a = warp_max(member ? x.x : -inf) - warp_min(member ? x.x : inf);
+    const float b = warp_max(member ? x.y : -inf) - warp_min(member ? x.y : inf);
+    const float c = warp_max(member ? x.z : -inf) - warp_min(member ? x.z : inf);
+    const float r = warp_max(member ? ub : 0.0f);
+    const float k = (float)targs().k;
+    if (mid == 0) {
+        const float lo = fminf(a, fminf(b, c)), hi = fmaxf(a, fmaxf(b, c)), md = a + b + c - lo - hi;
+        return k * __fdividef(hi * md + 2.0f * (hi + md) * r + 3.1415927f * r * r, 3.1415927f * mean * mean);
+    }
+    const float v = a * b * c + 2.0f * (a * b + b * c + c * a) * r + 3.1415927f * (a + b + c) * r * r +
+                    4.1887902f * r * r * r;
+    return k * __fdividef(v, 4.1887902f * mean * mean * mean);
+}
+
 // One chunk (groups of 32 consecutive queries of the sorted order, from
 // query chunk * 32 * groups) of a scene, with the warp's arguments set.
 template <int S>
 __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf, const MapView &vol,
                                            const float4 *qa, const float4 *qd, const uint32_t *order,
-                                           uint32_t n, uint32_t chunk, float anchor, int groups,
+                                           uint32_t n, uint32_t chunk, int groups,
                                            float r2cap, bool raw, float4 *out) {
     TileScratch &ts = scratch();
     const int lane = threadIdx.x & 31;
     const float rcap = sqrtf(r2cap);
     const uint32_t wfirst = chunk * (uint32_t)(32 * groups);
-    // exact distances known so far: the anchor, later the previous group
-    int nknown = 1, wkind;
-    {
-        const uint32_t ai = order[wfirst + min((uint32_t)kAnchorAt, n - 1 - wfirst)];
-        const float4 a = qa[ai];
-        wkind = __float_as_int(a.w) != kNone ? 0 : 1;
-        if (lane == 0) ts.known[0] = make_float4(a.x, a.y, a.z, anchor);
-    }
+    // exact distances known so far: those of the previous group
+    int nknown = 0, wkind = -1;
     for (int g = 0; g < groups; ++g) {
         const uint32_t first = wfirst + (uint32_t)(32 * g);
         if (first >= n) break;
@@ -521,14 +611,40 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
             ts.qd[lane] = make_float4(q.dirv.x, q.dirv.y, q.dirv.z, __uint_as_float(q.out));
             __syncwarp();
             // segments of the members in spatial order: the whole group,
-            // then halves of a segment whose set does not fit, down to
-            // single queries (growing again after a fit); each finished
-            // segment tightens the bounds of the rest
+            // then halves of a segment whose set does not fit (or is not
+            // expected to), down to single queries (growing again after a
+            // fit); each finished segment tightens the bounds of the rest
             unsigned rem = members;
             int sz = 32;
+            if (nknown == 0) {
+                // nothing bounds the group yet: its middle query by itself first
+                const int j = __fns(members, 0, (__popc(members) + 1) >> 1);
+                if (alone<S>(q.x, ub, gkind, j, &dnew)) {
+                    if (lane == j) ts.known[0] = make_float4(q.x.x, q.x.y, q.x.z, dnew);
+                    __syncwarp();
+                    nknown = 1;
+                    ub = bound_by(ts.known, 1, q.x, ub);
+                    ts.qx[lane].w = ub;
+                    __syncwarp();
+                } else {
+                    defer(q.out, 1u << j);
+                }
+                rem &= ~(1u << j);
+            }
+            // the mean known distance: the density the sets are expected at
+            const float kw = lane < nknown ? ts.known[lane].w : -1.0f;
+            const int kn = __popc(__ballot_sync(kFull, kw >= 0.0f));
+            float mean = kw >= 0.0f ? kw : 0.0f;
+#pragma unroll
+            for (int o = 16; o; o >>= 1) mean += __shfl_xor_sync(kFull, mean, o);
+            mean = kn ? __fdividef(mean, (float)kn) : -1.0f;
             while (rem) {
                 const unsigned seg = __popc(rem) <= sz ? rem : rem & ((1u << __fns(rem, 0, sz + 1)) - 1u);
                 const int j = __ffs(seg) - 1;
+                if (__popc(seg) > 1 && expected(q.x, ub, gkind, seg, mean) > (float)kTileCap) {
+                    sz = __popc(seg) >> 1;
+                    continue;
+                }
                 bool done = tile_queries<S>(q.x, ub, gkind, seg, &dnew);
                 if (!done && __popc(seg) > 1) {
                     count(kStHalvings);
@@ -538,16 +654,7 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
                 if (done) {
                     sz = min(2 * sz, 32);
                 } else {
-                    float u = 0.0f;
-                    if (shrink_single(gkind, j, &u)) {
-                        __syncwarp();
-                        if (lane == j) {
-                            ub = u;
-                            ts.qx[j].w = u;
-                        }
-                        __syncwarp();
-                        done = tile_queries<S>(q.x, ub, gkind, seg, &dnew);
-                    }
+                    done = alone<S>(q.x, ub, gkind, j, &dnew);
                     if (done) count(kStShrunk);
                     else defer(q.out, seg);
                 }
@@ -576,7 +683,7 @@ template <int S>
 __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     query_knn_tile_kernel(PScene Sc, MapView surf, MapView vol, const float4 *qa, const float4 *qd,
                           const uint32_t *order, uint32_t n, const uint32_t *n_dev, int groups,
-                          const float *anchor_d, int k, float r2cap, bool raw, float4 *out,
+                          int k, float r2cap, bool raw, float4 *out,
                           uint32_t *defer_list, uint32_t *defer_n, uint32_t *chunk_counter,
                           unsigned long long *stats) {
     const int lane = threadIdx.x & 31;
@@ -594,7 +701,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
         if (lane == 0) chunk = atomicAdd(chunk_counter, 1u);
         chunk = __shfl_sync(kFull, chunk, 0);
         if (chunk >= nchunks) break;
-        tile_chunk<S>(Sc, surf, vol, qa, qd, order, n, chunk, anchor_d[chunk], groups, r2cap, raw, out);
+        tile_chunk<S>(Sc, surf, vol, qa, qd, order, n, chunk, groups, r2cap, raw, out);
     }
     __syncwarp();
     if (stats && lane < kStCount && ts.st[lane]) atomicAdd(&stats[lane], ts.st[lane]);
@@ -616,7 +723,7 @@ __device__ __forceinline__ int scene_of_chunk(const TileScene *scenes, int nsc, 
 template <int S>
 __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     query_knn_tile_multi_kernel(const TileScene *scenes, int nsc, uint32_t total_chunks, int groups,
-                                const float *anchor_d, bool raw, uint32_t *defer_list,
+                                bool raw, uint32_t *defer_list,
                                 uint32_t *defer_sc, uint32_t *defer_n, uint32_t *chunk_counter,
                                 unsigned long long *stats) {
     const int lane = threadIdx.x & 31;
@@ -636,51 +743,11 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
                       d.k, raw);
             cur = sidx;
         }
-        tile_chunk<S>(*d.sc, d.surf, d.vol, d.qa, d.qd, d.order, d.n, chunk - d.chunk_begin, anchor_d[chunk],
-                      groups, d.r2cap, raw, d.val);
+        tile_chunk<S>(*d.sc, d.surf, d.vol, d.qa, d.qd, d.order, d.n, chunk - d.chunk_begin, groups,
+                      d.r2cap, raw, d.val);
     }
     __syncwarp();
     if (stats && lane < kStCount && ts.st[lane]) atomicAdd(&stats[lane], ts.st[lane]);
-}
-
-// Exact capped k-th distance of each warp chunk's anchor query (list search).
-template <int S>
-__global__ void __launch_bounds__(128)
-    anchor_kernel(MapView surf, MapView vol, const float4 *qa, const uint32_t *order, uint32_t n,
-                  const uint32_t *n_dev, int groups, int k, float r2cap, float *anchor_d) {
-    __shared__ WarpScratch ws[4];
-    if (n_dev) n = min(n, *n_dev);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t chunk = blockIdx.x * 4 + wib;
-    const uint32_t wfirst = chunk * (uint32_t)(32 * groups);
-    if (wfirst >= n) return;
-    const float4 a = qa[order[wfirst + min((uint32_t)kAnchorAt, n - 1 - wfirst)]];
-    const MapView &m = __float_as_int(a.w) != kNone ? surf : vol;
-    const uint64_t cap = make_key(r2cap, 0xffffffffu);
-    Knn<S> kn;
-    kn.reset(cap, k);
-    knn_search<S>(m, mk3(a.x, a.y, a.z), kn, ws[wib], lane, cap);
-    if (lane == 0) anchor_d[chunk] = kn.worst < cap ? sqrtf(key_d2(kn.worst)) : sqrtf(r2cap);
-}
-
-// The anchors of the chunks of many scenes (global chunk numbering).
-template <int S>
-__global__ void __launch_bounds__(128)
-    anchor_multi_kernel(const TileScene *scenes, int nsc, uint32_t total_chunks, int groups,
-                        float *anchor_d) {
-    __shared__ WarpScratch ws[4];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t chunk = blockIdx.x * 4 + wib;
-    if (chunk >= total_chunks) return;
-    const TileScene &d = scenes[scene_of_chunk(scenes, nsc, chunk)];
-    const uint32_t wfirst = (chunk - d.chunk_begin) * (uint32_t)(32 * groups);
-    const float4 a = d.qa[d.order[wfirst + min((uint32_t)kAnchorAt, d.n - 1 - wfirst)]];
-    const MapView &m = __float_as_int(a.w) != kNone ? d.surf : d.vol;
-    const uint64_t cap = make_key(d.r2cap, 0xffffffffu);
-    Knn<S> kn;
-    kn.reset(cap, d.k);
-    knn_search<S>(m, mk3(a.x, a.y, a.z), kn, ws[wib], lane, cap);
-    if (lane == 0) anchor_d[chunk] = kn.worst < cap ? sqrtf(key_d2(kn.worst)) : sqrtf(d.r2cap);
 }
 
 // The deferred queries of many scenes (defer_sc: each one's scene).
@@ -739,10 +806,10 @@ __global__ void __launch_bounds__(128)
 
 cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView &vol,
                              const float4 *qa, const float4 *qd, const uint32_t *order, uint32_t n,
-                             const uint32_t *n_dev, int groups, int k, float radius, bool raw,
-                             float4 *val, const TileBuffers &buf, int sm_count, cudaStream_t s) {
+                             const uint32_t *n_dev, int k, float radius, bool raw, float4 *val,
+                             const TileBuffers &buf, int sm_count, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    if (groups < 1 || groups > 4) return cudaErrorInvalidValue;
+    const int groups = tile_groups(n, sm_count);
     const float r2 = radius * radius;
     const uint32_t chunks = tile_chunks(n, groups);
     const dim3 grid((chunks + kTileWarps - 1) / kTileWarps), block(kTileWarps * 32);
@@ -754,13 +821,12 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
     int per_sm = 1;
     // persistent tile launch: as many blocks as fit on the GPU at once
 #define PM_TILE_LAUNCH(SL)                                                                              \
-    anchor_kernel<SL><<<grid, block, 0, s>>>(surf, vol, qa, order, n, n_dev, groups, k, r2, buf.anchor_d); \
     e = cudaFuncSetAttribute(query_knn_tile_kernel<SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
     if (e != cudaSuccess) return e;                                                                     \
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, query_knn_tile_kernel<SL>, kTileWarps * 32, smem); \
     if (e != cudaSuccess) return e;                                                                     \
     query_knn_tile_kernel<SL><<<std::min<uint32_t>(grid.x, (uint32_t)std::max(sm_count, 1) * (uint32_t)std::max(per_sm, 1)), \
-                                block, smem, s>>>(S, surf, vol, qa, qd, order, n, n_dev, groups, buf.anchor_d, k, \
+                                block, smem, s>>>(S, surf, vol, qa, qd, order, n, n_dev, groups, k, \
                                                   r2, raw, val, buf.defer, buf.defer_n, buf.defer_n + 1, buf.stats); \
     deferred_kernel<SL><<<dgrid, 128, 0, s>>>(S, surf, vol, qa, qd, buf.defer, buf.defer_n, k, r2, raw, val)
     switch ((k + 31) / 32) {
@@ -770,7 +836,7 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
         default: PM_TILE_LAUNCH(4); break;
     }
 #undef PM_TILE_LAUNCH
-    note_launches(3);
+    note_launches(2);
     return cudaGetLastError();
 }
 
@@ -786,13 +852,12 @@ cudaError_t knn_values_tiles_multi(const TileScene *scenes, int nsc, uint32_t to
     if (e != cudaSuccess) return e;
     int per_sm = 1;
 #define PM_MULTI_LAUNCH(SL)                                                                              \
-    anchor_multi_kernel<SL><<<agrid, block, 0, s>>>(scenes, nsc, total_chunks, groups, buf.anchor_d);   \
     e = cudaFuncSetAttribute(query_knn_tile_multi_kernel<SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
     if (e != cudaSuccess) return e;                                                                     \
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, query_knn_tile_multi_kernel<SL>, kTileWarps * 32, smem); \
     if (e != cudaSuccess) return e;                                                                     \
     query_knn_tile_multi_kernel<SL><<<std::min<uint32_t>(agrid.x, (uint32_t)std::max(sm_count, 1) * (uint32_t)std::max(per_sm, 1)), \
-                                      block, smem, s>>>(scenes, nsc, total_chunks, groups, buf.anchor_d, raw, \
+                                      block, smem, s>>>(scenes, nsc, total_chunks, groups, raw, \
                                                         buf.defer, defer_sc, buf.defer_n, buf.defer_n + 1, buf.stats); \
     deferred_multi_kernel<SL><<<dgrid, 128, 0, s>>>(scenes, buf.defer, defer_sc, buf.defer_n, raw)
     switch (slots) {
@@ -802,10 +867,22 @@ cudaError_t knn_values_tiles_multi(const TileScene *scenes, int nsc, uint32_t to
         default: PM_MULTI_LAUNCH(4); break;
     }
 #undef PM_MULTI_LAUNCH
-    note_launches(3);
+    note_launches(2);
     return cudaGetLastError();
 }
 
 uint32_t tile_chunks(uint32_t n, int groups) { return (n + 32u * groups - 1) / (32u * groups); }
+
+// A chunk's first group costs a bound of its own, its later ones have the
+// group before; the fewer chunks a warp gets, the longer the last ones leave
+// the others idle. Measured (ms, 1 / 2 / 4 groups, per query count): 2.1M
+// 2.4 / 2.6 / 3.3 (with 8 candidates a lane), 11M 12.5 / 11.5 / 11.4, 21M - /
+// 25.4 / 25.9, 46M - / 62.6 / 59.8: four from 64 chunks a warp on, one below
+// 8 chunks of two.
+int tile_groups(uint64_t n, int sm_count) {
+    const uint64_t warps = (uint64_t)std::max(sm_count, 1) * kTileBlocks * kTileWarps;
+    if (n >= 128u * 64u * warps) return 4;
+    return n >= 64u * 8u * warps ? 2 : 1;
+}
 
 }  // namespace pm
