@@ -34,8 +34,6 @@ struct CacheState {
 
 namespace pm {
 
-constexpr int kTargetRun = 8;  // training targets warm-started in runs of this length
-
 namespace {
 template <typename T>
 cudaError_t talloc(T **p, size_t count) {
@@ -57,7 +55,7 @@ cudaError_t train_scratch_alloc(uint32_t ns, TrainScratch *t) {
     TS_TRY(talloc(&t->sval_tmp, ns));
     TS_TRY(talloc(&t->shist, radix_sort_hist_words(ns)));
     TS_TRY(talloc(&t->sn, 1));
-    TS_TRY(talloc(&t->run_ctr, 1));
+    TS_TRY(talloc(&t->defer_n, 2));
     TS_TRY(talloc(&t->pqa, ns));
     TS_TRY(talloc(&t->pqd, ns));
     TS_TRY(talloc(&t->pval, ns));
@@ -74,7 +72,7 @@ cudaError_t train_scratch_alloc(uint32_t ns, TrainScratch *t) {
 
 void train_scratch_free(TrainScratch &t) {
     cudaFree(t.sel); cudaFree(t.skey); cudaFree(t.sval); cudaFree(t.skey_tmp); cudaFree(t.sval_tmp);
-    cudaFree(t.shist); cudaFree(t.sn); cudaFree(t.run_ctr);
+    cudaFree(t.shist); cudaFree(t.sn); cudaFree(t.defer_n);
     cudaFree(t.pqa); cudaFree(t.pqd); cudaFree(t.pval); cudaFree(t.pord);
     cudaFree(t.tqa); cudaFree(t.tqd); cudaFree(t.tgt); cudaFree(t.tsel); cudaFree(t.scale_sum);
     t = TrainScratch();
@@ -180,8 +178,10 @@ cudaError_t cache_pick_and_target(const pm_cache_config &cfg, const CacheGrid &g
     CT_TRY(radix_sort_pairs_u32(t.skey, t.sval, t.skey_tmp, t.sval_tmp, t.sn, ns, 0, 31, t.shist, stream, &ok_keys,
                                 &ok_vals));
     CT_TRY(cache_pick_records(ok_vals, t.sel, qa, qd, ns, t.pqa, t.pqd, t.pord, stream));
-    CT_TRY(cache_knn_values_runs(S, surf, vol, t.pqa, t.pqd, nullptr, t.pord, ns, kTargetRun, k, radius, false,
-                                 t.pval, t.run_ctr, sm_count, stream));
+    // the picks' sort keys are done with: room for the deferred ones
+    const TileBuffers buf{ok_keys, t.defer_n, nullptr};
+    CT_TRY(knn_values_tiles(S, surf, vol, t.pqa, t.pqd, t.pord, ns, nullptr, k, radius, false, t.pval, buf,
+                            sm_count, stream));
     CT_TRY(cache_train_order(t.pqa, t.pqd, t.pval, ok_vals, t.sel, ns, cache_batch_count(ns, cfg.batch), t.tqa,
                              t.tqd, t.tgt, t.tsel, stream));
 #undef CT_TRY

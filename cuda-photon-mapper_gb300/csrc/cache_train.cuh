@@ -17,7 +17,7 @@ struct TrainScratch {
     uint32_t *sel = nullptr;            // picked queries
     uint32_t *skey = nullptr, *sval = nullptr, *skey_tmp = nullptr, *sval_tmp = nullptr;
     uint32_t *shist = nullptr, *sn = nullptr;
-    uint32_t *run_ctr = nullptr;        // the target launch's run counter
+    uint32_t *defer_n = nullptr;        // the target pass's two counters
     float4 *pqa = nullptr, *pqd = nullptr, *pval = nullptr;  // sorted picks: records, targets
     uint32_t *pord = nullptr;           // identity order of the sorted picks
     float4 *tqa = nullptr, *tqd = nullptr, *tgt = nullptr;   // training order: records, targets
@@ -51,9 +51,10 @@ void cache_batch_range(uint32_t ns, uint32_t nb, uint32_t b, uint32_t *o, uint32
 // frame number `frame`, or *frame_dev when set) of the query list
 // qa/qd[0..nq) with diffuse queries slist[0..nsurf), and their k-NN targets,
 // into t in training order. The picks are sorted by (map, Morton code),
-// their records gathered in that order and estimated in runs of
-// warm-started list searches (picks this sparse are too far apart to share
-// candidate sets), then batch b takes every nb-th sorted pick.
+// their records gathered in that order and estimated by the render's pass
+// (knn_values_tiles: dense picks share candidate sets, sparse ones are bounded
+// by themselves; 2^20 picks of preset 2 take 4.0 ms, as warm-started list
+// searches they took 7.3 ms), then batch b takes every nb-th sorted pick.
 cudaError_t cache_pick_and_target(const pm_cache_config &cfg, const CacheGrid &grid, uint32_t frame,
                                   const unsigned long long *frame_dev, const PScene &S, const MapView &surf,
                                   const MapView &vol, int k, float radius, const float4 *qa, const float4 *qd,

@@ -1,7 +1,6 @@
-// gather.cu -- the k-NN queries of pm_knn, the single-kernel frame render
-// (eye rays, specular chains, volume march; one warp per pixel), the batched
-// multi-scene render, and the k-NN estimates of query lists. The warp k-NN
-// search and the estimate sum live in knn_core.cuh.
+// gather.cu -- the single-kernel frame render (eye rays, specular chains,
+// volume march; one warp per pixel) and the batched multi-scene render. The
+// warp k-NN search and the estimate sum live in knn_core.cuh.
 #include "launch_count.cuh"
 
 #include <atomic>
@@ -14,29 +13,6 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;
 using namespace wknn;
-
-template <int S>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32) knn_kernel(MapView m, const float4 *q,
-                                                                  uint32_t nq, int k, float r2cap,
-                                                                  uint32_t *idx_out, float *d2_out) {
-    __shared__ WarpScratch ws[kWarpsPerBlock];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t qi = blockIdx.x * kWarpsPerBlock + wib;
-    if (qi >= nq) return;
-    float4 qq = q[qi];
-    const uint64_t cap = make_key(r2cap, 0xffffffffu);
-    Knn<S> kn;
-    kn.reset(cap, k);
-    knn_search<S>(m, mk3(qq.x, qq.y, qq.z), kn, ws[wib], lane, cap);
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-        const int j = lane * S + s;
-        if (j < k) {
-            idx_out[(size_t)qi * k + j] = (uint32_t)kn.key[s];
-            d2_out[(size_t)qi * k + j] = key_d2(kn.key[s]);
-        }
-    }
-}
 
 // One pixel (one warp): eye ray, specular chain, volume march with a k-NN
 // in-scattering estimate per step, k-NN estimate at the diffuse hit.
@@ -221,98 +197,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 5)
     }
 }
 
-// k-NN estimates of runs of spatially sorted queries: warp w takes queries
-// order[w * run .. (w + 1) * run) (indices into sel, or the queries
-// themselves when sel is null), each warm-started from the previous query's
-// list when both read the same map and the previous one found k records --
-// the march's warm start, applied to spatial neighbours. Results land at
-// out[order[j]]: the exact estimate query_knn_kernel computes, or with raw
-// set the flux sum and the squared radius (-1 when nothing was found), from
-// which the render's own arithmetic finishes the estimate.
-// 9 blocks of 4 warps per SM (registers capped): the residency that measured
-// fastest (7 by registers alone, 12 spilled too much).
-template <int S>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 9)
-    query_knn_run_kernel(PScene Sc, MapView surf, MapView vol, const float4 *qa, const float4 *qd,
-                         const uint32_t *sel, const uint32_t *order, uint32_t n, int run, int k,
-                         float r2cap, bool raw, float4 *out, uint32_t *run_ctr) {
-    __shared__ WarpScratch ws[kWarpsPerBlock];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t nruns = (n + (uint32_t)run - 1) / (uint32_t)run;
-    const uint64_t cap = make_key(r2cap, 0xffffffffu);
-    // with run_ctr, persistent warps take runs from the counter until none
-    // is left; without, warp w of the grid takes run w
-    uint32_t r = blockIdx.x * kWarpsPerBlock + wib;
-    for (;;) {
-    if (run_ctr) {
-        if (lane == 0) r = atomicAdd(run_ctr, 1u);
-        r = __shfl_sync(0xffffffffu, r, 0);
-    }
-    if (r >= nruns) break;
-    const uint32_t first = r * (uint32_t)run;
-    const uint32_t last = min(first + (uint32_t)run, n);
-    Knn<S> kn;
-    kn.reset(cap, k);
-    int prev_kind = -1;  // 0 surface, 1 volume
-    bool warm = false;
-    for (uint32_t j = first; j < last; ++j) {
-        const uint32_t i = order[j];
-        const uint32_t src = sel ? sel[i] : i;
-        const float4 a = qa[src], d = qd[src];
-        const int obj = __float_as_int(a.w);
-        const v3 x = mk3(a.x, a.y, a.z), wo = mk3(d.x, d.y, d.z);
-        const bool surface = obj != kNone;
-        const int kind = surface ? 0 : 1;
-        const MapView &m = surface ? surf : vol;
-        v3 e = mk3(0.f, 0.f, 0.f);
-        float r2out = -1.0f;
-        bool found_k = false;
-        if (m.n > 0) {
-            const bool use_warm = warm && kind == prev_kind;
-            if (use_warm) rescore<S>(m, x, kn, ws[wib], cap, lane);
-            else kn.reset(cap, k);
-            knn_search<S>(m, x, kn, ws[wib], lane, cap, use_warm);
-            int found;
-            float r2;
-            const v3 dirv = surface ? facing_normal(Sc, obj, x, wo) : wo;
-            e = flux_sum<S>(kn, m, lane, surface ? 0 : 1, dirv, Sc.g, cap, r2cap, &found, &r2);
-            found_k = found == k;
-            if (found > 0) {
-                r2out = r2;
-                if (!raw) {
-                    const float sc = surface ? (1.0f / (3.14159265f * r2)) * 0.318309886f
-                                             : 1.0f / (4.18879020f * r2 * sqrtf(r2));
-                    e = e * sc;
-                }
-            } else {
-                e = mk3(0.f, 0.f, 0.f);
-            }
-        }
-        if (lane == 0) out[i] = make_float4(e.x, e.y, e.z, raw ? r2out : 0.0f);
-        warm = found_k;
-        prev_kind = kind;
-    }
-    if (!run_ctr) break;
-    }  // runs
-}
-
 int slots_for(int k) { return (k + 31) / 32; }
 
 }  // namespace
-
-cudaError_t knn_query(const MapView &m, const float4 *q, uint32_t nq, int k, float radius,
-                      uint32_t *idx, float *d2, cudaStream_t s) {
-    if (nq == 0) return cudaSuccess;
-    const float r2 = radius * radius;
-    const dim3 grid((nq + kWarpsPerBlock - 1) / kWarpsPerBlock), block(kWarpsPerBlock * 32);
-    switch (slots_for(k)) {
-        case 1: knn_kernel<1><<<grid, block, 0, s>>>(m, q, nq, k, r2, idx, d2); note_launch(); break;
-        case 2: knn_kernel<2><<<grid, block, 0, s>>>(m, q, nq, k, r2, idx, d2); note_launch(); break;
-        case 3: knn_kernel<3><<<grid, block, 0, s>>>(m, q, nq, k, r2, idx, d2); note_launch(); break;
-        default: knn_kernel<4><<<grid, block, 0, s>>>(m, q, nq, k, r2, idx, d2); note_launch(); break;
-    }
-    return cudaGetLastError();
-}
 
 cudaError_t render_batch(const BatchRenderScene *scenes, const uint32_t *chunk_prefix, int nscenes,
                          uint32_t *work, int sm_count, cudaStream_t s) {
@@ -352,42 +239,6 @@ cudaError_t render_frame(const PScene &S, const MapView &surf, const MapView &vo
         case 3: render_kernel<3><<<grid, block, 0, s>>>(S, surf, vol, R, rad, rgba); note_launch(); break;
         default: render_kernel<4><<<grid, block, 0, s>>>(S, surf, vol, R, rad, rgba); note_launch(); break;
     }
-    return cudaGetLastError();
-}
-
-cudaError_t cache_knn_values_runs(const PScene &S, const MapView &surf, const MapView &vol,
-                                  const float4 *qa, const float4 *qd, const uint32_t *sel,
-                                  const uint32_t *order, uint32_t n, int run, int k, float radius,
-                                  bool raw, float4 *val, uint32_t *run_ctr, int sm_count,
-                                  cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    const float r2 = radius * radius;
-    const uint32_t warps = (n + (uint32_t)run - 1) / (uint32_t)run;
-    dim3 grid((warps + kWarpsPerBlock - 1) / kWarpsPerBlock), block(kWarpsPerBlock * 32);
-    if (run_ctr) {
-        cudaError_t e = cudaMemsetAsync(run_ctr, 0, sizeof(uint32_t), s);
-        if (e != cudaSuccess) return e;
-    }
-#define PM_RUN_LAUNCH(SL)                                                                                   \
-    do {                                                                                                    \
-        if (run_ctr) {                                                                                      \
-            int per_sm = 1;                                                                                 \
-            cudaError_t eo = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, query_knn_run_kernel<SL>, \
-                                                                           kWarpsPerBlock * 32, 0);         \
-            if (eo != cudaSuccess) return eo;                                                               \
-            grid.x = std::min<uint32_t>(grid.x, (uint32_t)std::max(sm_count, 1) * (uint32_t)std::max(per_sm, 1)); \
-        }                                                                                                   \
-        query_knn_run_kernel<SL><<<grid, block, 0, s>>>(S, surf, vol, qa, qd, sel, order, n, run, k, r2, raw, val, \
-                                                        run_ctr);                                           \
-    } while (0)
-    switch (slots_for(k)) {
-        case 1: PM_RUN_LAUNCH(1); break;
-        case 2: PM_RUN_LAUNCH(2); break;
-        case 3: PM_RUN_LAUNCH(3); break;
-        default: PM_RUN_LAUNCH(4); break;
-    }
-#undef PM_RUN_LAUNCH
-    note_launch();
     return cudaGetLastError();
 }
 

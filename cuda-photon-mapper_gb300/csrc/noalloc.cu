@@ -178,7 +178,7 @@ extern "C" pm_status pm_knn_noalloc(const float4 *points, uint32_t n, const floa
             return PM_ERR_CUDA;
         }
     }
-    if (knn_query(m, queries, nq, k, radius, idx_out, d2_out, stream) != cudaSuccess) {
+    if (knn_query(m, 1, queries, nq, k, radius, idx_out, d2_out, stream) != cudaSuccess) {
         cudaGetLastError();
         return PM_ERR_CUDA;
     }

@@ -92,7 +92,7 @@ cudaError_t query_list_build(PhysicalState *st, bool force, cudaStream_t s);
 cudaError_t query_list_sort(PhysicalState *st, cudaStream_t s);
 void query_list_free(QueryList &ql);
 // Exact k-NN values of every query, raw (flux sum, squared radius or -1),
-// into ql.val: the list in spatial order, warm-started runs of queries.
+// into ql.val: the list in spatial order, shared candidate sets.
 cudaError_t knn_values_raw(PhysicalState *st, cudaStream_t s);
 constexpr int kGatherStats = 7;
 // Scratch of knn_values_tiles: defer[n], two defer_n words (deferred count,

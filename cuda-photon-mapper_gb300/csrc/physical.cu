@@ -285,7 +285,7 @@ pm_status pm_render(pm_ctx *ctx, float4 *radiance, uchar4 *rgba, cudaStream_t st
     DeviceGuard g(ctx->device);
     cudaError_t e;
     // The frame as its list of radiance queries (rebuilt on every call),
-    // estimated in spatial order by warm-started runs, then summed per pixel
+    // estimated in spatial order from shared candidate sets, then summed per pixel
     // in march order with the single-kernel render's arithmetic: the image
     // is bit-identical to render_frame's.
     PM_TRY(cudaEventRecord(st->ev[4], stream));
@@ -333,7 +333,7 @@ pm_status pm_knn(pm_ctx *ctx, int map, const float4 *queries, uint32_t nq, int k
     if (!st || !st->map[map].built) return fail(ctx, PM_ERR_STATE, "pm_knn before pm_build");
     DeviceGuard g(ctx->device);
     cudaError_t e;
-    PM_TRY(knn_query(view_of(st->map[map]), queries, nq, k, radius, idx_out, d2_out, stream));
+    PM_TRY(knn_query(view_of(st->map[map]), map, queries, nq, k, radius, idx_out, d2_out, stream));
     return PM_OK;
 }
 

@@ -1,5 +1,6 @@
 // tile_gather.cu -- k-NN radiance estimates of a query list in spatial
-// order, one candidate set per group of neighbouring queries.
+// order, one candidate set per group of neighbouring queries, and the k-NN
+// queries of points (pm_knn) by the same search.
 //
 // A warp takes chunks of 1, 2 or 4 consecutive groups of 32 queries of the
 // (map, Hilbert code) order. The k-th-neighbour distance d(x) (capped at the
@@ -58,8 +59,10 @@ constexpr int kTileWarps = 4;
 constexpr int kTileBlocks = 7;
 constexpr int kSlots = 10;
 constexpr int kTileCap = 32 * kSlots;        // candidate records per warp
+constexpr uint32_t kKnnLeft = 0xfffffffeu;   // mark of a query left to knn_rest_kernel (no record's index)
 constexpr float kRel = 2e-4f;                // relative and absolute margins of the distance bounds
 constexpr float kAbs = 1e-6f;
+constexpr float kOuter = 1.000001f;          // collected beyond a squared bound: above the bound's rounding
 
 // per-launch counters (pm_get_gather_stats)
 enum TileStat { kStTiled, kStList, kStShrunk, kStViolations, kStGroups, kStCandidates, kStHalvings, kStCount };
@@ -289,8 +292,8 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
 // addition per slot and one warp sum, the next threshold scales the last by
 // the density it found (r^3 in the medium, r^2 on surfaces), and the last one
 // or two candidates are stepped over one by one. Where the k-th distance
-// occurs more than once the photon index decides, and those left out get an
-// infinite distance. t: the first guess, at most capb (the squared gather
+// occurs more than once the photon index decides, and those left out get a
+// distance above all. t: the first guess, at most capb (the squared gather
 // radius), the search's upper end; on return the threshold, with *own the
 // candidates of this lane at or below it. Returns how many there are: k, or
 // all within the cap when fewer.
@@ -311,9 +314,9 @@ __device__ __forceinline__ int select_k(uint32_t (&d2)[kSlots], uint32_t &t, uin
         uint32_t nt = t;
         if (c < k && k - c <= 2) {
             for (int i = c; i < k; ++i) {
-                uint32_t v = 0x7f800000u;
+                uint32_t v = 0x7fffffffu;
 #pragma unroll
-                for (int s = 0; s < kSlots; ++s) v = min(v, d2[s] > nt ? d2[s] : 0x7f800000u);
+                for (int s = 0; s < kSlots; ++s) v = min(v, d2[s] > nt ? d2[s] : 0x7fffffffu);
                 nt = __reduce_min_sync(kFull, v);
             }
             nt = min(nt, capb);
@@ -342,7 +345,7 @@ __device__ __forceinline__ int select_k(uint32_t (&d2)[kSlots], uint32_t &t, uin
         id[s] = 0xffffffffu;
         if (d2[s] == t) {
             id[s] = __float_as_uint(__ldg(&m.pos[scratch().cat[cat_at(kSlots * lane + s)]]).w);
-            d2[s] = 0x7f800000u;
+            d2[s] = 0xffffffffu;
         }
         less += d2[s] < t ? 1 : 0;
     }
@@ -366,30 +369,29 @@ __device__ __forceinline__ int select_k(uint32_t (&d2)[kSlots], uint32_t &t, uin
     return k;
 }
 
-// The queries of `mask` (one map, lane order = spatial order; this lane's at
-// x, bounded by ub) from one shared candidate set. Returns false when the
-// set does not fit; otherwise sets d_lane to the capped k-th distance of the
-// lane's query (-1 if it was deferred).
-template <int S>
-__device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask, float *d_lane) {
-    TileScratch &ts = scratch();
-    const int lane = threadIdx.x & 31;
-    const int k = targs().k;
-    const MapView &m = targs().map[mid];
-    const bool member = (mask >> lane) & 1u;
+// The candidate set of the queries of `mask` (this lane's at x, bounded by
+// ub): every record within their largest bound of their box. Returns its
+// size, -1 when it does not fit.
+__device__ __forceinline__ int collect_for(v3 x, float ub, int mid, unsigned mask) {
+    const bool member = (mask >> (threadIdx.x & 31)) & 1u;
     const float inf = __int_as_float(0x7f800000);
     const v3 lo = mk3(warp_min(member ? x.x : inf), warp_min(member ? x.y : inf), warp_min(member ? x.z : inf));
     const v3 hi = mk3(warp_max(member ? x.x : -inf), warp_max(member ? x.y : -inf), warp_max(member ? x.z : -inf));
     const float rho = warp_max(member ? ub : 0.0f);
-    const int n = collect(mid, lo, hi, rho * rho);
-    if (n < 0) return false;
-    count(kStGroups);
-    count(kStCandidates, (unsigned long long)n);
-    // the candidates, kSlots consecutive ones (neighbours in the tree) to a lane
-    float px[kSlots], py[kSlots], pz[kSlots];
+    return collect(mid, lo, hi, rho * rho * kOuter);
+}
+
+// The positions of the n candidates in cat, kSlots consecutive ones
+// (neighbours in the tree) to a lane; empty slots hold NaN, whose distance is
+// above every other.
+__device__ __forceinline__ void load_candidates(const MapView &m, int n, float (&px)[kSlots], float (&py)[kSlots],
+                                                float (&pz)[kSlots]) {
+    const TileScratch &ts = scratch();
+    const int lane = threadIdx.x & 31;
+    const float none = __int_as_float(0x7fffffff);
 #pragma unroll
     for (int s = 0; s < kSlots; ++s) {
-        px[s] = py[s] = pz[s] = inf;
+        px[s] = py[s] = pz[s] = none;
         if (kSlots * lane + s < n) {
             const float4 p = __ldg(&m.pos[ts.cat[cat_at(kSlots * lane + s)]]);
             px[s] = p.x;
@@ -397,6 +399,22 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
             pz[s] = p.z;
         }
     }
+}
+
+// The queries of `mask` (one map, lane order = spatial order) from the n
+// candidates in cat, which hold every record within each query's bound.
+// Sets d_lane to the capped k-th distance of the lane's query (-1 if it was
+// deferred).
+template <int S>
+__device__ __noinline__ void tile_queries(int mid, int n, unsigned mask, float *d_lane) {
+    TileScratch &ts = scratch();
+    const int lane = threadIdx.x & 31;
+    const int k = targs().k;
+    const MapView &m = targs().map[mid];
+    count(kStGroups);
+    count(kStCandidates, (unsigned long long)n);
+    float px[kSlots], py[kSlots], pz[kSlots];
+    load_candidates(m, n, px, py, pz);
     const float r2cap = targs().r2cap, rcap = targs().rcap;
     const uint32_t capb = __float_as_uint(r2cap);
     const float expo = mid == 0 ? 1.0f : 0.6666667f;
@@ -464,16 +482,16 @@ __device__ __noinline__ bool tile_queries(v3 x, float ub, int mid, unsigned mask
         if (lane == j) *d_lane = found == k ? sqrtf(kd2) : rcap;
         count(kStTiled);
     }
-    return true;
 }
 
 // A radius around query j of the group that at least k and at most kTileCap
 // records of map `mid` lie within (or the gather radius, when fewer do), at
-// most `hi`; -1 when none turns up. The first radius is that of k records at
-// the density of the leaf nearest to the query (volume for the medium, area
-// for surfaces); it then grows by the density found and, between a radius
+// most `hi`; -1 when none turns up. The records are then in cat, *count of
+// them. The first radius is that of k records at
+// the density of the leaf nearest to the query (by volume, by area where the
+// leaf is flat); it then grows by the density found and, between a radius
 // that overflows and one with too few, is bisected in r^3.
-__device__ __noinline__ float single_bound(int mid, int j, float hi) {
+__device__ __noinline__ float single_bound(int mid, int j, float hi, int *count) {
     const int k = targs().k, lane = threadIdx.x & 31;
     const MapView &m = targs().map[mid];
     const float4 q = scratch().qx[j];
@@ -496,21 +514,23 @@ __device__ __noinline__ float single_bound(int mid, int j, float hi) {
     const float4 bl = __ldg(&m.lo[node]), bh = __ldg(&m.hi[node]);
     const float ex = bh.x - bl.x, ey = bh.y - bl.y, ez = bh.z - bl.z;
     const float f = (float)k / (float)(32 << m.leaf_shift);
-    const float area = fmaxf(ex * ey, fmaxf(ey * ez, ez * ex));
-    float r = mid == 0 ? approx_sqrt(f * area * 0.31830989f) : cbrtf(f * ex * ey * ez * 0.23873241f);
-    r = 1.1f * r + approx_sqrt(dist);
+    const float c = fminf(ex, fminf(ey, ez)), a = fmaxf(ex, fmaxf(ey, ez)), b = ex + ey + ez - a - c;
+    float r = c > 0.25f * b ? cbrtf(f * a * b * c * 0.23873241f) : approx_sqrt(f * a * b * 0.31830989f);
+    if (!(r > 0.0f)) r = 0.5f * f * a;  // records on a line
+    r = 1.18f * r + approx_sqrt(dist);
     hi = fminf(hi, rcap);
     r = r > 0.0f ? fminf(r, hi) : hi;  // and NaN
     float lo = 0.0f;
     bool over = false;
     for (int it = 0; it < 32; ++it) {
-        const int n = collect(mid, x, x, r * r);
+        const int n = collect(mid, x, x, r * r * kOuter);
         if (n < 0) {
             hi = r;
             over = true;
         } else if (n < k && r < rcap) {
             lo = r;
         } else {
+            *count = n;
             return r;
         }
         if (over) r = lo > 0.0f ? cbrtf(0.5f * (lo * lo * lo + hi * hi * hi)) : 0.75f * hi;
@@ -537,14 +557,16 @@ __device__ __forceinline__ float bound_by(const float4 *known, int n, v3 x, floa
 // Query j of the group by itself, its bound found first (below ub); false:
 // to be deferred.
 template <int S>
-__device__ __noinline__ bool alone(v3 x, float ub, int mid, int j, float *d_lane) {
-    const float r = single_bound(mid, j, __shfl_sync(kFull, ub, j));
+__device__ __forceinline__ bool alone(float ub, int mid, int j, float *d_lane) {
+    int n = 0;
+    const float r = single_bound(mid, j, __shfl_sync(kFull, ub, j), &n);
     if (!(r >= 0.0f)) return false;
-    const float u = fminf(r * (1.0f + kRel) + kAbs, targs().rcap);
     __syncwarp();
-    if ((threadIdx.x & 31) == j) scratch().qx[j].w = u;
+    // the bound of the set just collected: all records within r are in it
+    if ((threadIdx.x & 31) == j) scratch().qx[j].w = r < targs().rcap ? r * (1.0f + kRel) : targs().rcap;
     __syncwarp();
-    return tile_queries<S>(x, u, mid, 1u << j, d_lane);
+    tile_queries<S>(mid, n, 1u << j, d_lane);
+    return true;
 }
 
 // The records expected in the candidate set of the queries of `mask`: the
@@ -619,7 +641,7 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
             if (nknown == 0) {
                 // nothing bounds the group yet: its middle query by itself first
                 const int j = __fns(members, 0, (__popc(members) + 1) >> 1);
-                if (alone<S>(q.x, ub, gkind, j, &dnew)) {
+                if (alone<S>(ub, gkind, j, &dnew)) {
                     if (lane == j) ts.known[0] = make_float4(q.x.x, q.x.y, q.x.z, dnew);
                     __syncwarp();
                     nknown = 1;
@@ -641,20 +663,23 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
             while (rem) {
                 const unsigned seg = __popc(rem) <= sz ? rem : rem & ((1u << __fns(rem, 0, sz + 1)) - 1u);
                 const int j = __ffs(seg) - 1;
-                if (__popc(seg) > 1 && expected(q.x, ub, gkind, seg, mean) > (float)kTileCap) {
+                const bool big = expected(q.x, ub, gkind, seg, mean) > (float)kTileCap;
+                if (big && __popc(seg) > 1) {
                     sz = __popc(seg) >> 1;
                     continue;
                 }
-                bool done = tile_queries<S>(q.x, ub, gkind, seg, &dnew);
-                if (!done && __popc(seg) > 1) {
+                const int nc = big ? -1 : collect_for(q.x, ub, gkind, seg);
+                if (nc < 0 && __popc(seg) > 1) {
                     count(kStHalvings);
                     sz = __popc(seg) >> 1;
                     continue;
                 }
+                bool done = nc >= 0;
                 if (done) {
+                    tile_queries<S>(gkind, nc, seg, &dnew);
                     sz = min(2 * sz, 32);
                 } else {
-                    done = alone<S>(q.x, ub, gkind, j, &dnew);
+                    done = alone<S>(ub, gkind, j, &dnew);
                     if (done) count(kStShrunk);
                     else defer(q.out, seg);
                 }
@@ -705,6 +730,146 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     }
     __syncwarp();
     if (stats && lane < kStCount && ts.st[lane]) atomicAdd(&stats[lane], ts.st[lane]);
+}
+
+// k nearest records of query points, sorted by (squared distance, index);
+// one warp per query, each bounded and selected by itself as above. The
+// selected records are put in order by their ranks: every lane counts the
+// distances below its own, and where two are equal the indices decide. A
+// query without a radius that fits its set (more records at one distance
+// than the registers hold) is marked in its first index and left to
+// knn_rest_kernel. Bound by instruction issue and the walk's L2 latency.
+// Measured (GB300; the list search before): 262,144 queries, k = 100, 1M
+// points 3.62 -> 1.59 ms; 32,768 queries, k = 32, 100,000 points 225 -> 110 us.
+template <int S>
+__global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
+    knn_kernel(MapView m, int mid, const float4 *q, uint32_t nq, int k, float r2cap, uint32_t *idx_out,
+               float *d2_out) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t qi = blockIdx.x * kTileWarps + (threadIdx.x >> 5);
+    if (qi >= nq) return;
+    set_targs(m, m, nullptr, nullptr, nullptr, nullptr, 0u, r2cap, 0.0f, k, true);
+    TileScratch &ts = scratch();
+    const float4 p = q[qi];
+    if (lane == 0) ts.qx[0] = make_float4(p.x, p.y, p.z, targs().rcap);
+    __syncwarp();
+    uint32_t *idx = idx_out + (size_t)qi * k;
+    float *dist = d2_out + (size_t)qi * k;
+    int n = 0, found = 0;
+    if (m.n > 0) {
+        const float r = single_bound(mid, 0, targs().rcap, &n);
+        if (!(r >= 0.0f)) {
+            if (lane == 0) idx[0] = kKnnLeft;
+            return;
+        }
+        __syncwarp();
+        float px[kSlots], py[kSlots], pz[kSlots];
+        load_candidates(m, n, px, py, pz);
+        uint32_t d2[kSlots];
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+            const float dx = px[s] - p.x, dy = py[s] - p.y, dz = pz[s] - p.z;
+            d2[s] = __float_as_uint(dx * dx + dy * dy + dz * dz);
+        }
+        const uint32_t capb = __float_as_uint(r2cap);
+        const float expo = mid == 0 ? 1.0f : 0.6666667f;
+        uint32_t t = min(__float_as_uint(r * r * __powf(__fdividef((float)k, (float)max(n, k)), expo)), capb);
+        int own;
+        found = select_k(d2, t, capb, k, expo, m, &own);
+        int at = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, at, o);
+            if (lane >= o) at += v;
+        }
+        at -= own;
+        uint32_t *key = reinterpret_cast<uint32_t *>(ts.qd);  // 128 distances
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s)
+            if (d2[s] <= t) {
+                key[at] = d2[s];
+                ts.sel[at++] = ts.cat[cat_at(kSlots * lane + s)];
+            }
+        if (lane < 4 && found + lane < 128) key[found + lane] = 0xffffffffu;
+        __syncwarp();
+        uint32_t mine[S], id[S];
+        int rank[S];
+        uint32_t sum = 0;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const int e = lane + 32 * s;
+            mine[s] = e < found ? key[e] : 0u;
+            id[s] = e < found ? __float_as_uint(__ldg(&m.pos[ts.sel[e]]).w) : 0xffffffffu;
+            rank[s] = 0;
+        }
+        for (int f = 0; f < found; f += 4) {
+            const uint4 w = reinterpret_cast<const uint4 *>(key)[f >> 2];
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                rank[s] += (w.x < mine[s] ? 1 : 0) + (w.y < mine[s] ? 1 : 0) + (w.z < mine[s] ? 1 : 0) +
+                           (w.w < mine[s] ? 1 : 0);
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) sum += lane + 32 * s < found ? (uint32_t)rank[s] : 0u;
+        sum = __reduce_add_sync(kFull, sum);
+        __syncwarp();
+        if (sum != (uint32_t)(found * (found - 1) / 2)) {  // equal distances
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                if (lane + 32 * s < found) ts.sel[lane + 32 * s] = id[s];
+            __syncwarp();
+            for (int f = 0; f < found; ++f) {
+                const uint32_t w = key[f], o = ts.sel[f];
+#pragma unroll
+                for (int s = 0; s < S; ++s) rank[s] += w == mine[s] && o < id[s] ? 1 : 0;
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            if (lane + 32 * s < found) {
+                key[rank[s]] = mine[s];
+                ts.sel[rank[s]] = id[s];
+            }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int e = lane + 32 * s;
+        if (e < k) {
+            idx[e] = e < found ? ts.sel[e] : 0xffffffffu;
+            dist[e] = e < found ? __uint_as_float(reinterpret_cast<const uint32_t *>(ts.qd)[e]) : r2cap;
+        }
+    }
+}
+
+// The queries knn_kernel left, by the list search (grid-stride, 32 queries'
+// marks at a time).
+template <int S>
+__global__ void __launch_bounds__(128) knn_rest_kernel(MapView m, const float4 *q, uint32_t nq, int k, float r2cap,
+                                                       uint32_t *idx_out, float *d2_out) {
+    __shared__ WarpScratch ws[4];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint64_t cap = make_key(r2cap, 0xffffffffu);
+    for (uint64_t base = ((uint64_t)blockIdx.x * 4 + wib) * 32; base < nq; base += (uint64_t)gridDim.x * 128) {
+        const uint64_t mine = base + lane;
+        unsigned left = __ballot_sync(kFull, mine < nq && idx_out[mine * k] == kKnnLeft);
+        for (; left; left &= left - 1) {
+            const uint64_t qi = base + __ffs(left) - 1;
+            const float4 p = q[qi];
+            Knn<S> kn;
+            kn.reset(cap, k);
+            knn_search<S>(m, mk3(p.x, p.y, p.z), kn, ws[wib], lane, cap);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int j = lane * S + s;
+                if (j < k) {
+                    idx_out[qi * k + j] = (uint32_t)kn.key[s];
+                    d2_out[qi * k + j] = key_d2(kn.key[s]);
+                }
+            }
+        }
+    }
 }
 
 // The scene of global chunk c: the last descriptor whose chunk_begin <= c.
@@ -836,6 +1001,27 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
         default: PM_TILE_LAUNCH(4); break;
     }
 #undef PM_TILE_LAUNCH
+    note_launches(2);
+    return cudaGetLastError();
+}
+
+cudaError_t knn_query(const MapView &m, int map, const float4 *q, uint32_t nq, int k, float radius,
+                      uint32_t *idx, float *d2, cudaStream_t s) {
+    if (nq == 0) return cudaSuccess;
+    const float r2 = radius * radius;
+    const dim3 grid((nq + kTileWarps - 1) / kTileWarps), block(kTileWarps * 32);
+    const dim3 rest(std::min<uint32_t>((nq + 127) / 128, 1024));
+    const int smem = (int)(kTileWarps * sizeof(TileScratch));
+#define PM_KNN_LAUNCH(SL)                                                                 \
+    knn_kernel<SL><<<grid, block, smem, s>>>(m, map, q, nq, k, r2, idx, d2);              \
+    knn_rest_kernel<SL><<<rest, 128, 0, s>>>(m, q, nq, k, r2, idx, d2)
+    switch ((k + 31) / 32) {
+        case 1: PM_KNN_LAUNCH(1); break;
+        case 2: PM_KNN_LAUNCH(2); break;
+        case 3: PM_KNN_LAUNCH(3); break;
+        default: PM_KNN_LAUNCH(4); break;
+    }
+#undef PM_KNN_LAUNCH
     note_launches(2);
     return cudaGetLastError();
 }

@@ -442,7 +442,7 @@ PM_API pm_status pm_cache_get_queries(pm_ctx *ctx, float4 *qa, float4 *qd, uint3
  * record was found). PM_ERR_STATE after a pm_render, which reuses them. */
 PM_API pm_status pm_cache_get_values(pm_ctx *ctx, float4 *val, uint32_t cap, uint32_t *count);
 /* The k-NN targets of the next training frame, as pm_cache_train computes
- * them (spatially sorted, warm-started runs), without training: host copies
+ * them (in spatial order, shared candidate sets), without training: host copies
  * of train_samples targets and the query index of each (both nullable).
  * For checking the targets against per-query k-NN values. */
 PM_API pm_status pm_cache_debug_targets(pm_ctx *ctx, float4 *targets, uint32_t *query);
