@@ -942,8 +942,7 @@ pm_status pm_batch_create(pm_ctx *ctx, int n, const pm_scene *scenes, const pm_c
             j.total = w + (m == 0 ? W_TOTAL_S : W_TOTAL_V);
             j.extent = w + (m == 0 ? W_EXT_S : W_EXT_V);
         }
-        TraceParams P;
-        memset(&P, 0, sizeof(P));
+        TraceParams P = {};
         P.seed = c.seed;
         P.scene_id = c.scene_id;
         P.max_bounces = c.max_bounces;

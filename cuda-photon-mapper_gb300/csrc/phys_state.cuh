@@ -3,6 +3,7 @@
 #pragma once
 #include "gather.cuh"
 #include "pm.h"
+#include "trace.cuh"
 
 // The frame as a list of radiance queries (every volume march sample and
 // every diffuse hit of every eye path, as the render visits them; see
@@ -54,6 +55,10 @@ struct PhysicalState {
         int leaf_shift = 0;
         bool built = false;
     } map[2];
+    uint4 *near = nullptr;       // the tracer's sphere lists, for near_gen's scene (0: none yet)
+    pm::NearLists near_desc;
+    int near_g = 0;
+    uint64_t near_gen = 0;
     void *kd_scratch = nullptr;  // tree builds
     size_t kd_bytes = 0;
     unsigned long long *gctr = nullptr;

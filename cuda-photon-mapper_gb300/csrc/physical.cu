@@ -40,6 +40,7 @@ void free_state(PhysicalState *st) {
         cudaFree(m.lo); cudaFree(m.hi);
     }
     cudaFree(st->kd_scratch);
+    cudaFree(st->near);
     cudaFree(st->gctr);
     for (auto &e : st->ev)
         if (e) cudaEventDestroy(e);
@@ -67,6 +68,36 @@ cudaError_t kd_reserve(PhysicalState *st) {
     cudaError_t e = cudaMalloc(&st->kd_scratch, bytes);
     if (e == cudaSuccess) st->kd_bytes = bytes;
     return e;
+}
+
+// Room for the tracer's sphere lists of the installed scene.
+cudaError_t near_reserve(PhysicalState *st) {
+    const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
+    st->near_desc = NearLists();
+    st->near_gen = 0;
+    if (g > st->near_g) {
+        cudaFree(st->near);
+        st->near = nullptr;
+        st->near_g = 0;
+        cudaError_t e = cudaMalloc(&st->near, sizeof(uint4) * near_lists_words(g));
+        if (e != cudaSuccess) return e;
+        st->near_g = g;
+    }
+    return cudaSuccess;
+}
+
+// The sphere lists of the installed scene, built on the first emission after
+// it changed.
+cudaError_t near_update(PhysicalState *st, cudaStream_t s) {
+    if (st->near_gen == st->gen) return cudaSuccess;
+    const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
+    st->near_desc = NearLists();
+    if (g > 0) {
+        cudaError_t e = build_near_lists(st->dscene, g, st->near, &st->near_desc, s);
+        if (e != cudaSuccess) return e;
+    }
+    st->near_gen = st->gen;
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -132,6 +163,7 @@ pm_status pm_set_scene(pm_ctx *ctx, const pm_scene *scene, const pm_config *cfg)
         PM_TRY(dalloc(&mp.hi, tree_nodes(mp.cap)));
     }
     PM_TRY(kd_reserve(st));
+    PM_TRY(near_reserve(st));
     PM_TRY(dalloc(&st->gctr, 2));
     if (scene->het_res > 0) {
         const size_t nv = (size_t)scene->het_res * scene->het_res * scene->het_res;
@@ -167,6 +199,8 @@ pm_status pm_update_scene(pm_ctx *ctx, const pm_scene *scene) {
     }
     st->dscene = to_device_scene(*scene, st->het);
     st->gen = next_scene_gen();
+    cudaError_t en = near_reserve(st);
+    if (en != cudaSuccess) return check_cuda(ctx, en, "near_reserve");
     return PM_OK;
 }
 
@@ -179,8 +213,9 @@ pm_status pm_emit(pm_ctx *ctx, cudaStream_t stream) {
 #define PM_TRY(x) do { e = (x); if (e != cudaSuccess) return check_cuda(ctx, e, #x); } while (0)
     PM_TRY(cudaEventRecord(st->ev[0], stream));
     PM_TRY(cudaMemsetAsync(st->words, 0, 16 * sizeof(uint32_t), stream));
-    TraceParams P;
-    memset(&P, 0, sizeof(P));
+    PM_TRY(near_update(st, stream));
+    TraceParams P = {};
+    P.near = st->near_desc;
     P.seed = st->cfg.seed;
     P.scene_id = st->cfg.scene_id;
     P.max_bounces = st->mb;

@@ -7,6 +7,29 @@ namespace pm {
 // Bound on tentative collisions per path segment under delta tracking.
 constexpr uint32_t kMaxDeltaSteps = 4096;
 
+// The spheres a photon segment can meet, by where it starts and which way
+// it goes: a grid of g^3 cells over the scene box, kNearDirs direction bins
+// (the faces of a cube in 4 x 4 parts), and for each pair the list of spheres
+// that some ray from the cell in the bin reaches, by increasing least
+// distance. An entry is 16 bits: the sphere and the distance in units (down
+// to a whole one); kNearEnd closes a list, kNearMore one of more than
+// kNearList - 1 spheres.
+constexpr int kNearFace = 4, kNearDirs = 6 * kNearFace * kNearFace;
+constexpr int kNearList = 32;                 // entries, 64 bytes
+constexpr uint32_t kNearEnd = 0xff, kNearMore = 0xfe;
+struct NearLists {
+    const uint4 *list = nullptr;  // nullable: none, every sphere is tested
+    int g = 0;
+    float lo[3], inv[3];          // box corner, cells per unit length
+    float unit;
+};
+// Cells per axis for a scene of ns spheres whose larger map holds `target`
+// records (0: no lists), and the table's length.
+int near_lists_grid(int ns, uint32_t target);
+size_t near_lists_words(int g);
+// Builds the table of a scene into list and describes it.
+cudaError_t build_near_lists(const PScene &S, int g, uint4 *list, NearLists *out, cudaStream_t s);
+
 struct TraceParams {
     uint64_t seed;
     uint32_t scene_id;
@@ -30,6 +53,7 @@ struct TraceParams {
     // list[0 .. *list_n), instead of every id below the extents whose
     // counts are nonzero.
     const uint32_t *list, *list_n;
+    NearLists near;
 };
 
 // One persistent launch over the photon paths (counting or writing pass).
