@@ -40,7 +40,8 @@ constexpr int kTableGradShift = 44;
 struct CacheGrid {
     int levels;              // <= kCacheMaxLevels
     uint32_t log2_t;         // entries per level = 2^log2_t
-    int res[kCacheMaxLevels];
+    int res[kCacheMaxLevels];  // not decreasing
+    int dense;               // the first levels, those with (res + 1)^3 <= 2^log2_t
     float lo[3], inv_size[3];  // world box -> [0,1]^3
 };
 

@@ -94,6 +94,11 @@ void cache_grid_init(const pm_cache_config &cfg, CacheGrid *g) {
     g->log2_t = (uint32_t)cfg.log2_table;
     const double b = cfg.levels > 1 ? std::exp(std::log((double)cfg.max_res / cfg.base_res) / (cfg.levels - 1)) : 1.0;
     for (int l = 0; l < cfg.levels; ++l) g->res[l] = (int)std::floor(cfg.base_res * std::pow(b, l) + 1e-6);
+    while (g->dense < cfg.levels) {
+        const uint64_t n = (uint64_t)g->res[g->dense] + 1u;
+        if (n * n * n > (1ull << g->log2_t)) break;
+        ++g->dense;
+    }
     for (int a = 0; a < 3; ++a) {
         g->lo[a] = 0.0f;
         g->inv_size[a] = 1.0f;
