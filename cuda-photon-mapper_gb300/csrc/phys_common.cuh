@@ -90,22 +90,26 @@ __device__ __forceinline__ PHit intersect(const PScene &S, v3 o, v3 d, float tma
     return h;
 }
 
+// The plane's axis is the same for the whole warp: a branch, not selects.
+template <int A>
+__device__ __forceinline__ void plane_hit(const PScene &S, int i, v3 o, v3 d, PHit &h) {
+    constexpr int B = A == 0 ? 1 : 0, C = A == 2 ? 1 : 2;
+    const float da = vget(d, A);
+    const float t = (S.pl_off[i] - vget(o, A)) / da;
+    if (da != 0.0f && t > kRayEps && t < h.t) {
+        const float p1 = vget(o, B) + vget(d, B) * t, p2 = vget(o, C) + vget(d, C) * t;
+        if (p1 >= S.bmin[B] && p1 <= S.bmax[B] && p2 >= S.bmin[C] && p2 <= S.bmax[C]) {
+            h.t = t;
+            h.obj = -1 - i;
+        }
+    }
+}
 __device__ __forceinline__ void plane_hits(const PScene &S, v3 o, v3 d, PHit &h) {
     for (int i = 0; i < S.np; ++i) {
-        int a = S.pl_axis[i];
-        float da = vget(d, a);
-        if (da != 0.0f) {
-            float t = (S.pl_off[i] - vget(o, a)) / da;
-            if (t > kRayEps && t < h.t) {
-                v3 p = o + d * t;
-                int a1 = a == 0 ? 1 : 0, a2 = a == 2 ? 1 : 2;
-                float p1 = vget(p, a1), p2 = vget(p, a2);
-                if (p1 >= S.bmin[a1] && p1 <= S.bmax[a1] && p2 >= S.bmin[a2] && p2 <= S.bmax[a2]) {
-                    h.t = t;
-                    h.obj = -1 - i;
-                }
-            }
-        }
+        const int a = S.pl_axis[i];
+        if (a == 0) plane_hit<0>(S, i, o, d, h);
+        else if (a == 1) plane_hit<1>(S, i, o, d, h);
+        else plane_hit<2>(S, i, o, d, h);
     }
 }
 
@@ -272,20 +276,18 @@ PM_HD v3 sample_cosine(v3 n, float u1, float u2) {
     return normalize(from_local(n, r * c, r * s, sqrtf(fmaxf(0.0f, 1.0f - u1))));
 }
 
-// Henyey-Greenstein direction around the travel direction d.
-PM_HD v3 sample_hg(v3 d, float g, float u1, float u2) {
+// Cosine and sine to the travel direction of a Henyey-Greenstein event.
+PM_HD void hg_cosine(float g, float u, float *ct_out, float *st) {
     float ct;
     if (fabsf(g) < 1e-3f) {
-        ct = 1.0f - 2.0f * u1;
+        ct = 1.0f - 2.0f * u;
     } else {
-        float sq = (1.0f - g * g) / (1.0f - g + 2.0f * g * u1);
+        float sq = (1.0f - g * g) / (1.0f - g + 2.0f * g * u);
         ct = (1.0f + g * g - sq * sq) / (2.0f * g);
     }
     ct = fminf(1.0f, fmaxf(-1.0f, ct));
-    float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-    float s, c;
-    pm_sincos2pi(u2, &s, &c);
-    return normalize(from_local(d, st * c, st * s, ct));
+    *ct_out = ct;
+    *st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
 }
 
 // HG phase function value for the cosine between the photon's travel

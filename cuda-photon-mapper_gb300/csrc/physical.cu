@@ -70,7 +70,8 @@ cudaError_t kd_reserve(PhysicalState *st) {
     return e;
 }
 
-// Room for the tracer's sphere lists of the installed scene.
+// Room for the tracer's sphere lists of the installed scene; without it, no
+// lists.
 cudaError_t near_reserve(PhysicalState *st) {
     const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
     st->near_desc = NearLists();
@@ -80,6 +81,11 @@ cudaError_t near_reserve(PhysicalState *st) {
         st->near = nullptr;
         st->near_g = 0;
         cudaError_t e = cudaMalloc(&st->near, sizeof(uint4) * near_lists_words(g));
+        if (e == cudaErrorMemoryAllocation) {
+            st->near = nullptr;
+            cudaGetLastError();
+            return cudaSuccess;
+        }
         if (e != cudaSuccess) return e;
         st->near_g = g;
     }
@@ -92,7 +98,7 @@ cudaError_t near_update(PhysicalState *st, cudaStream_t s) {
     if (st->near_gen == st->gen) return cudaSuccess;
     const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
     st->near_desc = NearLists();
-    if (g > 0) {
+    if (g > 0 && g <= st->near_g) {
         cudaError_t e = build_near_lists(st->dscene, g, st->near, &st->near_desc, s);
         if (e != cudaSuccess) return e;
     }

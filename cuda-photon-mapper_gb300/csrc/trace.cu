@@ -117,9 +117,13 @@ __global__ void __launch_bounds__(256) near_list_kernel(const __grid_constant__ 
 // Equal distances keep the lower index, so the hit is intersect()'s. An origin
 // outside the box, and a list that does not hold all its spheres, test every
 // sphere. The lanes' rays differ, so a warp waits for its longest list: in the
-// 64-sphere preset a lane tests 4.7 of 13.6 listed spheres, a warp's longest
-// about 13, instead of 64.
-__device__ __forceinline__ PHit intersect_near(const PScene &S, const NearLists &N, v3 o, v3 d, float tmax) {
+// 64-sphere preset a lane tests 4 spheres, a warp's longest about 11, instead
+// of 64. An entry is one 16-bit load a test ahead of its use (entries shifted
+// out of registers, the distance as a float compared: 34.3 -> 33.3 ms for 8M
+// records); whoever has more to test keeps the warp (lanes left walking while
+// the others go on: 33.7).
+__device__ __forceinline__ PHit intersect_near(const PScene &S, const PScene &U, const NearLists &N, v3 o, v3 d,
+                                               float tmax) {
     PHit h;
     h.t = tmax;
     h.obj = kNone;
@@ -129,36 +133,27 @@ __device__ __forceinline__ PHit intersect_near(const PScene &S, const NearLists 
     if (!all) {
         const int g1 = N.g - 1;
         const int cx = min(max((int)f[0], 0), g1), cy = min(max((int)f[1], 0), g1), cz = min(max((int)f[2], 0), g1);
-        const uint4 *row = N.list + ((size_t)((cz * N.g + cy) * N.g + cx) * kNearDirs + near_bin(d)) * (kNearList / 8);
-        uint4 v = __ldg(row);
-        for (int i = 0;; ++i) {
-            const uint32_t e = v.x & 0xffffu, k = e & 255u;
-            if (k >= kNearMore) {
-                all = k == kNearMore;
-                break;
-            }
-            if (h.t <= (float)(e >> 8) * N.unit) break;
+        const uint16_t *at = reinterpret_cast<const uint16_t *>(N.list) +
+                             ((size_t)((cz * N.g + cy) * N.g + cx) * kNearDirs + near_bin(d)) * kNearList;
+        uint32_t e = __ldg(at), lim = 0xfe00u;  // entries from lim on are no nearer than the hit
+        while (e < lim) {
+            const uint32_t k = e & 255u;
+            e = __ldg(++at);
             const float t = sphere_t(S.sph[k], o, d);
             if (t > kRayEps && (t < h.t || (t == h.t && h.obj != kNone && (int)k < h.obj))) {
                 h.t = t;
                 h.obj = (int)k;
-            }
-            if ((i & 7) == 7) {
-                v = __ldg(row + ((i + 1) >> 3));
-            } else {
-                v.x = __funnelshift_r(v.x, v.y, 16);
-                v.y = __funnelshift_r(v.y, v.z, 16);
-                v.z = __funnelshift_r(v.z, v.w, 16);
-                v.w >>= 16;
+                lim = ((uint32_t)fminf(t * N.inv_unit, 252.0f) + 1u) << 8;
             }
         }
+        all = e == kNearMore;
     }
     if (all)
         for (int i = 0; i < S.ns; ++i) {
             const float t = sphere_t(S.sph[i], o, d);
             if (t > kRayEps && (t < h.t || (t == h.t && h.obj != kNone && i < h.obj))) { h.t = t; h.obj = i; }
         }
-    plane_hits(S, o, d, h);
+    plane_hits(U, o, d, h);
     return h;
 }
 
@@ -198,29 +193,40 @@ struct MapOut {
     float scale;
 };
 
-// One interaction of path p; returns false when the path ends.
+// One interaction of path p; returns false when the path ends. S is read at
+// each lane's own object, U (the same scene) at one place by the whole warp.
+//
+// The instructions issued bound it, and how few lanes share them (15 of 32 in
+// preset 3). So the lanes meet again after the hit and after the tracking,
+// whose loop the compiler leaves in groups (39.1 -> 35.5 ms for 8M records of
+// preset 3); a surface and the medium share the scattered direction's sine,
+// frame and record, all kinds the last normalisation (with the planes' axes
+// told apart by branches and read from the parameters 35.5 -> 34.3; preset 2,
+// 1M records: 1.73 -> 1.63).
 template <bool kNear>
-__device__ bool step_path(const PScene &S, const TraceParams &P, Path &p, const MapOut &ms,
-                          const MapOut &mv) {
+__device__ __forceinline__ bool step_path(const PScene &S, const PScene &U, const TraceParams &P, Path &p,
+                                          const MapOut &ms, const MapOut &mv) {
     p.ev += 1;
     pm_u32x4 r = philox(P.seed, p.id, (uint32_t)p.ev, 0u, P.scene_id);
     float u0 = pm_u01(r.v[0]), u1 = pm_u01(r.v[1]), u2 = pm_u01(r.v[2]), u3 = pm_u01(r.v[3]);
     // without lists a uniform loop over the spheres beats divergent walks
     // of a grid
-    PHit h = kNear ? intersect_near(S, P.near, p.o, p.d, 3.0e38f) : intersect(S, p.o, p.d, 3.0e38f);
-    float seg = h.obj != kNone ? h.t : box_exit(S, p.o, p.d);
+    const unsigned together = __activemask();
+    const PHit h = kNear ? intersect_near(S, U, P.near, p.o, p.d, 3.0e38f) : intersect(U, p.o, p.d, 3.0e38f);
+    float seg = h.obj != kNone ? h.t : box_exit(U, p.o, p.d);
+    __syncwarp(together);
     bool vol = false;
     v3 x = p.o;
     float ss = 0.0f, st = 1.0f;
-    if (S.sigma_max > 0.0f && !p.glass) {
-        if (S.het_res <= 0) {
-            st = S.sigma_s + S.sigma_a;
-            if (S.sigma_s > 0.0f) {
+    if (U.sigma_max > 0.0f && !p.glass) {
+        if (U.het_res <= 0) {
+            st = U.sigma_s + U.sigma_a;
+            if (U.sigma_s > 0.0f) {
                 float t = -pm_logf(1.0f - u0) / st;
                 if (t < seg) {
                     vol = true;
                     x = p.o + p.d * t;
-                    ss = S.sigma_s;
+                    ss = U.sigma_s;
                 }
             }
         } else {
@@ -232,12 +238,12 @@ __device__ bool step_path(const PScene &S, const TraceParams &P, Path &p, const 
             for (uint32_t j = 0; j < kMaxDeltaSteps; ++j) {
                 if ((j & 1u) == 0u) q = philox(P.seed, p.id, (uint32_t)p.ev, 1u + (j >> 1), P.scene_id);
                 const uint32_t ua = (j & 1u) ? q.v[2] : q.v[0], ub = (j & 1u) ? q.v[3] : q.v[1];
-                t += -pm_logf(1.0f - pm_u01(ua)) * S.inv_sigma_max;
+                t += -pm_logf(1.0f - pm_u01(ua)) * U.inv_sigma_max;
                 if (!(t < seg)) break;
                 v3 y = p.o + p.d * t;
-                float s = sigma_s_at(S, y);
-                float sty = s + S.sigma_a;
-                if (pm_u01(ub) * S.sigma_max < sty) {
+                float s = sigma_s_at(U, y);
+                float sty = s + U.sigma_a;
+                if (pm_u01(ub) * U.sigma_max < sty) {
                     vol = true;
                     x = y;
                     ss = s;
@@ -247,39 +253,48 @@ __device__ bool step_path(const PScene &S, const TraceParams &P, Path &p, const 
             }
         }
     }
-    if (vol) {
-        if (P.store) {
-            uint32_t j = p.ov + p.nv;
-            if (j < mv.n) store(P.vpos, P.vpow, j, x, p.thr, p.d, mv.scale);
-        }
-        p.nv += 1;
-        if (!(u1 < P.rr)) return false;
-        float f = (ss / st) / P.rr;
-        p.thr = p.thr * f;
-        p.d = sample_hg(p.d, S.g, u2, u3);
-        p.o = x;
-        return p.ev < P.max_bounces;
+    __syncwarp(together);
+    v3 n = mk3(0.0f, 0.0f, 0.0f);
+    float dn = 0.0f;
+    int kind = PM_MAT_DIFFUSE;
+    if (!vol) {
+        if (h.obj == kNone) return false;  // leaves through the open side
+        x = p.o + p.d * h.t;
+        n = outward_normal(S, h.obj, x);
+        kind = material_kind(S, h.obj);
+        dn = dot(n, p.d);
     }
-    if (h.obj == kNone) return false;  // leaves through the open side
-    v3 hp = p.o + p.d * h.t;
-    v3 n = outward_normal(S, h.obj, hp);
-    int kind = material_kind(S, h.obj);
-    float dn = dot(n, p.d);
-    v3 nf = dn < 0.0f ? n : n * -1.0f;
-    if (kind == PM_MAT_DIFFUSE) {
+    v3 v;  // the new direction, not normalised
+    if (kind == PM_MAT_DIFFUSE) {  // or in the medium
         if (P.store) {
-            uint32_t j = p.os + p.ns;
-            if (j < ms.n) store(P.spos, P.spow, j, hp, p.thr, p.d, ms.scale);
+            const uint32_t j = vol ? p.ov + p.nv : p.os + p.ns;
+            if (j < (vol ? mv.n : ms.n))
+                store(vol ? P.vpos : P.spos, vol ? P.vpow : P.spow, j, x, p.thr, p.d, vol ? mv.scale : ms.scale);
         }
-        p.ns += 1;
+        p.nv += vol ? 1 : 0;
+        p.ns += vol ? 0 : 1;
         if (!(u1 < P.rr)) return false;
-        v3 a = material_albedo(S, h.obj);
-        p.thr = mk3(p.thr.x * a.x / P.rr, p.thr.y * a.y / P.rr, p.thr.z * a.z / P.rr);
-        p.d = sample_cosine(nf, u2, u3);
-        p.o = hp + nf * kOffset;
+        float r, z;
+        v3 axis;
+        if (vol) {
+            p.thr = p.thr * ((ss / st) / P.rr);
+            hg_cosine(S.g, u2, &z, &r);
+            axis = p.d;
+            p.o = x;
+        } else {
+            const v3 a = material_albedo(S, h.obj);
+            p.thr = mk3(p.thr.x * a.x / P.rr, p.thr.y * a.y / P.rr, p.thr.z * a.z / P.rr);
+            axis = dn < 0.0f ? n : n * -1.0f;
+            r = sqrtf(u2);
+            z = sqrtf(fmaxf(0.0f, 1.0f - u2));
+            p.o = x + axis * kOffset;
+        }
+        float sn, cs;
+        pm_sincos2pi(u3, &sn, &cs);
+        v = from_local(axis, r * cs, r * sn, z);
     } else if (kind == PM_MAT_MIRROR) {
-        p.d = normalize(p.d - n * (2.0f * dn));
-        p.o = hp + nf * kOffset;
+        v = p.d - n * (2.0f * dn);
+        p.o = x + (dn < 0.0f ? n : n * -1.0f) * kOffset;
     } else {
         float ci = -dn;
         bool entering = ci > 0.0f;
@@ -290,14 +305,15 @@ __device__ bool step_path(const PScene &S, const TraceParams &P, Path &p, const 
         float ct;
         float F = fresnel(ci, eta, &ct);
         if (u1 < F) {
-            p.d = normalize(p.d + nn * (2.0f * ci));
-            p.o = hp + nn * kOffset;
+            v = p.d + nn * (2.0f * ci);
+            p.o = x + nn * kOffset;
         } else {
-            p.d = normalize(p.d * eta + nn * (eta * ci - ct));
-            p.o = hp - nn * kOffset;
+            v = p.d * eta + nn * (eta * ci - ct);
+            p.o = x - nn * kOffset;
             p.glass = entering;
         }
     }
+    p.d = normalize(v);
     return p.ev < P.max_bounces;
 }
 
@@ -318,7 +334,7 @@ constexpr uint32_t kIdBlock = 32;
 // The persistent per-warp loop of one scene: keep 32 live paths, refill
 // empty lanes from the warp's pool of path ids until no ids are left.
 template <bool kNear>
-__device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P) {
+__device__ __forceinline__ void trace_loop(const PScene &S, const PScene &U, const TraceParams &P) {
     const int lane = threadIdx.x & 31;
     MapOut ms = {0u, 0u, 0.0f}, mv = {0u, 0u, 0.0f};
     uint32_t cap = P.path_cap;
@@ -398,7 +414,7 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
             continue;
         }
         if (live) {
-            if (!step_path<kNear>(S, P, p, ms, mv)) {
+            if (!step_path<kNear>(S, U, P, p, ms, mv)) {
                 if (!P.store) {
                     uint32_t ns = min(p.ns, (uint32_t)P.max_bounces);
                     uint32_t nv = min(p.nv, (uint32_t)P.max_bounces);
@@ -413,25 +429,29 @@ __device__ __forceinline__ void trace_loop(const PScene &S, const TraceParams &P
     }
 }
 
-// The scene is read from shared memory: the lanes' materials and normals
-// sit at different objects, which the constant bank serves one at a time
-// (preset 3, 87.6M paths: 57.8 -> 56.1 ms). 8 blocks per SM: 64 registers.
+// What the lanes read at their own objects (materials, normals, listed
+// spheres) is read from shared memory: the constant bank serves one address at
+// a time (preset 3, 87.6M paths: 57.8 -> 56.1 ms). Blocks per SM: the lists'
+// loads want the ninth (56 registers; 32.3 -> 31.5 ms), small scenes have no
+// use for it (0.37 / 0.38 ms in preset 1: more paths beyond the last needed).
+constexpr int trace_blocks(bool near) { return near ? 9 : 8; }
 template <bool kNear>
-__global__ void __launch_bounds__(128, 8) trace_kernel(const __grid_constant__ PScene S,
-                                                       const __grid_constant__ TraceParams P) {
+__global__ void __launch_bounds__(128, trace_blocks(kNear)) trace_kernel(const __grid_constant__ PScene S,
+                                                                          const __grid_constant__ TraceParams P) {
     __shared__ PScene sS;
     const uint32_t *a = reinterpret_cast<const uint32_t *>(&S);
     uint32_t *b = reinterpret_cast<uint32_t *>(&sS);
     for (int i = threadIdx.x; i < (int)(offsetof(PScene, cell_mask) / 4); i += blockDim.x) b[i] = a[i];
     __syncthreads();
-    trace_loop<kNear>(sS, P);
+    trace_loop<kNear>(sS, S, P);
 }
 
 // Many scenes in one persistent launch: every block walks the scene list
 // (starting at a different scene per block, so scenes are worked on side
 // by side), stages the scene in shared memory and traces its paths with
-// the single-scene loop until the scene's path ids run out.
-__global__ void __launch_bounds__(128) trace_batch_kernel(const PScene *scenes,
+// the single-scene loop until the scene's path ids run out. 64 registers for
+// 8 blocks an SM, as the grid has (72: six scenes' frame 48.5 ms, 64: 48.0).
+__global__ void __launch_bounds__(128, 8) trace_batch_kernel(const PScene *scenes,
                                                           const TraceParams *params, int n) {
     __shared__ PScene sS;
     __shared__ TraceParams sP;
@@ -445,7 +465,7 @@ __global__ void __launch_bounds__(128) trace_batch_kernel(const PScene *scenes,
         uint32_t *d = reinterpret_cast<uint32_t *>(&sP);
         for (int i = threadIdx.x; i < (int)(sizeof(TraceParams) / 4); i += blockDim.x) d[i] = c[i];
         __syncthreads();
-        trace_loop<false>(sS, sP);
+        trace_loop<false>(sS, sS, sP);
     }
 }
 
@@ -563,13 +583,18 @@ cudaError_t needed_paths(uint32_t issued, const uint32_t *cnt_s, const uint32_t 
 size_t near_lists_words(int g) { return (size_t)g * g * g * kNearDirs * (kNearList / 8); }
 
 int near_lists_grid(int ns, uint32_t target) {
-    // emission (ms) without and with the lists: 16 spheres, 1M records 3.69 /
-    // 3.71; 32 spheres 4.77 / 4.43; 48 spheres 5.63 / 4.72, 100,000 records
-    // 0.98 / 0.82; 64 spheres 7.9 / 5.8, 8M records 56.1 / 42.3 (24 cells an
-    // axis: 40.0, 12: 45.4, 8: 54.1); against 0.35 ms for a table of 16^3 cells
-    // and 1.65 ms for one of 24^3, built when the scene has changed
-    if (ns < 32 || target < (ns < 48 ? 2000000u : 500000u)) return 0;
-    return ns >= 48 && target >= 4000000u ? 24 : 16;
+    // What the lists save grows with the spheres beyond about a dozen and with
+    // the records; the table costs 0.3 (12 cells an axis), 0.7 (16) or 1.5 ms
+    // (20) when the scene has changed, and every emission of 14M units or more
+    // wins that back. Emission (ms) without the lists / with them and the table's
+    // building / with a table kept, at 12 cells: 48 spheres, 300,000 records 1.99
+    // / 1.95 / 1.65; 32, 500,000 2.44 / 2.49 / 2.22 and 1M 4.35 / 4.16 / 3.91;
+    // 24, 1M 3.94 / 3.99 / 3.74; 16, 2M 5.94 / 6.04 / 5.79 and 4M 11.43 / 11.32 /
+    // 11.08. 64 spheres: 1M 7.00, 5.21 / 4.85 at 12, 5.32 / 4.54 at 16, 5.90 /
+    // 4.39 at 20; 8M 51.0, 33.4 / 32.6 at 16, 33.0 / 31.5 at 20, 33.5 / 30.9 at 24.
+    const uint64_t units = ns > 12 ? (uint64_t)(ns - 12) * target : 0;
+    if (units < 14000000ull) return 0;
+    return units < 40000000ull ? 12 : (units < 160000000ull ? 16 : 20);
 }
 
 cudaError_t build_near_lists(const PScene &S, int g, uint4 *list, NearLists *out, cudaStream_t s) {
@@ -584,6 +609,7 @@ cudaError_t build_near_lists(const PScene &S, int g, uint4 *list, NearLists *out
         diag += ext * ext;
     }
     N.unit = sqrtf(diag) / 250.0f;
+    N.inv_unit = 1.00001f / N.unit;
     *out = N;
     const uint32_t lists = (uint32_t)g * g * g * kNearDirs;
     near_list_kernel<<<(lists + 7) / 8, 256, 0, s>>>(S, N, lists, reinterpret_cast<uint16_t *>(list)); note_launch();
@@ -591,9 +617,8 @@ cudaError_t build_near_lists(const PScene &S, int g, uint4 *list, NearLists *out
 }
 
 cudaError_t trace_photons(const PScene &S, const TraceParams &P, int sm_count, cudaStream_t s) {
-    // 4 warps per CTA, enough CTAs to fill every SM several times over.
-    if (P.near.list) trace_kernel<true><<<sm_count * 8, 128, 0, s>>>(S, P);
-    else trace_kernel<false><<<sm_count * 8, 128, 0, s>>>(S, P);
+    if (P.near.list) trace_kernel<true><<<sm_count * trace_blocks(true), 128, 0, s>>>(S, P);
+    else trace_kernel<false><<<sm_count * trace_blocks(false), 128, 0, s>>>(S, P);
     note_launch();
     return cudaGetLastError();
 }

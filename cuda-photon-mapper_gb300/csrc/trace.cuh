@@ -9,19 +9,19 @@ constexpr uint32_t kMaxDeltaSteps = 4096;
 
 // The spheres a photon segment can meet, by where it starts and which way
 // it goes: a grid of g^3 cells over the scene box, kNearDirs direction bins
-// (the faces of a cube in 4 x 4 parts), and for each pair the list of spheres
+// (the faces of a cube in 5 x 5 parts), and for each pair the list of spheres
 // that some ray from the cell in the bin reaches, by increasing least
 // distance. An entry is 16 bits: the sphere and the distance in units (down
 // to a whole one); kNearEnd closes a list, kNearMore one of more than
 // kNearList - 1 spheres.
-constexpr int kNearFace = 4, kNearDirs = 6 * kNearFace * kNearFace;
+constexpr int kNearFace = 5, kNearDirs = 6 * kNearFace * kNearFace;
 constexpr int kNearList = 32;                 // entries, 64 bytes
-constexpr uint32_t kNearEnd = 0xff, kNearMore = 0xfe;
+constexpr uint32_t kNearEnd = 0xffff, kNearMore = 0xfffe;  // above every entry
 struct NearLists {
     const uint4 *list = nullptr;  // nullable: none, every sphere is tested
     int g = 0;
     float lo[3], inv[3];          // box corner, cells per unit length
-    float unit;
+    float unit, inv_unit;         // of least distance; its inverse a little enlarged
 };
 // Cells per axis for a scene of ns spheres whose larger map holds `target`
 // records (0: no lists), and the table's length.

@@ -11,7 +11,7 @@ import oracle  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
-TARGET = 500000  # the smallest map for which the lists are built
+TARGET = 500000  # enough for the lists at 48 spheres and more
 
 
 @pytest.mark.parametrize("spheres,radii,light", [
