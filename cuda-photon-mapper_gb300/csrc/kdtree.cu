@@ -15,23 +15,24 @@
 // deterministic. It does not affect a query's result: the boxes that are
 // tested are the exact bounds of each node's records.
 //
-// Nodes of more than kSubMax records ("split levels") take three launches
-// per level over tiles of kTile records: bins and histogram, per-tile
-// counts, partition (which also collects the children's boxes). A node of
-// at most kSubMax records is finished by one CTA in shared memory: the
-// remaining levels, the records and directions in tree order and the boxes
-// of all its nodes; the last CTA of a map to finish combines the boxes of
-// the nodes above.
+// Nodes of more than 32,768 records take three launches per level over tiles
+// of kTile records: bins and histogram, per-tile counts, partition (which
+// also collects the children's boxes). Smaller nodes are split by a cluster
+// of 8 CTAs in its shared memory, down to nodes of at most kSubMax records,
+// and each of those is finished by one CTA: the remaining levels, the
+// records and directions in tree order and the boxes of all its nodes; the
+// last CTA of a map to finish combines the boxes of the nodes above.
 //
 // Against sorting every level (two 8-bit radix passes over 12-byte pairs
 // and a key pass), a level moves each record once, 16 B read and written,
 // and its 2-byte bin three times. Measured (GB300, both maps): 2 x 8M records
-// 15.8 -> 3.4 ms, 2 x 100,000 records 1.65 -> 0.15 ms, one map of 20,011
-// 0.47 -> 0.11 ms.
+// 15.8 -> 3.3 ms, 2 x 1M 2.75 -> 0.39 ms, 2 x 100,000 1.46 -> 0.10 ms, one map
+// of 20,011 0.44 -> 0.065 ms.
 #include "launch_count.cuh"
 #include "kdtree.cuh"
 
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cstring>
 
 namespace pm {
@@ -51,6 +52,10 @@ constexpr int kTileItems = (int)(kTile / kTileThreads);
 
 // Subtrees.
 constexpr int kSubMax = 2048;
+// Split levels of a cluster of 8 CTAs, a tile of records each.
+constexpr int kMidLevels = 4;
+constexpr int kMidCtas = (kSubMax << kMidLevels) / (int)kTile;
+static_assert(kMidCtas == 8, "the portable cluster size");
 constexpr int kSubThreads = 512;
 constexpr int kSubWarps = kSubThreads / 32;
 constexpr int kSubItems = kSubMax / kSubThreads;
@@ -64,6 +69,7 @@ struct Maps2 {
     KdMap m[2];
     int n;
     __device__ __forceinline__ const KdMap &of_tile(uint32_t t) const { return m[n > 1 && t >= m[1].tile0 ? 1 : 0]; }
+    __device__ __forceinline__ const KdMap &of_mid(uint32_t c) const { return m[n > 1 && c >= m[1].mid0 ? 1 : 0]; }
     __device__ __forceinline__ const KdMap &of_sub(uint32_t b) const { return m[n > 1 && b >= m[1].sub0 ? 1 : 0]; }
 };
 // Any number of maps in device memory.
@@ -72,6 +78,14 @@ struct MapsN {
     const uint32_t *tile_map, *sub_first;
     int n;
     __device__ __forceinline__ const KdMap &of_tile(uint32_t t) const { return m[tile_map[t]]; }
+    __device__ __forceinline__ const KdMap &of_mid(uint32_t c) const {
+        int lo = 0, hi = n - 1;  // the last map whose first cluster <= c
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (m[mid].mid0 <= c) lo = mid; else hi = mid - 1;
+        }
+        return m[lo];
+    }
     __device__ __forceinline__ const KdMap &of_sub(uint32_t b) const {
         int lo = 0, hi = n - 1;  // the last map whose first subtree <= b
         while (lo < hi) {
@@ -253,7 +267,7 @@ __global__ void __launch_bounds__(kTileThreads)
     const TileNode n = tile_node(m, blockIdx.x, level);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint4 sp = thr[n.node];
-    const bool boxes = level + 1 < m.lf;
+    const bool boxes = level + 1 < m.lf;  // split again, by launches or a cluster
     if (threadIdx.x < 12) bb[threadIdx.x] = 0u;
     // the node's earlier tiles
     uint32_t pl = 0, pe = 0;
@@ -341,6 +355,203 @@ __global__ void __launch_bounds__(kTileThreads)
         const uint32_t j = n.node - m.node0, side = threadIdx.x / 6, a = threadIdx.x % 6;
         atomicMax(&box[8 * (size_t)(m.node0 + 2 * j + side) + a], bb[threadIdx.x]);
     }
+}
+
+struct MidScratch {
+    float4 p[kTile];
+    uint32_t hist[kBins];
+    uint32_t box[2][6];  // a node's first CTA: its box, by the level's parity
+    uint32_t bb[12];
+    uint32_t wsum[kTileWarps], wcnt[kTileWarps], pre[kTileWarps];
+    uint4 split;
+};
+
+extern __shared__ __align__(16) unsigned char mid_smem[];
+
+// The split levels from a node of at most 32,768 records down to subtrees,
+// by a cluster of 8 CTAs that hold a tile each: the same bins, medians and
+// stable partition as the launches above (and so the same layout), with two
+// cluster barriers a level in place of three launches. A CTA reads the
+// node's other histograms in their shared memory and writes its records to
+// their place there. Bound by latency: four levels of a small map in 24 us
+// (launches: 19.5 us a level), of 2 x 8M records in 0.58 ms (0.82). Two CTAs
+// an SM against one: 2 x 8M built in 3.30 / 3.64 ms, small maps the same;
+// clusters of 16 CTAs and five levels: 100,000 records 5 us faster, 8M 0.3 ms
+// slower.
+template <class Maps>
+__global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads, 2)
+    kd_mid_kernel(const __grid_constant__ Maps maps, const uint32_t *box) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    MidScratch &ms = *reinterpret_cast<MidScratch *>(mid_smem);
+    constexpr int kPer = kTileItems;          // records per lane
+    constexpr int kBinPer = kBins / kTileThreads;
+    const uint32_t id = blockIdx.x / kMidCtas;
+    const KdMap &m = maps.of_mid(id);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int q = (int)cluster.block_rank();
+    const uint32_t c = id - m.mid0;
+    const int levels = m.lf - m.ls;
+    const uint32_t span0 = (uint32_t)kSubMax << levels;
+    const uint32_t first = c * span0;          // the cluster's first record
+    const uint32_t start = first + (uint32_t)q * kTile;
+    const int cnt = q * (int)kTile < (int)span0 && start < m.n ? (int)min(kTile, m.n - start) : 0;
+    const int wfirst = warp * 32 * kPer;
+    float4 p[kPer];
+    {
+        const float4 *src = level_src(m, m.ls) + start;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+            if (wfirst + 32 * i + lane < cnt) p[i] = src[wfirst + 32 * i + lane];
+    }
+    if (threadIdx.x < 12) (&ms.box[0][0])[threadIdx.x] = 0u;
+    // zeroed before another CTA's records reach them: its first barrier
+    for (int l = 0; l < levels; ++l) {
+        const int span = (int)(span0 >> l), ctas = span / (int)kTile;
+        const int f = q / ctas * ctas;          // the node's first CTA
+        const uint32_t nstart = first + (uint32_t)f * kTile;
+        const uint32_t ncnt = nstart < m.n ? min((uint32_t)span, m.n - nstart) : 0u;
+        const uint32_t half = min((uint32_t)span >> 1, ncnt);
+        const bool boxes = l + 1 < levels;
+        Cut cut;
+        if (l > 0) cut = cut_of_words(cluster.map_shared_rank(&ms.box[l & 1][0], f), (float)kBins);
+        else if (m.ls == 0 && !m.root_boxed) cut = cut_of(m.root_lo, m.root_hi, (float)kBins);
+        else cut = cut_of_words(box + 8 * (size_t)(m.node0 + (1u << m.ls) + c), (float)kBins);
+        for (int i = threadIdx.x; i < kBins; i += kTileThreads) ms.hist[i] = 0;
+        if (threadIdx.x < 12) ms.bb[threadIdx.x] = 0u;
+        __syncthreads();
+        uint32_t b[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            b[i] = wfirst + 32 * i + lane < cnt ? bin_of(cut, p[i], kBins) : (uint32_t)kBins;
+            int all;
+            __match_all_sync(kFull, b[i], &all);
+            if (all) {
+                if (lane == 0 && b[i] < kBins) atomicAdd(&ms.hist[b[i]], 32u);
+            } else if (b[i] < kBins) {
+                atomicAdd(&ms.hist[b[i]], 1u);
+            }
+        }
+        cluster.sync();  // histograms complete; every record of the node is in registers
+        uint32_t tot[kBinPer], pre[kBinPer], sum = 0;
+#pragma unroll
+        for (int i = 0; i < kBinPer; ++i) tot[i] = pre[i] = 0;
+        for (int o = 0; o < ctas; ++o) {
+            const uint32_t *h = cluster.map_shared_rank(&ms.hist[0], f + o) + threadIdx.x * kBinPer;
+#pragma unroll
+            for (int i = 0; i < kBinPer; ++i) {
+                const uint32_t v = h[i];
+                tot[i] += v;
+                if (f + o < q) pre[i] += v;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kBinPer; ++i) sum += tot[i];
+        if (threadIdx.x == 0) ms.split = make_uint4(kBins, ncnt, 0u, 0u);  // no right child: all below
+        if (threadIdx.x < 6) ms.box[l & 1][threadIdx.x] = 0u;              // read before the barrier
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) ms.wsum[warp] = incl;
+        __syncthreads();
+        uint32_t run = __reduce_add_sync(kFull, lane < warp ? ms.wsum[lane] : 0u) + incl - sum;
+        if (ncnt > half) {
+#pragma unroll
+            for (int i = 0; i < kBinPer; ++i) {
+                if (run <= half && half < run + tot[i])
+                    ms.split = make_uint4(threadIdx.x * kBinPer + i, run, half - run, tot[i]);
+                run += tot[i];
+            }
+        }
+        __syncthreads();
+        const uint4 sp = ms.split;
+        // records of the node's earlier tiles below the median's bin and in
+        // it (at most 7 tiles of 4096: 16 bits each)
+        uint32_t before = 0;
+#pragma unroll
+        for (int i = 0; i < kBinPer; ++i) {
+            const uint32_t bin = threadIdx.x * kBinPer + i;
+            before += bin < sp.x ? pre[i] : (bin == sp.x ? pre[i] << 16 : 0u);
+        }
+        before = __reduce_add_sync(kFull, before);
+        uint32_t ml[kPer], me[kPer], own = 0;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            ml[i] = __ballot_sync(kFull, b[i] < sp.x && b[i] < kBins);
+            me[i] = __ballot_sync(kFull, b[i] == sp.x && b[i] < kBins);
+            own += __popc(ml[i]) | ((uint32_t)__popc(me[i]) << 16);
+        }
+        if (lane == 0) {
+            ms.pre[warp] = before;
+            ms.wcnt[warp] = own;
+        }
+        __syncthreads();
+        uint32_t less, eq;
+        {
+            const uint32_t w = __reduce_add_sync(kFull, lane < warp ? ms.wcnt[lane] : 0u);
+            const uint32_t t = __reduce_add_sync(kFull, lane < kTileWarps ? ms.pre[lane] : 0u);
+            less = (w & 0xffffu) + (t & 0xffffu);
+            eq = (w >> 16) + (t >> 16);
+        }
+        uint32_t wl[6] = {0, 0, 0, 0, 0, 0}, wr[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int r = wfirst + 32 * i + lane;
+            if (r < cnt) {
+                const uint32_t lb = less + __popc(ml[i] & lt), eb = eq + __popc(me[i] & lt);
+                const bool is_l = (ml[i] >> lane) & 1u, is_e = (me[i] >> lane) & 1u;
+                uint32_t at;
+                bool left = true;
+                if (is_l) {
+                    at = lb;
+                } else if (is_e && eb < sp.z) {
+                    at = sp.y + eb;
+                } else {
+                    left = false;
+                    at = is_e ? half + (eb - sp.z)
+                              : half + (sp.w - sp.z) + ((uint32_t)((q - f) * (int)kTile + r) - lb - eb);
+                }
+                cluster.map_shared_rank(&ms.p[0], f + (int)(at / kTile))[at % kTile] = p[i];
+                if (boxes) {
+                    const uint32_t w[6] = {min_word(p[i].x), min_word(p[i].y), min_word(p[i].z),
+                                           max_word(p[i].x), max_word(p[i].y), max_word(p[i].z)};
+#pragma unroll
+                    for (int a = 0; a < 6; ++a) {
+                        if (left) wl[a] = max(wl[a], w[a]);
+                        else wr[a] = max(wr[a], w[a]);
+                    }
+                }
+            }
+            less += __popc(ml[i]);
+            eq += __popc(me[i]);
+        }
+        if (boxes) {
+#pragma unroll
+            for (int a = 0; a < 6; ++a) {
+                const uint32_t x = __reduce_max_sync(kFull, wl[a]), y = __reduce_max_sync(kFull, wr[a]);
+                if (lane == 0) {
+                    if (x) atomicMax(&ms.bb[a], x);
+                    if (y) atomicMax(&ms.bb[6 + a], y);
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x < 12 && ms.bb[threadIdx.x]) {
+                const int side = threadIdx.x / 6, a = threadIdx.x % 6;
+                atomicMax(cluster.map_shared_rank(&ms.box[(l + 1) & 1][a], f + side * (ctas / 2)), ms.bb[threadIdx.x]);
+            }
+        }
+        cluster.sync();  // records in place, boxes complete, histograms read
+        if (boxes) {
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                if (wfirst + 32 * i + lane < cnt) p[i] = ms.p[wfirst + 32 * i + lane];
+        }
+    }
+    for (int r = threadIdx.x; r < cnt; r += kTileThreads) m.pos_out[start + r] = ms.p[r];
 }
 
 struct SubScratch {
@@ -449,7 +660,7 @@ __global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_
     const int cnt = start < m.n ? (int)min((uint32_t)span0, m.n - start) : 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float inf = __int_as_float(0x7f800000);
-    const float4 *src = level_src(m, m.lf);
+    const float4 *src = m.lf == 0 ? m.pos : m.pos_out;
     for (int t = tid; t < cnt; t += kSubThreads) {
         ss.p[t] = src[start + t];
         ss.ord[0][t] = (uint16_t)t;
@@ -674,6 +885,9 @@ uint32_t tiles_of(uint32_t n) { return (n + kTile - 1) / kTile; }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// The level from which a map's nodes are split by clusters.
+int mid_level(int lf) { return std::max(lf - kMidLevels, 0); }
+
 // Scratch layout of a set of maps: the words zeroed by each build
 // (histograms, boxes, finished-subtree counters), the splits, the tile
 // counts, then the bins and the partner buffer of every map.
@@ -691,9 +905,9 @@ Layout layout_of(const uint32_t *n, const int *leaf_shift, int maps) {
         if (n[i] == 0) continue;
         L.tiles += tiles_of(n[i]);
         L.subs += 1u << lf;
-        if (lf == 0) continue;  // never split by the level launches: no scratch
-        L.nodes += 1u << lf;
-        records += (n[i] + 127u) & ~(size_t)127u;
+        if (lf == 0) continue;  // one subtree: no scratch
+        L.nodes += 2u << mid_level(lf);  // down to those the clusters split
+        if (mid_level(lf) > 0) records += (n[i] + 127u) & ~(size_t)127u;
     }
     L.box = align256(L.hist + sizeof(uint32_t) * kBins * (size_t)L.nodes);
     L.done = align256(L.box + sizeof(uint32_t) * 8 * (size_t)L.nodes);
@@ -714,7 +928,7 @@ int finish_level_of(const KdBuildArgs &a) {
 // records.
 void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, void *scratch, KdMap *out) {
     unsigned char *base = (unsigned char *)scratch;
-    uint32_t tile = 0, sub = 0, node = 0;
+    uint32_t tile = 0, sub = 0, node = 0, mid = 0;
     size_t rec = 0;
     for (int i = 0; i < count; ++i) {
         const KdBuildArgs &b = a[idx[i]];
@@ -736,15 +950,20 @@ void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, 
         m.depth = tree_depth(b.n, b.leaf_shift);
         m.leaf_shift = b.leaf_shift;
         m.lf = first_finish_level(m.depth, 32u << b.leaf_shift);
+        m.ls = mid_level(m.lf);
         m.tile0 = tile;
         m.sub0 = sub;
         m.node0 = node;
+        m.mid0 = mid;
         tile += tiles_of(b.n);
         sub += 1u << m.lf;
         if (m.lf > 0) {
+            mid += 1u << m.ls;
+            node += 2u << m.ls;
+        }
+        if (m.ls > 0) {
             m.tmp = (float4 *)(base + L.tmp) + rec;
             m.bins = (uint16_t *)(base + L.bins) + rec;
-            node += 1u << m.lf;
             rec += (b.n + 127u) & ~(size_t)127u;
         }
     }
@@ -753,17 +972,27 @@ void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, 
 template <class Maps>
 cudaError_t launch_build(const Maps &maps, const KdMap *host, int count, uint32_t subs, uint32_t *hist,
                          uint32_t *box, uint4 *thr, uint2 *tile_cnt, cudaStream_t s) {
-    for (int l = 0; l < host[0].lf; ++l) {
+    for (int l = 0; l < host[0].ls; ++l) {
         // the maps split at this level come first
         uint32_t t = 0;
-        for (int i = 0; i < count && host[i].lf > l; ++i) t = host[i].tile0 + tiles_of(host[i].n);
+        for (int i = 0; i < count && host[i].ls > l; ++i) t = host[i].tile0 + tiles_of(host[i].n);
         kd_hist_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, box, hist);
         kd_count_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, hist, thr, tile_cnt);
         kd_split_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, thr, tile_cnt, box);
         note_launches(3);
     }
+    cudaError_t e;
+    uint32_t mids = 0;
+    for (int i = 0; i < count && host[i].lf > 0; ++i) mids = host[i].mid0 + (1u << host[i].ls);
+    if (mids) {
+        const int smem = (int)sizeof(MidScratch);
+        e = cudaFuncSetAttribute(kd_mid_kernel<Maps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        kd_mid_kernel<Maps><<<mids * kMidCtas, kTileThreads, smem, s>>>(maps, box);
+        note_launch();
+    }
     const int smem = (int)sizeof(SubScratch);
-    cudaError_t e = cudaFuncSetAttribute(kd_finish_kernel<Maps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(kd_finish_kernel<Maps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     kd_finish_kernel<Maps><<<subs, kSubThreads, smem, s>>>(maps);
     note_launch();

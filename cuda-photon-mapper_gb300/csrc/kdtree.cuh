@@ -37,8 +37,9 @@ struct KdMap {
     uint32_t *done;                        // finished subtrees (zero between builds)
     const uint32_t *pad_count;             // nullable
     float3 root_lo, root_hi;
-    uint32_t n, tile0, sub0, node0;        // first tile, subtree and node words of this map in the launch
-    int depth, lf, leaf_shift, root_boxed;
+    uint32_t n, tile0, mid0, sub0, node0;  // first tile, cluster, subtree and node words of this map in the launch
+    int depth, leaf_shift, root_boxed;
+    int ls, lf;                            // the first level split by clusters, the level of the subtrees
 };
 
 // Scratch of build_trees over these maps (one or two, built in shared

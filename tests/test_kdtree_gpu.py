@@ -3,8 +3,8 @@ nearest records of any point set are those of a brute-force sort by
 (squared distance, index), whatever the set's size and shape.
 
 Sizes sit at the edges of the build's parts: leaves of 32, warp splits of 64
-and 128, subtrees of 2,048 records, tiles of 4,096, one to seven split
-levels, both maps in shared launches and (above 4M records) apart."""
+and 128, subtrees of 2,048 records, tiles of 4,096, clusters of 32,768, one to
+seven split levels, both maps in shared launches and (above 4M records) apart."""
 import numpy as np
 import pytest
 
@@ -46,7 +46,8 @@ def brute(p, q, k, radius):
     return idx, d2
 
 
-CASES = [(n, "box", ls) for n in (1, 32, 33, 64, 65, 128, 129, 2047, 2048, 2049, 4096, 4097, 8193, 65537)
+CASES = [(n, "box", ls) for n in (1, 32, 33, 64, 65, 128, 129, 2047, 2048, 2049, 4096, 4097, 8193,
+                                              32767, 32769, 65537)
          for ls in (32,)]
 CASES += [(n, "box", ls) for n in (100, 128, 129, 5000, 131073) for ls in (64, 128)]
 CASES += [(n, kind, 32) for n in (3000, 40001, 300007) for kind in ("wall", "point", "outlier", "nonfinite")]
