@@ -150,7 +150,7 @@ pm_status pm_set_scene(pm_ctx *ctx, const pm_scene *scene, const pm_config *cfg)
     for (auto &p : st->off) PM_TRY(dalloc(&p, st->path_cap));
     PM_TRY(dalloc(&st->scan_tmp, scan_tile_count(st->path_cap) + 1));
     PM_TRY(dalloc(&st->need_list, st->path_cap));
-    PM_TRY(dalloc(&st->need_tile, needed_tiles(st->path_cap)));
+    PM_TRY(dalloc(&st->need_tile, needed_words(st->path_cap)));
     PM_TRY(dalloc(&st->need_tile_off, needed_tiles(st->path_cap)));
     PM_TRY(dalloc(&st->words, 16));
     PM_TRY(cudaMemset(st->words, 0, 16 * sizeof(uint32_t)));

@@ -58,48 +58,108 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const uint32_t *in, 
     if (threadIdx.x == 0 && total_out) *total_out = total;
 }
 
+constexpr int kSortWarps = kSortThreads / 32;
+
+// The block's sum of v, on every thread.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *warp_sums) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t w = __reduce_add_sync(0xffffffffu, v);
+    if (lane == 0) warp_sums[threadIdx.x >> 5] = w;
+    __syncthreads();
+    const uint32_t r = __reduce_add_sync(0xffffffffu, lane < kSortWarps ? warp_sums[lane] : 0u);
+    __syncthreads();
+    return r;
+}
+
 // Per-tile sums for the large scan (tile = kSortTile elements).
 __global__ void __launch_bounds__(kSortThreads) tile_sum_kernel(const uint32_t *in, uint32_t n,
                                                                 uint32_t *sums) {
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t total;
-    const uint32_t base = blockIdx.x * kSortTile + threadIdx.x * kSortItems;
+    __shared__ uint32_t warp_sums[kSortWarps];
+    const uint32_t base = blockIdx.x * kSortTile;
     uint32_t s = 0;
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        uint32_t idx = base + i;
-        if (idx < n) s += in[idx];
+    for (int i = 0; i < kSortItems / 4; ++i) {
+        const uint4 v = load_words4(in, base + 4 * ((uint32_t)i * kSortThreads + threadIdx.x), n);
+        s += v.x + v.y + v.z + v.w;
     }
-    block_exclusive_scan(s, warp_sums, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+    s = block_sum(s, warp_sums);
+    if (threadIdx.x == 0) sums[blockIdx.x] = s;
 }
 
-// With seg_tab (per tile: the first tile of its segment, the segment's
-// tiles) each segment's scan starts at 0: the tile's offset less that of
-// its segment's first tile.
+// A tile's scan, its first value from the tiles before it: offs holds their
+// scan, or (raw) the tiles' sums, which the block adds up itself. With
+// seg_tab (per tile: the first tile of its segment, the segment's tiles) each
+// segment's scan starts at 0: the tile's offset less that of its segment's
+// first tile. A warp scans 512 consecutive elements, 128 at a time in 16-byte
+// loads and stores. Bound by them: 88M words 2 x 0.35 GB in 96 us (one thread
+// per 16 consecutive words: 380).
 __global__ void __launch_bounds__(kSortThreads) tile_scan_kernel(const uint32_t *in, uint32_t *out,
-                                                                 uint32_t n,
-                                                                 const uint32_t *offs,
-                                                                 const uint2 *seg_tab) {
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t total;
-    const uint32_t base = blockIdx.x * kSortTile + threadIdx.x * kSortItems;
-    uint32_t v[kSortItems];
-    uint32_t s = 0;
+                                                                 uint32_t n, const uint32_t *offs, bool raw,
+                                                                 uint32_t *total_out, const uint2 *seg_tab) {
+    __shared__ uint32_t warp_sums[kSortWarps];
+    constexpr int kRounds = kSortItems / 4;
+    const bool aligned = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t base = blockIdx.x * kSortTile + (uint32_t)warp * (32u * kSortItems) + 4u * lane;
+    uint4 v[kRounds];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        uint32_t idx = base + i;
-        v[i] = idx < n ? in[idx] : 0u;
-        s += v[i];
+    for (int r = 0; r < kRounds; ++r) v[r] = load_words4(in, base + 128u * r, n);
+    uint32_t first;
+    if (raw) {
+        uint32_t s = 0;
+        for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kSortThreads) s += offs[t];
+        first = block_sum(s, warp_sums);
+    } else {
+        first = offs[blockIdx.x];
+        if (seg_tab) first -= offs[seg_tab[blockIdx.x].x];
     }
-    uint32_t run = block_exclusive_scan(s, warp_sums, &total) + offs[blockIdx.x];
-    if (seg_tab) run -= offs[seg_tab[blockIdx.x].x];
+    uint32_t pre[kRounds], run = 0;  // of this lane's words within the warp's
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        uint32_t idx = base + i;
-        if (idx < n) out[idx] = run;
-        run += v[i];
+    for (int r = 0; r < kRounds; ++r) {
+        const uint32_t s = v[r].x + v[r].y + v[r].z + v[r].w;
+        uint32_t incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        pre[r] = run + incl - s;
+        run += __shfl_sync(0xffffffffu, incl, 31);
     }
+    if (lane == 0) warp_sums[warp] = run;
+    __syncthreads();
+    const uint32_t all = lane < kSortWarps ? warp_sums[lane] : 0u;
+    first += __reduce_add_sync(0xffffffffu, lane < warp ? all : 0u);
+    if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == kSortThreads - 1) *total_out = first + run;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const uint32_t i = base + 128u * r, a = first + pre[r];
+        const uint4 o = make_uint4(a, a + v[r].x, a + v[r].x + v[r].y, a + v[r].x + v[r].y + v[r].z);
+        if (aligned && i + 4 <= n) {
+            *reinterpret_cast<uint4 *>(out + i) = o;
+        } else {
+            if (i < n) out[i] = o.x;
+            if (i + 1 < n) out[i + 1] = o.y;
+            if (i + 2 < n) out[i + 2] = o.z;
+            if (i + 3 < n) out[i + 3] = o.w;
+        }
+    }
+}
+
+// The launches of a scan of n words over its tiles, their sums in tmp. Up to
+// kRawTiles tiles each block adds up the sums before its own (16 KB at most)
+// instead of a launch of their scan.
+constexpr uint32_t kRawTiles = 4096;
+void scan_tiles(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total, uint32_t *tmp, const uint2 *seg_tab,
+                bool pooled, cudaStream_t stream) {
+    const uint32_t tiles = scan_tile_count(n);
+    const bool raw = !pooled && tiles <= kRawTiles;
+    tile_sum_kernel<<<tiles, kSortThreads, 0, stream>>>(in, n, tmp); note_launch();
+    if (!raw) {
+        scan_kernel<<<1, kScanThreads, 0, stream>>>(tmp, tmp, tiles, total); note_launch();
+    }
+    tile_scan_kernel<<<tiles, kSortThreads, 0, stream>>>(in, out, n, tmp, raw, raw ? total : nullptr, seg_tab);
+    note_launch();
 }
 
 // Position of the (digit d, tile t) count in the scanned array: digit-major;
@@ -114,6 +174,8 @@ __device__ __forceinline__ uint32_t count_at(uint32_t d, uint32_t t, uint32_t nt
     return d * ntiles + t;
 }
 
+// A tile's digit counts: bound by latency in short sorts (5 tiles: 11 -> 4.7 us
+// with the tile's loads issued together, 16 bytes each).
 __global__ void __launch_bounds__(kSortThreads) hist_kernel(const uint32_t *keys, const uint32_t *n_dev,
                                                             int shift, uint32_t *hist,
                                                             uint32_t ntiles, const uint2 *seg_tab) {
@@ -122,9 +184,17 @@ __global__ void __launch_bounds__(kSortThreads) hist_kernel(const uint32_t *keys
     __syncthreads();
     const uint32_t n = *n_dev;
     const uint32_t base = blockIdx.x * kSortTile;
-    for (uint32_t i = threadIdx.x; i < kSortTile; i += kSortThreads) {
-        uint32_t idx = base + i;
-        if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1u);
+    uint4 v[kSortItems / 4];  // all loads in flight before the first count
+#pragma unroll
+    for (int i = 0; i < kSortItems / 4; ++i)
+        v[i] = load_words4(keys, base + 4u * ((uint32_t)i * kSortThreads + threadIdx.x), n);
+#pragma unroll
+    for (int i = 0; i < kSortItems / 4; ++i) {
+        const uint32_t idx = base + 4u * ((uint32_t)i * kSortThreads + threadIdx.x);
+        if (idx < n) atomicAdd(&h[(v[i].x >> shift) & 255u], 1u);
+        if (idx + 1 < n) atomicAdd(&h[(v[i].y >> shift) & 255u], 1u);
+        if (idx + 2 < n) atomicAdd(&h[(v[i].z >> shift) & 255u], 1u);
+        if (idx + 3 < n) atomicAdd(&h[(v[i].w >> shift) & 255u], 1u);
     }
     __syncthreads();
     hist[count_at(threadIdx.x, blockIdx.x, ntiles, seg_tab)] = h[threadIdx.x];
@@ -227,10 +297,7 @@ cudaError_t radix_sort_pairs_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_
         if (hn <= kSortTile && !seg_tab) {
             scan_kernel<<<1, kScanThreads, 0, stream>>>(hist, hist, hn, nullptr); note_launch();
         } else {
-            const uint32_t tiles = scan_tile_count(hn);
-            tile_sum_kernel<<<tiles, kSortThreads, 0, stream>>>(hist, hn, partials); note_launch();
-            scan_kernel<<<1, kScanThreads, 0, stream>>>(partials, partials, tiles, nullptr); note_launch();
-            tile_scan_kernel<<<tiles, kSortThreads, 0, stream>>>(hist, hist, hn, partials, nullptr); note_launch();
+            scan_tiles(hist, hist, hn, nullptr, partials, nullptr, seg_tab != nullptr, stream);
         }
         scatter_kernel<<<ntiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n_dev, shift,
                                                                hist, ntiles, seg_tab); note_launch();
@@ -250,20 +317,14 @@ uint32_t scan_tile_count(uint32_t n) {
 cudaError_t exclusive_scan_u32_large(const uint32_t *in, uint32_t *out, uint32_t n,
                                      uint32_t *total, uint32_t *tmp, cudaStream_t stream) {
     if (n <= 65536) return exclusive_scan_u32(in, out, n, total, stream);
-    uint32_t tiles = scan_tile_count(n);
-    tile_sum_kernel<<<tiles, kSortThreads, 0, stream>>>(in, n, tmp); note_launch();
-    scan_kernel<<<1, kScanThreads, 0, stream>>>(tmp, tmp, tiles, total); note_launch();
-    tile_scan_kernel<<<tiles, kSortThreads, 0, stream>>>(in, out, n, tmp, nullptr); note_launch();
+    scan_tiles(in, out, n, total, tmp, nullptr, false, stream);
     return cudaGetLastError();
 }
 
 cudaError_t exclusive_scan_u32_segmented(const uint32_t *in, uint32_t *out, uint32_t n, const uint2 *seg_tab,
                                          uint32_t *tmp, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    const uint32_t tiles = scan_tile_count(n);
-    tile_sum_kernel<<<tiles, kSortThreads, 0, stream>>>(in, n, tmp); note_launch();
-    scan_kernel<<<1, kScanThreads, 0, stream>>>(tmp, tmp, tiles, nullptr); note_launch();
-    tile_scan_kernel<<<tiles, kSortThreads, 0, stream>>>(in, out, n, tmp, seg_tab); note_launch();
+    scan_tiles(in, out, n, nullptr, tmp, seg_tab, true, stream);
     return cudaGetLastError();
 }
 

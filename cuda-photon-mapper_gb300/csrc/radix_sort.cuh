@@ -18,6 +18,18 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
 constexpr uint32_t kSortTile = kSortThreads * kSortItems;
 
+// Four consecutive words from in[i] (i a multiple of 4), zero past n: one
+// 16-byte load where the array and n allow it.
+__device__ __forceinline__ uint4 load_words4(const uint32_t *in, uint32_t i, uint32_t n) {
+    if ((reinterpret_cast<uintptr_t>(in) & 15u) == 0 && i + 4 <= n) return *reinterpret_cast<const uint4 *>(in + i);
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (i < n) v.x = in[i];
+    if (i + 1 < n) v.y = in[i + 1];
+    if (i + 2 < n) v.z = in[i + 2];
+    if (i + 3 < n) v.w = in[i + 3];
+    return v;
+}
+
 // Number of uint32 words of scratch the sort needs for max_n elements: the
 // digit counts of every tile plus the partial sums of their scan.
 inline size_t radix_sort_hist_words(uint32_t max_n) {
@@ -44,9 +56,9 @@ cudaError_t radix_sort_pairs_u32(uint32_t *keys, uint32_t *vals, uint32_t *keys_
 cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total,
                                cudaStream_t stream);
 
-// Exclusive prefix sum of in[0..n) for large n: per-tile sums, one scan of
-// the tile sums, then per-tile scans. tmp must hold scan_tile_count(n) + 1
-// words. *total (device) receives the sum.
+// Exclusive prefix sum of in[0..n) for large n: per-tile sums, for many tiles
+// one scan of the sums, then per-tile scans. tmp must hold scan_tile_count(n)
+// + 1 words. *total (device) receives the sum.
 uint32_t scan_tile_count(uint32_t n);
 cudaError_t exclusive_scan_u32_large(const uint32_t *in, uint32_t *out, uint32_t n,
                                      uint32_t *total, uint32_t *tmp, cudaStream_t stream);

@@ -82,9 +82,11 @@ cudaError_t map_extents_multi(const ExtentJob *jobs, int n, cudaStream_t s);
 // The ids below `issued` of the paths that hold a record of a map (id <
 // ext_s[1] with cnt_s > 0, or id < ext_v[1] with cnt_v > 0), in increasing
 // order, into list[0 .. *list_n): per-tile counts, a scan of them, then each
-// tile's ids placed at its offset. tile_cnt / tile_off hold
-// needed_tiles(issued) words; scan_tmp as exclusive_scan_u32_large's.
+// tile's ids placed at its offset. tile_cnt holds needed_words(issued) words
+// (the counts and a bit per id), tile_off needed_tiles(issued); scan_tmp as
+// exclusive_scan_u32_large's.
 uint32_t needed_tiles(uint32_t n);
+uint32_t needed_words(uint32_t n);
 cudaError_t needed_paths(uint32_t issued, const uint32_t *cnt_s, const uint32_t *cnt_v,
                          const uint32_t *ext_s, const uint32_t *ext_v, uint32_t *tile_cnt,
                          uint32_t *tile_off, uint32_t *scan_tmp, uint32_t *list, uint32_t *list_n,
