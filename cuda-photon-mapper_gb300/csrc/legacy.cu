@@ -290,32 +290,30 @@ __device__ v3 interpolate_slab(const float4 *__restrict__ slab, v3 p, int type, 
 // A photon's path is traced by kPhotonLanes lanes together: the path is the
 // same on each of them, a wall's splat window of up to 36 cells takes a cell
 // per lane. 8 lanes: the path's arithmetic is repeated eight times, the
-// window's is spread over them. The writing launch takes 61 us, the counting
-// one, which needs no windows, 37 us (a thread per photon, which walks a
-// bounce's 72 cells one by one: 121 us each).
+// window's is spread over them: 55 us (a thread per photon, which walks a
+// bounce's 72 cells one by one: 121 us). One launch: a photon's deposits go to
+// its own places and are closed up afterwards in 8 us, where a launch that
+// only counted them took 37.
 constexpr int kPhotonLanes = 8;
 __device__ __forceinline__ int photon_lane() { return (int)(threadIdx.x & (kPhotonLanes - 1)); }
 __device__ __forceinline__ unsigned photon_mask() {
     return ((1u << kPhotonLanes) - 1u) << (threadIdx.x & (31u & ~(kPhotonLanes - 1u)));
 }
 
-// Records a photon's grid deposits in the order the reference applies them.
-// The counting pass (kWrite false) only counts; the writing pass stores
-// (voxel, value) at this photon's offset.
-template <bool kWrite>
+// Records a photon's grid deposits in the order the reference applies them,
+// (voxel, value) from place `off` on.
 struct Deposits {
-    uint32_t *keys, *idx;
+    uint32_t *keys;
     float4 *vals;
     const float *inv;  // 1 / sqrt(i), i < kInvN
     uint32_t off, n;
     __device__ __forceinline__ void store(uint32_t at, int vox, v3 e) {
         keys[at] = (uint32_t)vox;
-        idx[at] = at;
         vals[at] = make_float4(e.x, e.y, e.z, 0.0f);
     }
     // One deposit (the same on every lane).
     __device__ __forceinline__ void put(int vox, v3 e) {
-        if (kWrite && photon_lane() == 0) store(off + n, vox, e);
+        if (photon_lane() == 0) store(off + n, vox, e);
         ++n;
     }
     // One deposit on each lane with `on`, in lane order.
@@ -349,8 +347,7 @@ __device__ __forceinline__ I3 clamped_voxel(v3 p) {
 // the reference's row order, a cell per lane. A cell's value is the energy's
 // twentieth over its distance (:1059-1071), whose reciprocal depends only on
 // the squared distance in cells and is read from a table.
-template <bool kWrite>
-__device__ __forceinline__ void store_surface(Deposits<kWrite> &d, int type, int id, v3 loc, v3 e) {
+__device__ __forceinline__ void store_surface(Deposits &d, int type, int id, v3 loc, v3 e) {
     I3 c = clamped_voxel(loc);
     if (type != 0) d.put(vox_index(c.x, c.y, c.z), e);
     if (type != 1 || id < 0 || id > 4) return;
@@ -360,10 +357,6 @@ __device__ __forceinline__ void store_surface(Deposits<kWrite> &d, int type, int
     const int ca = on_x ? c.y : c.x, cb = on_x || on_y ? c.z : c.y, cf = on_x ? c.x : (on_y ? c.y : c.z);
     const int a0 = lo_edge(ca, 0), a1 = hi_edge(ca, G), b0 = lo_edge(cb, 0), b1 = hi_edge(cb, G);
     const int nb = b1 - b0, cells = (a1 - a0) * nb;  // 3 to 6 a side
-    if (!kWrite) {
-        d.n += (uint32_t)(cells - (cf == fixed ? 1 : 0));  // the photon's own cell is left out
-        return;
-    }
     const v3 e20 = e * 0.05f;
     const int rcp = 65536 / nb + 1;  // t / nb for t < 64
     const int df = cf - fixed;
@@ -372,7 +365,7 @@ __device__ __forceinline__ void store_surface(Deposits<kWrite> &d, int type, int
         const int row = (t * rcp) >> 16, a = a0 + row, b = b0 + (t - row * nb);
         const int i = on_x ? fixed : a, j = on_y ? fixed : (on_x ? a : b), k = on_x || on_y ? b : fixed;
         const int da = ca - a, db = cb - b, d2 = da * da + db * db + df * df;
-        const bool on = t < cells && d2 > 0;
+        const bool on = t < cells && d2 > 0;  // the photon's own cell is left out
         d.put_lanes(on, vox_index(i, j, k), e20 * (on ? d.inv[d2] : 0.0f));
     }
 }
@@ -414,9 +407,8 @@ struct Mwc {
 
 // emitPhotons (:1215-1375) for photon `index`; the medium steps draw from
 // the generator positioned at this photon's first draw.
-template <bool kWrite>
 __device__ void emit_one(const Scene &sc, const float4 *__restrict__ table, int index, bool media,
-                         Mwc rng, Deposits<kWrite> &d) {
+                         Mwc rng, Deposits &d) {
     int bounces = 1;
     v3 rgb = mk3(10.0f, 10.0f, 10.0f);
     float4 t = table[index];
@@ -513,31 +505,51 @@ __device__ __forceinline__ Mwc jump_photon(const JumpTable &J, uint32_t z0, uint
 }
 
 // Bound by the latency of a photon's serial bounces and their arithmetic.
-template <bool kWrite>
 __global__ void __launch_bounds__(256) emit_kernel(Scene sc, const float4 *__restrict__ table, bool media,
                                                    uint32_t z0, uint32_t w0, JumpTable jump, uint32_t *counts,
-                                                   const uint32_t *offsets, uint32_t *keys, uint32_t *idx,
-                                                   float4 *vals) {
-    __shared__ float inv[kWrite ? kInvN : 1];
-    if (kWrite) {
-        for (int i = threadIdx.x; i < kInvN; i += blockDim.x) inv[i] = 1.0f / sqrtf((float)i);
-        __syncthreads();
-    }
+                                                   uint32_t *keys, float4 *vals) {
+    __shared__ float inv[kInvN];
+    for (int i = threadIdx.x; i < kInvN; i += blockDim.x) inv[i] = 1.0f / sqrtf((float)i);
+    __syncthreads();
     const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kPhotonLanes);
     if (p >= kLegacyPhotons) return;  // whole photons
     Mwc rng;
     rng.z = z0;
     rng.w = w0;
-    if (kWrite && media) rng = jump_photon(jump, z0, w0, p);  // the draws do not change the count
-    Deposits<kWrite> d;
+    if (media) rng = jump_photon(jump, z0, w0, p);
+    Deposits d;
     d.keys = keys;
-    d.idx = idx;
     d.vals = vals;
     d.inv = inv;
-    d.off = kWrite ? offsets[p] : 0u;
+    d.off = (uint32_t)p * kLegacyMaxDepositsPerPhoton;
     d.n = 0;
     emit_one(sc, table, p, media, rng, d);
-    if (!kWrite && photon_lane() == 0) counts[p] = d.n;
+    if (photon_lane() == 0) counts[p] = d.n;
+}
+
+// The photons' deposits one after another: voxel and place, for the sort. A
+// warp per photon; a block adds up the counts of the photons before its own.
+constexpr int kClosePhotons = 32;
+__global__ void __launch_bounds__(kClosePhotons * 32) close_up_kernel(const uint32_t *__restrict__ counts,
+                                                                      const uint32_t *__restrict__ slots,
+                                                                      uint32_t *keys, uint32_t *idx, uint32_t *total) {
+    __shared__ uint32_t sums[kClosePhotons];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * kClosePhotons;
+    uint32_t s = 0;
+    for (int i = threadIdx.x; i < first; i += kClosePhotons * 32) s += counts[i];
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) sums[warp] = s;
+    const uint32_t c = first + lane < kLegacyPhotons ? counts[first + lane] : 0u;
+    __syncthreads();
+    const uint32_t off = __reduce_add_sync(0xffffffffu, sums[lane] + (lane < warp ? c : 0u));
+    const uint32_t n = __shfl_sync(0xffffffffu, c, warp);
+    const uint32_t from = (uint32_t)(first + warp) * kLegacyMaxDepositsPerPhoton;
+    for (uint32_t i = lane; i < n; i += 32) {
+        keys[off + i] = slots[from + i];
+        idx[off + i] = from + i;
+    }
+    if (first + warp == kLegacyPhotons - 1 && lane == 0) *total = off + n;
 }
 
 // Deposit values in sorted order (one parallel gather), so that each
@@ -722,7 +734,6 @@ cudaError_t legacy_alloc(LegacyState &st) {
     PM_ALLOC(st.vol_win, sizeof(float4) * kVolWindows);
     PM_ALLOC(st.slab_win, sizeof(float4) * kSlabWindows);
     PM_ALLOC(st.counts, sizeof(uint32_t) * kLegacyPhotons);
-    PM_ALLOC(st.offsets, sizeof(uint32_t) * kLegacyPhotons);
     PM_ALLOC(st.total, sizeof(uint32_t));
     PM_ALLOC(st.start, sizeof(uint32_t) * (kLegacyVoxels + 1));
     PM_ALLOC(st.keys, sizeof(uint32_t) * kLegacyMaxDeposits);
@@ -745,7 +756,7 @@ cudaError_t legacy_alloc(LegacyState &st) {
 void legacy_free(LegacyState &st) {
     cudaFree(st.table); cudaFree(st.grid3); cudaFree(st.grid4); cudaFree(st.counts);
     cudaFree(st.vol_win); cudaFree(st.slab_win);
-    cudaFree(st.offsets); cudaFree(st.total); cudaFree(st.start); cudaFree(st.keys); cudaFree(st.keys_tmp);
+    cudaFree(st.total); cudaFree(st.start); cudaFree(st.keys); cudaFree(st.keys_tmp);
     cudaFree(st.idx); cudaFree(st.idx_tmp); cudaFree(st.dep); cudaFree(st.sdep); cudaFree(st.hist);
     st = LegacyState();
 }
@@ -770,14 +781,12 @@ cudaError_t legacy_emit(LegacyState &st, float anim_time, int flags, cudaStream_
         jump.w[i] = mwc_jump_host(1u, kMwcAw, kMwcMw, 9ull << i);
     }
     const int blocks = (kLegacyPhotons * kPhotonLanes + 255) / 256;
-    emit_kernel<false><<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, jump, st.counts, nullptr, nullptr,
-                                              nullptr, nullptr); note_launch();
-    cudaError_t e = exclusive_scan_u32(st.counts, st.offsets, kLegacyPhotons, st.total, s);
-    if (e != cudaSuccess) return e;
-    emit_kernel<true><<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, jump, st.counts, st.offsets, st.keys,
-                                             st.idx, st.dep); note_launch();
+    emit_kernel<<<blocks, 256, 0, s>>>(sc, st.table, media, z0, w0, jump, st.counts, st.keys_tmp, st.dep); note_launch();
+    close_up_kernel<<<(kLegacyPhotons + kClosePhotons - 1) / kClosePhotons, kClosePhotons * 32, 0, s>>>(
+        st.counts, st.keys_tmp, st.keys, st.idx, st.total);
+    note_launch();
     uint32_t *sk = nullptr, *si = nullptr;
-    e = radix_sort_pairs_u32(st.keys, st.idx, st.keys_tmp, st.idx_tmp, st.total, kLegacyMaxDeposits,
+    cudaError_t e = radix_sort_pairs_u32(st.keys, st.idx, st.keys_tmp, st.idx_tmp, st.total, kLegacyMaxDeposits,
                              0, 16, st.hist, s, &sk, &si);
     if (e != cudaSuccess) return e;
     gather_deposits_kernel<<<512, 256, 0, s>>>(sk, si, st.dep, st.total, st.sdep, st.start); note_launch();

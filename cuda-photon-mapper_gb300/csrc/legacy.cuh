@@ -32,12 +32,11 @@ struct LegacyState {
     float4 *vol_win = nullptr;    // the render's window sums of the grid (media march)
     float4 *slab_win = nullptr;   // (wall slabs)
     uint32_t *counts = nullptr;   // deposits per photon
-    uint32_t *offsets = nullptr;  // exclusive scan of counts
     uint32_t *total = nullptr;    // total deposits (device scalar)
     uint32_t *start = nullptr;    // per voxel: its first sorted deposit (+ the total)
-    uint32_t *keys = nullptr, *keys_tmp = nullptr;
+    uint32_t *keys = nullptr, *keys_tmp = nullptr;  // keys_tmp: at first the photons' own places
     uint32_t *idx = nullptr, *idx_tmp = nullptr;
-    float4 *dep = nullptr;        // deposit values in photon order
+    float4 *dep = nullptr;        // deposit values, kLegacyMaxDepositsPerPhoton places a photon
     float4 *sdep = nullptr;       // the same, in (voxel, photon order) order
     uint32_t *hist = nullptr;
     uint64_t rng_draws = 0;       // draws taken from the shared generator so far
