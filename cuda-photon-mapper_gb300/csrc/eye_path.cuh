@@ -18,6 +18,9 @@ namespace pm {
 constexpr int kMaxSpecular = 8;
 constexpr uint32_t kEyeSalt = 0xE7E5A17Bu;
 constexpr int kMaxMarchSteps = 1 << 16;  // per segment
+// March samples whose densities are looked up together (the query list of
+// 1920 x 1080 pixels 431 -> 397 us; small frames wait for their longest path).
+constexpr int kMarchAhead = 4;
 
 // Sink interface:
 //   void volume(v3 x, v3 wo, float w)         in-scattering query, w = T(mid) * dt
@@ -48,17 +51,25 @@ __device__ __forceinline__ void walk_eye(const PScene &Sc, const RenderParams &R
                 const v3 wo = d * -1.0f;
                 if constexpr (Sink::kCountOnly) {
                     if (vol_on) sink.volume_steps(nst);
-                } else for (int j = 0; j < nst; ++j) {
-                    const float ta = t0 + (float)j * R.step;
-                    const float tb = fminf(t0 + (float)(j + 1) * R.step, t1);
-                    const float dt = tb - ta;
-                    const float tm = 0.5f * (ta + tb);
-                    const v3 x = o + d * tm;
-                    const float ss = Sc.het_res > 0 ? sigma_s_at(Sc, x) : Sc.sigma_s;
-                    const float st = ss + Sc.sigma_a;
-                    const float tau_mid = tau + st * (0.5f * dt);
-                    if (vol_on) sink.volume(x, wo, pm_expf(-tau_mid) * dt);
-                    tau = tau + st * dt;
+                } else for (int j = 0; j < nst; j += kMarchAhead) {
+                    v3 x[kMarchAhead];
+                    float dt[kMarchAhead], ss[kMarchAhead];
+#pragma unroll
+                    for (int q = 0; q < kMarchAhead; ++q) {  // the density is looked up for all of them at once
+                        const float ta = t0 + (float)(j + q) * R.step;
+                        const float tb = fminf(t0 + (float)(j + q + 1) * R.step, t1);
+                        dt[q] = tb - ta;
+                        x[q] = o + d * (0.5f * (ta + tb));
+                        ss[q] = Sc.het_res > 0 && j + q < nst ? sigma_s_at(Sc, x[q]) : Sc.sigma_s;
+                    }
+#pragma unroll
+                    for (int q = 0; q < kMarchAhead; ++q)
+                        if (j + q < nst) {
+                            const float st = ss[q] + Sc.sigma_a;
+                            const float tau_mid = tau + st * (0.5f * dt[q]);
+                            if (vol_on) sink.volume(x[q], wo, pm_expf(-tau_mid) * dt[q]);
+                            tau = tau + st * dt[q];
+                        }
                 }
             }
         }

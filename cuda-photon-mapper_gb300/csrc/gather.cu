@@ -122,9 +122,9 @@ __device__ __forceinline__ void render_pixel(const PScene &Sc, const MapView &su
     if (lane == 0) {
         if (rad) rad[pix] = make_float4(L.x, L.y, L.z, 1.0f);
         if (rgba)
-            rgba[pix] = make_uchar4(to_u8_sat((double)(L.x * R.exposure) * 255.0),
-                                    to_u8_sat((double)(L.y * R.exposure) * 255.0),
-                                    to_u8_sat((double)(L.z * R.exposure) * 255.0), 255);
+            rgba[pix] = make_uchar4(unit_to_u8(L.x * R.exposure),
+                                    unit_to_u8(L.y * R.exposure),
+                                    unit_to_u8(L.z * R.exposure), 255);
         if (R.counters) {
             if (nsurf) atomicAdd(&R.counters[0], (unsigned long long)nsurf);
             if (nvol) atomicAdd(&R.counters[1], (unsigned long long)nvol);

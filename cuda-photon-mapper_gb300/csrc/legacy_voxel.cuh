@@ -14,15 +14,6 @@
 #pragma once
 #include "pm_vec.cuh"
 
-#if defined(__CUDACC__)
-#define PM_FMAF(a, b, c) fmaf(a, b, c)
-#define PM_FLOORF(a) floorf(a)
-#else
-#include <cmath>
-#define PM_FMAF(a, b, c) std::fmaf(a, b, c)
-#define PM_FLOORF(a) std::floor(a)
-#endif
-
 namespace pm {
 
 PM_HD int legacy_voxel_xy_general(float x) { return d2i_sat((((double)x + 1.5) / 3.0) * 32.0); }
@@ -64,16 +55,6 @@ PM_HD float legacy_world_xy(int v) {
 PM_HD float legacy_world_z(int v) {
     if (v > -(1 << 20) && v < (1 << 20)) return ((float)v / 32.0f) * 6.0f;
     return (float)((double)((float)v / 32.0f) * 6.0);
-}
-
-// to_u8_sat((double)c * 255.0): the float product is at most one too large
-// when truncated (it can round up to the next integer), and the fused
-// remainder's sign says so.
-PM_HD unsigned char unit_to_u8(float c) {
-    if (!(c > 0.0f)) return 0;
-    if (c >= 1.0f) return 255;
-    const int k = (int)(c * 255.0f);
-    return (unsigned char)(PM_FMAF(c, 255.0f, -(float)k) < 0.0f ? k - 1 : k);
 }
 
 }  // namespace pm

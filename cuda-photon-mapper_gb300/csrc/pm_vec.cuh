@@ -11,8 +11,13 @@
 
 #if defined(__CUDACC__)
 #define PM_HD __host__ __device__ __forceinline__
+#define PM_FMAF(a, b, c) fmaf(a, b, c)
+#define PM_FLOORF(a) floorf(a)
 #else
+#include <cmath>
 #define PM_HD inline
+#define PM_FMAF(a, b, c) std::fmaf(a, b, c)
+#define PM_FLOORF(a) std::floor(a)
 #endif
 
 namespace pm {
@@ -50,6 +55,16 @@ PM_HD unsigned char to_u8_sat(double v) {
     double c = v > 255.0 ? 255.0 : v;
     if (!(c > 0.0)) return 0;
     return (unsigned char)(int)c;
+}
+
+// to_u8_sat((double)c * 255.0): the float product is at most one too large
+// when truncated (it can round up to the next integer), and the fused
+// remainder's sign says so.
+PM_HD unsigned char unit_to_u8(float c) {
+    if (!(c > 0.0f)) return 0;
+    if (c >= 1.0f) return 255;
+    const int k = (int)(c * 255.0f);
+    return (unsigned char)(PM_FMAF(c, 255.0f, -(float)k) < 0.0f ? k - 1 : k);
 }
 
 }  // namespace pm
