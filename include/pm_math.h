@@ -107,12 +107,11 @@ PMM_FN void pm_sincos2pi(float u, float *s, float *c) {
     cp = fmaf(x2, cp, 4.16666667e-02f);
     cp = fmaf(x2, cp, -0.5f);
     float cs = fmaf(x2, cp, 1.0f);
-    switch (quad) {
-        case 0: *s = sn; *c = cs; break;
-        case 1: *s = cs; *c = -sn; break;
-        case 2: *s = -sn; *c = -cs; break;
-        default: *s = -cs; *c = sn; break;
-    }
+    /* the quarter turn by selects: lanes at different quarters do not take
+     * turns (emission of 64 spheres 30.2 -> 29.8 ms) */
+    const float a = (quad & 1) ? cs : sn, b = (quad & 1) ? sn : cs;
+    *s = (quad & 2) ? -a : a;
+    *c = ((quad + 1) & 2) ? -b : b;
 }
 
 /* exp(x) for x <= 0 (returns 0 below -87). */
