@@ -58,7 +58,7 @@ cudaError_t render_batch(const BatchRenderScene *scenes, const uint32_t *chunk_p
 // k nearest records of each point, sorted by (squared distance, index).
 // `map` only steers: 0 where the records lie on surfaces, 1 in a volume.
 cudaError_t knn_query(const MapView &m, int map, const float4 *q, uint32_t nq, int k, float radius,
-                      uint32_t *idx, float *d2, cudaStream_t s);
+                      uint32_t *idx, float *d2, cudaStream_t s, bool thin = false);
 cudaError_t radius_gather(const MapView &m, const float4 *pts, const float4 *nrm, uint32_t nq,
                           float sq_radius, float exposure, float4 *out, cudaStream_t s);
 cudaError_t render_frame(const PScene &S, const MapView &surf, const MapView &vol,

@@ -374,7 +374,15 @@ pm_status pm_knn(pm_ctx *ctx, int map, const float4 *queries, uint32_t nq, int k
     if (!st || !st->map[map].built) return fail(ctx, PM_ERR_STATE, "pm_knn before pm_build");
     DeviceGuard g(ctx->device);
     cudaError_t e;
-    PM_TRY(knn_query(view_of(st->map[map]), map, queries, nq, k, radius, idx_out, d2_out, stream));
+    // With fewer than two dozen records expected in reach there is little to
+    // select, and one launch of the list search is faster: 5,000 records at
+    // radius 0.1 of a unit box, 5,000 queries 16.6 us (21.7 by the selection),
+    // 20,000 at 0.05 with 20,000 queries 39 (41). Beyond, 60,000 at 0.05: k = 1
+    // 56 (43), k = 50 64 (66), k = 100 82 (76); 20,000 at 0.1: 77 (56).
+    const pm_scene &sc = st->scene;
+    const float box = (sc.box_max[0] - sc.box_min[0]) * (sc.box_max[1] - sc.box_min[1]) * (sc.box_max[2] - sc.box_min[2]);
+    const bool thin = (float)st->map[map].n * 4.18879020f * radius * radius * radius <= 24.0f * box;
+    PM_TRY(knn_query(view_of(st->map[map]), map, queries, nq, k, radius, idx_out, d2_out, stream, thin));
     return PM_OK;
 }
 

@@ -763,75 +763,103 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
             return;
         }
         __syncwarp();
-        float px[kSlots], py[kSlots], pz[kSlots];
-        load_candidates(m, n, px, py, pz);
-        uint32_t d2[kSlots];
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s) {
-            const float dx = px[s] - p.x, dy = py[s] - p.y, dz = pz[s] - p.z;
-            d2[s] = __float_as_uint(dx * dx + dy * dy + dz * dz);
-        }
-        const uint32_t capb = __float_as_uint(r2cap);
-        const float expo = mid == 0 ? 1.0f : 0.6666667f;
-        uint32_t t = min(__float_as_uint(r * r * __powf(__fdividef((float)k, (float)max(n, k)), expo)), capb);
-        int own;
-        found = select_k(d2, t, capb, k, expo, m, &own);
-        int at = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(kFull, at, o);
-            if (lane >= o) at += v;
-        }
-        at -= own;
-        uint32_t *key = reinterpret_cast<uint32_t *>(ts.qd);  // 128 distances
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s)
-            if (d2[s] <= t) {
-                key[at] = d2[s];
-                ts.sel[at++] = ts.cat[cat_at(kSlots * lane + s)];
+        if (n <= 32) {
+            // A record a lane, its place by comparing with every other: 20,000
+            // queries of 200,000 records with k = 1 49.5 -> 43.3 us, k = 12 68.4
+            // -> 64.
+            uint32_t *key = reinterpret_cast<uint32_t *>(ts.qd);
+            uint32_t mine = 0xffffffffu, id = 0xffffffffu;
+            if (lane < n) {
+                const float4 c = __ldg(&m.pos[ts.cat[cat_at(lane)]]);
+                const float dx = c.x - p.x, dy = c.y - p.y, dz = c.z - p.z;
+                const uint32_t d2 = __float_as_uint(dx * dx + dy * dy + dz * dz);
+                if (d2 <= __float_as_uint(r2cap)) {
+                    mine = d2;
+                    id = __float_as_uint(c.w);
+                }
             }
-        if (lane < 4 && found + lane < 128) key[found + lane] = 0xffffffffu;
-        __syncwarp();
-        uint32_t mine[S], id[S];
-        int rank[S];
-        uint32_t sum = 0;
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const int e = lane + 32 * s;
-            mine[s] = e < found ? key[e] : 0u;
-            id[s] = e < found ? __float_as_uint(__ldg(&m.pos[ts.sel[e]]).w) : 0xffffffffu;
-            rank[s] = 0;
-        }
-        for (int f = 0; f < found; f += 4) {
-            const uint4 w = reinterpret_cast<const uint4 *>(key)[f >> 2];
-#pragma unroll
-            for (int s = 0; s < S; ++s)
-                rank[s] += (w.x < mine[s] ? 1 : 0) + (w.y < mine[s] ? 1 : 0) + (w.z < mine[s] ? 1 : 0) +
-                           (w.w < mine[s] ? 1 : 0);
-        }
-#pragma unroll
-        for (int s = 0; s < S; ++s) sum += lane + 32 * s < found ? (uint32_t)rank[s] : 0u;
-        sum = __reduce_add_sync(kFull, sum);
-        __syncwarp();
-        if (sum != (uint32_t)(found * (found - 1) / 2)) {  // equal distances
-#pragma unroll
-            for (int s = 0; s < S; ++s)
-                if (lane + 32 * s < found) ts.sel[lane + 32 * s] = id[s];
-            __syncwarp();
-            for (int f = 0; f < found; ++f) {
-                const uint32_t w = key[f], o = ts.sel[f];
-#pragma unroll
-                for (int s = 0; s < S; ++s) rank[s] += w == mine[s] && o < id[s] ? 1 : 0;
+            int rank = 0;
+            for (int o = 0; o < n; ++o) {
+                const uint32_t w = __shfl_sync(kFull, mine, o), i = __shfl_sync(kFull, id, o);
+                rank += w < mine || (w == mine && i < id) ? 1 : 0;
+            }
+            found = min(k, __popc(__ballot_sync(kFull, mine != 0xffffffffu)));
+            if (mine != 0xffffffffu && rank < k) {
+                key[rank] = mine;
+                ts.sel[rank] = id;
             }
             __syncwarp();
-        }
+        } else {
+            float px[kSlots], py[kSlots], pz[kSlots];
+            load_candidates(m, n, px, py, pz);
+            uint32_t d2[kSlots];
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-            if (lane + 32 * s < found) {
-                key[rank[s]] = mine[s];
-                ts.sel[rank[s]] = id[s];
+            for (int s = 0; s < kSlots; ++s) {
+                const float dx = px[s] - p.x, dy = py[s] - p.y, dz = pz[s] - p.z;
+                d2[s] = __float_as_uint(dx * dx + dy * dy + dz * dz);
             }
-        __syncwarp();
+            const uint32_t capb = __float_as_uint(r2cap);
+            const float expo = mid == 0 ? 1.0f : 0.6666667f;
+            uint32_t t = min(__float_as_uint(r * r * __powf(__fdividef((float)k, (float)max(n, k)), expo)), capb);
+            int own;
+            found = select_k(d2, t, capb, k, expo, m, &own);
+            int at = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, at, o);
+                if (lane >= o) at += v;
+            }
+            at -= own;
+            uint32_t *key = reinterpret_cast<uint32_t *>(ts.qd);  // 128 distances
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s)
+                if (d2[s] <= t) {
+                    key[at] = d2[s];
+                    ts.sel[at++] = ts.cat[cat_at(kSlots * lane + s)];
+                }
+            if (lane < 4 && found + lane < 128) key[found + lane] = 0xffffffffu;
+            __syncwarp();
+            uint32_t mine[S], id[S];
+            int rank[S];
+            uint32_t sum = 0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int e = lane + 32 * s;
+                mine[s] = e < found ? key[e] : 0u;
+                id[s] = e < found ? __float_as_uint(__ldg(&m.pos[ts.sel[e]]).w) : 0xffffffffu;
+                rank[s] = 0;
+            }
+            for (int f = 0; f < found; f += 4) {
+                const uint4 w = reinterpret_cast<const uint4 *>(key)[f >> 2];
+#pragma unroll
+                for (int s = 0; s < S; ++s)
+                    rank[s] += (w.x < mine[s] ? 1 : 0) + (w.y < mine[s] ? 1 : 0) + (w.z < mine[s] ? 1 : 0) +
+                               (w.w < mine[s] ? 1 : 0);
+            }
+#pragma unroll
+            for (int s = 0; s < S; ++s) sum += lane + 32 * s < found ? (uint32_t)rank[s] : 0u;
+            sum = __reduce_add_sync(kFull, sum);
+            __syncwarp();
+            if (sum != (uint32_t)(found * (found - 1) / 2)) {  // equal distances
+#pragma unroll
+                for (int s = 0; s < S; ++s)
+                    if (lane + 32 * s < found) ts.sel[lane + 32 * s] = id[s];
+                __syncwarp();
+                for (int f = 0; f < found; ++f) {
+                    const uint32_t w = key[f], o = ts.sel[f];
+#pragma unroll
+                    for (int s = 0; s < S; ++s) rank[s] += w == mine[s] && o < id[s] ? 1 : 0;
+                }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                if (lane + 32 * s < found) {
+                    key[rank[s]] = mine[s];
+                    ts.sel[rank[s]] = id[s];
+                }
+            __syncwarp();
+        }
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -843,6 +871,25 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     }
 }
 
+// One query by the list search.
+template <int S>
+__device__ __forceinline__ void list_query(const MapView &m, const float4 *q, size_t qi, int k, float r2cap,
+                                           uint32_t *idx_out, float *d2_out, WarpScratch &ws, int lane) {
+    const uint64_t cap = make_key(r2cap, 0xffffffffu);
+    const float4 p = q[qi];
+    Knn<S> kn;
+    kn.reset(cap, k);
+    knn_search<S>(m, mk3(p.x, p.y, p.z), kn, ws, lane, cap);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int j = lane * S + s;
+        if (j < k) {
+            idx_out[qi * k + j] = (uint32_t)kn.key[s];
+            d2_out[qi * k + j] = key_d2(kn.key[s]);
+        }
+    }
+}
+
 // The queries knn_kernel left, by the list search (grid-stride, 32 queries'
 // marks at a time).
 template <int S>
@@ -850,26 +897,23 @@ __global__ void __launch_bounds__(128) knn_rest_kernel(MapView m, const float4 *
                                                        uint32_t *idx_out, float *d2_out) {
     __shared__ WarpScratch ws[4];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint64_t cap = make_key(r2cap, 0xffffffffu);
     for (uint64_t base = ((uint64_t)blockIdx.x * 4 + wib) * 32; base < nq; base += (uint64_t)gridDim.x * 128) {
         const uint64_t mine = base + lane;
         unsigned left = __ballot_sync(kFull, mine < nq && idx_out[mine * k] == kKnnLeft);
         for (; left; left &= left - 1) {
             const uint64_t qi = base + __ffs(left) - 1;
-            const float4 p = q[qi];
-            Knn<S> kn;
-            kn.reset(cap, k);
-            knn_search<S>(m, mk3(p.x, p.y, p.z), kn, ws[wib], lane, cap);
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-                const int j = lane * S + s;
-                if (j < k) {
-                    idx_out[qi * k + j] = (uint32_t)kn.key[s];
-                    d2_out[qi * k + j] = key_d2(kn.key[s]);
-                }
-            }
+            list_query<S>(m, q, qi, k, r2cap, idx_out, d2_out, ws[wib], lane);
         }
     }
+}
+
+// Every query by the list search: thin maps.
+template <int S>
+__global__ void __launch_bounds__(128) knn_list_kernel(MapView m, const float4 *q, uint32_t nq, int k, float r2cap,
+                                                       uint32_t *idx_out, float *d2_out) {
+    __shared__ WarpScratch ws[4];
+    const uint32_t qi = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (qi < nq) list_query<S>(m, q, qi, k, r2cap, idx_out, d2_out, ws[threadIdx.x >> 5], threadIdx.x & 31);
 }
 
 // The scene of global chunk c: the last descriptor whose chunk_begin <= c.
@@ -1006,15 +1050,19 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
 }
 
 cudaError_t knn_query(const MapView &m, int map, const float4 *q, uint32_t nq, int k, float radius,
-                      uint32_t *idx, float *d2, cudaStream_t s) {
+                      uint32_t *idx, float *d2, cudaStream_t s, bool thin) {
     if (nq == 0) return cudaSuccess;
     const float r2 = radius * radius;
     const dim3 grid((nq + kTileWarps - 1) / kTileWarps), block(kTileWarps * 32);
     const dim3 rest(std::min<uint32_t>((nq + 127) / 128, 1024));
     const int smem = (int)(kTileWarps * sizeof(TileScratch));
 #define PM_KNN_LAUNCH(SL)                                                                 \
-    knn_kernel<SL><<<grid, block, smem, s>>>(m, map, q, nq, k, r2, idx, d2);              \
-    knn_rest_kernel<SL><<<rest, 128, 0, s>>>(m, q, nq, k, r2, idx, d2)
+    if (thin) {                                                                           \
+        knn_list_kernel<SL><<<(nq + 3) / 4, 128, 0, s>>>(m, q, nq, k, r2, idx, d2);       \
+    } else {                                                                              \
+        knn_kernel<SL><<<grid, block, smem, s>>>(m, map, q, nq, k, r2, idx, d2);          \
+        knn_rest_kernel<SL><<<rest, 128, 0, s>>>(m, q, nq, k, r2, idx, d2);               \
+    }
     switch ((k + 31) / 32) {
         case 1: PM_KNN_LAUNCH(1); break;
         case 2: PM_KNN_LAUNCH(2); break;
@@ -1022,7 +1070,7 @@ cudaError_t knn_query(const MapView &m, int map, const float4 *q, uint32_t nq, i
         default: PM_KNN_LAUNCH(4); break;
     }
 #undef PM_KNN_LAUNCH
-    note_launches(2);
+    note_launches(thin ? 1 : 2);
     return cudaGetLastError();
 }
 
