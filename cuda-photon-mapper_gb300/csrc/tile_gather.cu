@@ -592,9 +592,9 @@ __device__ __forceinline__ float expected(v3 x, float ub, int mid, unsigned mask
     return k * __fdividef(v, 4.1887902f * mean * mean * mean);
 }
 
-// One chunk (groups of 32 consecutive queries of the sorted order, from
-// query chunk * 32 * groups) of a scene, with the warp's arguments set.
-template <int S>
+// One chunk (groups of W consecutive queries of the sorted order, from query
+// chunk * W * groups) of a scene, with the warp's arguments set.
+template <int S, uint32_t W>
 __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf, const MapView &vol,
                                            const float4 *qa, const float4 *qd, const uint32_t *order,
                                            uint32_t n, uint32_t chunk, int groups,
@@ -602,13 +602,13 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
     TileScratch &ts = scratch();
     const int lane = threadIdx.x & 31;
     const float rcap = sqrtf(r2cap);
-    const uint32_t wfirst = chunk * (uint32_t)(32 * groups);
+    const uint32_t wfirst = chunk * (W * (uint32_t)groups);
     // exact distances known so far: those of the previous group
     int nknown = 0, wkind = -1;
     for (int g = 0; g < groups; ++g) {
-        const uint32_t first = wfirst + (uint32_t)(32 * g);
+        const uint32_t first = wfirst + W * (uint32_t)g;
         if (first >= n) break;
-        const uint32_t cnt = min(32u, n - first);
+        const uint32_t cnt = min(W, n - first);
         Query q;
         q.x = q.dirv = mk3(0.f, 0.f, 0.f);
         q.map = 1;
@@ -704,7 +704,7 @@ __device__ __forceinline__ void tile_chunk(const PScene &Sc, const MapView &surf
     }
 }
 
-template <int S>
+template <int S, uint32_t W>
 __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     query_knn_tile_kernel(PScene Sc, MapView surf, MapView vol, const float4 *qa, const float4 *qd,
                           const uint32_t *order, uint32_t n, const uint32_t *n_dev, int groups,
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     TileScratch &ts = scratch();
     if (lane < kStCount) ts.st[lane] = 0;
     __syncwarp();
-    const uint32_t nchunks = (n + 32u * (uint32_t)groups - 1u) / (32u * (uint32_t)groups);
+    const uint32_t nchunks = (n + W * (uint32_t)groups - 1u) / (W * (uint32_t)groups);
     // persistent warps: each takes the next chunk from the counter until
     // none is left, so a block's resources are never held by finished warps
     // waiting on a slow one
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
         if (lane == 0) chunk = atomicAdd(chunk_counter, 1u);
         chunk = __shfl_sync(kFull, chunk, 0);
         if (chunk >= nchunks) break;
-        tile_chunk<S>(Sc, surf, vol, qa, qd, order, n, chunk, groups, r2cap, raw, out);
+        tile_chunk<S, W>(Sc, surf, vol, qa, qd, order, n, chunk, groups, r2cap, raw, out);
     }
     __syncwarp();
     if (stats && lane < kStCount && ts.st[lane]) atomicAdd(&stats[lane], ts.st[lane]);
@@ -952,7 +952,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
                       d.k, raw);
             cur = sidx;
         }
-        tile_chunk<S>(*d.sc, d.surf, d.vol, d.qa, d.qd, d.order, d.n, chunk - d.chunk_begin, groups,
+        tile_chunk<S, 32>(*d.sc, d.surf, d.vol, d.qa, d.qd, d.order, d.n, chunk - d.chunk_begin, groups,
                       d.r2cap, raw, d.val);
     }
     __syncwarp();
@@ -1013,6 +1013,9 @@ __global__ void __launch_bounds__(128)
 
 }  // namespace
 
+// The estimate pass's warps on the GPU at once.
+static uint32_t tile_warps(int sm_count) { return (uint32_t)std::max(sm_count, 1) * kTileBlocks * kTileWarps; }
+
 cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView &vol,
                              const float4 *qa, const float4 *qd, const uint32_t *order, uint32_t n,
                              const uint32_t *n_dev, int k, float radius, bool raw, float4 *val,
@@ -1020,7 +1023,12 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
     if (n == 0) return cudaSuccess;
     const int groups = tile_groups(n, sm_count);
     const float r2 = radius * radius;
-    const uint32_t chunks = tile_chunks(n, groups);
+    // Few queries: groups of 8, so that no warp waits for 32 of them while
+    // others have none. 2^14 picks, k = 128, 1M records 1.22 -> 0.53 ms; 2^17,
+    // k = 16, 20,000 records 0.49 -> 0.38; 2^18, k = 16 0.58 -> 0.55; 2^19 0.78 ->
+    // 0.88, k = 128 2.61 -> 2.54.
+    const bool few = n < 64u * tile_warps(sm_count);
+    const uint32_t chunks = few ? (n + 7) / 8 : tile_chunks(n, groups);
     const dim3 grid((chunks + kTileWarps - 1) / kTileWarps), block(kTileWarps * 32);
     const int smem = (int)(kTileWarps * sizeof(TileScratch));
     const dim3 dgrid(std::max(sm_count, 1) * 8);
@@ -1029,14 +1037,16 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
     if (e != cudaSuccess) return e;
     int per_sm = 1;
     // persistent tile launch: as many blocks as fit on the GPU at once
+#define PM_TILE_KERNEL(SL, W)                                                                           \
+    e = cudaFuncSetAttribute(query_knn_tile_kernel<SL, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+    if (e != cudaSuccess) return e;                                                                     \
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, query_knn_tile_kernel<SL, W>, kTileWarps * 32, smem); \
+    if (e != cudaSuccess) return e;                                                                     \
+    query_knn_tile_kernel<SL, W><<<std::min<uint32_t>(grid.x, (uint32_t)std::max(sm_count, 1) * (uint32_t)std::max(per_sm, 1)), \
+                                   block, smem, s>>>(S, surf, vol, qa, qd, order, n, n_dev, groups, k, \
+                                                     r2, raw, val, buf.defer, buf.defer_n, buf.defer_n + 1, buf.stats)
 #define PM_TILE_LAUNCH(SL)                                                                              \
-    e = cudaFuncSetAttribute(query_knn_tile_kernel<SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
-    if (e != cudaSuccess) return e;                                                                     \
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, query_knn_tile_kernel<SL>, kTileWarps * 32, smem); \
-    if (e != cudaSuccess) return e;                                                                     \
-    query_knn_tile_kernel<SL><<<std::min<uint32_t>(grid.x, (uint32_t)std::max(sm_count, 1) * (uint32_t)std::max(per_sm, 1)), \
-                                block, smem, s>>>(S, surf, vol, qa, qd, order, n, n_dev, groups, k, \
-                                                  r2, raw, val, buf.defer, buf.defer_n, buf.defer_n + 1, buf.stats); \
+    if (few) { PM_TILE_KERNEL(SL, 8); } else { PM_TILE_KERNEL(SL, 32); }                                \
     deferred_kernel<SL><<<dgrid, 128, 0, s>>>(S, surf, vol, qa, qd, buf.defer, buf.defer_n, k, r2, raw, val)
     switch ((k + 31) / 32) {
         case 1: PM_TILE_LAUNCH(1); break;
@@ -1045,6 +1055,7 @@ cudaError_t knn_values_tiles(const PScene &S, const MapView &surf, const MapView
         default: PM_TILE_LAUNCH(4); break;
     }
 #undef PM_TILE_LAUNCH
+#undef PM_TILE_KERNEL
     note_launches(2);
     return cudaGetLastError();
 }
@@ -1114,7 +1125,7 @@ uint32_t tile_chunks(uint32_t n, int groups) { return (n + 32u * groups - 1) / (
 // 25.4 / 25.9, 46M - / 62.6 / 59.8: four from 64 chunks a warp on, one below
 // 8 chunks of two.
 int tile_groups(uint64_t n, int sm_count) {
-    const uint64_t warps = (uint64_t)std::max(sm_count, 1) * kTileBlocks * kTileWarps;
+    const uint64_t warps = tile_warps(sm_count);
     if (n >= 128u * 64u * warps) return 4;
     return n >= 64u * 8u * warps ? 2 : 1;
 }
