@@ -714,7 +714,7 @@ def estimate_roofline(r, steps, k, peak, peak_kind, traffic):
             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
             "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes,
             "formula": "gathers x (32 B x k + 52 B), over the CUDA-event time of the k-NN "
-                       "estimate pass (anchor, shared-candidate and deferred launches; events "
+                       "estimate pass (shared-candidate and deferred launches; events "
                        "on the render stream)"}
 
 

@@ -2,8 +2,8 @@
 // order, one candidate set per group of neighbouring queries, and the k-NN
 // queries of points (pm_knn) by the same search.
 //
-// A warp takes chunks of 1, 2 or 4 consecutive groups of 32 queries of the
-// (map, Hilbert code) order. The k-th-neighbour distance d(x) (capped at the
+// A warp takes chunks of 1, 2 or 4 consecutive groups of 32 queries (where
+// queries are few, one group of 8) of the (map, Hilbert code) order. The k-th-neighbour distance d(x) (capped at the
 // gather radius) is 1-Lipschitz in the query position, so exact distances d_j
 // at points x_j bound it everywhere: d(x) <= min_j (d_j + |x - x_j|). A
 // chunk's first group is bounded by its middle query, which is answered by
@@ -25,8 +25,9 @@
 // estimate's sum is order-independent (knn_core.cuh), so every value is
 // bit-identical to the list search's.
 //
-// Bound by instruction issue (75 % of the slots with 7 warps a scheduler);
-// the selected records' flux comes from L1 and L2. Candidates in registers
+// Bound by instructions and the latency between them (64 % of the issue slots
+// with 7 warps a scheduler on preset 2, 58 % on preset 3); the selected
+// records' flux comes from L1 and L2. Candidates in registers
 // instead of shared memory make a query's distances and counts straight-line
 // code without loads, need no lists of the certain and the doubtful
 // candidates, and leave most of the L1 to the flux. Estimate pass (GB300,
@@ -34,8 +35,8 @@
 // two bounds ranked, 16.9 / 113.0 / 45.4 ms; in registers 12.0 / 76.0 / 34.5;
 // Hilbert instead of Morton order, a lane per channel for the last rounding
 // 10.0 / 64.0 / 29.9; expected set sizes instead of failed collections 9.8 /
-// 62.6 / 29.7; no separate anchor launch, 10 candidates per lane 10.0 / 59.8 /
-// 25.9.
+// 62.6 / 29.7; the first bound found in the pass instead of a launch before it,
+// 10 candidates per lane 10.0 / 59.8 / 25.9; now 10.2 / 60.0 / 24.7.
 #include <algorithm>
 
 #include "cache.cuh"

@@ -205,7 +205,7 @@ PM_API pm_status pm_update_scene(pm_ctx *ctx, const pm_scene *scene);
  * the stream once to learn the map sizes. */
 PM_API pm_status pm_emit(pm_ctx *ctx, cudaStream_t stream);
 /* Builds the kd-tree of each map: level-by-level median splits along each
- * cell's longest axis (stable radix sort per level) and tight node boxes. */
+ * node's longest axis (histogram and stable partition) and tight node boxes. */
 PM_API pm_status pm_build(pm_ctx *ctx, cudaStream_t stream);
 /* Renders one frame: eye rays, specular chains, the volume march and the
  * surface radiance estimate. radiance (nullable, device): width*height
@@ -216,7 +216,7 @@ PM_API pm_status pm_render(pm_ctx *ctx, float4 *radiance, uchar4 *rgba, cudaStre
  * query list: no host synchronisation, slower on large frames. pm_render
  * builds the frame's query list (one stream synchronisation to size it),
  * estimates the queries in spatial order from one shared candidate set per
- * group of 32 neighbours, and sums them per pixel with this kernel's
+ * group of up to 32 neighbours, and sums them per pixel with this kernel's
  * arithmetic; the k-NN sets are exact and the estimate sum is independent
  * of the order of the records, so the two are bit-identical. */
 PM_API pm_status pm_render_single_kernel(pm_ctx *ctx, float4 *radiance, uchar4 *rgba,
