@@ -26,8 +26,8 @@
 // Against sorting every level (two 8-bit radix passes over 12-byte pairs
 // and a key pass), a level moves each record once, 16 B read and written,
 // and its 2-byte bin three times. Measured (GB300, both maps): 2 x 8M records
-// 15.8 -> 3.3 ms, 2 x 1M 2.75 -> 0.39 ms, 2 x 100,000 1.46 -> 0.10 ms, one map
-// of 20,011 0.44 -> 0.065 ms.
+// 15.8 -> 3.13 ms, 2 x 1M 2.75 -> 0.36 ms, 2 x 100,000 1.46 -> 0.09 ms, one map
+// of 20,011 0.44 -> 0.06 ms.
 #include "launch_count.cuh"
 #include "kdtree.cuh"
 
@@ -102,6 +102,19 @@ __device__ __forceinline__ float coord(float4 p, int a) { return a == 0 ? p.x : 
 // not finite, which the box leaves out.
 __device__ __forceinline__ uint32_t min_word(float x) { return isfinite(x) ? ~kd_flip(x) : 0u; }
 __device__ __forceinline__ uint32_t max_word(float x) { return isfinite(x) ? kd_flip(x) : 0u; }
+
+// Lane a's value is the warp's maximum of w[a] (a < N): one addition to a box
+// then takes one atomic of N lanes.
+template <int N>
+__device__ __forceinline__ uint32_t box_lane(const uint32_t (&w)[N], int lane) {
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int a = 0; a < N; ++a) {
+        const uint32_t x = __reduce_max_sync(0xffffffffu, w[a]);
+        if (lane == a) mine = x;
+    }
+    return mine;
+}
 
 // The split axis, the box's lower side along it and bins per unit length. A
 // box without finite records, or of no extent, puts every record in bin 0.
@@ -342,14 +355,9 @@ __global__ void __launch_bounds__(kTileThreads)
         eq += __popc(me[i]);
     }
     if (!boxes) return;
-#pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        const uint32_t x = __reduce_max_sync(kFull, wl[a]), y = __reduce_max_sync(kFull, wr[a]);
-        if (lane == 0) {
-            if (x) atomicMax(&bb[a], x);
-            if (y) atomicMax(&bb[6 + a], y);
-        }
-    }
+    const uint32_t wb[12] = {wl[0], wl[1], wl[2], wl[3], wl[4], wl[5], wr[0], wr[1], wr[2], wr[3], wr[4], wr[5]};
+    const uint32_t mine = box_lane(wb, lane);
+    if (mine) atomicMax(&bb[lane], mine);
     __syncthreads();
     if (threadIdx.x < 12 && bb[threadIdx.x]) {
         const uint32_t j = n.node - m.node0, side = threadIdx.x / 6, a = threadIdx.x % 6;
@@ -373,7 +381,7 @@ extern __shared__ __align__(16) unsigned char mid_smem[];
 // stable partition as the launches above (and so the same layout), with two
 // cluster barriers a level in place of three launches. A CTA reads the
 // node's other histograms in their shared memory and writes its records to
-// their place there. Bound by latency: four levels of a small map in 24 us
+// their place there. Bound by latency: four levels of a small map in 23 us
 // (launches: 19.5 us a level), of 2 x 8M records in 0.58 ms (0.82). Two CTAs
 // an SM against one: 2 x 8M built in 3.30 / 3.64 ms, small maps the same;
 // clusters of 16 CTAs and five levels: 100,000 records 5 us faster, 8M 0.3 ms
@@ -530,14 +538,9 @@ __global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads,
             eq += __popc(me[i]);
         }
         if (boxes) {
-#pragma unroll
-            for (int a = 0; a < 6; ++a) {
-                const uint32_t x = __reduce_max_sync(kFull, wl[a]), y = __reduce_max_sync(kFull, wr[a]);
-                if (lane == 0) {
-                    if (x) atomicMax(&ms.bb[a], x);
-                    if (y) atomicMax(&ms.bb[6 + a], y);
-                }
-            }
+            const uint32_t wb[12] = {wl[0], wl[1], wl[2], wl[3], wl[4], wl[5], wr[0], wr[1], wr[2], wr[3], wr[4], wr[5]};
+            const uint32_t mine = box_lane(wb, lane);
+            if (mine) atomicMax(&ms.bb[lane], mine);
             __syncthreads();
             if (threadIdx.x < 12 && ms.bb[threadIdx.x]) {
                 const int side = threadIdx.x / 6, a = threadIdx.x % 6;
@@ -646,10 +649,11 @@ __device__ __forceinline__ void warp_split(SubScratch &ss, uint16_t *ord, int ba
 // histogram per node and five barriers per level; nodes of 128 and 64 are
 // sorted by one warp in registers. Only the 2-byte places move; the records
 // stay where they were loaded. Bound by latency (barriers, shared-memory
-// round trips): 3 CTAs per SM, 0.50 ms for 8M records (sorting every level
-// of the subtree in shared memory: 2.27 ms), 32 us for a small map.
+// round trips): 0.44 ms for 8M records (sorting every level of the subtree in
+// shared memory: 2.27 ms), 27 us for a small map. 2 CTAs per SM at 64 registers
+// (3 at 40, which spill: 0.50 ms and 31 us; 1: 8M slower by a quarter).
 template <class Maps>
-__global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_constant__ Maps maps) {
+__global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_constant__ Maps maps) {
     SubScratch &ss = *reinterpret_cast<SubScratch *>(sub_smem);
     const KdMap &m = maps.of_sub(blockIdx.x);
     const uint32_t j = blockIdx.x - m.sub0;
@@ -690,11 +694,8 @@ __global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_
             }
         }
         if (warp * kWarpSpan < cnt) {
-#pragma unroll
-            for (int a = 0; a < 6; ++a) {
-                const uint32_t x = __reduce_max_sync(kFull, w[a]);
-                if (lane == 0 && x) atomicMax(&ss.bb[node][a], x);
-            }
+            const uint32_t mine = box_lane(w, lane);
+            if (mine) atomicMax(&ss.bb[node][lane], mine);
         }
         __syncthreads();
         uint32_t b[kSubItems];
@@ -715,9 +716,13 @@ __global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_
             const int ncnt = min(span, cnt - warp * span), half = min(span >> 1, ncnt);
             uint32_t v[kSubBins / 32], s = 0;
 #pragma unroll
-            for (int i = 0; i < kSubBins / 32; ++i) {
-                v[i] = ss.hist[warp * kSubBins + lane * (kSubBins / 32) + i];
-                s += v[i];
+            for (int i = 0; i < kSubBins / 32; i += 4) {
+                const uint4 h = *reinterpret_cast<const uint4 *>(&ss.hist[warp * kSubBins + lane * (kSubBins / 32) + i]);
+                v[i] = h.x;
+                v[i + 1] = h.y;
+                v[i + 2] = h.z;
+                v[i + 3] = h.w;
+                s += (h.x + h.y) + (h.z + h.w);
             }
             uint32_t incl = s;
 #pragma unroll
@@ -750,7 +755,8 @@ __global__ void __launch_bounds__(kSubThreads, 3) kd_finish_kernel(const __grid_
             }
         }
         if (lane == 0) ss.wcnt[warp] = tot;
-        for (int i = tid; i < kSubMax / 256 * kSubBins; i += kSubThreads) ss.hist[i] = 0;
+        for (int i = 4 * tid; i < kSubMax / 256 * kSubBins; i += 4 * kSubThreads)
+            *reinterpret_cast<uint4 *>(&ss.hist[i]) = make_uint4(0u, 0u, 0u, 0u);
         for (int i = tid; i < kSubMax / 256 * 6; i += kSubThreads) (&ss.bb[0][0])[i] = 0;
         __syncthreads();
         if (warp * kWarpSpan < cnt) {
