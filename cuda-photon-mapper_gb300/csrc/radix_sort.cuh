@@ -5,7 +5,7 @@
 // (count -> scan -> sort -> reduce) runs without a host round trip; max_n
 // only sizes the grids. Each 8-bit pass is reduce-then-scan: a per-tile
 // digit histogram, one exclusive scan over all (digit, tile) counts, and a
-// scatter in which every tile ranks its items with warp match masks, so
+// scatter in which every tile ranks its items with warp ballots, so
 // equal keys keep their input order.
 #pragma once
 #include <cuda_runtime.h>
