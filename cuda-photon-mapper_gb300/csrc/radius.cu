@@ -12,12 +12,12 @@
 // per-lane Kahan sums meet in a compensated butterfly. The reference's
 // double literals promote the weight, w * (1 - sqrt(d)) / exposure, to double
 // precision, which this GPU runs at a small fraction of its single-precision
-// rate; it is taken here as unevaluated sums of two floats (Dekker 1971), some
-// 47 bits, and rounded once: 131,072 points over 500,000 records 688 -> 165 us.
-// An exposure whose reciprocal
-// such a sum cannot hold keeps the double expression.
+// rate; radius_weight.cuh finds the same bits in single precision, and takes
+// the double expression where it cannot tell them: 131,072 points over 500,000
+// records 688 -> 165 us.
 #include "gather.cuh"
 #include "launch_count.cuh"
+#include "radius_weight.cuh"
 
 namespace pm {
 namespace {
@@ -48,22 +48,6 @@ __device__ __forceinline__ float warp_total(float sum, float comp) {
     return s + e;
 }
 
-// w * (1 - s) / exposure, rounded to float once; inv: 1 / exposure as two
-// floats.
-__device__ __forceinline__ float weight_of(float w, float s, float2 inv) {
-    // 1 - s exactly: u + ul
-    const float u = 1.0f - s;
-    const float bb = u - 1.0f;
-    const float ul = (1.0f - (u - bb)) + (-s - bb);
-    // times inv: p + pl
-    const float p = u * inv.x;
-    const float pl = __fmaf_rn(u, inv.x, -p) + __fmaf_rn(u, inv.y, ul * inv.x);
-    // times w
-    const float r = w * p;
-    return r + (__fmaf_rn(w, p, -r) + w * pl);
-}
-
-template <bool kDouble>
 __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const float4 *pts,
                                                              const float4 *nrm, uint32_t nq,
                                                              float sq_radius, float exposure, float2 inv,
@@ -101,9 +85,7 @@ __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const fl
                         const float4 pw = __ldg(&m.pow[r]);
                         const float4 dir = __ldg(&m.dir[r]);
                         const float nd = nv.x * dir.x + nv.y * dir.y + nv.z * dir.z;
-                        float w = fmaxf(0.0f, -nd);
-                        if (kDouble) w = (float)((double)w * ((1.0 - (double)sqrtf(d)) / (double)exposure));
-                        else w = weight_of(w, sqrtf(d), inv);
+                        const float w = radius_weight(fmaxf(0.0f, -nd), sqrtf(d), exposure, inv.x, inv.y);
                         kahan(sx, cx, pw.x * w);
                         kahan(sy, cy, pw.y * w);
                         kahan(sz, cz, pw.z * w);
@@ -139,17 +121,9 @@ __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const fl
 cudaError_t radius_gather(const MapView &m, const float4 *pts, const float4 *nrm, uint32_t nq,
                           float sq_radius, float exposure, float4 *out, cudaStream_t s) {
     if (nq == 0) return cudaSuccess;
-    // 1 / exposure as a float and the float nearest to the rest
-    const double r = 1.0 / (double)exposure;
-    const bool fits = r > -1e30 && r < 1e30 && (r > 1e-20 || r < -1e-20);
-    float2 inv = make_float2(0.0f, 0.0f);
-    if (fits) {
-        inv.x = (float)r;
-        inv.y = (float)(r - (double)inv.x);
-    }
-    const dim3 grid((nq + kWarps - 1) / kWarps), block(kWarps * 32);
-    if (fits) radius_kernel<false><<<grid, block, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
-    else radius_kernel<true><<<grid, block, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
+    float2 inv;
+    radius_inverse(exposure, &inv.x, &inv.y);
+    radius_kernel<<<(nq + kWarps - 1) / kWarps, kWarps * 32, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
     note_launch();
     return cudaGetLastError();
 }
