@@ -738,8 +738,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
 // selected records are put in order by their ranks: every lane counts the
 // distances below its own, and where two are equal the indices decide. A
 // query without a radius that fits its set (more records at one distance
-// than the registers hold) is marked in its first index and left to
-// knn_rest_kernel. Bound by instruction issue and the walk's L2 latency.
+// than the registers hold), or whose set holds records without a distance, is
+// marked in its first index and left to knn_rest_kernel. Bound by instruction issue and the walk's L2 latency.
 // Measured (GB300; the list search before): 262,144 queries, k = 100, 1M
 // points 3.62 -> 1.59 ms; 32,768 queries, k = 32, 100,000 points 225 -> 110 us.
 template <int S>
@@ -757,8 +757,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     uint32_t *idx = idx_out + (size_t)qi * k;
     float *dist = d2_out + (size_t)qi * k;
     int n = 0, found = 0;
+    float r = targs().rcap;
     if (m.n > 0) {
-        const float r = single_bound(mid, 0, targs().rcap, &n);
+        r = single_bound(mid, 0, targs().rcap, &n);
         if (!(r >= 0.0f)) {
             if (lane == 0) idx[0] = kKnnLeft;
             return;
@@ -861,6 +862,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
                 }
             __syncwarp();
         }
+    }
+    // fewer than k within a radius that held k records: some of those have no
+    // distance (NaN), others may lie beyond the radius
+    if (found < k && r < targs().rcap) {
+        if (lane == 0) idx[0] = kKnnLeft;
+        return;
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) {
