@@ -7,10 +7,12 @@
 // the level), so no child pointers or ranges are stored.
 //
 // Top-down. A node is split at its median along the longest axis of its
-// records' bounding box (the root: of the scene box): the coordinate is cut
-// into bins of that box, a histogram finds the bin holding the median, and
-// one stable partition moves the records below the bin to the left child,
-// those above it to the right, and the bin's own records left until the
+// records' bounding box (the root: of the scene box): the coordinate is
+// quantised to 16 bits of that box, a histogram over its upper bits finds the
+// bin holding the median -- and one over the lower bits the part of that bin,
+// where the bin holds more of the node than an even spread would put there --
+// and one stable partition moves the records below that bin (or part) to the
+// left child, those above it to the right, and its own records left until the
 // left child is full, in their present order. The layout is therefore
 // deterministic. It does not affect a query's result: the boxes that are
 // tested are the exact bounds of each node's records.
@@ -25,9 +27,9 @@
 //
 // Against sorting every level (two 8-bit radix passes over 12-byte pairs
 // and a key pass), a level moves each record once, 16 B read and written,
-// and its 2-byte bin three times. Measured (GB300, both maps): 2 x 8M records
-// 15.8 -> 3.13 ms, 2 x 1M 2.75 -> 0.36 ms, 2 x 100,000 1.46 -> 0.09 ms, one map
-// of 20,011 0.44 -> 0.06 ms.
+// and its 2-byte key three times. Measured (GB300, both maps): 2 x 8M records
+// 15.7 -> 3.03 ms, 2 x 1M 2.75 -> 0.36 ms, 2 x 100,000 1.46 -> 0.10 ms, one map
+// of 20,011 0.44 -> 0.06 ms (half of it in one clump: 0.074).
 #include "launch_count.cuh"
 #include "kdtree.cuh"
 
@@ -40,11 +42,23 @@ namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
 
+constexpr uint32_t kKeys = 65536;  // values of a split coordinate
+
 // Split levels. 1024 bins: the records of the median's bin that go left by
 // their order alone are 1/1024 of the node's extent thick, a few percent of
-// a leaf's width at the root of an 8M-record map, and less below; 4 KB of
-// shared histogram.
+// a leaf's width at the root of an 8M-record map of even density, and less
+// below; 4 KB of shared histogram. A bin that holds more than 1/64 of its node
+// (16 times the even share) is cut into its 64 key values: the children of a
+// node with a dense clump would overlap in the clump, level after level. Leaves
+// within reach of a k = 100 query in a clump of 0.0003 of the box that holds a
+// fifth of 262,144 records: 34.6 by 1024 bins alone, 16.2 (a clump of 0.0001
+// with half of them: 120 and 19.9; even density 15.9 both; limits of 1/16 to
+// 1/256 the same within 2 %); 65,536 such queries 2.91 -> 0.72 ms (5.09 -> 1.54).
 constexpr int kBins = 1024;
+constexpr int kSub = (int)kKeys / kBins, kSubShift = 6;
+constexpr int kRow = kBins + kSub;     // words of a node's histograms
+constexpr uint32_t kCrowd = 64;        // a bin of more than a node's records / kCrowd
+static_assert(kSub == 1 << kSubShift && kSub == 64, "two values of a bin a lane");
 constexpr uint32_t kTile = 4096;
 constexpr int kTileThreads = 512;
 constexpr int kTileWarps = kTileThreads / 32;
@@ -59,7 +73,9 @@ static_assert(kMidCtas == 8, "the portable cluster size");
 constexpr int kSubThreads = 512;
 constexpr int kSubWarps = kSubThreads / 32;
 constexpr int kSubItems = kSubMax / kSubThreads;
-constexpr int kSubBins = 256;
+constexpr int kSubBins = 256;           // each of 256 key values
+constexpr uint32_t kSubCrowd = 16;
+constexpr uint32_t kMark = 0x80000000u;  // of a crowded bin
 constexpr int kWarpSpan = kSubMax / kSubWarps;   // records of a warp: nodes this small are split by one warp
 constexpr int kSubLeaves = kSubMax / 32;
 static_assert(kWarpSpan == 128, "the warp-level splits sort 4 records per lane");
@@ -116,29 +132,70 @@ __device__ __forceinline__ uint32_t box_lane(const uint32_t (&w)[N], int lane) {
     return mine;
 }
 
-// The split axis, the box's lower side along it and bins per unit length. A
-// box without finite records, or of no extent, puts every record in bin 0.
+// The split axis, the box's lower side along it and key values per unit
+// length. A box without finite records, or of no extent, gives every record
+// key 0.
 struct Cut {
     int axis;
     float lo, inv;
 };
-__device__ __forceinline__ Cut cut_of(float3 lo, float3 hi, float bins) {
+__device__ __forceinline__ Cut cut_of(float3 lo, float3 hi) {
     const float ex = hi.x - lo.x, ey = hi.y - lo.y, ez = hi.z - lo.z;
     Cut c;
     c.axis = (ex >= ey && ex >= ez) ? 0 : (ey >= ez ? 1 : 2);
     c.lo = c.axis == 0 ? lo.x : (c.axis == 1 ? lo.y : lo.z);
     const float e = c.axis == 0 ? ex : (c.axis == 1 ? ey : ez);
-    c.inv = e > 0.0f ? bins / e : 0.0f;
+    c.inv = e > 0.0f ? (float)kKeys / e : 0.0f;
     return c;
 }
-__device__ __forceinline__ Cut cut_of_words(const uint32_t *w, float bins) {
+__device__ __forceinline__ Cut cut_of_words(const uint32_t *w) {
     return cut_of(make_float3(kd_unflip(~w[0]), kd_unflip(~w[1]), kd_unflip(~w[2])),
-                  make_float3(kd_unflip(w[3]), kd_unflip(w[4]), kd_unflip(w[5])), bins);
+                  make_float3(kd_unflip(w[3]), kd_unflip(w[4]), kd_unflip(w[5])));
 }
-// NaN and everything below the box: 0; +inf and above: the last bin.
-__device__ __forceinline__ uint32_t bin_of(const Cut &c, float4 p, uint32_t bins) {
+// The key of a record. NaN and everything below the box: 0; +inf and above:
+// the last.
+__device__ __forceinline__ uint32_t key_of(const Cut &c, float4 p) {
     const float f = (coord(p, c.axis) - c.lo) * c.inv;
-    return !(f > 0.0f) ? 0u : (f >= (float)(bins - 1u) ? bins - 1u : (uint32_t)f);
+    return !(f > 0.0f) ? 0u : (f >= (float)(kKeys - 1u) ? kKeys - 1u : (uint32_t)f);
+}
+constexpr uint32_t kNoKey = 2u * kKeys - 1u;  // of no record: in no bin, beyond every key
+
+// A node's split: its records with keys below lo (there are `less`) go first,
+// then those with keys from lo to lo + span (`equal` of them), then the others,
+// each in their present order. The left child ends among the middle ones.
+struct Split {
+    uint32_t lo, span, less, equal;
+    // the place in the node of a record at pos, lb and eb of those before it
+    // being below and in the middle
+    __device__ __forceinline__ uint32_t place(bool below, bool middle, uint32_t pos, uint32_t lb, uint32_t eb) const {
+        return below ? lb : (middle ? less + eb : less + equal + (pos - lb - eb));
+    }
+};
+
+// The part of the median's bin that holds the median: lane l has the records
+// a and b of the bin's values 2l and 2l + 1. less are below the bin.
+__device__ __forceinline__ Split split_bin(uint32_t bin, uint32_t less, uint32_t half, uint32_t a, uint32_t b,
+                                           int lane) {
+    uint32_t incl = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const uint32_t before = less + incl - a - b;
+    const unsigned at = __ballot_sync(kFull, before <= half && half < before + a + b);
+    const int src = __ffs(at) - 1;  // one lane: half is within the bin's records
+    const bool second = half >= before + a;
+    Split sp;
+    sp.lo = (bin << kSubShift) + 2u * (uint32_t)src + __shfl_sync(kFull, second ? 1u : 0u, src);
+    sp.span = 0u;
+    sp.less = __shfl_sync(kFull, second ? before + a : before, src);
+    sp.equal = __shfl_sync(kFull, second ? b : a, src);
+    return sp;
+}
+// The split at a whole bin.
+__device__ __forceinline__ Split split_at(uint4 thr) {
+    return Split{thr.x << kSubShift, (uint32_t)kSub - 1u, thr.y, thr.z};
 }
 
 // The buffer a split level reads: level 0 the input, then the partner
@@ -166,7 +223,7 @@ __device__ __forceinline__ TileNode tile_node(const KdMap &m, uint32_t t, int l)
     return n;
 }
 
-// Launch 1 of a split level: every record's bin, and the node's histogram.
+// Launch 1 of a split level: every record's key, and the node's histogram.
 // Bound by the records' read (16 B each): 32 us for 8M records.
 template <class Maps>
 __global__ void __launch_bounds__(kTileThreads)
@@ -175,18 +232,19 @@ __global__ void __launch_bounds__(kTileThreads)
     const KdMap &m = maps.of_tile(blockIdx.x);
     const TileNode n = tile_node(m, blockIdx.x, level);
     for (int i = threadIdx.x; i < kBins; i += kTileThreads) h[i] = 0;
-    const Cut c = level == 0 && !m.root_boxed ? cut_of(m.root_lo, m.root_hi, (float)kBins)
-                                              : cut_of_words(box + 8 * (size_t)n.node, (float)kBins);
+    const Cut c = level == 0 && !m.root_boxed ? cut_of(m.root_lo, m.root_hi)
+                                              : cut_of_words(box + 8 * (size_t)n.node);
     const float4 *src = level_src(m, level) + n.start;
-    uint16_t *bins = m.bins + n.start;
+    uint16_t *keys = m.keys + n.start;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kTileItems; ++i) {
         const uint32_t r = (uint32_t)i * kTileThreads + threadIdx.x;
         uint32_t b = kBins;
         if (r < n.cnt) {
-            b = bin_of(c, src[r], kBins);
-            bins[r] = (uint16_t)b;
+            const uint32_t key = key_of(c, src[r]);
+            keys[r] = (uint16_t)key;
+            b = key >> kSubShift;
         }
         // records of one wall share a bin: one addition for a warp of them
         int all;
@@ -199,30 +257,42 @@ __global__ void __launch_bounds__(kTileThreads)
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kBins; i += kTileThreads)
-        if (h[i]) atomicAdd(&hist[(size_t)n.node * kBins + i], h[i]);
+        if (h[i]) atomicAdd(&hist[(size_t)n.node * kRow + i], h[i]);
 }
 
-// Launch 2: the node's split (every tile of the node finds the same one;
-// its first tile writes it for launch 3) and the tile's records below the
-// median's bin and in it: 12 us for 8M records (their bins, 2 B each). thr:
-// {bin, records below it, of its records those that go left, its records}.
+// Launch 2: the node's bin (every tile of the node finds the same one; its
+// first tile writes it for launch 3) and the tile's records below the
+// median's bin and in it: 12 us for 8M records (their keys, 2 B each). thr:
+// {bin, records below it, its records}. Where the bin is crowded, also the
+// bin's records by their key: the node's counts beside its histogram, and the
+// tile's up to each of them.
+__device__ __forceinline__ bool crowded(uint4 thr, uint32_t ncnt) { return (uint64_t)thr.z * kCrowd > ncnt; }
+
 template <class Maps>
 __global__ void __launch_bounds__(kTileThreads)
-    kd_count_kernel(const __grid_constant__ Maps maps, int level, const uint32_t *hist, uint4 *thr,
-                    uint2 *tile_cnt) {
+    kd_count_kernel(const __grid_constant__ Maps maps, int level, uint32_t *hist, uint4 *thr,
+                    uint2 *tile_cnt, uint32_t *tile_sub) {
     constexpr int kPer = kBins / kTileThreads;
     __shared__ uint32_t wsum[kTileWarps];
     __shared__ uint4 split;
+    __shared__ uint32_t sub[kSub];
     const KdMap &m = maps.of_tile(blockIdx.x);
     const TileNode n = tile_node(m, blockIdx.x, level);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t key[kTileItems];
+#pragma unroll
+    for (int i = 0; i < kTileItems; ++i) {
+        const uint32_t r = (uint32_t)i * kTileThreads + threadIdx.x;
+        key[i] = r < n.cnt ? m.keys[n.start + r] : kNoKey;
+    }
     uint32_t v[kPer], s = 0;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-        v[i] = hist[(size_t)n.node * kBins + threadIdx.x * kPer + i];
+        v[i] = hist[(size_t)n.node * kRow + threadIdx.x * kPer + i];
         s += v[i];
     }
     if (threadIdx.x == 0) split = make_uint4(kBins, n.ncnt, 0u, 0u);  // no right child: all below
+    if (threadIdx.x < kSub) sub[threadIdx.x] = 0u;
     uint32_t incl = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -237,21 +307,27 @@ __global__ void __launch_bounds__(kTileThreads)
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
             if (run <= n.half && n.half < run + v[i])
-                split = make_uint4(threadIdx.x * kPer + i, run, n.half - run, v[i]);
+                split = make_uint4(threadIdx.x * kPer + i, run, v[i], 0u);
             run += v[i];
         }
     }
     __syncthreads();
     const uint32_t tb = split.x;
+    const bool crowd = crowded(split, n.ncnt);
     if (threadIdx.x == 0 && n.start == n.nstart) thr[n.node] = split;
     uint32_t less = 0, eq = 0;
 #pragma unroll
     for (int i = 0; i < kTileItems; ++i) {
-        const uint32_t r = (uint32_t)i * kTileThreads + threadIdx.x;
-        if (r < n.cnt) {
-            const uint32_t b = m.bins[n.start + r];
-            less += b < tb ? 1u : 0u;
-            eq += b == tb ? 1u : 0u;
+        less += key[i] >> kSubShift < tb ? 1u : 0u;
+        eq += key[i] >> kSubShift == tb ? 1u : 0u;
+    }
+    if (crowd) {
+#pragma unroll
+        for (int i = 0; i < kTileItems; ++i) {  // records of one wall share a key too
+            int all;
+            __match_all_sync(kFull, key[i], &all);
+            if (key[i] >> kSubShift == tb && (!all || lane == 0))
+                atomicAdd(&sub[key[i] & (kSub - 1u)], all ? 32u : 1u);
         }
     }
     const uint32_t both = __reduce_add_sync(kFull, less | (eq << 16));  // at most 256 each
@@ -262,6 +338,19 @@ __global__ void __launch_bounds__(kTileThreads)
         // 16-bit halves hold at most kTile
         const uint32_t t = __reduce_add_sync(kFull, lane < kTileWarps ? wsum[lane] : 0u);
         if (lane == 0) tile_cnt[blockIdx.x] = make_uint2(t & 0xffffu, t >> 16);
+        if (crowd) {
+            const uint32_t a = sub[2 * lane], b = sub[2 * lane + 1];
+            uint32_t *node_sub = hist + (size_t)n.node * kRow + kBins;
+            if (a) atomicAdd(&node_sub[2 * lane], a);
+            if (b) atomicAdd(&node_sub[2 * lane + 1], b);
+            uint32_t upto = a + b;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(kFull, upto, o);
+                if (lane >= o) upto += x;
+            }
+            tile_sub[(size_t)blockIdx.x * (kSub / 2) + lane] = (upto - b) | (upto << 16);
+        }
     }
 }
 
@@ -272,14 +361,32 @@ __global__ void __launch_bounds__(kTileThreads)
 // records, 4.9 TB/s; the writes of a warp are runs of consecutive records.
 template <class Maps>
 __global__ void __launch_bounds__(kTileThreads)
-    kd_split_kernel(const __grid_constant__ Maps maps, int level, const uint4 *thr, const uint2 *tile_cnt,
-                    uint32_t *box) {
+    kd_split_kernel(const __grid_constant__ Maps maps, int level, const uint32_t *hist, const uint4 *thr,
+                    const uint2 *tile_cnt, const uint32_t *tile_sub, uint32_t *box) {
     __shared__ uint32_t wcnt[kTileWarps], pre_l[kTileWarps], pre_e[kTileWarps];
     __shared__ uint32_t bb[12];
     const KdMap &m = maps.of_tile(blockIdx.x);
     const TileNode n = tile_node(m, blockIdx.x, level);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint4 sp = thr[n.node];
+    constexpr int kPer = kTileItems;  // records per lane
+    const uint32_t wfirst = n.start + (uint32_t)warp * (32u * kPer);
+    const float4 *src = level_src(m, level);
+    float4 *dst = level_dst(m, level);
+    float4 p[kPer];
+    uint32_t key[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t r = wfirst + 32u * i + lane;
+        key[i] = r < m.n ? m.keys[r] : kNoKey;
+        if (r < m.n) p[i] = src[r];
+    }
+    const uint4 bin = thr[n.node];
+    const bool crowd = crowded(bin, n.ncnt);
+    Split sp = split_at(bin);
+    if (crowd) {
+        const uint2 h = reinterpret_cast<const uint2 *>(hist + (size_t)n.node * kRow + kBins)[lane];
+        sp = split_bin(bin.x, bin.y, n.half, h.x, h.y, lane);
+    }
     const bool boxes = level + 1 < m.lf;  // split again, by launches or a cluster
     if (threadIdx.x < 12) bb[threadIdx.x] = 0u;
     // the node's earlier tiles
@@ -288,7 +395,14 @@ __global__ void __launch_bounds__(kTileThreads)
     for (uint32_t t = first + threadIdx.x; t < blockIdx.x; t += kTileThreads) {
         const uint2 c = tile_cnt[t];
         pl += c.x;
-        pe += c.y;
+        if (crowd) {
+            const uint16_t *u = reinterpret_cast<const uint16_t *>(tile_sub + (size_t)t * (kSub / 2));
+            const uint32_t q = sp.lo & (kSub - 1u), below = q ? u[q - 1] : 0u;
+            pl += below;
+            pe += u[q] - below;
+        } else {
+            pe += c.y;
+        }
     }
     pl = __reduce_add_sync(kFull, pl);
     pe = __reduce_add_sync(kFull, pe);
@@ -296,21 +410,12 @@ __global__ void __launch_bounds__(kTileThreads)
         pre_l[warp] = pl;
         pre_e[warp] = pe;
     }
-    constexpr int kPer = kTileItems;  // records per lane
-    const uint32_t wfirst = n.start + (uint32_t)warp * (32u * kPer);
-    const float4 *src = level_src(m, level);
-    float4 *dst = level_dst(m, level);
-    float4 p[kPer];
     uint32_t ml[kPer], me[kPer];
     uint32_t nl = 0, ne = 0;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-        const uint32_t r = wfirst + 32u * i + lane;
-        const bool valid = r < m.n;
-        const uint32_t b = valid ? m.bins[r] : 0xffffu;
-        if (valid) p[i] = src[r];
-        ml[i] = __ballot_sync(kFull, b < sp.x);
-        me[i] = __ballot_sync(kFull, b == sp.x);
+        ml[i] = __ballot_sync(kFull, key[i] < sp.lo);
+        me[i] = __ballot_sync(kFull, key[i] - sp.lo <= sp.span);
         nl += __popc(ml[i]);
         ne += __popc(me[i]);
     }
@@ -330,16 +435,8 @@ __global__ void __launch_bounds__(kTileThreads)
         if (r < m.n) {
             const uint32_t lb = less + __popc(ml[i] & lt), eb = eq + __popc(me[i] & lt);
             const bool is_l = (ml[i] >> lane) & 1u, is_e = (me[i] >> lane) & 1u;
-            uint32_t at;
-            bool left = true;
-            if (is_l) {
-                at = lb;
-            } else if (is_e && eb < sp.z) {
-                at = sp.y + eb;
-            } else {
-                left = false;
-                at = is_e ? n.half + (eb - sp.z) : n.half + (sp.w - sp.z) + ((r - n.nstart) - lb - eb);
-            }
+            const uint32_t at = sp.place(is_l, is_e, r - n.nstart, lb, eb);
+            const bool left = at < n.half;
             dst[n.nstart + at] = p[i];
             if (boxes) {
                 const uint32_t c[6] = {min_word(p[i].x), min_word(p[i].y), min_word(p[i].z),
@@ -368,16 +465,19 @@ __global__ void __launch_bounds__(kTileThreads)
 struct MidScratch {
     float4 p[kTile];
     uint32_t hist[kBins];
+    uint16_t key[kTile];
+    uint32_t sub[2][kSub];  // the median's bin by its values where it is crowded: the node's, the earlier tiles'
     uint32_t box[2][6];  // a node's first CTA: its box, by the level's parity
     uint32_t bb[12];
     uint32_t wsum[kTileWarps], wcnt[kTileWarps], pre[kTileWarps];
-    uint4 split;
+    uint4 split;      // {lo, span, less, equal} of the node's split
+    uint32_t earlier; // added to the earlier tiles' records below the split and in it (upper half)
 };
 
 extern __shared__ __align__(16) unsigned char mid_smem[];
 
 // The split levels from a node of at most 32,768 records down to subtrees,
-// by a cluster of 8 CTAs that hold a tile each: the same bins, medians and
+// by a cluster of 8 CTAs that hold a tile each: the same keys, medians and
 // stable partition as the launches above (and so the same layout), with two
 // cluster barriers a level in place of three launches. A CTA reads the
 // node's other histograms in their shared memory and writes its records to
@@ -423,40 +523,50 @@ __global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads,
         const uint32_t half = min((uint32_t)span >> 1, ncnt);
         const bool boxes = l + 1 < levels;
         Cut cut;
-        if (l > 0) cut = cut_of_words(cluster.map_shared_rank(&ms.box[l & 1][0], f), (float)kBins);
-        else if (m.ls == 0 && !m.root_boxed) cut = cut_of(m.root_lo, m.root_hi, (float)kBins);
-        else cut = cut_of_words(box + 8 * (size_t)(m.node0 + (1u << m.ls) + c), (float)kBins);
+        if (l > 0) cut = cut_of_words(cluster.map_shared_rank(&ms.box[l & 1][0], f));
+        else if (m.ls == 0 && !m.root_boxed) cut = cut_of(m.root_lo, m.root_hi);
+        else cut = cut_of_words(box + 8 * (size_t)(m.node0 + (1u << m.ls) + c));
         for (int i = threadIdx.x; i < kBins; i += kTileThreads) ms.hist[i] = 0;
         if (threadIdx.x < 12) ms.bb[threadIdx.x] = 0u;
+        if (threadIdx.x < 2 * kSub) (&ms.sub[0][0])[threadIdx.x] = 0u;
         __syncthreads();
-        uint32_t b[kPer];
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
-            b[i] = wfirst + 32 * i + lane < cnt ? bin_of(cut, p[i], kBins) : (uint32_t)kBins;
+            const int at = wfirst + 32 * i + lane;
+            uint32_t bin = kBins;
+            if (at < cnt) {
+                const uint32_t key = key_of(cut, p[i]);
+                ms.key[at] = (uint16_t)key;
+                bin = key >> kSubShift;
+            }
             int all;
-            __match_all_sync(kFull, b[i], &all);
+            __match_all_sync(kFull, bin, &all);
             if (all) {
-                if (lane == 0 && b[i] < kBins) atomicAdd(&ms.hist[b[i]], 32u);
-            } else if (b[i] < kBins) {
-                atomicAdd(&ms.hist[b[i]], 1u);
+                if (lane == 0 && bin < kBins) atomicAdd(&ms.hist[bin], 32u);
+            } else if (bin < kBins) {
+                atomicAdd(&ms.hist[bin], 1u);
             }
         }
-        cluster.sync();  // histograms complete; every record of the node is in registers
+        cluster.sync();  // histograms and keys complete; every record of the node is in registers
         uint32_t tot[kBinPer], pre[kBinPer], sum = 0;
 #pragma unroll
         for (int i = 0; i < kBinPer; ++i) tot[i] = pre[i] = 0;
+#pragma unroll 4
         for (int o = 0; o < ctas; ++o) {
-            const uint32_t *h = cluster.map_shared_rank(&ms.hist[0], f + o) + threadIdx.x * kBinPer;
-#pragma unroll
-            for (int i = 0; i < kBinPer; ++i) {
-                const uint32_t v = h[i];
-                tot[i] += v;
-                if (f + o < q) pre[i] += v;
+            const uint2 v = reinterpret_cast<const uint2 *>(cluster.map_shared_rank(&ms.hist[0], f + o))[threadIdx.x];
+            tot[0] += v.x;
+            tot[1] += v.y;
+            if (f + o < q) {
+                pre[0] += v.x;
+                pre[1] += v.y;
             }
         }
 #pragma unroll
         for (int i = 0; i < kBinPer; ++i) sum += tot[i];
-        if (threadIdx.x == 0) ms.split = make_uint4(kBins, ncnt, 0u, 0u);  // no right child: all below
+        if (threadIdx.x == 0) {
+            ms.split = make_uint4(kKeys, 0u, ncnt, 0u);  // no right child: all below
+            ms.earlier = 0u;
+        }
         if (threadIdx.x < 6) ms.box[l & 1][threadIdx.x] = 0u;              // read before the barrier
         uint32_t incl = sum;
 #pragma unroll
@@ -471,26 +581,64 @@ __global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads,
 #pragma unroll
             for (int i = 0; i < kBinPer; ++i) {
                 if (run <= half && half < run + tot[i])
-                    ms.split = make_uint4(threadIdx.x * kBinPer + i, run, half - run, tot[i]);
+                    ms.split = make_uint4((threadIdx.x * kBinPer + i) << kSubShift, kSub - 1u, run, tot[i]);
                 run += tot[i];
             }
         }
         __syncthreads();
-        const uint4 sp = ms.split;
+        if (ms.split.w * kCrowd > ncnt) {
+            // by the bin's values: each CTA reads the keys of all the node's,
+            // without a barrier that the other nodes' CTAs would have to meet
+            const uint32_t bin = ms.split.x >> kSubShift, below = ms.split.z;
+#pragma unroll 1
+            for (int o = f; o < f + ctas; ++o) {
+                const uint32_t first_o = first + (uint32_t)o * kTile;
+                const int n_o = first_o < m.n ? (int)min(kTile, m.n - first_o) - 8 * (int)threadIdx.x : 0;
+                const uint4 w = reinterpret_cast<const uint4 *>(cluster.map_shared_rank(&ms.key[0], o))[threadIdx.x];
+                const uint32_t k[4] = {w.x, w.y, w.z, w.w};
+                uint32_t last = kNoKey, same = 0;  // a run of one key: records of one wall share it
+#pragma unroll
+                for (int i = 0; i < 9; ++i) {
+                    const uint32_t v = i < 8 && i < n_o ? (k[(i >> 1) & 3] >> (16 * (i & 1))) & 0xffffu : kNoKey;
+                    if (v != last && last >> kSubShift == bin) {
+                        atomicAdd(&ms.sub[0][last & (kSub - 1u)], same);
+                        if (o < q) atomicAdd(&ms.sub[1][last & (kSub - 1u)], same);
+                    }
+                    same = v == last ? same + 1u : 1u;
+                    last = v;
+                }
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const Split sp = split_bin(bin, below, half, ms.sub[0][2 * lane], ms.sub[0][2 * lane + 1], lane);
+                const uint32_t at = sp.lo & (kSub - 1u), x = 2u * lane, y = x + 1u, ex = ms.sub[1][x], ey = ms.sub[1][y];
+                const uint32_t e = __reduce_add_sync(kFull, (x < at ? ex : (x == at ? 0u : 0u - (ex << 16))) +
+                                                                (y < at ? ey : (y == at ? 0u : 0u - (ey << 16))) -
+                                                                (x < at ? ex << 16 : 0u) - (y < at ? ey << 16 : 0u));
+                if (lane == 0) {
+                    ms.split = make_uint4(sp.lo, sp.span, sp.less, sp.equal);
+                    ms.earlier = e;
+                }
+            }
+            __syncthreads();
+        }
+        const Split sp{ms.split.x, ms.split.y, ms.split.z, ms.split.w};
         // records of the node's earlier tiles below the median's bin and in
         // it (at most 7 tiles of 4096: 16 bits each)
         uint32_t before = 0;
 #pragma unroll
         for (int i = 0; i < kBinPer; ++i) {
             const uint32_t bin = threadIdx.x * kBinPer + i;
-            before += bin < sp.x ? pre[i] : (bin == sp.x ? pre[i] << 16 : 0u);
+            before += bin < sp.lo >> kSubShift ? pre[i] : (bin == sp.lo >> kSubShift ? pre[i] << 16 : 0u);
         }
         before = __reduce_add_sync(kFull, before);
         uint32_t ml[kPer], me[kPer], own = 0;
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
-            ml[i] = __ballot_sync(kFull, b[i] < sp.x && b[i] < kBins);
-            me[i] = __ballot_sync(kFull, b[i] == sp.x && b[i] < kBins);
+            const int at = wfirst + 32 * i + lane;
+            const uint32_t key = at < cnt ? ms.key[at] : kNoKey;
+            ml[i] = __ballot_sync(kFull, key < sp.lo);
+            me[i] = __ballot_sync(kFull, key - sp.lo <= sp.span);
             own += __popc(ml[i]) | ((uint32_t)__popc(me[i]) << 16);
         }
         if (lane == 0) {
@@ -501,7 +649,7 @@ __global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads,
         uint32_t less, eq;
         {
             const uint32_t w = __reduce_add_sync(kFull, lane < warp ? ms.wcnt[lane] : 0u);
-            const uint32_t t = __reduce_add_sync(kFull, lane < kTileWarps ? ms.pre[lane] : 0u);
+            const uint32_t t = __reduce_add_sync(kFull, lane < kTileWarps ? ms.pre[lane] : 0u) + ms.earlier;
             less = (w & 0xffffu) + (t & 0xffffu);
             eq = (w >> 16) + (t >> 16);
         }
@@ -512,17 +660,8 @@ __global__ void __cluster_dims__(kMidCtas, 1, 1) __launch_bounds__(kTileThreads,
             if (r < cnt) {
                 const uint32_t lb = less + __popc(ml[i] & lt), eb = eq + __popc(me[i] & lt);
                 const bool is_l = (ml[i] >> lane) & 1u, is_e = (me[i] >> lane) & 1u;
-                uint32_t at;
-                bool left = true;
-                if (is_l) {
-                    at = lb;
-                } else if (is_e && eb < sp.z) {
-                    at = sp.y + eb;
-                } else {
-                    left = false;
-                    at = is_e ? half + (eb - sp.z)
-                              : half + (sp.w - sp.z) + ((uint32_t)((q - f) * (int)kTile + r) - lb - eb);
-                }
+                const uint32_t at = sp.place(is_l, is_e, (uint32_t)((q - f) * (int)kTile + r), lb, eb);
+                const bool left = at < half;
                 cluster.map_shared_rank(&ms.p[0], f + (int)(at / kTile))[at % kTile] = p[i];
                 if (boxes) {
                     const uint32_t w[6] = {min_word(p[i].x), min_word(p[i].y), min_word(p[i].z),
@@ -623,12 +762,12 @@ __device__ __forceinline__ void warp_split(SubScratch &ss, uint16_t *ord, int ba
     }
 #pragma unroll
     for (int a = 0; a < 6; ++a) w[a] = __reduce_max_sync(mask, w[a]);
-    const Cut c = cut_of_words(w, 65536.0f);
+    const Cut c = cut_of_words(w);
     uint32_t k[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int e = lane * 4 + r;
-        k[r] = base + e < cnt ? (bin_of(c, p[r], 65536u) << 16) | (uint32_t)e : 0xffffff00u | (uint32_t)e;
+        k[r] = base + e < cnt ? (key_of(c, p[r]) << 16) | (uint32_t)e : 0xffffff00u | (uint32_t)e;
     }
     warp_sort4<kN>(k, lane);
     // an empty place's key is above every record's, so the node's first
@@ -646,12 +785,76 @@ __device__ __forceinline__ void warp_split(SubScratch &ss, uint16_t *ord, int ba
 // One subtree per CTA: the levels from a node of at most kSubMax records
 // down to its leaves, the records in tree order and the boxes. Nodes of
 // more than 128 records split as in the split levels, with a 256-bin shared
-// histogram per node and five barriers per level; nodes of 128 and 64 are
+// histogram per node and five barriers per level (seven where a node's median
+// lies in a bin of more than 1/16 of it, which is split by its 256 values);
+// nodes of 128 and 64 are
 // sorted by one warp in registers. Only the 2-byte places move; the records
 // stay where they were loaded. Bound by latency (barriers, shared-memory
 // round trips): 0.44 ms for 8M records (sorting every level of the subtree in
 // shared memory: 2.27 ms), 27 us for a small map. 2 CTAs per SM at 64 registers
 // (3 at 40, which spill: 0.50 ms and 31 us; 1: 8M slower by a quarter).
+
+// The bin of a node's 256 (its row of the histograms, 8 consecutive bins a
+// lane) that holds place `half`, `less` records lying below the row: {first +
+// bin * step | mark, records below it, its records} into *thr by the lane that
+// finds it, marked where it holds more than `many`. Returns (warp-uniform)
+// whether it does.
+__device__ __forceinline__ bool row_split(const uint32_t *row, uint32_t less, uint32_t half, uint32_t first,
+                                          uint32_t step, uint32_t many, uint4 *thr, int lane) {
+    uint32_t v[kSubBins / 32], s = 0;
+#pragma unroll
+    for (int i = 0; i < kSubBins / 32; i += 4) {
+        const uint4 h = *reinterpret_cast<const uint4 *>(row + lane * (kSubBins / 32) + i);
+        v[i] = h.x;
+        v[i + 1] = h.y;
+        v[i + 2] = h.z;
+        v[i + 3] = h.w;
+        s += (h.x + h.y) + (h.z + h.w);
+    }
+    uint32_t incl = s;
+#pragma unroll
+    for (int q = 1; q < 32; q <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, q);
+        if (lane >= q) incl += t;
+    }
+    uint32_t run = less + incl - s;
+    bool crowd = false;
+#pragma unroll
+    for (int i = 0; i < kSubBins / 32; ++i) {
+        if (run <= half && half < run + v[i]) {
+            crowd = v[i] > many;
+            *thr = make_uint4((first + (uint32_t)(lane * (kSubBins / 32) + i) * step) | (crowd ? kMark : 0u), run, v[i], 0u);
+        }
+        run += v[i];
+    }
+    return __any_sync(kFull, crowd);
+}
+
+// The crowded bins of a subtree's level: their records (keys b of this thread,
+// node: this warp's, or -1) counted by the key's lower half, and the marked
+// splits made by it (crowd: that of node `warp` is). Returns how many key
+// values the middle of this warp's split has, less one. Out of line: the usual
+// level keeps its registers.
+__device__ __noinline__ uint32_t split_crowded(SubScratch &ss, int node, bool crowd, int span, int cnt, uint4 b) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = node >= 0 ? ss.thr[node].x : 0u;
+    const uint32_t k[kSubItems] = {b.x, b.y, b.z, b.w};
+    if (first & kMark) {
+#pragma unroll
+        for (int u = 0; u < kSubItems; ++u)
+            if (k[u] >> 8 == (first & ~kMark) >> 8) atomicAdd(&ss.hist[node * kSubBins + (k[u] & 255u)], 1u);
+    }
+    __syncthreads();
+    if (crowd) {
+        const uint4 t = ss.thr[warp];
+        const int half = min(span >> 1, cnt - warp * span);
+        __syncwarp();
+        row_split(&ss.hist[warp * kSubBins], t.y, (uint32_t)half, t.x & ~kMark, 1u, kKeys, &ss.thr[warp], lane);
+    }
+    __syncthreads();
+    return first & kMark ? 0u : kSubBins - 1u;
+}
+
 template <class Maps>
 __global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_constant__ Maps maps) {
     SubScratch &ss = *reinterpret_cast<SubScratch *>(sub_smem);
@@ -700,49 +903,36 @@ __global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_
         __syncthreads();
         uint32_t b[kSubItems];
         if (warp * kWarpSpan < cnt) {
-            const Cut c = cut_of_words(ss.bb[node], (float)kSubBins);
+            const Cut c = cut_of_words(ss.bb[node]);
 #pragma unroll
             for (int u = 0; u < kSubItems; ++u) {
-                b[u] = 0xffffu;
+                b[u] = kNoKey;
                 if (warp * kWarpSpan + u * 32 + lane < cnt) {
-                    b[u] = bin_of(c, p[u], kSubBins);
-                    atomicAdd(&ss.hist[node * kSubBins + b[u]], 1u);
+                    b[u] = key_of(c, p[u]);
+                    atomicAdd(&ss.hist[node * kSubBins + (b[u] >> 8)], 1u);
                 }
             }
         }
         __syncthreads();
+        // one warp per node; its split at a whole bin, or (crowded) the bin's
+        // records counted by their key's lower half and split there
+        bool crowd = false;
         if (warp < nodes) {
-            // one warp per node: 8 consecutive bins per lane
             const int ncnt = min(span, cnt - warp * span), half = min(span >> 1, ncnt);
-            uint32_t v[kSubBins / 32], s = 0;
-#pragma unroll
-            for (int i = 0; i < kSubBins / 32; i += 4) {
-                const uint4 h = *reinterpret_cast<const uint4 *>(&ss.hist[warp * kSubBins + lane * (kSubBins / 32) + i]);
-                v[i] = h.x;
-                v[i + 1] = h.y;
-                v[i + 2] = h.z;
-                v[i + 3] = h.w;
-                s += (h.x + h.y) + (h.z + h.w);
-            }
-            uint32_t incl = s;
-#pragma unroll
-            for (int q = 1; q < 32; q <<= 1) {
-                const uint32_t t = __shfl_up_sync(kFull, incl, q);
-                if (lane >= q) incl += t;
-            }
-            if (ncnt == half) {
-                if (lane == 0) ss.thr[warp] = make_uint4(kSubBins, (uint32_t)ncnt, 0u, 0u);
+            uint32_t *row = &ss.hist[warp * kSubBins];
+            if (ncnt == half) {  // no right child: all below
+                if (lane == 0) ss.thr[warp] = make_uint4(kKeys, (uint32_t)ncnt, 0u, 0u);
             } else {
-                uint32_t run = incl - s;
+                crowd = row_split(row, 0u, (uint32_t)half, 0u, 256u, (uint32_t)ncnt / kSubCrowd, &ss.thr[warp], lane);
+            }
+            if (crowd) {
 #pragma unroll
-                for (int i = 0; i < kSubBins / 32; ++i) {
-                    if (run <= (uint32_t)half && (uint32_t)half < run + v[i])
-                        ss.thr[warp] = make_uint4((uint32_t)(lane * (kSubBins / 32) + i), run, (uint32_t)half - run, v[i]);
-                    run += v[i];
-                }
+                for (int i = 0; i < kSubBins; i += 32) row[i + lane] = 0u;
             }
         }
-        __syncthreads();
+        uint32_t wide = kSubBins - 1u;  // the split's keys
+        if (__syncthreads_or(crowd))
+            wide = split_crowded(ss, warp * kWarpSpan < cnt ? node : -1, crowd, span, cnt, make_uint4(b[0], b[1], b[2], b[3]));
         uint32_t ml[kSubItems], me[kSubItems], tot = 0;
         uint4 sp = make_uint4(0u, 0u, 0u, 0u);
         if (warp * kWarpSpan < cnt) {
@@ -750,7 +940,7 @@ __global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_
 #pragma unroll
             for (int u = 0; u < kSubItems; ++u) {
                 ml[u] = __ballot_sync(kFull, b[u] < sp.x);
-                me[u] = __ballot_sync(kFull, b[u] == sp.x);
+                me[u] = __ballot_sync(kFull, b[u] - sp.x <= wide);
                 tot += __popc(ml[u]) | ((uint32_t)__popc(me[u]) << 16);
             }
         }
@@ -764,16 +954,13 @@ __global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_
             const uint32_t pre = __reduce_add_sync(kFull, lane >= nwarp && lane < warp ? ss.wcnt[lane] : 0u);
             uint32_t less = pre & 0xffffu, eq = pre >> 16;
             const unsigned lt = (1u << lane) - 1u;
-            const uint32_t half = (uint32_t)min(span >> 1, cnt - node * span);
 #pragma unroll
             for (int u = 0; u < kSubItems; ++u) {
                 const int at = warp * kWarpSpan + u * 32 + lane;
                 if (at < cnt) {
+                    const bool lower = (ml[u] >> lane) & 1u, middle = (me[u] >> lane) & 1u;
                     const uint32_t lb = less + __popc(ml[u] & lt), eb = eq + __popc(me[u] & lt);
-                    uint32_t to;
-                    if ((ml[u] >> lane) & 1u) to = lb;
-                    else if ((me[u] >> lane) & 1u) to = eb < sp.z ? sp.y + eb : half + (eb - sp.z);
-                    else to = half + (sp.w - sp.z) + ((uint32_t)(at - node * span) - lb - eb);
+                    const uint32_t to = lower ? lb : (middle ? sp.y + eb : sp.y + sp.z + ((uint32_t)(at - node * span) - lb - eb));
                     ss.ord[cur ^ 1][node * span + (int)to] = o[u];
                 }
                 less += __popc(ml[u]);
@@ -895,11 +1082,11 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 int mid_level(int lf) { return std::max(lf - kMidLevels, 0); }
 
 // Scratch layout of a set of maps: the words zeroed by each build
-// (histograms, boxes, finished-subtree counters), the splits, the tile
-// counts, then the bins and the partner buffer of every map.
+// (histograms, boxes, finished-subtree counters), the splits, the tiles'
+// counts, then the keys and the partner buffer of every map.
 struct Layout {
     uint32_t tiles = 0, subs = 0, nodes = 0;
-    size_t hist = 0, box = 0, done = 0, clear = 0, thr = 0, tile_cnt = 0, bins = 0, tmp = 0, total = 0;
+    size_t hist = 0, box = 0, done = 0, clear = 0, thr = 0, tile_cnt = 0, tile_sub = 0, keys = 0, tmp = 0, total = 0;
 };
 
 Layout layout_of(const uint32_t *n, const int *leaf_shift, int maps) {
@@ -915,13 +1102,14 @@ Layout layout_of(const uint32_t *n, const int *leaf_shift, int maps) {
         L.nodes += 2u << mid_level(lf);  // down to those the clusters split
         if (mid_level(lf) > 0) records += (n[i] + 127u) & ~(size_t)127u;
     }
-    L.box = align256(L.hist + sizeof(uint32_t) * kBins * (size_t)L.nodes);
+    L.box = align256(L.hist + sizeof(uint32_t) * kRow * (size_t)L.nodes);
     L.done = align256(L.box + sizeof(uint32_t) * 8 * (size_t)L.nodes);
     L.clear = align256(L.done + sizeof(uint32_t) * (size_t)std::max(maps, 1));
     L.thr = L.clear;
     L.tile_cnt = align256(L.thr + sizeof(uint4) * (size_t)L.nodes);
-    L.bins = align256(L.tile_cnt + sizeof(uint2) * (size_t)L.tiles);
-    L.tmp = align256(L.bins + sizeof(uint16_t) * records);
+    L.tile_sub = align256(L.tile_cnt + sizeof(uint2) * (size_t)L.tiles);
+    L.keys = align256(L.tile_sub + sizeof(uint16_t) * kSub * (size_t)L.tiles);
+    L.tmp = align256(L.keys + sizeof(uint16_t) * records);
     L.total = align256(L.tmp + sizeof(float4) * records);
     return L;
 }
@@ -969,7 +1157,7 @@ void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, 
         }
         if (m.ls > 0) {
             m.tmp = (float4 *)(base + L.tmp) + rec;
-            m.bins = (uint16_t *)(base + L.bins) + rec;
+            m.keys = (uint16_t *)(base + L.keys) + rec;
             rec += (b.n + 127u) & ~(size_t)127u;
         }
     }
@@ -977,14 +1165,14 @@ void describe(const KdBuildArgs *a, const int *idx, int count, const Layout &L, 
 
 template <class Maps>
 cudaError_t launch_build(const Maps &maps, const KdMap *host, int count, uint32_t subs, uint32_t *hist,
-                         uint32_t *box, uint4 *thr, uint2 *tile_cnt, cudaStream_t s) {
+                         uint32_t *box, uint4 *thr, uint2 *tile_cnt, uint32_t *tile_sub, cudaStream_t s) {
     for (int l = 0; l < host[0].ls; ++l) {
         // the maps split at this level come first
         uint32_t t = 0;
         for (int i = 0; i < count && host[i].ls > l; ++i) t = host[i].tile0 + tiles_of(host[i].n);
         kd_hist_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, box, hist);
-        kd_count_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, hist, thr, tile_cnt);
-        kd_split_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, thr, tile_cnt, box);
+        kd_count_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, hist, thr, tile_cnt, tile_sub);
+        kd_split_kernel<Maps><<<t, kTileThreads, 0, s>>>(maps, l, hist, thr, tile_cnt, tile_sub, box);
         note_launches(3);
     }
     cudaError_t e;
@@ -1057,7 +1245,7 @@ cudaError_t build_trees(const KdBuildArgs *a, int maps, void *scratch, cudaStrea
     describe(a, idx, count, L, scratch, m.m);
     unsigned char *base = (unsigned char *)scratch;
     return launch_build(m, m.m, count, L.subs, (uint32_t *)(base + L.hist), (uint32_t *)(base + L.box),
-                        (uint4 *)(base + L.thr), (uint2 *)(base + L.tile_cnt), s);
+                        (uint4 *)(base + L.thr), (uint2 *)(base + L.tile_cnt), (uint32_t *)(base + L.tile_sub), s);
 }
 
 namespace {
@@ -1094,6 +1282,7 @@ cudaError_t kd_multi_create(const std::vector<KdBuildArgs> &args, KdMulti *k) {
     k->box = (uint32_t *)(base + L.box);
     k->thr = (uint4 *)(base + L.thr);
     k->tile_cnt = (uint2 *)(base + L.tile_cnt);
+    k->tile_sub = (uint32_t *)(base + L.tile_sub);
     std::vector<uint32_t> tile_map(std::max<uint32_t>(L.tiles, 1), 0), sub_first(k->nmaps + 1, 0);
     for (int i = 0; i < k->nmaps; ++i) {
         const KdMap &m = k->maps[i];
@@ -1132,7 +1321,7 @@ cudaError_t kd_multi_build(KdMulti &k, cudaStream_t s) {
         kd_pad_kernel<MapsN><<<k.tiles, kTileThreads, 0, s>>>(m);
         note_launch();
     }
-    return launch_build(m, k.maps.data(), k.nmaps, k.subs, k.hist, k.box, k.thr, k.tile_cnt, s);
+    return launch_build(m, k.maps.data(), k.nmaps, k.subs, k.hist, k.box, k.thr, k.tile_cnt, k.tile_sub, s);
 }
 
 }  // namespace pm

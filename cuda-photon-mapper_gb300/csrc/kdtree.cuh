@@ -33,7 +33,7 @@ struct KdMap {
     float4 *pos_out, *pow_out, *dir_out;   // tree order
     float4 *lo, *hi;                       // node boxes
     float4 *tmp;                           // n records: the other buffer of the split levels
-    uint16_t *bins;                        // n: each record's bin at the current level
+    uint16_t *keys;                        // n: each record's split coordinate at the current level
     uint32_t *done;                        // finished subtrees (zero between builds)
     const uint32_t *pad_count;             // nullable
     float3 root_lo, root_hi;
@@ -82,6 +82,7 @@ struct KdMulti {
     uint32_t *box = nullptr;
     uint4 *thr = nullptr;
     uint2 *tile_cnt = nullptr;
+    uint32_t *tile_sub = nullptr;
     size_t clear_bytes = 0;             // of scratch, zeroed by each build
 };
 // Plans the build of the maps args[i] and allocates its tables and scratch.
