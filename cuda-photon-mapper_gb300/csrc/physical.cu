@@ -70,33 +70,30 @@ cudaError_t kd_reserve(PhysicalState *st) {
     return e;
 }
 
-// Room for the tracer's sphere lists of the installed scene; without it, no
-// lists.
+int near_grid(const PhysicalState *st, int spheres) {
+    return near_lists_grid(spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
+}
+
+// Room for the tracer's sphere lists of any scene that pm_update_scene may
+// install, which allocates nothing; without it, no lists.
 cudaError_t near_reserve(PhysicalState *st) {
-    const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
-    st->near_desc = NearLists();
-    st->near_gen = 0;
-    if (g > st->near_g) {
-        cudaFree(st->near);
+    const int g = near_grid(st, PM_MAX_SPHERES);
+    if (g == 0) return cudaSuccess;
+    cudaError_t e = cudaMalloc(&st->near, sizeof(uint4) * near_lists_words(g));
+    if (e == cudaErrorMemoryAllocation) {
         st->near = nullptr;
-        st->near_g = 0;
-        cudaError_t e = cudaMalloc(&st->near, sizeof(uint4) * near_lists_words(g));
-        if (e == cudaErrorMemoryAllocation) {
-            st->near = nullptr;
-            cudaGetLastError();
-            return cudaSuccess;
-        }
-        if (e != cudaSuccess) return e;
-        st->near_g = g;
+        cudaGetLastError();
+        return cudaSuccess;
     }
-    return cudaSuccess;
+    if (e == cudaSuccess) st->near_g = g;
+    return e;
 }
 
 // The sphere lists of the installed scene, built on the first emission after
 // it changed.
 cudaError_t near_update(PhysicalState *st, cudaStream_t s) {
     if (st->near_gen == st->gen) return cudaSuccess;
-    const int g = near_lists_grid(st->scene.num_spheres, std::max(st->cfg.surface_photons, st->cfg.volume_photons));
+    const int g = near_grid(st, st->scene.num_spheres);
     st->near_desc = NearLists();
     if (g > 0 && g <= st->near_g) {
         cudaError_t e = build_near_lists(st->dscene, g, st->near, &st->near_desc, s);
@@ -205,8 +202,6 @@ pm_status pm_update_scene(pm_ctx *ctx, const pm_scene *scene) {
     }
     st->dscene = to_device_scene(*scene, st->het);
     st->gen = next_scene_gen();
-    cudaError_t en = near_reserve(st);
-    if (en != cudaSuccess) return check_cuda(ctx, en, "near_reserve");
     return PM_OK;
 }
 
