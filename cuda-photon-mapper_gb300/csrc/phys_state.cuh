@@ -55,10 +55,17 @@ struct PhysicalState {
         int leaf_shift = 0;
         bool built = false;
     } map[2];
-    uint4 *near = nullptr;       // the tracer's sphere lists, for near_gen's scene (0: none yet)
+    // the tracer's sphere lists: room for near_g cells an axis; the lists in it
+    // (near_desc, empty: none) and the spheres and box that they were built from
+    struct NearKey {
+        float4 sph[PM_MAX_SPHERES];
+        float lo[3], hi[3];
+        int spheres, pad;
+    };
+    uint4 *near = nullptr;
     pm::NearLists near_desc;
     int near_g = 0;
-    uint64_t near_gen = 0;
+    NearKey near_key = {};
     void *kd_scratch = nullptr;  // tree builds
     size_t kd_bytes = 0;
     unsigned long long *gctr = nullptr;
