@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -89,13 +90,26 @@ cudaError_t near_reserve(PhysicalState *st) {
     return e;
 }
 
+// The lists enlarge a cell by a hundredth of its half diagonal, which has to
+// cover a few roundings of its coordinates: boxes of a finite size and within a
+// thousand times that size of the origin (cells of 1/20 of a side, a float's
+// spacing there 1/400 of a cell). Elsewhere every sphere is tested.
+bool near_box_fits(const pm_scene &sc) {
+    for (int a = 0; a < 3; ++a) {
+        const float ext = sc.box_max[a] - sc.box_min[a];
+        const float far = std::max(std::fabs(sc.box_min[a]), std::fabs(sc.box_max[a]));
+        if (!std::isfinite(ext) || !(far <= 1000.0f * ext)) return false;
+    }
+    return true;
+}
+
 // The sphere lists of the installed scene, built on the first emission after
 // its spheres or its box changed (a camera, light, material or medium that
 // changes leaves them: 1.5 ms of preset 3's 30).
 cudaError_t near_update(PhysicalState *st, cudaStream_t s) {
     const pm_scene &sc = st->scene;
     const int g = near_grid(st, sc.num_spheres);
-    if (g == 0 || g > st->near_g) {
+    if (g == 0 || g > st->near_g || !near_box_fits(sc)) {
         st->near_desc = NearLists();
         return cudaSuccess;
     }
