@@ -54,6 +54,7 @@ struct PhysicalState {
         int depth = 0;
         int leaf_shift = 0;
         bool built = false;
+        float ext[3] = {0.0f, 0.0f, 0.0f};  // sides of a box around the records
     } map[2];
     // the tracer's sphere lists: room for near_g cells an axis; the lists in it
     // (near_desc, empty: none) and the spheres and box that they were built from

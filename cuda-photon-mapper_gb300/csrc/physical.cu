@@ -289,6 +289,7 @@ pm_status pm_emit(pm_ctx *ctx, cudaStream_t stream) {
         st->map[m].paths = ext[2 * m + 1];
         st->map[m].built = false;
         st->map[m].depth = tree_depth(ext[2 * m], st->map[m].leaf_shift);
+        for (int a = 0; a < 3; ++a) st->map[m].ext[a] = st->scene.box_max[a] - st->scene.box_min[a];
         st->stats.map_size[m] = ext[2 * m];
         st->stats.map_paths[m] = ext[2 * m + 1];
     }
@@ -398,10 +399,16 @@ pm_status pm_knn(pm_ctx *ctx, int map, const float4 *queries, uint32_t nq, int k
     // select, and one launch of the list search is faster: 5,000 records at
     // radius 0.1 of a unit box, 5,000 queries 16.6 us (21.7 by the selection),
     // 20,000 at 0.05 with 20,000 queries 39 (41). Beyond, 60,000 at 0.05: k = 1
-    // 56 (43), k = 50 64 (66), k = 100 82 (76); 20,000 at 0.1: 77 (56).
-    const pm_scene &sc = st->scene;
-    const float box = (sc.box_max[0] - sc.box_min[0]) * (sc.box_max[1] - sc.box_min[1]) * (sc.box_max[2] - sc.box_min[2]);
-    const bool thin = (float)st->map[map].n * 4.18879020f * radius * radius * radius <= 24.0f * box;
+    // 56 (43), k = 50 64 (66), k = 100 82 (76); 20,000 at 0.1: 77 (56). Expected
+    // by the records' own box, a side shorter than the ball's counted as full:
+    // points that fill a part of the scene box (20,000 in 0.001 of it, k = 32,
+    // 20,000 queries 272 -> 60 us), lie beyond it (400,000 over a thousand times
+    // it, k = 8: 51 -> 42 us) or in a plane.
+    const auto &mp = st->map[map];
+    float reach = (float)mp.n * 0.52359878f;
+    for (int a = 0; a < 3; ++a)
+        if (mp.ext[a] > 2.0f * radius) reach *= 2.0f * radius / mp.ext[a];
+    const bool thin = reach <= 24.0f;
     PM_TRY(knn_query(view_of(st->map[map]), map, queries, nq, k, radius, idx_out, d2_out, stream, thin));
     return PM_OK;
 }
@@ -520,11 +527,22 @@ pm_status pm_set_photons(pm_ctx *ctx, int map, const float4 *pos, const float4 *
     }
     std::vector<float4> tmp(pos, pos + n);
     for (uint32_t i = 0; i < n; ++i) memcpy(&tmp[i].w, &i, 4);
+    // the box of a thousand of them (all of them: 1 ns a record)
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = 0; i < n; i += n / 1024u + 1u) {
+        const float c[3] = {tmp[i].x, tmp[i].y, tmp[i].z};
+        for (int a = 0; a < 3; ++a)
+            if (std::isfinite(c[a])) {
+                lo[a] = std::min(lo[a], c[a]);
+                hi[a] = std::max(hi[a], c[a]);
+            }
+    }
     if (n) {
         PM_TRY(cudaMemcpy(mp.pos, tmp.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
         PM_TRY(cudaMemcpy(mp.pow, pw, sizeof(float4) * n, cudaMemcpyHostToDevice));
     }
     PM_TRY(cudaMemcpy(st->words + 4 + 2 * map, &n, sizeof(uint32_t), cudaMemcpyHostToDevice));
+    for (int a = 0; a < 3; ++a) mp.ext[a] = hi[a] >= lo[a] ? hi[a] - lo[a] : 0.0f;
     mp.n = n;
     mp.paths = 0;
     mp.built = false;
