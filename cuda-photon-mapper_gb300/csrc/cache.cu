@@ -34,6 +34,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace pm {
 namespace {
@@ -360,7 +361,6 @@ __device__ __forceinline__ void relu_grad(uint32_t taddr, const unsigned char *h
 // layout the training kernel copies into its first activation buffer. One
 // thread per sample: the 128 hash-table reads of an encoding run at full
 // occupancy here instead of on the tensor-core kernel's critical path.
-template <int kDense>
 __global__ void __launch_bounds__(256)
     encode_kernel(CacheGrid g, const __half2 *tab, PScene Sc, const float4 *qa, const float4 *qd,
                   const uint32_t *sel, uint32_t n, uint32_t rows, unsigned char *xt, float *x_out) {
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(256)
             a = qa[qi];
             d = qd[qi];
         }
-        encode_row<kDense>(xt + (size_t)(i >> 7) * kXTile, kActSbo, (int)(i & 127u), g, tab, Sc, a, d, valid,
+        encode_row<-1>(xt + (size_t)(i >> 7) * kXTile, kActSbo, (int)(i & 127u), g, tab, Sc, a, d, valid,
                    (valid && x_out) ? x_out + (size_t)i * 64 : nullptr);
     }
 }
@@ -1262,11 +1262,28 @@ __global__ void schedule_kernel(float *sched, unsigned long long *step, float lr
 }  // namespace
 
 namespace {
-// The encoding compiled for a grid: the dense levels of the 16 (3 to 5 for
-// tables of 2^15 to 2^19 entries at the default resolutions), -1 for any
-// other grid.
-int dense_case(const CacheGrid &g) {
-    return g.levels == kCacheMaxLevels && g.dense >= 3 && g.dense <= 5 ? g.dense : -1;
+// Calls f with the number of the grid's dense levels as a constant, where
+// inference is compiled for it: all 16 levels, 0 to 8 of them dense (every
+// table size at the default resolutions); -1 for any other grid. Preset 2's
+// 46M queries by table size, 2^10 / 2^14 / 2^19 / 2^22: 5.44 / 5.85 / 5.90 / 6.74
+// ms with the kind of index found at run time, 4.81 / 4.73 / 4.87 / 5.05 so. The
+// training's encoding gains nothing by it (a frame's steps 2.95 ms both at 2^19)
+// and has one form.
+template <class F>
+cudaError_t with_dense(const CacheGrid &g, F &&f) {
+    using std::integral_constant;
+    switch (g.levels == kCacheMaxLevels ? g.dense : -1) {
+        case 0: return f(integral_constant<int, 0>());
+        case 1: return f(integral_constant<int, 1>());
+        case 2: return f(integral_constant<int, 2>());
+        case 3: return f(integral_constant<int, 3>());
+        case 4: return f(integral_constant<int, 4>());
+        case 5: return f(integral_constant<int, 5>());
+        case 6: return f(integral_constant<int, 6>());
+        case 7: return f(integral_constant<int, 7>());
+        case 8: return f(integral_constant<int, 8>());
+        default: return f(integral_constant<int, -1>());
+    }
 }
 }  // namespace
 
@@ -1447,12 +1464,7 @@ cudaError_t cache_backward(const CacheGrid &g, const CacheParams &p, const PScen
     const uint32_t rows = ntiles * kThreads;
     const uint32_t egrid = std::min<uint32_t>((rows + 255) / 256, (uint32_t)sm_count * 16);
     unsigned char *xt = reinterpret_cast<unsigned char *>(p.xt);
-    switch (dense_case(g)) {
-        case 3: encode_kernel<3><<<egrid, 256, 0, s>>>(g, p.table_h, S, qa, qd, sel, n, rows, xt, x_out); break;
-        case 4: encode_kernel<4><<<egrid, 256, 0, s>>>(g, p.table_h, S, qa, qd, sel, n, rows, xt, x_out); break;
-        case 5: encode_kernel<5><<<egrid, 256, 0, s>>>(g, p.table_h, S, qa, qd, sel, n, rows, xt, x_out); break;
-        default: encode_kernel<-1><<<egrid, 256, 0, s>>>(g, p.table_h, S, qa, qd, sel, n, rows, xt, x_out); break;
-    }
+    encode_kernel<<<egrid, 256, 0, s>>>(g, p.table_h, S, qa, qd, sel, n, rows, xt, x_out);
     note_launch();
     const uint32_t grid = std::min<uint32_t>(
         ntiles, (uint32_t)std::min(sm_count, p.parts_cap));
@@ -1513,17 +1525,9 @@ cudaError_t cache_infer(const CacheGrid &g, const CacheParams &p, const PScene &
         kernel<<<grid, kThreads * kInferPipes, kInferSmem, s>>>(g, p, S, qa, qd, order, n, out_scale, val);
         return cudaSuccess;
     };
-    cudaError_t e;
-    if (p.wait_polls != kMbarSpin) {
-        e = launch(infer_kernel<true, -1>);
-    } else {
-        switch (dense_case(g)) {
-            case 3: e = launch(infer_kernel<false, 3>); break;
-            case 4: e = launch(infer_kernel<false, 4>); break;
-            case 5: e = launch(infer_kernel<false, 5>); break;
-            default: e = launch(infer_kernel<false, -1>); break;
-        }
-    }
+    const cudaError_t e = p.wait_polls != kMbarSpin
+                              ? launch(infer_kernel<true, -1>)
+                              : with_dense(g, [&](auto dense) { return launch(infer_kernel<false, dense()>); });
     if (e != cudaSuccess) return e;
     note_launch();
     return cudaGetLastError();
