@@ -12,9 +12,11 @@
 // per-lane Kahan sums meet in a compensated butterfly. The reference's
 // double literals promote the weight, w * (1 - sqrt(d)) / exposure, to double
 // precision, which this GPU runs at a small fraction of its single-precision
-// rate; radius_weight.cuh finds the same bits in single precision, and takes
-// the double expression where it cannot tell them: 131,072 points over 500,000
-// records 688 -> 165 us.
+// rate; radius_weight.cuh takes it as pairs of floats: 131,072 points over
+// 500,000 records 688 -> 165 us. An exposure beyond the pairs' range keeps the
+// double expression. (Taking in double precision only the weights whose
+// rounding the pairs leave open, one in 50,000, made every weight the same and
+// the kernel 212 us: 48 registers instead of 32.)
 #include "gather.cuh"
 #include "launch_count.cuh"
 #include "radius_weight.cuh"
@@ -48,6 +50,7 @@ __device__ __forceinline__ float warp_total(float sum, float comp) {
     return s + e;
 }
 
+template <bool kDouble>
 __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const float4 *pts,
                                                              const float4 *nrm, uint32_t nq,
                                                              float sq_radius, float exposure, float2 inv,
@@ -56,7 +59,8 @@ __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const fl
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t qi = blockIdx.x * kWarps + wib;
     if (qi >= nq) return;
-    const float4 q = pts[qi], nv = nrm[qi];
+    const float4 q = pts[qi];
+    const float4 nv = nrm[qi];
     float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
     if (m.n > 0) {
         uint32_t *st = stack[wib];
@@ -85,7 +89,9 @@ __global__ void __launch_bounds__(kWarps * 32) radius_kernel(MapView m, const fl
                         const float4 pw = __ldg(&m.pow[r]);
                         const float4 dir = __ldg(&m.dir[r]);
                         const float nd = nv.x * dir.x + nv.y * dir.y + nv.z * dir.z;
-                        const float w = radius_weight(fmaxf(0.0f, -nd), sqrtf(d), exposure, inv.x, inv.y);
+                        float w = fmaxf(0.0f, -nd);
+                        w = kDouble ? radius_weight_double(w, sqrtf(d), exposure)
+                                    : radius_weight(w, sqrtf(d), inv.x, inv.y);
                         kahan(sx, cx, pw.x * w);
                         kahan(sy, cy, pw.y * w);
                         kahan(sz, cz, pw.z * w);
@@ -122,8 +128,10 @@ cudaError_t radius_gather(const MapView &m, const float4 *pts, const float4 *nrm
                           float sq_radius, float exposure, float4 *out, cudaStream_t s) {
     if (nq == 0) return cudaSuccess;
     float2 inv;
-    radius_inverse(exposure, &inv.x, &inv.y);
-    radius_kernel<<<(nq + kWarps - 1) / kWarps, kWarps * 32, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
+    const bool fits = radius_inverse(exposure, &inv.x, &inv.y);
+    const dim3 grid((nq + kWarps - 1) / kWarps), block(kWarps * 32);
+    if (fits) radius_kernel<false><<<grid, block, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
+    else radius_kernel<true><<<grid, block, 0, s>>>(m, pts, nrm, nq, sq_radius, exposure, inv, out);
     note_launch();
     return cudaGetLastError();
 }
