@@ -782,18 +782,6 @@ __device__ __forceinline__ void warp_split(SubScratch &ss, uint16_t *ord, int ba
     __syncwarp();
 }
 
-// One subtree per CTA: the levels from a node of at most kSubMax records
-// down to its leaves, the records in tree order and the boxes. Nodes of
-// more than 128 records split as in the split levels, with a 256-bin shared
-// histogram per node and five barriers per level (seven where a node's median
-// lies in a bin of more than 1/16 of it, which is split by its 256 values);
-// nodes of 128 and 64 are
-// sorted by one warp in registers. Only the 2-byte places move; the records
-// stay where they were loaded. Bound by latency (barriers, shared-memory
-// round trips): 0.44 ms for 8M records (sorting every level of the subtree in
-// shared memory: 2.27 ms), 27 us for a small map. 2 CTAs per SM at 64 registers
-// (3 at 40, which spill: 0.50 ms and 31 us; 1: 8M slower by a quarter).
-
 // The bin of a node's 256 (its row of the histograms, 8 consecutive bins a
 // lane) that holds place `half`, `less` records lying below the row: {first +
 // bin * step | mark, records below it, its records} into *thr by the lane that
@@ -855,6 +843,17 @@ __device__ __noinline__ uint32_t split_crowded(SubScratch &ss, int node, bool cr
     return first & kMark ? 0u : kSubBins - 1u;
 }
 
+// One subtree per CTA: the levels from a node of at most kSubMax records
+// down to its leaves, the records in tree order and the boxes. Nodes of more
+// than 128 records split as in the split levels, with a 256-bin shared
+// histogram per node and five barriers per level (seven where a node's median
+// lies in a bin of more than 1/16 of it, which is split by its 256 values);
+// nodes of 128 and 64 are sorted by one warp in registers. Only the 2-byte
+// places move; the records stay where they were loaded. Bound by latency
+// (barriers, shared-memory round trips): 0.44 ms for 8M records (sorting every
+// level of the subtree in shared memory: 2.27 ms), 28 us for a small map. 2 CTAs
+// per SM at 64 registers (3 at 40, which spill: 0.50 ms and 31 us; 1: 8M slower
+// by a quarter).
 template <class Maps>
 __global__ void __launch_bounds__(kSubThreads, 2) kd_finish_kernel(const __grid_constant__ Maps maps) {
     SubScratch &ss = *reinterpret_cast<SubScratch *>(sub_smem);
