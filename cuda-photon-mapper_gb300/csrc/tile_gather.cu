@@ -173,9 +173,14 @@ __device__ __forceinline__ float approx_sqrt(float v) {
     return r;
 }
 
-__device__ __forceinline__ float gap(float lo, float hi, float v) {
-    return fmaxf(fmaxf(lo - v, v - hi), 0.0f);
+// How far v lies outside [lo, hi]. NaN where a coordinate is: a record or a
+// query without one is in no set.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
+__device__ __forceinline__ float gap(float lo, float hi, float v) { return max_nan(max_nan(lo - v, v - hi), 0.0f); }
 
 __device__ __forceinline__ void count(int i, unsigned long long v = 1) {
     if ((threadIdx.x & 31) == 0) scratch().st[i] += v;
@@ -271,9 +276,9 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
             bool ok = false;
             if (lane < nc) {
                 const float4 bl = __ldg(&m.lo[child]), bh = __ldg(&m.hi[child]);
-                const float gx = fmaxf(fmaxf(bl.x - hi.x, lo.x - bh.x), 0.0f);
-                const float gy = fmaxf(fmaxf(bl.y - hi.y, lo.y - bh.y), 0.0f);
-                const float gz = fmaxf(fmaxf(bl.z - hi.z, lo.z - bh.z), 0.0f);
+                const float gx = max_nan(max_nan(bl.x - hi.x, lo.x - bh.x), 0.0f);
+                const float gy = max_nan(max_nan(bl.y - hi.y, lo.y - bh.y), 0.0f);
+                const float gz = max_nan(max_nan(bl.z - hi.z, lo.z - bh.z), 0.0f);
                 ok = gx * gx + gy * gy + gz * gz <= rho2;
             }
             const unsigned mk = __ballot_sync(kFull, ok);
@@ -491,7 +496,11 @@ __device__ __noinline__ void tile_queries(int mid, int n, unsigned mask, float *
 // them. The first radius is that of k records at
 // the density of the leaf nearest to the query (by volume, by area where the
 // leaf is flat); it then grows by the density found and, between a radius
-// that overflows and one with too few, is bisected in r^3.
+// that overflows and one with too few, is bisected in r^3. For points of any
+// kind (kPoints) nothing is looked for beside four leaves that are one place,
+// and far from the map (64 times the ball's radius) the radius grows and is
+// bisected beyond the distance to the leaf.
+template <bool kPoints>
 __device__ __noinline__ float single_bound(int mid, int j, float hi, int *count) {
     const int k = targs().k, lane = threadIdx.x & 31;
     const MapView &m = targs().map[mid];
@@ -518,12 +527,21 @@ __device__ __noinline__ float single_bound(int mid, int j, float hi, int *count)
     const float c = fminf(ex, fminf(ey, ez)), a = fmaxf(ex, fmaxf(ey, ez)), b = ex + ey + ez - a - c;
     float r = c > 0.25f * b ? cbrtf(f * a * b * c * 0.23873241f) : approx_sqrt(f * a * b * 0.31830989f);
     if (!(r > 0.0f)) r = 0.5f * f * a;  // records on a line
-    r = 1.18f * r + approx_sqrt(dist);
+    if (kPoints && a == 0.0f && m.depth >= 2) {
+        const float4 pl = __ldg(&m.lo[node >> 2]), ph = __ldg(&m.hi[node >> 2]);
+        if (pl.x == ph.x && pl.y == ph.y && pl.z == ph.z) return -1.0f;
+    }
     hi = fminf(hi, rcap);
+    float base = 0.0f;
+    if (kPoints) {
+        const float d = approx_sqrt(dist);
+        if (d > 64.0f * r && d < hi) base = d;
+    }
+    r = 1.18f * r + approx_sqrt(dist);
     r = r > 0.0f ? fminf(r, hi) : hi;  // and NaN
     float lo = 0.0f;
     bool over = false;
-    for (int it = 0; it < 32; ++it) {
+    for (int it = 0; it < (kPoints ? 20 : 32); ++it) {
         const int n = collect(mid, x, x, r * r * kOuter);
         if (n < 0) {
             hi = r;
@@ -534,7 +552,11 @@ __device__ __noinline__ float single_bound(int mid, int j, float hi, int *count)
             *count = n;
             return r;
         }
-        if (over) r = lo > 0.0f ? cbrtf(0.5f * (lo * lo * lo + hi * hi * hi)) : 0.75f * hi;
+        if (kPoints && base > 0.0f) {
+            if (!over) r = fminf(base + 2.0f * (lo - base), hi);
+            else r = base + (lo > base ? approx_sqrt((lo - base) * (hi - base)) : 0.25f * (hi - base));
+            if (over && !(r < hi)) return -1.0f;
+        } else if (over) r = lo > 0.0f ? cbrtf(0.5f * (lo * lo * lo + hi * hi * hi)) : 0.75f * hi;
         else r = fminf(lo * fminf(fmaxf(__powf(__fdividef(1.4f * (float)k, (float)max(n, 1)), mid == 0 ? 0.5f : 0.3333333f), 1.05f), 2.0f), hi);
         if (!(r > lo)) return -1.0f;
     }
@@ -560,7 +582,7 @@ __device__ __forceinline__ float bound_by(const float4 *known, int n, v3 x, floa
 template <int S>
 __device__ __forceinline__ bool alone(float ub, int mid, int j, float *d_lane) {
     int n = 0;
-    const float r = single_bound(mid, j, __shfl_sync(kFull, ub, j), &n);
+    const float r = single_bound<false>(mid, j, __shfl_sync(kFull, ub, j), &n);
     if (!(r >= 0.0f)) return false;
     __syncwarp();
     // the bound of the set just collected: all records within r are in it
@@ -759,7 +781,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     int n = 0, found = 0;
     float r = targs().rcap;
     if (m.n > 0) {
-        r = single_bound(mid, 0, targs().rcap, &n);
+        r = single_bound<true>(mid, 0, targs().rcap, &n);
         if (!(r >= 0.0f)) {
             if (lane == 0) idx[0] = kKnnLeft;
             return;
@@ -898,18 +920,20 @@ __device__ __forceinline__ void list_query(const MapView &m, const float4 *q, si
     }
 }
 
-// The queries knn_kernel left, by the list search (grid-stride, 32 queries'
-// marks at a time).
+// The queries knn_kernel left, by the list search. A warp looks at the marks of
+// 32 queries at a time, a grid of warps apart, so that queries left side by side
+// (all of them, where the records are piles) go to different warps.
 template <int S>
 __global__ void __launch_bounds__(128) knn_rest_kernel(MapView m, const float4 *q, uint32_t nq, int k, float r2cap,
                                                        uint32_t *idx_out, float *d2_out) {
     __shared__ WarpScratch ws[4];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (uint64_t base = ((uint64_t)blockIdx.x * 4 + wib) * 32; base < nq; base += (uint64_t)gridDim.x * 128) {
-        const uint64_t mine = base + lane;
+    const uint64_t warps = (uint64_t)gridDim.x * 4;
+    for (uint64_t base = (uint64_t)blockIdx.x * 4 + wib; base < nq; base += 32 * warps) {
+        const uint64_t mine = base + lane * warps;
         unsigned left = __ballot_sync(kFull, mine < nq && idx_out[mine * k] == kKnnLeft);
         for (; left; left &= left - 1) {
-            const uint64_t qi = base + __ffs(left) - 1;
+            const uint64_t qi = base + (__ffs(left) - 1) * warps;
             list_query<S>(m, q, qi, k, r2cap, idx_out, d2_out, ws[wib], lane);
         }
     }
@@ -1073,7 +1097,7 @@ cudaError_t knn_query(const MapView &m, int map, const float4 *q, uint32_t nq, i
     if (nq == 0) return cudaSuccess;
     const float r2 = radius * radius;
     const dim3 grid((nq + kTileWarps - 1) / kTileWarps), block(kTileWarps * 32);
-    const dim3 rest(std::min<uint32_t>((nq + 127) / 128, 1024));
+    const dim3 rest(std::min<uint32_t>((nq + 3) / 4, 2432));  // 16 blocks on each of 152 SMs
     const int smem = (int)(kTileWarps * sizeof(TileScratch));
 #define PM_KNN_LAUNCH(SL)                                                                 \
     if (thin) {                                                                           \
