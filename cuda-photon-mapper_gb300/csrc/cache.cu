@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Inference: kInferPipes independent 128-query pipelines per CTA share one
 // copy of the weights; each has its own activation tile, TMEM columns,
 // mbarrier and named barrier, so while one pipeline waits on the tensor core
-// or on hash-table reads the others issue. Bound by instruction issue (65 % of
+// or on hash-table reads the others issue. Bound by instruction issue (61 % of
 // the slots with 16 warps) and the latency of the 128 table reads of a query:
 // one CTA per SM, so that the compiler may keep them in flight in up to 128
 // registers. 46M queries of preset 2: 6.9 -> 4.85 ms with the levels' kind of

@@ -93,9 +93,9 @@ cudaError_t cache_composite(const PScene &S, const uint32_t *off, const float4 *
 cudaError_t render_composite(const PScene &S, const uint32_t *off, const float4 *qa,
                              const float4 *qd, const float4 *raw, uint32_t npix, float exposure,
                              float4 *rad, uchar4 *rgba, cudaStream_t s);
-// keys[i] = (1 for a volume query, 0 for a diffuse one) << 30 | the 30-bit
-// (map, Morton code) of query sel[i] -- or (map, Hilbert code) of query i, sel null -- in the
-// grid box; vals[i] = i.
+// keys[i] = (1 for a volume query, 0 for a diffuse one) << 30 | a 30-bit code of
+// the position in the grid box: the Morton code of query sel[i], or with sel
+// null the Hilbert code of query i; vals[i] = i.
 cudaError_t cache_sample_keys(const CacheGrid &g, const float4 *qa, const uint32_t *sel, uint32_t n,
                               uint32_t *keys, uint32_t *vals, cudaStream_t s);
 

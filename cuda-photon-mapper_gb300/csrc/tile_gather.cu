@@ -30,13 +30,14 @@
 // records' flux comes from L1 and L2. Candidates in registers
 // instead of shared memory make a query's distances and counts straight-line
 // code without loads, need no lists of the certain and the doubtful
-// candidates, and leave most of the L1 to the flux. Estimate pass (GB300,
-// presets 1 / 2 / 3): candidates in shared memory, scanned, the band between
-// two bounds ranked, 16.9 / 113.0 / 45.4 ms; in registers 12.0 / 76.0 / 34.5;
-// Hilbert instead of Morton order, a lane per channel for the last rounding
-// 10.0 / 64.0 / 29.9; expected set sizes instead of failed collections 9.8 /
-// 62.6 / 29.7; the first bound found in the pass instead of a launch before it,
-// 10 candidates per lane 10.0 / 59.8 / 25.9; now 10.2 / 60.0 / 24.7.
+// candidates, and leave most of the L1 to the flux. Estimate pass (GB300, ms,
+// presets 1 / 2 / 3 at seed 0x5EED0003: 11.0M, 46.0M and 20.8M queries):
+// candidates in shared memory, scanned, the band between two bounds ranked,
+// 16.9 / 113.0 / 45.4; in registers 12.0 / 76.0 / 34.5; Hilbert instead of
+// Morton order, a lane per channel for the last rounding 10.0 / 64.0 / 29.9;
+// expected set sizes instead of failed collections 9.8 / 62.6 / 29.7; the first
+// bound found in the pass instead of a launch before it, 10 candidates per lane
+// 10.0 / 59.8 / 25.9; now 10.2 / 60.0 / 24.7.
 #include <algorithm>
 
 #include "cache.cuh"

@@ -194,7 +194,10 @@ typedef struct pm_frame_stats {
  * Host only; needs no GPU. */
 PM_API pm_status pm_preset(int preset, uint64_t seed, pm_scene *scene, pm_config *cfg);
 
-/* Installs a scene and configuration (copies both); allocates the maps. */
+/* Installs a scene and configuration (copies both); allocates the maps and,
+ * from 270,000 records a map on, the photon tracer's sphere lists (17, 39 or 77
+ * MB by the larger target, for any scene pm_update_scene may install; where
+ * the memory is short every sphere is tested instead). */
 PM_API pm_status pm_set_scene(pm_ctx *ctx, const pm_scene *scene, const pm_config *cfg);
 /* Replaces the scene of the next frame (geometry, materials, light, medium
  * coefficients, camera) without reallocating: sphere and plane counts may
@@ -227,7 +230,7 @@ PM_API pm_status pm_render_single_kernel(pm_ctx *ctx, float4 *radiance, uchar4 *
  * [3] results that contradicted their upper bound and were redone by the
  * list search (0 while the bounds hold), [4] candidate sets collected,
  * [5] candidates collected, [6] segments halved because their set did not
- * fit in shared memory. */
+ * fit in a warp's registers. */
 PM_API pm_status pm_get_gather_stats(pm_ctx *ctx, uint64_t *out, int n);
 /* k nearest photons of map `map` for nq query points (device float4
  * xyz), within radius; idx_out / d2_out (device, nq*k) receive photon
