@@ -174,8 +174,8 @@ __device__ __forceinline__ float approx_sqrt(float v) {
     return r;
 }
 
-// How far v lies outside [lo, hi]. NaN where a coordinate is: a record or a
-// query without one is in no set.
+// How far v lies outside [lo, hi]. NaN where a coordinate is: a record without
+// one is in no set.
 __device__ __forceinline__ float max_nan(float a, float b) {
     float r;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
@@ -277,9 +277,9 @@ __device__ __noinline__ int collect(int mid, v3 lo, v3 hi, float rho2) {
             bool ok = false;
             if (lane < nc) {
                 const float4 bl = __ldg(&m.lo[child]), bh = __ldg(&m.hi[child]);
-                const float gx = max_nan(max_nan(bl.x - hi.x, lo.x - bh.x), 0.0f);
-                const float gy = max_nan(max_nan(bl.y - hi.y, lo.y - bh.y), 0.0f);
-                const float gz = max_nan(max_nan(bl.z - hi.z, lo.z - bh.z), 0.0f);
+                const float gx = fmaxf(fmaxf(bl.x - hi.x, lo.x - bh.x), 0.0f);
+                const float gy = fmaxf(fmaxf(bl.y - hi.y, lo.y - bh.y), 0.0f);
+                const float gz = fmaxf(fmaxf(bl.z - hi.z, lo.z - bh.z), 0.0f);
                 ok = gx * gx + gy * gy + gz * gz <= rho2;
             }
             const unsigned mk = __ballot_sync(kFull, ok);
@@ -761,8 +761,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
 // selected records are put in order by their ranks: every lane counts the
 // distances below its own, and where two are equal the indices decide. A
 // query without a radius that fits its set (more records at one distance
-// than the registers hold), or whose set holds records without a distance, is
-// marked in its first index and left to knn_rest_kernel. Bound by instruction issue and the walk's L2 latency.
+// than the registers hold) is marked in its first index and left to
+// knn_rest_kernel. Bound by instruction issue and the walk's L2 latency.
 // Measured (GB300; the list search before): 262,144 queries, k = 100, 1M
 // points 3.62 -> 1.59 ms; 32,768 queries, k = 32, 100,000 points 225 -> 110 us.
 template <int S>
@@ -781,7 +781,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
     float *dist = d2_out + (size_t)qi * k;
     int n = 0, found = 0;
     float r = targs().rcap;
-    if (m.n > 0) {
+    if (m.n > 0 && p.x == p.x && p.y == p.y && p.z == p.z) {  // nothing is near a NaN
         r = single_bound<true>(mid, 0, targs().rcap, &n);
         if (!(r >= 0.0f)) {
             if (lane == 0) idx[0] = kKnnLeft;
@@ -886,8 +886,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks)
             __syncwarp();
         }
     }
-    // fewer than k within a radius that held k records: some of those have no
-    // distance (NaN), others may lie beyond the radius
+    // fewer than k of a radius's k records: their distance beside the gather
+    // radius's rounding, or none at all (infinity less infinity); others may lie
+    // beyond that radius
     if (found < k && r < targs().rcap) {
         if (lane == 0) idx[0] = kKnnLeft;
         return;

@@ -20,6 +20,8 @@ def records(kind, n, rs):
             p[a::3, a] = np.nan
     elif kind == "nan_most":    # nine of ten lack all three
         p[np.arange(n) % 10 != 0, :3] = np.nan
+    elif kind == "infinite":    # beside queries at infinity: no distance, and boxes without end
+        p[::5, 0], p[1::7, 1], p[2::9, :3] = -np.inf, np.inf, -np.inf
     elif kind == "piles":       # places of 1, 20, 400 and 1,000 records
         for i, m in enumerate((1000, 400, 20)):
             p[i: i + 4 * m: 4, :3] = np.float32([0.1 * i, 0.5, 0.0])
@@ -60,7 +62,8 @@ def brute(p, q, k, radius):
 @pytest.mark.parametrize("k,radius", [(1, 0.3), (10, 0.4), (33, 2.0), (128, 5.0), (20, np.inf)])
 @pytest.mark.parametrize("n,kind,qkind", [(300, "nan_axis", "plain"), (5000, "nan_axis", "plain"),
                                           (6000, "nan_most", "odd"), (5000, "piles", "plain"),
-                                          (25, "box", "odd"), (5000, "box", "odd")])
+                                          (25, "box", "odd"), (5000, "box", "odd"), (90, "infinite", "odd"),
+                                          (4000, "infinite", "odd")])
 def test_odd_sets(n, kind, qkind, k, radius, noalloc):
     rs = np.random.RandomState(n + k)
     p = records(kind, n, rs)
